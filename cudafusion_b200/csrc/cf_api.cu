@@ -108,11 +108,11 @@ void dfree(T*& p) {
 
 void free_pattern(Pattern& p) {
   dfree(p.row_ptr); dfree(p.col_idx); dfree(p.diag_pos); dfree(p.trans_pos);
-  dfree(p.upper_pos); dfree(p.upper_row); dfree(p.arap_row_ptr); dfree(p.arap_row_inc);
+  dfree(p.upper_row); dfree(p.arap_row_ptr); dfree(p.arap_row_inc);
   dfree(p.arap_blk_ptr); dfree(p.arap_blk_edge); dfree(p.edge_ijk); dfree(p.values);
   dfree(p.seg_off); dfree(p.seg_cnt); dfree(p.pcg_row_begin);
-  dfree(p.clu_row_begin); dfree(p.ustart); dfree(p.low_ptr); dfree(p.clu_opnd); dfree(p.clu_push);
-  dfree(p.clu_halo_ptr); dfree(p.clu_halo); dfree(p.g_vidx); dfree(p.g_halo_ptr); dfree(p.g_halo_col);
+  dfree(p.clu_row_begin); dfree(p.ustart); dfree(p.clu_vidx); dfree(p.clu_halo);
+  dfree(p.clu_halo_ptr); dfree(p.g_vidx); dfree(p.g_halo_ptr); dfree(p.g_halo_col);
   dfree(p.off_upper); dfree(p.pcg_cta_off); dfree(p.pcg_prob); dfree(p.prob_edge_off);
   dfree(p.st_tile_ptr); dfree(p.st_tile_row); dfree(p.st_tile_cols); dfree(p.edge_terms); dfree(p.edge_energy);
   p = Pattern();
@@ -517,37 +517,21 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
     edge_off[q] = (q < P) ? e : n_edges;
   }
 
-  // single-cluster PCG plan: rows split over C CTAs in contiguous ranges of
-  // balanced UPPER block counts (what each CTA keeps in shared memory and
-  // multiplies twice).  Per upper block: the operand slot of its column (own
-  // row, or the CTA's halo) and, off the diagonal, where its transposed
-  // product goes: the owner of the column and the receive slot of the lower
-  // block there (row j's lower blocks in order of their row i).
-  std::vector<int> ustart(N + 1, 0), low_ptr(N + 1, 0), low_of_upper(std::max(1, n_upper), -1);
+  std::vector<int> ustart(N + 1, 0);
   for (int i = 0; i < N; i++) ustart[i + 1] = ustart[i] + (row_ptr[i + 1] - diag_pos[i]);
-  {
-    std::vector<std::vector<std::pair<int, int>>> lows(N);  // row i: (j, u of (j, i)), j < i
-    for (int j = 0; j < N; j++)
-      for (int q = diag_pos[j] + 1; q < row_ptr[j + 1]; q++) lows[col_idx[q]].push_back({j, upper_of_pos[q]});
-    for (int i = 0; i < N; i++) {
-      std::sort(lows[i].begin(), lows[i].end());
-      low_ptr[i + 1] = low_ptr[i] + (int)lows[i].size();
-      for (size_t k = 0; k < lows[i].size(); k++) low_of_upper[lows[i][k].second] = low_ptr[i] + (int)k;
-    }
-  }
-  int clu_C = 0, clu_smem = 0, clu_nup = 0, clu_nlow = 0, clu_rows = 0, clu_nhalo = 0;
-  std::vector<int> clu_rb, clu_opnd(std::max(1, n_upper)), clu_push(std::max(1, n_upper)), clu_hptr, clu_halo;
+  // single-cluster PCG plan: rows split over C CTAs in contiguous ranges of
+  // balanced block counts.  Per block the operand slot of its column (own row,
+  // or the CTA's halo); per halo row its owner and its row there.
+  int clu_C = 0, clu_smem = 0, clu_blk = 0, clu_rows = 0, clu_nhalo = 0;
+  std::vector<int> clu_rb, clu_vidx(std::max(1, nnzb)), clu_hptr, clu_halo;
   if (h->pcg_mode != 1 && h->pcg_mode != 3 && !stream && P == 1) {
     const int cands[2] = {16, 8};
     for (int ci = 0; ci < 2 && !clu_C; ci++) {
       const int C = cands[ci];
       if (N < C) continue;
-      // automatic choice: the cluster's 16 SMs win while each holds few rows
-      // (measured on B200: 54 vs 62 us per PCG at 16 rows per CTA, 169 vs 107
-      // at 128); past ~32 rows per CTA the grid-wide kernel is faster
       if (h->pcg_mode == 0 && N > kClusterAutoRows * C) continue;
       std::vector<int> rb(1, 0);
-      const long long target = ((long long)n_upper + C - 1) / C;
+      const long long target = ((long long)nnzb + C - 1) / C;
       int start = 0;
       for (int c = 0; c < C; c++) {
         const int rem = C - c;
@@ -555,47 +539,40 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
         if (rem == 1) {
           end = N;
         } else {
-          while (end < N - (rem - 1) && ustart[end] - ustart[start] < target) end++;
+          while (end < N - (rem - 1) && row_ptr[end] - row_ptr[start] < target) end++;
         }
         rb.push_back(end);
         start = end;
       }
-      std::vector<int> owner(N);
+      std::vector<int> owner(N), hptr(1, 0), halo;
       for (int c = 0; c < C; c++)
         for (int r = rb[c]; r < rb[c + 1]; r++) owner[r] = c;
-      std::vector<int> hptr(1, 0), halo;
-      int nu = 0, nl = 0, nr = 0, nh = 0;
+      int nb = 0, nr = 0, nh = 0;
       for (int c = 0; c < C; c++) {
         const int r0 = rb[c], r1 = rb[c + 1];
-        std::vector<int> cols;  // remote columns of the CTA's upper blocks (all > r1 - 1)
-        for (int u = ustart[r0]; u < ustart[r1]; u++) {
-          const int j = col_idx[upper_pos[u]];
-          if (j >= r1) cols.push_back(j);
-        }
+        std::vector<int> cols;  // the CTA's halo
+        for (int q = row_ptr[r0]; q < row_ptr[r1]; q++)
+          if (col_idx[q] < r0 || col_idx[q] >= r1) cols.push_back(col_idx[q]);
         std::sort(cols.begin(), cols.end());
         cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-        for (int u = ustart[r0]; u < ustart[r1]; u++) {
-          const int q = upper_pos[u], j = col_idx[q];
-          clu_opnd[u] = (j < r1) ? j - r0
-                                 : (r1 - r0) + (int)(std::lower_bound(cols.begin(), cols.end(), j) - cols.begin());
-          clu_push[u] = (q == diag_pos[upper_row[u]])
-                            ? -1
-                            : (owner[j] << 24) | (low_of_upper[u] - low_ptr[rb[owner[j]]]);
+        for (int q = row_ptr[r0]; q < row_ptr[r1]; q++) {
+          const int j = col_idx[q];
+          clu_vidx[q] = (j >= r0 && j < r1) ? j - r0
+                                            : (r1 - r0) + (int)(std::lower_bound(cols.begin(), cols.end(), j) - cols.begin());
         }
         for (int j : cols) halo.push_back((owner[j] << 24) | (j - rb[owner[j]]));
         hptr.push_back((int)halo.size());
-        nu = std::max(nu, ustart[r1] - ustart[r0]);
-        nl = std::max(nl, low_ptr[r1] - low_ptr[r0]);
+        nb = std::max(nb, row_ptr[r1] - row_ptr[r0]);
         nr = std::max(nr, r1 - r0);
         nh = std::max(nh, (int)cols.size());
       }
-      const int sm = pcg_cluster_smem_bytes(nu, nl, nr, nh, C);
+      if (nr > pcg_cluster_max_rows() || nr + nh > 0xffff) continue;
+      const int sm = pcg_cluster_smem_bytes(nb, nr, nh, C);
       if (sm > 227 * 1024 - 1024) continue;
-      if (pcg_cluster_max_active(C, sm) < 1) continue;
+      if (pcg_cluster_max_active(C, nr, sm) < 1) continue;
       clu_C = C;
       clu_smem = sm;
-      clu_nup = nu;
-      clu_nlow = nl;
+      clu_blk = nb;
       clu_rows = nr;
       clu_nhalo = nh;
       clu_rb = rb;
@@ -626,7 +603,6 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
   CF_TRY(up(&p.col_idx, col_idx));
   CF_TRY(up(&p.diag_pos, diag_pos));
   CF_TRY(up(&p.trans_pos, trans_pos));
-  CF_TRY(up(&p.upper_pos, upper_pos));
   CF_TRY(up(&p.upper_row, upper_row));
   CF_TRY(up(&p.arap_row_ptr, arow_ptr));
   CF_TRY(up(&p.arap_row_inc, arow_inc));
@@ -656,16 +632,13 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
   p.use_cluster = clu_C ? 1 : 0;
   p.clu_C = clu_C;
   p.clu_smem = clu_smem;
-  p.clu_nup_max = clu_nup;
-  p.clu_nlow_max = clu_nlow;
+  p.clu_blk_max = clu_blk;
   p.clu_rows_max = clu_rows;
   p.clu_halo_max = clu_nhalo;
   CF_TRY(up(&p.ustart, ustart));
-  CF_TRY(up(&p.low_ptr, low_ptr));
   if (clu_C) {
     CF_TRY(up(&p.clu_row_begin, clu_rb));
-    CF_TRY(up(&p.clu_opnd, clu_opnd));
-    CF_TRY(up(&p.clu_push, clu_push));
+    CF_TRY(up(&p.clu_vidx, clu_vidx));
     CF_TRY(up(&p.clu_halo_ptr, clu_hptr));
     CF_TRY(up(&p.clu_halo, clu_halo.empty() ? std::vector<int>(1, 0) : clu_halo));
   }

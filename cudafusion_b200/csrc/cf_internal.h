@@ -75,7 +75,6 @@ struct Pattern {
   int* col_idx = nullptr;   // [nnzb]
   int* diag_pos = nullptr;  // [N]
   int* trans_pos = nullptr; // [nnzb] position of the transposed block
-  int* upper_pos = nullptr; // [n_upper]
   int* upper_row = nullptr; // [n_upper]
   int* arap_row_ptr = nullptr;  // [N+1]
   int* arap_row_inc = nullptr;  // (edge << 1) | role, role 0 = lower endpoint
@@ -94,13 +93,11 @@ struct Pattern {
   int use_cluster = 0;
   int clu_C = 0;
   int clu_smem = 0;
-  int clu_nup_max = 0, clu_nlow_max = 0, clu_rows_max = 0, clu_halo_max = 0;
+  int clu_blk_max = 0, clu_rows_max = 0, clu_halo_max = 0;
   int* clu_row_begin = nullptr;  // [clu_C+1]
   int* ustart = nullptr;         // [N+1] first upper index of each row
-  int* low_ptr = nullptr;        // [N+1] lower blocks (j, i), j < i, of row i, in order of j
-  int* clu_opnd = nullptr;       // [n_upper] operand slot of the block's column in its CTA: own row, or rows + halo slot
-  int* clu_push = nullptr;       // [n_upper] off-diagonal (i, j): (owner of row j << 24) | receive slot of (j, i) there; -1 diagonal
-  int* clu_halo_ptr = nullptr;   // [clu_C+1]
+  int* clu_vidx = nullptr;       // [nnzb] operand slot of the block's column in its CTA: own row, or rows + halo slot
+  int* clu_halo_ptr = nullptr;   // [clu_C+1] halo rows before each CTA's
   int* clu_halo = nullptr;       // per CTA, its remote columns: (owner << 24) | row local to the owner
   // grid PCG partition
   int pcg_ctas = 0;
@@ -167,7 +164,11 @@ constexpr int kEnergyCtas = 512;  // residual/energy CTAs of a single solve (wit
 constexpr int kMaxPcgCtas = 1024;
 constexpr int kSortCorrs = 4096;     // correspondences per sort CTA of a batched solve (at least)
 constexpr int kMaxSortCtas = 1 << 16;
-constexpr int kClusterAutoRows = 32;  // rows per CTA up to which mode 0 picks the single-cluster PCG
+// Rows per CTA up to which mode 0 picks the single-cluster PCG.  Its exchanges
+// are shorter than the grid's, its 16 SMs hold more rows each; per launch of 12-13
+// iterations on B200: 256 nodes 52 us (grid 78), 512 nodes 52 (grid 70), 1024
+// nodes 75 (grid 72), 2048 nodes 105 (grid 81).
+constexpr int kClusterAutoRows = 48;
 constexpr int kMaxProblems = 1024;       // problems per batched solve
 constexpr int kMaxProblemNodes = 48000;  // nodes per problem (per-CTA histograms in shared memory)
 
@@ -309,8 +310,9 @@ int pcg_grid_smem_bytes(int nblk, int nrows, int nhalo, bool a_in_smem, bool pip
 int pcg_max_active_ctas(int smem, bool a_in_smem, bool pipelined);
 int expand_smem_bytes(int max_upper_row, int N);
 
-int pcg_cluster_smem_bytes(int nup_max, int nlow_max, int rows_max, int nhalo_max, int C);
-int pcg_cluster_max_active(int C, int smem);
+int pcg_cluster_max_rows();
+int pcg_cluster_smem_bytes(int blk_max, int rows_max, int nhalo_max, int C);
+int pcg_cluster_max_active(int C, int rows_max, int smem);
 cudaError_t launch_pcg_cluster(const Work& w, const Pattern& p, const SolveArgs& a, int gn_slot, cudaStream_t s);
 
 // The learned initial increment (cf_mpnn.cu): parameters, graph, activations.

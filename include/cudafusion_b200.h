@@ -155,12 +155,12 @@ CF_API cf_status cf_gn_linearize_solve(cf_gn* h, const cf_correspondence* d_corr
  *                          update.  With 0 the GN energy can rise for large
  *                          lambda_smooth, exactly as in the reference.
  *  CF_OPT_PCG_CTAS         CTAs of the grid-wide PCG kernel (0 = automatic).
- *  CF_OPT_PCG_MODE         0: automatic (single cluster up to 32 rows per
+ *  CF_OPT_PCG_MODE         0: automatic (single cluster up to 48 rows per
  *                          CTA of a 16-CTA cluster, else grid-wide or, past
  *                          the GPU's shared memory, streaming); 1: grid-wide
  *                          cooperative PCG with the system in shared memory
  *                          (streaming when it does not fit); 2: single-
- *                          cluster PCG (upper blocks in distributed shared
+ *                          cluster PCG (full rows in distributed shared 
  *                          memory) when the system fits the cluster's shared
  *                          memory (else grid-wide); 3: streaming PCG (A re-read from HBM
  *                          through TMA bulk copies every iteration, vectors
