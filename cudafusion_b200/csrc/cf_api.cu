@@ -20,13 +20,13 @@ using namespace cf;
 
 // Phase slots of the profiler (cf_gn_profile_*).
 enum ProfSlot {
-  kProfPack = 0, kProfBinScan, kProfScatter, kProfExpand, kProfNodePlain, kProfResidual, kProfAssemble,
-  kProfPcg, kProfEnergy, kProfTwist, kProfSkin, kProfOther
+  kProfPack = 0, kProfBinScan, kProfScatter, kProfSort, kProfNodePlain, kProfResidual, kProfAssemble,
+  kProfPcg, kProfEnergy, kProfTwist, kProfLists, kProfOther
 };
 constexpr int kProfLearned = kProfTwist;  // the learned start: features, network, apply, gate
-static const char* kProfNames[CF_PROF_SLOTS] = {"pack_count", "bin_scan", "bin_scatter", "expand",
+static const char* kProfNames[CF_PROF_SLOTS] = {"key_count", "bin_scan", "bin_scatter", "bucket_sort",
                                                 "node_plain", "residual", "assemble", "pcg",
-                                                "final_energy", "apply_twist", "skin_points", "other"};
+                                                "final_energy", "apply_twist", "node_lists", "other"};
 
 struct ProfEvent {
   int slot;
@@ -107,22 +107,22 @@ void dfree(T*& p) {
 }
 
 void free_pattern(Pattern& p) {
-  dfree(p.row_ptr); dfree(p.col_idx); dfree(p.diag_pos); dfree(p.trans_pos);
-  dfree(p.upper_row); dfree(p.arap_row_ptr); dfree(p.arap_row_inc);
+  dfree(p.row_ptr); dfree(p.col_idx); dfree(p.diag_pos);
+  dfree(p.upper_meta); dfree(p.arap_row_ptr); dfree(p.arap_row_inc);
   dfree(p.arap_blk_ptr); dfree(p.arap_blk_edge); dfree(p.edge_ijk); dfree(p.values);
-  dfree(p.seg_off); dfree(p.seg_cnt); dfree(p.pcg_row_begin);
+  dfree(p.pcg_row_begin);
   dfree(p.clu_row_begin); dfree(p.ustart); dfree(p.clu_vidx); dfree(p.clu_halo);
   dfree(p.clu_halo_ptr); dfree(p.g_vidx); dfree(p.g_halo_ptr); dfree(p.g_halo_col);
-  dfree(p.off_upper); dfree(p.pcg_cta_off); dfree(p.pcg_prob); dfree(p.prob_edge_off);
+  dfree(p.pcg_cta_off); dfree(p.pcg_prob); dfree(p.prob_edge_off);
   dfree(p.st_tile_ptr); dfree(p.st_tile_row); dfree(p.st_tile_cols); dfree(p.edge_terms); dfree(p.edge_energy);
   p = Pattern();
 }
 
 void free_work(Work& w) {
-  dfree(w.pk_src); dfree(w.pk_dst); dfree(w.pk_nrm); dfree(w.pk_ids); dfree(w.pk_ws);
-  dfree(w.c_srcfw); dfree(w.c_nres); dfree(w.c_fr); dfree(w.cnt); dfree(w.node_total); dfree(w.row_order); dfree(w.asm_meta); dfree(w.inc_start);
-  dfree(w.inc); dfree(w.trip); dfree(w.ekeys); dfree(w.rhs); dfree(w.plain); dfree(w.x); dfree(w.z); dfree(w.p0); dfree(w.p1);
-  dfree(w.partials); dfree(w.barrier); dfree(w.err); dfree(w.e_data_part); dfree(w.e_arap_part); dfree(w.stats); dfree(w.timers);
+  dfree(w.key); dfree(w.order); dfree(w.sorted); dfree(w.npos); dfree(w.sp_src); dfree(w.sp_dst); dfree(w.sp_nrm); dfree(w.sp_uw); dfree(w.task);
+  dfree(w.cell_ids); dfree(w.rec); dfree(w.raw); dfree(w.cstat); dfree(w.cl_total); dfree(w.cl_start);
+  dfree(w.cl_cur); dfree(w.clist); dfree(w.cdesc); dfree(w.cnt); dfree(w.node_total); dfree(w.inc_start); dfree(w.rhs); dfree(w.plain); dfree(w.x); dfree(w.z); dfree(w.p0); dfree(w.p1);
+  dfree(w.partials); dfree(w.barrier); dfree(w.err); dfree(w.done); dfree(w.e_data_part); dfree(w.e_arap_part); dfree(w.stats); dfree(w.timers);
   dfree(w.nodes_cat); dfree(w.T_cat); dfree(w.r); dfree(w.ap); dfree(w.minv32);
   w.cnt_cap = 0;
 }
@@ -139,16 +139,16 @@ cudaError_t alloc_work(Work& w, int max_nodes, int max_corrs, int bin_ctas_max) 
   size_t M = (size_t)max_corrs, N = (size_t)max_nodes;
   cudaError_t e;
 #define A_(ptr, n) if ((e = dalloc(&(ptr), (n))) != cudaSuccess) return e
-  A_(w.pk_src, M); A_(w.pk_dst, M); A_(w.pk_nrm, M); A_(w.pk_ids, M); A_(w.pk_ws, M);
-  A_(w.c_srcfw, M); A_(w.c_nres, M); A_(w.c_fr, M);
-  A_(w.node_total, N); A_(w.row_order, N); A_(w.asm_meta, 3 * N); A_(w.inc_start, N + 1);
-  A_(w.inc, 4 * M); A_(w.trip, 16 * M); A_(w.ekeys, 4 * M);
+  A_(w.key, M); A_(w.order, M); A_(w.sorted, M); A_(w.npos, N); A_(w.sp_src, M); A_(w.sp_dst, M); A_(w.sp_nrm, M); A_(w.sp_uw, M);
+  A_(w.task, M); A_(w.cell_ids, M); A_(w.rec, (M / kRecMin + 2) * kRecFloats); A_(w.raw, M); A_(w.cstat, M);
+  A_(w.node_total, N); A_(w.inc_start, N + 1);
+  A_(w.cl_total, N); A_(w.cl_start, N + 1); A_(w.cl_cur, N); A_(w.clist, 4 * M); A_(w.cdesc, 4 * M);
   A_(w.rhs, 6 * N); A_(w.plain, N); A_(w.x, 6 * N); A_(w.z, 6 * N); A_(w.p0, 6 * N); A_(w.p1, 6 * N);
   A_(w.partials, (size_t)2 * 3 * kMaxPcgCtas); A_(w.barrier, (size_t)kMaxPcgCtas); A_(w.err, 1);
-  A_(w.e_data_part, (size_t)(kEnergyCtas + kMaxProblems)); A_(w.e_arap_part, N); A_(w.stats, (size_t)kMaxProblems);
-  A_(w.timers, (size_t)kTimerSlots);
+  A_(w.e_data_part, (size_t)(kMaxEnergyCtas + kMaxProblems)); A_(w.e_arap_part, N); A_(w.stats, (size_t)kMaxProblems);
+  A_(w.timers, (size_t)kTimerSlots); A_(w.done, 1);
 #undef A_
-  return cudaSuccess;
+  return cudaMemset(w.done, 0, sizeof(unsigned));
 }
 
 int cdiv(int a, int b) { return (a + b - 1) / b; }
@@ -222,6 +222,7 @@ cf_status prepare_table(cf_gn* h, std::vector<ProbDesc> in, bool single, cudaStr
   // kSortCorrs correspondences, shared out in proportion to the problems' sizes
   const int B = single ? w.bin_ctas_max
                        : (int)std::max<long long>(w.bin_ctas_max, std::min<long long>(kMaxSortCtas, (Mt + kSortCorrs - 1) / kSortCorrs));
+  const long long e_total = std::min<long long>(kMaxEnergyCtas, std::max<long long>(kEnergyCtas, Mt / kEnergyMinPerCta));
   std::vector<int> bin_prob, e_prob;
   long long cnt = 0;
   int corr_off = 0, node_off = 0;
@@ -243,14 +244,14 @@ cf_status prepare_table(cf_gn* h, std::vector<ProbDesc> in, bool single, cudaStr
     cnt += (long long)bc * d.N;
     bin_prob.insert(bin_prob.end(), bc, p);
     const int ec = single ? kEnergyCtas
-                          : std::max(1, (int)((double)kEnergyCtas * d.M / (double)std::max(1LL, Mt) + 0.5));
+                          : std::max(1, (int)((double)e_total * d.M / (double)std::max(1LL, Mt) + 0.5));
     d.e_cta0 = (int)e_prob.size();
     d.e_ctas = ec;
     e_prob.insert(e_prob.end(), ec, p);
     corr_off += d.M;
     node_off += d.N;
   }
-  if ((int)e_prob.size() > kEnergyCtas + kMaxProblems) return CF_ERR_CAPACITY;
+  if ((int)e_prob.size() > kMaxEnergyCtas + kMaxProblems) return CF_ERR_CAPACITY;
   if (cnt > w.cnt_cap) {
     dfree(w.cnt);
     w.cnt_cap = 0;
@@ -259,7 +260,7 @@ cf_status prepare_table(cf_gn* h, std::vector<ProbDesc> in, bool single, cudaStr
   }
   if (!t.desc) {
     CF_TRY(dalloc(&t.desc, (size_t)kMaxProblems));
-    CF_TRY(dalloc(&t.e_prob, (size_t)(kEnergyCtas + kMaxProblems)));
+    CF_TRY(dalloc(&t.e_prob, (size_t)(kMaxEnergyCtas + kMaxProblems)));
     CF_TRY(dalloc(&t.node_prob, (size_t)w.max_nodes));
   }
   if ((long long)bin_prob.size() > t.bin_cap) {
@@ -321,7 +322,6 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
     return (it != e && *it == c) ? (int)(it - col_idx.begin()) : -1;
   };
   std::vector<int> diag_pos(N), trans_pos(nnzb), upper_pos, upper_row, upper_of_pos(nnzb, -1);
-  int max_up = 1;
   for (int i = 0; i < N; i++) {
     diag_pos[i] = find(i, i);
     for (int q = row_ptr[i]; q < row_ptr[i + 1]; q++) trans_pos[q] = find(col_idx[q], i);
@@ -330,7 +330,6 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
       upper_pos.push_back(q);
       upper_row.push_back(i);
     }
-    max_up = std::max(max_up, row_ptr[i + 1] - diag_pos[i]);
   }
   const int n_upper = (int)upper_pos.size();
   // ARAP edges in the reference's visiting order (solver_kernels.cu:225-233)
@@ -587,7 +586,6 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
   p.nnzb = nnzb;
   p.n_upper = n_upper;
   p.n_edges = n_edges;
-  p.max_upper_row = max_up;
   p.pcg_ctas = G;
   p.pcg_smem = smem;
   p.pcg_a_in_smem = a_smem ? 1 : 0;
@@ -602,8 +600,15 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
   CF_TRY(up(&p.row_ptr, row_ptr));
   CF_TRY(up(&p.col_idx, col_idx));
   CF_TRY(up(&p.diag_pos, diag_pos));
-  CF_TRY(up(&p.trans_pos, trans_pos));
-  CF_TRY(up(&p.upper_row, upper_row));
+  {
+    std::vector<int4> meta(n_upper);
+    for (int u = 0; u < n_upper; u++) {
+      const int q = upper_pos[u];
+      meta[u] = make_int4(upper_row[u], q, col_idx[q], trans_pos[q]);
+    }
+    CF_TRY(dalloc(&p.upper_meta, (size_t)n_upper));
+    CF_TRY(cudaMemcpy(p.upper_meta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  }
   CF_TRY(up(&p.arap_row_ptr, arow_ptr));
   CF_TRY(up(&p.arap_row_inc, arow_inc));
   CF_TRY(up(&p.arap_blk_ptr, ablk_ptr));
@@ -643,16 +648,7 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
     CF_TRY(up(&p.clu_halo, clu_halo.empty() ? std::vector<int>(1, 0) : clu_halo));
   }
   CF_TRY(dalloc(&p.values, (size_t)nnzb * 36));
-  CF_TRY(dalloc(&p.seg_off, (size_t)nnzb));
-  CF_TRY(dalloc(&p.seg_cnt, (size_t)nnzb));
   CF_TRY(cudaMemset(p.values, 0, sizeof(float) * (size_t)std::max(1, nnzb) * 36));
-  {
-    std::vector<int> off_upper;
-    for (int u = 0; u < n_upper; u++)
-      if (col_idx[upper_pos[u]] != upper_row[u]) off_upper.push_back(u);
-    p.n_off = (int)off_upper.size();
-    CF_TRY(up(&p.off_upper, off_upper));
-  }
   h->h_row_ptr = row_ptr;
   h->h_col_idx = col_idx;
   h->pattern_version++;
@@ -700,21 +696,23 @@ cf_status ensure_pattern_batch(cf_gn* h, const std::vector<ProbDesc>& pr, cudaSt
   return st;
 }
 
-// Per-solve binning of correspondence incidences (counting sort by node,
-// then per-row grouping by block column).
-cf_status bin_correspondences(cf_gn* h, cudaStream_t s) {
+// Per-solve sort of the correspondences by their node sets (counting sort by
+// the first node, then within each node's bucket) and the nodes' task lists;
+// resets the error word and, when asked, the statistics, and sets up the nodes.
+cf_status bin_correspondences(cf_gn* h, bool reset_stats, cudaStream_t s) {
   Work& w = h->w;
   const Table& t = h->tb;
   if (t.n_bin > 0) {
-    { Timed tm(h, s, kProfPack, 1); CF_TRY(launch_pack_count(w, t, s)); }
-    { Timed tm(h, s, kProfBinScan, 2); CF_TRY(launch_bin_scan(w, t, s)); }
+    { Timed tm(h, s, kProfPack, 1); CF_TRY(launch_key_count(w, t, s)); }
+    { Timed tm(h, s, kProfBinScan, 2); CF_TRY(launch_bin_scan(w, t, reset_stats, s)); }
     { Timed tm(h, s, kProfScatter, 1); CF_TRY(launch_bin_scatter(w, t, s)); }
+    { Timed tm(h, s, kProfSort, 1); CF_TRY(launch_bucket_sort(w, t, s)); }
+    { Timed tm(h, s, kProfLists, 3); CF_TRY(launch_list_scan(w, t, s)); CF_TRY(launch_node_lists(w, t, h->p, s)); }
   } else {
     CF_TRY(cudaMemsetAsync(w.inc_start, 0, sizeof(int) * (size_t)(t.N + 1), s));
-    CF_TRY(cudaMemsetAsync(w.node_total, 0, sizeof(int) * (size_t)t.N, s));
-    { Timed tm(h, s, kProfBinScan, 1); CF_TRY(launch_row_order(w, t.N, s)); }
+    CF_TRY(cudaMemsetAsync(w.cl_start, 0, sizeof(int) * (size_t)(t.N + 1), s));
+    { Timed tm(h, s, kProfBinScan, 1); CF_TRY(launch_node_setup(w, t, reset_stats, s)); }
   }
-  { Timed tm(h, s, kProfExpand, 1); CF_TRY(launch_expand(w, h->p, t.N, s)); }
   return CF_OK;
 }
 
@@ -765,14 +763,13 @@ namespace {
 // G GN iterations and the final energy over the current table.
 cf_status run_gn(cf_gn* h, SolveArgs& a, cudaStream_t s) {
   Work& w = h->w;
-  { Timed t(h, s, kProfNodePlain, 1); CF_TRY(launch_node_plain(w, a.nodes, a.transforms, a.N, s)); }
   const int G = h->params.gn_iterations;
   for (int g = 0; g < G; g++) {
     { Timed t(h, s, kProfResidual, 1); CF_TRY(launch_residual(w, h->tb, h->p, a, a.transforms, true, s)); }
-    { Timed t(h, s, kProfAssemble, 1); CF_TRY(launch_assemble(w, h->p, a, a.transforms, s)); }
+    { Timed t(h, s, kProfAssemble, 1); CF_TRY(launch_assemble(w, h->p, a, s)); }
     { Timed t(h, s, kProfPcg, 1); CF_TRY(launch_pcg_any(h, a, g, s)); }
   }
-  { Timed t(h, s, kProfEnergy, 2); CF_TRY(launch_final_energy(w, h->p, a, G, s)); }
+  { Timed t(h, s, kProfEnergy, a.tb.P > 1 ? 2 : 1); CF_TRY(launch_final_energy(w, h->p, a, G, s)); }
   h->last_gn = G;
   return CF_OK;
 }
@@ -817,30 +814,26 @@ cf_status read_stats(cf_gn* h, cf_solve_stats* stats, const std::vector<int>& sl
 // (batched: scatter).  kind 0: single problem, 1: batch.
 cf_status enqueue_solve(cf_gn* h, int kind, SolveArgs& a, cudaStream_t s) {
   Work& w = h->w;
-  CF_TRY(cudaMemsetAsync(w.stats, 0, sizeof(DevStats) * (size_t)h->tb.P, s));
-  CF_TRY(cudaMemsetAsync(w.err, 0, sizeof(int), s));
   if (kind == 1) {
     Timed t(h, s, kProfOther, 1);
     CF_TRY(launch_batch_gather(w, h->tb, s));
   }
-  cf_status st = bin_correspondences(h, s);
+  cf_status st = bin_correspondences(h, true, s);
   if (st != CF_OK) return st;
   if (kind == 2) {
     // learned start: features at the warm start, the network's increment,
     // kept only if it lowers the energy (the plain warm start otherwise)
     Mpnn& net = *h->learn_net;
-    { Timed t(h, s, kProfNodePlain, 1); CF_TRY(launch_node_plain(w, a.nodes, a.transforms, a.N, s)); }
-    { Timed t(h, s, kProfResidual, 1); CF_TRY(launch_residual(w, h->tb, h->p, a, a.transforms, true, s, true)); }
+      // the warm start's energy, and each task's residual statistics for the features
+    { Timed t(h, s, kProfEnergy, 1); CF_TRY(launch_final_energy(w, h->p, a, -1, s, true)); }
     {
       Timed t(h, s, kProfLearned, 6);
       CF_TRY(launch_features(w, a.transforms, h->learn_hist, a.N, net.feat, s));
       CF_TRY(mpnn_graph_from_nodes(net, a.nodes, a.N, s));
       CF_TRY(mpnn_forward(net, net.feat, net.out, s));
     }
-    // the warm start's energy from the residual launch above
-    { Timed t(h, s, kProfEnergy, 1); CF_TRY(launch_residual_energy(w, h->p, a, -1, s)); }
     { Timed t(h, s, kProfLearned, 1); CF_TRY(launch_apply_prediction(w, a.transforms, a.nodes, net.out, a.N, s)); }
-    { Timed t(h, s, kProfEnergy, 2); CF_TRY(launch_final_energy(w, h->p, a, -2, s)); }
+    { Timed t(h, s, kProfEnergy, 1); CF_TRY(launch_final_energy(w, h->p, a, -2, s)); }
     { Timed t(h, s, kProfLearned, 1); CF_TRY(launch_gate_prediction(w, a.transforms, a.nodes, a.N, s)); }
   }
   st = run_gn(h, a, s);
@@ -1084,14 +1077,12 @@ cf_status cf_gn_linearize_solve(cf_gn* h, const cf_correspondence* d_corrs, int 
                      true, s);
   if (st != CF_OK) return st;
   Work& w = h->w;
-  CF_TRY(cudaMemsetAsync(w.stats, 0, sizeof(DevStats), s));
-  CF_TRY(cudaMemsetAsync(w.err, 0, sizeof(int), s));
-  st = bin_correspondences(h, s);
+  st = bin_correspondences(h, true, s);
   if (st != CF_OK) return st;
   SolveArgs a = make_args(h, d_nodes, num_nodes, num_corrs);
   a.delta_x = d_delta_x;
   { Timed t(h, s, kProfResidual, 1); CF_TRY(launch_residual(w, h->tb, h->p, a, d_transforms, false, s)); }
-  { Timed t(h, s, kProfAssemble, 1); CF_TRY(launch_assemble(w, h->p, a, d_transforms, s)); }
+  { Timed t(h, s, kProfAssemble, 1); CF_TRY(launch_assemble(w, h->p, a, s)); }
   { Timed t(h, s, kProfPcg, 1); CF_TRY(launch_pcg_any(h, a, 0, s)); }
   h->last_gn = 1;
   return CF_OK;
@@ -1480,11 +1471,10 @@ cf_status cf_gn_features(cf_gn* h, const cf_problem* prob, const cf_dual_quat* d
                           true, s)) != CF_OK)
     return st;
   Work& w = h->w;
-  CF_TRY(cudaMemsetAsync(w.err, 0, sizeof(int), s));
-  if ((st = bin_correspondences(h, s)) != CF_OK) return st;
+  if ((st = bin_correspondences(h, false, s)) != CF_OK) return st;
   SolveArgs a = make_args(h, prob->nodes, N, M);
-  CF_TRY(launch_node_plain(w, prob->nodes, d_transforms, N, s));
-  CF_TRY(launch_residual(w, h->tb, h->p, a, d_transforms, true, s, true));
+  a.transforms = const_cast<cf_dual_quat*>(d_transforms);  // (read only here)
+  CF_TRY(launch_final_energy(w, h->p, a, kNoSlot, s, true));
   CF_TRY(launch_features(w, d_transforms, d_history, N, d_features, s));
   return CF_OK;
 }

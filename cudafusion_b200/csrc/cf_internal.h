@@ -70,12 +70,10 @@ struct Pattern {
   int nnzb = 0;
   int n_upper = 0;      // blocks with col >= row (incl. diagonal)
   int n_edges = 0;      // ARAP edges visited by the reference (lower endpoint owns)
-  int max_upper_row = 0;  // max upper blocks in one row
   int* row_ptr = nullptr;   // [N+1]
   int* col_idx = nullptr;   // [nnzb]
   int* diag_pos = nullptr;  // [N]
-  int* trans_pos = nullptr; // [nnzb] position of the transposed block
-  int* upper_row = nullptr; // [n_upper]
+  int4* upper_meta = nullptr; // [n_upper] row, position, column, position of the transpose
   int* arap_row_ptr = nullptr;  // [N+1]
   int* arap_row_inc = nullptr;  // (edge << 1) | role, role 0 = lower endpoint
   int* arap_blk_ptr = nullptr;  // [n_upper+1] over upper off-diagonal blocks
@@ -85,10 +83,6 @@ struct Pattern {
   double* edge_energy = nullptr; // [n_edges] per GN iteration: el |r|^2
   // per-pattern work arrays
   float* values = nullptr;  // [nnzb*36]
-  int* seg_off = nullptr;   // [nnzb]
-  int* seg_cnt = nullptr;   // [nnzb]
-  int n_off = 0;            // off-diagonal upper blocks
-  int* off_upper = nullptr; // [n_off] their upper indices
   // single-cluster PCG (cf_pcg_cluster.cu)
   int use_cluster = 0;
   int clu_C = 0;
@@ -120,23 +114,29 @@ struct Pattern {
 struct Work {
   int max_nodes = 0, max_corrs = 0;
   int bin_ctas_max = 0;
-  float4* pk_src = nullptr;  // xyz: canonical point (solve) or src (linearise); w: effective weight
-  float4* pk_dst = nullptr;
-  float4* pk_nrm = nullptr;
-  int4* pk_ids = nullptr;
-  float4* pk_ws = nullptr;
-  float4* c_srcfw = nullptr;  // skinned src, fw (0 = skipped)
-  float4* c_nres = nullptr;   // normal, residual
-  float2* c_fr = nullptr;     // (weight, residual) per correspondence, for the learned start's features
+  // the correspondences in the order of their node sets (cf_cells.cu)
+  uint2* key = nullptr;       // [max_corrs] per correspondence: its distinct nodes, ascending, 16-bit local ids
+  int* order = nullptr;       // [max_corrs] the correspondences in order of their first node
+  int* sorted = nullptr;      // [max_corrs] and in order of the whole set
+  float4* sp_src = nullptr;   // [max_corrs] canonical point (solve) or src (linearise), effective weight
+  float4* sp_dst = nullptr;   // target, which node of the set each slot names (3 bits per slot, 7: none)
+  float4* sp_nrm = nullptr;   // normal; w: residual (tasks without a record)
+  float4* sp_uw = nullptr;    // the skin weights of the set's nodes
+  unsigned char* task = nullptr;  // [max_corrs] size of the task that starts at the position, else 0
+  int4* cell_ids = nullptr;   // [max_corrs] at a task's first position: its nodes, ascending, -1 past the last
+  float* rec = nullptr;       // [max_corrs / kRecMin + 2][kRecFloats] the tasks' sums
+  float4* raw = nullptr;      // [max_corrs] skinned src, fw (0 = skipped) of tasks without a record
+  float4* cstat = nullptr;    // [max_corrs] at a task's first position: sum |r|, max |r|, count (learned start)
+  int* cl_total = nullptr;    // [max_nodes] tasks that contain the node
+  int* cl_start = nullptr;    // [max_nodes+1]
+  int* cl_cur = nullptr;      // [max_nodes]
+  float4* npos = nullptr;     // [max_nodes] node positions
+  int* clist = nullptr;       // [4*max_corrs] per node its tasks, in position order
   int* cnt = nullptr;         // per sort CTA, a histogram over its problem's nodes
   long long cnt_cap = 0;      // words allocated for cnt
   int* node_total = nullptr;  // [max_nodes]
-  int* row_order = nullptr;   // [max_nodes] rows by decreasing incidence count (launch order of the per-row kernels)
-  int4* asm_meta = nullptr;   // [3*max_nodes] per launch position: the assembly's row metadata, written by the expand
-  int* inc_start = nullptr;   // [max_nodes+1]
-  int* inc = nullptr;         // [4*max_corrs]: (c << 2) | a
-  int* trip = nullptr;        // [16*max_corrs]: (c << 4) | (a << 2) | b
-  int2* ekeys = nullptr;      // [4*max_corrs]: per incidence, column keys of its 4 slots
+  int* inc_start = nullptr;   // [max_nodes+1] first sorted position of each node's bucket
+  uint4* cdesc = nullptr;     // [4*max_corrs] their descriptions for the gather
   float* rhs = nullptr;       // [6*max_nodes]
   cf_dual_quat* plain = nullptr;  // [max_nodes]
   float* x = nullptr;         // [6*max_nodes]
@@ -146,7 +146,8 @@ struct Work {
   double* partials = nullptr;  // [2 bufs][3 slots][max pcg ctas]
   unsigned* barrier = nullptr;  // [max pcg ctas] one arrival counter per PCG CTA group
   int* err = nullptr;
-  double* e_data_part = nullptr;  // [kEnergyCtas + kMaxProblems] one partial per energy CTA
+  unsigned* done = nullptr;       // CTAs of an energy launch that have finished (0 between launches)
+  double* e_data_part = nullptr;  // [kMaxEnergyCtas + kMaxProblems] one partial per energy CTA
   double* e_arap_part = nullptr;  // [max_nodes] per row
   DevStats* stats = nullptr;      // [kMaxProblems]
   // streaming PCG: residual, A p and the FP32 block inverses in global memory
@@ -160,8 +161,20 @@ struct Work {
   long long* timers = nullptr;  // [kTimerSlots] phase cycles of the grid PCG (debug)
 };
 
-constexpr int kEnergyCtas = 512;  // residual/energy CTAs of a single solve (with the edge CTAs, one wave at 4 per SM)
+// CTAs of the data term.  A single solve's share it evenly in one wave (two per
+// SM; 148 SMs).  A batch's problems differ, so up to eight waves once each warp
+// still has 16 windows of 32 correspondences: a problem's CTAs are whole ones.
+constexpr int kEnergyCtas = 296;
+constexpr int kMaxEnergyCtas = 8 * kEnergyCtas;
+constexpr int kEnergyMinPerCta = 8 * 32 * 16;
 constexpr int kMaxPcgCtas = 1024;
+constexpr int kSortChunk = 512;  // sorted positions of a bucket's chunk (cf_cells.cu)
+// Tasks of at least kRecMin correspondences leave a record of sums; one that
+// starts at position q owns record ceil(q / kRecMin), which no other does,
+// so records are bounded by the correspondences.  In smaller ones (under 2 % of
+// the correspondences of a frame) the gather reads each correspondence.
+constexpr int kRecMin = 4;
+constexpr int kRecFloats = 236;  // 10 pairs x 21 sums, 4 x 6 right-hand sides, padded to 16 B
 constexpr int kSortCorrs = 4096;     // correspondences per sort CTA of a batched solve (at least)
 constexpr int kMaxSortCtas = 1 << 16;
 // Rows per CTA up to which mode 0 picks the single-cluster PCG.  Its exchanges
@@ -222,22 +235,23 @@ struct PhaseClock {
 
 
 // ---- launchers (cf_kernels.cu) ----
-cudaError_t launch_pack_count(const Work& w, const Table& tb, cudaStream_t s);
-cudaError_t launch_bin_scan(const Work& w, const Table& tb, cudaStream_t s);
-cudaError_t launch_row_order(const Work& w, int N, cudaStream_t s);
+cudaError_t launch_key_count(const Work& w, const Table& tb, cudaStream_t s);
+cudaError_t launch_bin_scan(const Work& w, const Table& tb, bool reset_stats, cudaStream_t s);
 cudaError_t launch_bin_scatter(const Work& w, const Table& tb, cudaStream_t s);
-cudaError_t launch_expand(const Work& w, const Pattern& p, int N, cudaStream_t s);
-cudaError_t launch_node_plain(const Work& w, const cf_deform_node* nodes, const cf_dual_quat* T, int N,
-                              cudaStream_t s);
+cudaError_t launch_node_setup(const Work& w, const Table& tb, bool reset_stats, cudaStream_t s);
+cudaError_t launch_list_scan(const Work& w, const Table& tb, cudaStream_t s);
+// cf_cells.cu
+cudaError_t launch_bucket_sort(const Work& w, const Table& tb, cudaStream_t s);
+cudaError_t launch_node_lists(const Work& w, const Table& tb, const Pattern& p, cudaStream_t s);
 cudaError_t launch_residual(const Work& w, const Table& tb, const Pattern& p, const SolveArgs& a,
-                            const cf_dual_quat* T, bool skin, cudaStream_t s, bool fr = false);
+                            const cf_dual_quat* T, bool skin, cudaStream_t s);
 cudaError_t launch_batch_gather(const Work& w, const Table& tb, cudaStream_t s);
 cudaError_t launch_batch_scatter(const Work& w, const Table& tb, cudaStream_t s);
-cudaError_t launch_assemble(const Work& w, const Pattern& p, const SolveArgs& a, const cf_dual_quat* T,
-                            cudaStream_t s);
+cudaError_t launch_assemble(const Work& w, const Pattern& p, const SolveArgs& a, cudaStream_t s);
 cudaError_t launch_pcg(const Work& w, const Pattern& p, const SolveArgs& a, int gn_slot, cudaStream_t s);
-cudaError_t launch_residual_energy(const Work& w, const Pattern& p, const SolveArgs& a, int slot, cudaStream_t s);
-cudaError_t launch_final_energy(const Work& w, const Pattern& p, const SolveArgs& a, int slot, cudaStream_t s);
+constexpr int kNoSlot = -1000;  // (launch_final_energy) the energy is not kept
+cudaError_t launch_final_energy(const Work& w, const Pattern& p, const SolveArgs& a, int slot, cudaStream_t s,
+                                bool stats = false);
 cudaError_t launch_apply_twist(cf_dual_quat* T, const float* dx, int N, float max_rot, float max_trans,
                                float scale, cudaStream_t s);
 // cf_corr.cu: projective correspondence search
@@ -308,7 +322,6 @@ cudaError_t launch_energy_noalloc(const cf_problem* pr, const cf_dual_quat* T, f
                                   cudaStream_t s);
 int pcg_grid_smem_bytes(int nblk, int nrows, int nhalo, bool a_in_smem, bool pipelined);
 int pcg_max_active_ctas(int smem, bool a_in_smem, bool pipelined);
-int expand_smem_bytes(int max_upper_row, int N);
 
 int pcg_cluster_max_rows();
 int pcg_cluster_smem_bytes(int blk_max, int rows_max, int nhalo_max, int C);

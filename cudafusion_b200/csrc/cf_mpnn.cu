@@ -475,36 +475,20 @@ __global__ void increments_kernel(const cf_dual_quat* __restrict__ to, const cf_
 // Features of every node at the warm start T (= T_{t-1}) with the history
 // hist = [T_{t-2}, T_{t-3}, T_{t-4}]: the three increments (scaled) and the
 // mean / max |residual| (mm) of the node's valid correspondences (the
-// residual launch at T must have run; warp per node over its incidences).
+// residual launch at T must have run; warp per node over its tasks).
 __global__ void features_kernel(const cf_dual_quat* __restrict__ T, const cf_dual_quat* __restrict__ hist, int N,
-                                const int* __restrict__ inc_start, const int* __restrict__ inc,
-                                const float2* __restrict__ c_fr, float* __restrict__ feat) {
+                                const int* __restrict__ cl_start, const int* __restrict__ clist,
+                                const float4* __restrict__ cstat, float* __restrict__ feat) {
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= N) return;
   float s = 0.f, mx = 0.f;
   int cnt = 0;
-  // 4 incidences per lane in flight: their ids, then the (weight, residual)
-  // pair of each (8 B, written by the residual launch), summed in incidence order
-  const int q1 = inc_start[i + 1];
-  for (int q0 = inc_start[i] + lane; q0 < q1; q0 += 4 * 32) {
-    int c[4];
-#pragma unroll
-    for (int b = 0; b < 4; b++) c[b] = q0 + 32 * b < q1 ? (inc[q0 + 32 * b] >> 2) : -1;
-    float f[4], r[4];
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const float2 fr = c[b] >= 0 ? __ldg(c_fr + c[b]) : make_float2(0.f, 0.f);
-      f[b] = fr.x;
-      r[b] = fr.y;
-    }
-#pragma unroll
-    for (int b = 0; b < 4; b++)
-      if (f[b] > 0.f) {
-        const float ra = fabsf(r[b]);
-        s += ra;
-        mx = fmaxf(mx, ra);
-        cnt++;
-      }
+  // the node's tasks (about 28), each with the sum, maximum and count of its |residuals|
+  for (int q = cl_start[i] + lane; q < cl_start[i + 1]; q += 32) {
+    const float4 v = __ldg(cstat + (clist[q] >> 2));
+    s += v.x;
+    mx = fmaxf(mx, v.y);
+    cnt += (int)v.z;
   }
   s = warp_sum_f(s);
 #pragma unroll
@@ -695,7 +679,7 @@ cudaError_t launch_increments(const cf_dual_quat* to, const cf_dual_quat* from, 
 cudaError_t launch_features(const Work& w, const cf_dual_quat* T, const cf_dual_quat* hist, int N, float* feat,
                             cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  features_kernel<<<cdiv(N * 32, 256), 256, 0, s>>>(T, hist, N, w.inc_start, w.inc, w.c_fr, feat);
+  features_kernel<<<cdiv(N * 32, 256), 256, 0, s>>>(T, hist, N, w.cl_start, w.clist, w.cstat, feat);
   return cudaGetLastError();
 }
 

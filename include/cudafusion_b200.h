@@ -160,7 +160,7 @@ CF_API cf_status cf_gn_linearize_solve(cf_gn* h, const cf_correspondence* d_corr
  *                          the GPU's shared memory, streaming); 1: grid-wide
  *                          cooperative PCG with the system in shared memory
  *                          (streaming when it does not fit); 2: single-
- *                          cluster PCG (full rows in distributed shared 
+ *                          cluster PCG (full rows in distributed shared
  *                          memory) when the system fits the cluster's shared
  *                          memory (else grid-wide); 3: streaming PCG (A re-read from HBM
  *                          through TMA bulk copies every iteration, vectors
