@@ -1639,8 +1639,13 @@ void corr_free(cf_corr_search* h) {
   cudaFree(h->keep);
   cudaFree(h->sc.A);
   cudaFree(h->sc.B);
-  cudaFree(h->sc.part_pd);
-  cudaFree(h->sc.part_idx);
+  cudaFree(h->sc.part_a);
+  cudaFree(h->sc.part_g);
+  cudaFree(h->sc.rows);
+  cudaFree(h->sc.box);
+  cudaFree(h->sc.pix_v);
+  cudaFree(h->sc.pix_n);
+  cudaFree(h->sc.pix_row);
   cudaFree(h->sc.flag);
 }
 }  // namespace
@@ -1660,8 +1665,14 @@ cf_status cf_corr_search_create(int max_width, int max_height, cf_corr_search** 
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sc.sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = dalloc(&h->sc.A, P);
   if (e == cudaSuccess) e = dalloc(&h->sc.B, P);
-  if (e == cudaSuccess) e = dalloc(&h->sc.part_pd, P * kCorrMaxChunks);
-  if (e == cudaSuccess) e = dalloc(&h->sc.part_idx, P * kCorrMaxChunks);
+  h->sc.chunk_cap = corr_chunk_cap(P);
+  if (e == cudaSuccess) e = dalloc(&h->sc.part_a, P * h->sc.chunk_cap);
+  if (e == cudaSuccess) e = dalloc(&h->sc.part_g, P * h->sc.chunk_cap);
+  if (e == cudaSuccess) e = dalloc(&h->sc.rows, corr_box_cap(P));
+  if (e == cudaSuccess) e = cudaMalloc(&h->sc.box, corr_box_cap(P) * corr_box_bytes());
+  if (e == cudaSuccess) e = dalloc(&h->sc.pix_v, P);
+  if (e == cudaSuccess) e = dalloc(&h->sc.pix_n, P);
+  if (e == cudaSuccess) e = dalloc(&h->sc.pix_row, P);
   if (e == cudaSuccess) e = dalloc(&h->sc.flag, 1);
   if (e != cudaSuccess) {
     corr_free(h);

@@ -26,41 +26,61 @@
 //                      unprojected point and the normal.  The two skip cases
 //                      are folded into z (0: no depth; -1: no normal) with x, y
 //                      and the normal's x so large that the record's
-//                      point-to-plane distance is +inf.
+//                      point-to-plane distance is +inf.  Per block of 16 x 16
+//                      pixels the box of its real points and its longest normal.
 //                      The reference recomputes the unprojection, two
 //                      divisions, for every (pixel, candidate) pair.
-//  corr_search_kernel  one thread per two vertically adjacent live pixels (one
-//                      shared-memory load serves both windows; each pixel still
-//                      meets its candidates in row-major order), 32 x 16 pixels
-//                      per CTA, and
-//                      blockIdx.z = one of C chunks of the rows that the CTA's
-//                      windows cover (C from a cost model of the waves of
-//                      tiles x C CTAs over the resident slots).  The CTA stages
-//                      its chunk in shared memory one band of rows at a time;
-//                      each thread scans its window's rows in the chunk in
-//                      row-major order with the reference's acceptance rule,
-//                      applied to groups of 4 consecutive candidates (one min
-//                      per candidate, one compare per group, the group's first
-//                      column found again at the end).  The Euclidean test
-//                      compares the
-//                      squared distance with the largest float whose IEEE
-//                      square root is within the cap (exact: the rounded
-//                      square root is monotonic), and is left out for a band
-//                      whose bounding box of real points lies within the cap.  With one chunk the kernel writes the
-//                      records itself; otherwise each (chunk, pixel) leaves its
-//                      best distance and candidate for
-//  corr_merge_kernel   which takes the chunks in row order with the same
-//                      strict-less rule.  That reproduces one sequential scan
-//                      because no distance can be NaN: every value entering
-//                      the search is finite and at most 1e18 in magnitude, so
-//                      no product sum overflows.  A pixel or frame holding any
-//                      other value is rescanned sequentially with the
-//                      reference's rule as it stands (a NaN distance is
-//                      accepted).  The record write gathers the pixel's node
-//                      lists and reduces the counters per warp.
+//                      The live pixels' camera-frame points, projections and
+//                      rejections are made here as well.
+//  corr_search_kernel  finds, for each pixel and chunk of image rows, the runs
+//                      of kGroup candidates that can hold the winner (below).
+//  corr_merge_kernel   evaluates those runs with the reference's arithmetic,
+//                      takes the least distance (of equal ones the first
+//                      candidate in row-major order: the strict-less rule of
+//                      one sequential scan, as no distance can be NaN: every
+//                      value entering the search is finite and at most 1e18 in
+//                      magnitude, so no product sum overflows), and writes the
+//                      record.  A pixel or frame holding any other value is
+//                      rescanned sequentially with the reference's rule as it
+//                      stands (a NaN distance is accepted).  Small windows it
+//                      scans itself, without a search before.
+//
+// The search.  A CTA takes 32 x 16 pixels, a warp 8 x 8 of them, a lane two.
+// The warp scans the union of its pixels' windows.  With o the centre of the
+// CTA's points, w = v - o, and per candidate c = n . (p - o), made once per CTA as
+// the records are staged, n . (v - p) is n . w - c: a contraction, done on the
+// tensor cores eight candidates by 16 pixels at a time, with n, w and c as sums
+// of two or three halfs (16 products per value).  It differs from the
+// reference's rounded distance by at most
+//   eps = u N (25 max |w| + 20 max |p - o|)       (u = 2^-24, N the longest normal):
+// 4 u (both terms) for the reference's roundings, u and 4 u for those of w and
+// c in FP32, 8 u for what two halfs leave of n and w, and 11 u for the tensor
+// core's sum, of which at most 2.7 u was seen over 10^7 sums of such terms
+// (0.7 u where they cancel).  That is some 3e-7 m.  Per run of up to kGroup
+// candidates of a row a lane takes the least |n . w - c| and keeps of these the
+// least L1, the second L2 (with their runs) and the third L3, each less eps.  The
+// winner's distance is at most U = min(L1 + 2 eps), so it is in a run of L <= U:
+// usually one, and if a chunk's L3 <= U its rows are scanned again.  A surface
+// with many equal distances (a plane seen head on) takes that path, at about
+// the cost of one exact scan.
+// With an angle threshold the values come from packed FP32 FMAs on the lane's own
+// two pixels (one shared-memory broadcast per candidate; eps = 14 u N (max |w| +
+// max |p - o|)), since that test needs each candidate's normal.  Where the boxes
+// do not prove every candidate within the Euclidean cap, or the values' ranges
+// leave no room in halfs, the CTA scans with the reference's arithmetic and cap
+// test instead (eps = 0).
+//
+// What bounds it: the legacy tensor path (8.2 clocks per step and SM quarter)
+// and instruction issue (two lane-minima per step and 16 pixels, the masks of
+// the windows' edges).  Measured on B200, 640 x 480: radius 50 585 us per call
+// (1825 with a thread per two pixels scanning its own windows in the reference's
+// arithmetic: its shared-memory reads and 11 instructions per candidate), with an
+// angle threshold 1411 (2656), past the cap 2122 (2868), radius 20 272 (463).
 #include <cfloat>
 #include <climits>
 #include <cmath>
+
+#include <cuda_fp16.h>
 
 #include "cf_internal.h"
 
@@ -68,13 +88,23 @@ namespace cf {
 
 namespace {
 
-constexpr int kCsTx = 32;
-constexpr int kCsTy = 8;
-constexpr int kCsPy = 2 * kCsTy;  // pixel rows per tile: each thread scans two
-constexpr int kCsThreads = kCsTx * kCsTy;
-constexpr int kCsSmem = 55 * 1024;  // one band of records; 4 CTAs per SM with the 1 KB reserve each
-constexpr int kCsCtasPerSm = 4;
-constexpr int kCsRecBytes = (int)(sizeof(float4) + sizeof(float2));
+constexpr int kCsTx = 32;  // pixels of a CTA
+constexpr int kCsTy = 16;
+constexpr int kCsThreads = 256;
+constexpr int kCsSmem = 72 * 1024;  // one band of records; 3 CTAs per SM with the 1 KB reserve each
+constexpr int kCsCtasPerSm = 3;
+constexpr int kCsBlock = 16;  // side of the blocks whose boxes are known
+constexpr int kGroup = 128;   // candidates of a run at most
+constexpr int kSub = 8;       // columns scanned with or without window masks together
+constexpr int kSlab = 768;    // columns staged at a time at most
+constexpr int kPad = 8;       // and the columns past them that a step may read
+constexpr float kFarS = 3e5f;  // (scaled) distance of what is not there, above every real one
+// Largest radius whose windows the merge scans itself, a lane per pixel: 640 x
+// 480 takes 84 us at radius 3 and 118 at 6 that way, 137 and 150 with the
+// search's fixed costs; at 8 152 (from the candidates' share) and 165.
+constexpr int kCsDirect = 8;
+constexpr float kCsNone = 1e30f;  // distance of what is not there
+constexpr float kU = 5.9604645e-8f;  // 2^-24
 constexpr float kCsBig = 1e18f;  // squares and three-term sums of such values stay finite in FP32
 constexpr float kCsFar = 1e30f;  // x, y and normal x of a skip record: its distance overflows to +inf
 
@@ -121,34 +151,6 @@ __device__ __forceinline__ float3 cs_normalize(float3 v) {
 __device__ __forceinline__ float cs_norm(float x, float y, float z) { return __fsqrt_rn(cs_dot(x, y, z, x, y, z)); }
 __device__ __forceinline__ bool cs_small(float v) { return fabsf(v) <= kCsBig; }  // false for NaN and inf
 
-__global__ void corr_prep_kernel(const float* __restrict__ depth, const float* __restrict__ dn, int W, int H,
-                                 float fx, float fy, float cx, float cy, float4* __restrict__ A,
-                                 float2* __restrict__ B, int* __restrict__ flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W * H) return;
-  const int y = i / W, x = i - y * W;
-  const float d = depth[i];
-  float4 a = make_float4(kCsFar, kCsFar, 0.f, kCsFar);
-  float2 b = make_float2(0.f, 0.f);
-  if (!(d <= 0.f)) {
-    const float nx = dn[3 * i], ny = dn[3 * i + 1], nz = dn[3 * i + 2];
-    if (cs_norm(nx, ny, nz) < 1e-6f) {
-      a.z = -1.f;
-    } else {
-      // CameraIntrinsics::unproject, include/types.h:157-161
-      a.x = __fdiv_rn(__fmul_rn(d, __fsub_rn((float)x, cx)), fx);
-      a.y = __fdiv_rn(__fmul_rn(d, __fsub_rn((float)y, cy)), fy);
-      a.z = d;
-      a.w = nx;
-      b = make_float2(ny, nz);
-      if (!(cs_small(a.x) && cs_small(a.y) && cs_small(d) && cs_small(nx) && cs_small(ny) && cs_small(nz)))
-        atomicOr(flag, 1);
-    }
-  }
-  A[i] = a;
-  B[i] = b;
-}
-
 // The per-pixel part of find_correspondences_kernel before the window scan.
 struct CsPixel {
   int code;      // debug counter when the pixel stops here, else -1
@@ -160,7 +162,7 @@ struct CsPixel {
 };
 
 __device__ __forceinline__ CsPixel cs_pixel(const CorrConsts& k, const float* __restrict__ lv,
-                                            const float* __restrict__ ln, int px, int frame_flag) {
+                                            const float* __restrict__ ln, int px) {
   CsPixel p;
   p.code = -1;
   p.search = false;
@@ -194,160 +196,319 @@ __device__ __forceinline__ CsPixel cs_pixel(const CorrConsts& k, const float* __
     return p;
   }
   p.search = true;
-  p.special = frame_flag != 0 || !(cs_small(p.vc.x) && cs_small(p.vc.y) && cs_small(p.vc.z) && cs_small(p.nc.x) &&
-                                   cs_small(p.nc.y) && cs_small(p.nc.z));
+  p.special = !(cs_small(p.vc.x) && cs_small(p.vc.y) && cs_small(p.vc.z) && cs_small(p.nc.x) && cs_small(p.nc.y) &&
+                cs_small(p.nc.z));
   return p;
 }
 
-// The scan state of one pixel: its projection, camera-frame point and normal,
-// and the best candidate so far.
-struct CsScan {
-  int pu, pv;
-  float vx, vy, vz, nx, ny, nz;
-  float best;
-  int bi;
-  bool on;  // the pixel is scanned here
+// A pixel's record: its camera-frame point and projection's column, its normal
+// and view cosine, and its projection's row, with bit 30 for a special one, or
+// -1 - the counter at which it stopped.
+struct CsPix {
+  float4* __restrict__ v;
+  float4* __restrict__ n;
+  int* __restrict__ row;
 };
+constexpr int kCsSpecial = 1 << 30;
+__device__ __forceinline__ CsPixel cs_load_pixel(const CsPix& x, int px) {
+  const int row = x.row[px];
+  const float4 v = x.v[px], n = x.n[px];
+  CsPixel p;
+  p.search = row >= 0;
+  p.code = row >= 0 ? -1 : -1 - row;
+  p.special = row >= 0 && (row & kCsSpecial) != 0;
+  p.pu = __float_as_int(v.w);
+  p.pv = row & (kCsSpecial - 1);
+  p.vl = make_float3(0.f, 0.f, 0.f);  // (the merge reads it when it is needed)
+  p.vc = make_float3(v.x, v.y, v.z);
+  p.nc = make_float3(n.x, n.y, n.z);
+  p.view_cos = n.w;
+  return p;
+}
 
-__device__ __forceinline__ CsScan cs_scan_state(const CsPixel& p, bool on, float dist_thr) {
-  CsScan q;
-  q.pu = p.pu;
-  q.pv = p.pv;
-  q.vx = p.vc.x;
-  q.vy = p.vc.y;
-  q.vz = p.vc.z;
-  q.nx = p.nc.x;
-  q.ny = p.nc.y;
-  q.nz = p.nc.z;
-  q.best = dist_thr;
-  q.bi = -1;
-  q.on = on;
-  return q;
+__device__ __forceinline__ float cs_warp_max(float v) {
+  float d;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(v));
+  return d;
+}
+
+// What is known of a block of 16 x 16 pixels.  Maxima throughout: of the
+// depth's real points -x, -y, -z, |n|^2, x, y, z (-inf: none; |n|^2: 0), and of
+// the live pixels that are scanned -pu, pu, -pv, pv (kCsOff: none) and their
+// points' -x, -y, -z, x, y, z.
+struct CsBox {
+  float d[8];  // (d[7] unused)
+  int p[4];
+  float v[6];
+  float pad[2];
+};
+static_assert(sizeof(CsBox) == 80, "whole 16-byte words");
+constexpr int kCsOff = -(1 << 30);
+
+// One thread per pixel: the depth's candidate record, the live pixel's record,
+// and the block's box.
+__global__ void __launch_bounds__(kCsBlock* kCsBlock)
+    corr_prep_kernel(const CorrConsts k, const float* __restrict__ depth, const float* __restrict__ dn,
+                     const float* __restrict__ lv, const float* __restrict__ ln, float4* __restrict__ A,
+                     float2* __restrict__ B, const CsPix pix, CsBox* __restrict__ box, int* __restrict__ flag,
+                     int* __restrict__ num_valid, int* __restrict__ stats) {
+  __shared__ float s_f[kCsBlock * kCsBlock / 32][13];
+  __shared__ int s_i[kCsBlock * kCsBlock / 32][4];
+  const int tid = threadIdx.x;
+  const int x = blockIdx.x * kCsBlock + (tid & (kCsBlock - 1)), y = blockIdx.y * kCsBlock + tid / kCsBlock;
+  if (blockIdx.x == 0 && blockIdx.y == 0) {  // (counted by the merge)
+    if (tid == 0) *num_valid = 0;
+    if (stats && tid < 6) stats[tid] = 0;
+  }
+  const float none = -INFINITY;
+  float f[13] = {none, none, none, 0.f, none, none, none, none, none, none, none, none, none};
+  int q[4] = {kCsOff, kCsOff, kCsOff, kCsOff};
+  if (x < k.W && y < k.H) {
+    const int i = y * k.W + x;
+    const float d = depth[i];
+    float4 a = make_float4(kCsFar, kCsFar, 0.f, kCsFar);
+    float2 b = make_float2(0.f, 0.f);
+    if (!(d <= 0.f)) {
+      const float nx = dn[3 * i], ny = dn[3 * i + 1], nz = dn[3 * i + 2];
+      if (cs_norm(nx, ny, nz) < 1e-6f) {
+        a.z = -1.f;
+      } else {
+        // CameraIntrinsics::unproject, include/types.h:157-161
+        a.x = __fdiv_rn(__fmul_rn(d, __fsub_rn((float)x, k.cx)), k.fx);
+        a.y = __fdiv_rn(__fmul_rn(d, __fsub_rn((float)y, k.cy)), k.fy);
+        a.z = d;
+        a.w = nx;
+        b = make_float2(ny, nz);
+        if (!(cs_small(a.x) && cs_small(a.y) && cs_small(d) && cs_small(nx) && cs_small(ny) && cs_small(nz)))
+          atomicOr(flag, 1);
+        f[0] = -a.x; f[1] = -a.y; f[2] = -a.z;
+        f[3] = nx * nx + ny * ny + nz * nz;
+        f[4] = a.x; f[5] = a.y; f[6] = a.z;
+      }
+    }
+    A[i] = a;
+    B[i] = b;
+    const CsPixel p = cs_pixel(k, lv, ln, i);
+    pix.row[i] = p.search ? p.pv | (p.special ? kCsSpecial : 0) : -1 - p.code;
+    pix.v[i] = make_float4(p.vc.x, p.vc.y, p.vc.z, __int_as_float(p.pu));
+    pix.n[i] = make_float4(p.nc.x, p.nc.y, p.nc.z, p.view_cos);
+    if (p.search && !p.special) {
+      q[0] = -p.pu; q[1] = p.pu; q[2] = -p.pv; q[3] = p.pv;
+      f[7] = -p.vc.x; f[8] = -p.vc.y; f[9] = -p.vc.z;
+      f[10] = p.vc.x; f[11] = p.vc.y; f[12] = p.vc.z;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 13; ++c) f[c] = cs_warp_max(f[c]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) q[c] = __reduce_max_sync(0xffffffffu, q[c]);
+  if ((tid & 31) == 0) {
+#pragma unroll
+    for (int c = 0; c < 13; ++c) s_f[tid >> 5][c] = f[c];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s_i[tid >> 5][c] = q[c];
+  }
+  __syncthreads();
+  CsBox* o = box + (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+  if (tid < 13) {
+    float m = s_f[0][tid];
+#pragma unroll
+    for (int w = 1; w < kCsBlock * kCsBlock / 32; ++w) m = fmaxf(m, s_f[w][tid]);
+    (tid < 7 ? o->d[tid] : o->v[tid - 7]) = m;
+  } else if (tid < 17) {
+    int m = s_i[0][tid - 13];
+#pragma unroll
+    for (int w = 1; w < kCsBlock * kCsBlock / 32; ++w) m = max(m, s_i[w][tid - 13]);
+    o->p[tid - 13] = m;
+  }
 }
 
 // A candidate's point-to-plane distance, +inf where the reference would skip
 // it (finite values only).  A skip record's far-away point and huge normal
-// make its distance +inf by themselves.  kCheckS: apply the Euclidean cap
-// (left out where the band's bounding box proves every record within it);
-// kAngle: apply the angle threshold.
-template <bool kAngle, bool kCheckS>
-__device__ __forceinline__ float cs_pd(const CsScan& q, const float4& a, const float2& b, const CorrConsts& k) {
-  const float ex = __fsub_rn(q.vx, a.x), ey = __fsub_rn(q.vy, a.y), ez = __fsub_rn(q.vz, a.z);
+// make its distance +inf by themselves.  kAngle: apply the angle threshold.
+template <bool kAngle>
+__device__ __forceinline__ float cs_pd(const float3& v, const float3& n, const float4& a, const float2& b,
+                                       const CorrConsts& k) {
+  const float ex = __fsub_rn(v.x, a.x), ey = __fsub_rn(v.y, a.y), ez = __fsub_rn(v.z, a.z);
   float pd = fabsf(cs_dot(a.w, b.x, b.y, ex, ey, ez));
-  if (kCheckS) pd = cs_dot(ex, ey, ez, ex, ey, ez) <= k.s_max ? pd : INFINITY;
-  if (kAngle) pd = fabsf(cs_dot(q.nx, q.ny, q.nz, a.w, b.x, b.y)) < k.angle_thr ? INFINITY : pd;
+  pd = cs_dot(ex, ey, ez, ex, ey, ez) <= k.s_max ? pd : INFINITY;
+  if (kAngle) pd = fabsf(cs_dot(n.x, n.y, n.z, a.w, b.x, b.y)) < k.angle_thr ? INFINITY : pd;
   return pd;
 }
 
-// The acceptance rule over columns lo..hi of one row, for one pixel or for
-// two at one load each, by groups of kCsGroup consecutive candidates: the
-// group's minimum distance (one min per candidate) replaces the best when
-// strictly below it, and q.bi keeps the first candidate of that group.  The
-// winning group is the first one holding the least distance, as in the
-// reference's scan; cs_resolve finds the first candidate in it reaching that
-// distance.  best starts at the distance bound and only falls, so a kept
-// distance is below the bound.
-constexpr int kCsGroup = 4;
-
-__device__ __forceinline__ void cs_keep(CsScan& q, float m, int idx) {
-  const bool acc = m < q.best;
-  q.best = acc ? m : q.best;
-  q.bi = acc ? idx : q.bi;
+__device__ __forceinline__ unsigned long long cs_pack(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 cs_unpack(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ unsigned long long cs_fma2(unsigned long long a, unsigned long long b,
+                                                      unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long cs_mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 
-template <bool kAngle, bool kCheckS>
-__device__ __forceinline__ void cs_seg1(const float4* ra, const float2* rb, int lo, int hi, int row_base, CsScan& q,
-                                        const CorrConsts& k) {
-  int xx = lo;
-  for (; xx + kCsGroup - 1 <= hi; xx += kCsGroup) {
-    float m = INFINITY;
+// One of a lane's two pixels.
+struct CsLane {
+  unsigned long long wx, wy, wz;  // its point less the origin, twice (filter), or its point (exact)
+  unsigned long long nx, ny, nz;  // its normal, twice (angle test)
+  int l;                          // its window's first column and the columns after it
+  unsigned span;
+  int pv;                         // its projection's row; off the image when it is not scanned
+  float L1, L2, L3;
+  int g1, g2;                     // the runs of L1 and L2: their first pixel
+};
+
+__device__ __forceinline__ float cs_min_abs(float a, float b, float c) {
+  float d;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Two candidates' distances from a pixel into m.  (col: the first one's
+// column, for the window mask.)
+template <bool kAngle, bool kMask>
+__device__ __forceinline__ float cs_pair(float m, const CsLane& q, const ulonglong2& xy, const ulonglong2& zc, int col,
+                                         float angle_thr) {
+  float2 f = cs_unpack(cs_fma2(xy.x, q.wx, cs_fma2(xy.y, q.wy, cs_fma2(zc.x, q.wz, zc.y))));
+  if (kAngle) {
+    const float2 t = cs_unpack(cs_fma2(q.nz, zc.x, cs_fma2(q.ny, xy.y, cs_mul2(q.nx, xy.x))));
+    f.x = fabsf(t.x) < angle_thr ? kCsNone : f.x;
+    f.y = fabsf(t.y) < angle_thr ? kCsNone : f.y;
+  }
+  if (kMask) {
+    f.x = (unsigned)(col - q.l) <= q.span ? f.x : kCsNone;
+    f.y = (unsigned)(col + 1 - q.l) <= q.span ? f.y : kCsNone;
+  }
+  return cs_min_abs(m, f.x, f.y);
+}
+
+// A run's least value into the pixel's three least.
+__device__ __forceinline__ void cs_track(CsLane& q, float m, float eps, int g) {
+  const float L = m - eps;
+  const bool c1 = L < q.L1, c2 = L < q.L2;
+  q.L3 = fminf(q.L3, fmaxf(q.L2, L));
+  q.L2 = fminf(q.L2, fmaxf(q.L1, L));
+  q.g2 = c1 ? q.g1 : c2 ? g : q.g2;
+  q.L1 = fminf(q.L1, L);
+  q.g1 = c1 ? g : q.g1;
+}
+
+// D = A B of one tensor-core step: 16 pixels by 8 candidates over 16 products.
+__device__ __forceinline__ void cs_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ unsigned cs_h2(float x, float y) {  // two halfs, x in the lower one
+  const __half2 h = __floats2half2_rn(x, y);
+  return reinterpret_cast<const unsigned&>(h);
+}
+// x as a sum of halfs: the nearest, and the nearest to what is left
+__device__ __forceinline__ float cs_hi(float x) { return __half2float(__float2half_rn(x)); }
+
+// The 16 products that make n . w - c: the high and low halfs of n and w
+// against each other, and c in three halfs against 4.  A candidate's halfs in
+// the order in which lanes read them: lane t of a quad those of the products
+// 2t, 2t + 1, 2t + 8, 2t + 9.
+//   0..2  w_hi n_hi    3..5  w_lo n_hi    6..8  w_hi n_lo    9..11  w_lo n_lo
+//   12..14  4 c'       (c' = -c / 4)      15  0
+__device__ __forceinline__ void cs_store_mma(float4* o, float nx, float ny, float nz, float mc) {
+  const float hx = cs_hi(nx), hy = cs_hi(ny), hz = cs_hi(nz), lx = nx - hx, ly = ny - hy, lz = nz - hz;
+  const float c1 = cs_hi(mc), c2 = cs_hi(mc - c1), c3 = mc - c1 - c2;
+  o[0] = make_float4(__uint_as_float(cs_h2(hx, hy)), __uint_as_float(cs_h2(lz, lx)), __uint_as_float(cs_h2(hz, hx)),
+                     __uint_as_float(cs_h2(ly, lz)));
+  o[1] = make_float4(__uint_as_float(cs_h2(hy, hz)), __uint_as_float(cs_h2(c1, c2)), __uint_as_float(cs_h2(lx, ly)),
+                     __uint_as_float(cs_h2(c3, 0.f)));
+}
+// Lane t's part of a pixel (scaled w): products 2t, 2t + 1 and 2t + 8, 2t + 9.
+__device__ __forceinline__ void cs_pixel_mma(float wx, float wy, float wz, int t, unsigned& k0, unsigned& k1) {
+  const float hx = cs_hi(wx), hy = cs_hi(wy), hz = cs_hi(wz), lx = wx - hx, ly = wy - hy, lz = wz - hz;
+  k0 = t == 0 ? cs_h2(hx, hy) : t == 1 ? cs_h2(hz, lx) : t == 2 ? cs_h2(ly, lz) : cs_h2(hx, hy);
+  k1 = t == 0 ? cs_h2(hz, lx) : t == 1 ? cs_h2(ly, lz) : t == 2 ? cs_h2(4.f, 4.f) : cs_h2(4.f, 0.f);
+}
+
+// Eight candidates against the warp's 64 pixels, four 16-pixel tiles: lane
+// 4 g + t has the values of the pixels g and g + 8 of each tile at the
+// candidates 2 t and 2 t + 1.  kLeft, kRight: some windows begin, end here
+// (first: their first columns, not clipped: outside the image nothing is there).
+template <bool kLeft, bool kRight>
+__device__ __forceinline__ void cs_step_mma(const uint2 b, const unsigned (&af)[4][4], const int (&first)[8], int col,
+                                            int far, float (&m)[8]) {
+  float d[4][4];
 #pragma unroll
-    for (int j = 0; j < kCsGroup; ++j) m = fminf(m, cs_pd<kAngle, kCheckS>(q, ra[xx + j], rb[xx + j], k));
-    cs_keep(q, m, row_base + xx);
-  }
-  for (; xx <= hi; ++xx) cs_keep(q, cs_pd<kAngle, kCheckS>(q, ra[xx], rb[xx], k), row_base + xx);
-}
-
-template <bool kAngle, bool kCheckS>
-__device__ __forceinline__ void cs_seg2(const float4* ra, const float2* rb, int lo, int hi, int row_base, CsScan& q0,
-                                        CsScan& q1, const CorrConsts& k) {
-  int xx = lo;
-  for (; xx + kCsGroup - 1 <= hi; xx += kCsGroup) {
-    float m0 = INFINITY, m1 = INFINITY;
+  for (int i = 0; i < 4; ++i) cs_mma(d[i], af[i], b.x, b.y);
 #pragma unroll
-    for (int j = 0; j < kCsGroup; ++j) {
-      const float4 a = ra[xx + j];
-      const float2 b = rb[xx + j];
-      m0 = fminf(m0, cs_pd<kAngle, kCheckS>(q0, a, b, k));
-      m1 = fminf(m1, cs_pd<kAngle, kCheckS>(q1, a, b, k));
-    }
-    cs_keep(q0, m0, row_base + xx);
-    cs_keep(q1, m1, row_base + xx);
-  }
-  for (; xx <= hi; ++xx) {
-    const float4 a = ra[xx];
-    const float2 b = rb[xx];
-    cs_keep(q0, cs_pd<kAngle, kCheckS>(q0, a, b, k), row_base + xx);
-    cs_keep(q1, cs_pd<kAngle, kCheckS>(q1, a, b, k), row_base + xx);
-  }
-}
-
-// The first candidate of the kept group whose distance equals the best
-// (recomputed with the cap test: where it was left out it holds anyway).
-template <bool kAngle>
-__device__ __forceinline__ void cs_resolve(CsScan& q, const float4* __restrict__ A, const float2* __restrict__ B,
-                                           const CorrConsts& k) {
-  if (!q.on || q.bi < 0) return;
-  const int last = min(q.bi + kCsGroup - 1, (q.bi / k.W) * k.W + k.W - 1);
-  for (int i = q.bi; i <= last; ++i)
-    if (cs_pd<kAngle, true>(q, A[i], B[i], k) == q.best) {
-      q.bi = i;
-      return;
-    }
-}
-
-// Row yy of the two pixels' windows (ra/rb: the row's records indexed by
-// image column).  Each pixel still meets its candidates in increasing column
-// order: the row splits into the part only one window covers on the left,
-// the shared part, and the part only one covers on the right.
-template <bool kAngle, bool kCheckS>
-__device__ __forceinline__ void cs_pair_row(const float4* ra, const float2* rb, int yy, CsScan& q0, CsScan& q1,
-                                            const CorrConsts& k) {
-  const int r = k.radius, row_base = yy * k.W;
-  const bool in0 = q0.on && yy >= q0.pv - r && yy <= q0.pv + r;
-  const bool in1 = q1.on && yy >= q1.pv - r && yy <= q1.pv + r;
-  const int l0 = max(0, q0.pu - r), h0 = min(k.W - 1, q0.pu + r);
-  const int l1 = max(0, q1.pu - r), h1 = min(k.W - 1, q1.pu + r);
-  if (in0 && in1) {
-    const int slo = max(l0, l1), shi = min(h0, h1);
-    if (slo <= shi) {
-      if (l0 < slo) cs_seg1<kAngle, kCheckS>(ra, rb, l0, slo - 1, row_base, q0, k);
-      else if (l1 < slo) cs_seg1<kAngle, kCheckS>(ra, rb, l1, slo - 1, row_base, q1, k);
-      cs_seg2<kAngle, kCheckS>(ra, rb, slo, shi, row_base, q0, q1, k);
-      if (h0 > shi) cs_seg1<kAngle, kCheckS>(ra, rb, shi + 1, h0, row_base, q0, k);
-      else if (h1 > shi) cs_seg1<kAngle, kCheckS>(ra, rb, shi + 1, h1, row_base, q1, k);
+  for (int i = 0; i < 8; ++i) {
+    const float x = d[i >> 1][2 * (i & 1)], y = d[i >> 1][2 * (i & 1) + 1];
+    if (!kLeft && !kRight) {
+      m[i] = cs_min_abs(m[i], x, y);
     } else {
-      cs_seg1<kAngle, kCheckS>(ra, rb, l0, h0, row_base, q0, k);
-      cs_seg1<kAngle, kCheckS>(ra, rb, l1, h1, row_base, q1, k);
+      if ((!kLeft || first[i] <= col) && (!kRight || first[i] >= far)) m[i] = fminf(m[i], fabsf(x));
+      if ((!kLeft || first[i] <= col + 1) && (!kRight || first[i] >= far + 1)) m[i] = fminf(m[i], fabsf(y));
     }
-  } else if (in0) {
-    cs_seg1<kAngle, kCheckS>(ra, rb, l0, h0, row_base, q0, k);
-  } else if (in1) {
-    cs_seg1<kAngle, kCheckS>(ra, rb, l1, h1, row_base, q1, k);
   }
 }
 
-// Whether every record of a band whose real points lie in the box lo..hi is
-// within the Euclidean cap of the pixel's point: the box's farthest corner,
-// with a relative margin of 1e-4 over the few-ulp rounding of the squared
-// distances, is below the bound.
-__device__ __forceinline__ bool cs_within_cap(const CsScan& q, const float* lo, const float* hi, float s_max) {
-  if (!q.on) return true;
-  if (lo[0] > hi[0]) return true;  // no real record in the band
-  const float dx = fmaxf(fabsf(q.vx - lo[0]), fabsf(q.vx - hi[0]));
-  const float dy = fmaxf(fabsf(q.vy - lo[1]), fabsf(q.vy - hi[1]));
-  const float dz = fmaxf(fabsf(q.vz - lo[2]), fabsf(q.vz - hi[2]));
-  return (dx * dx + dy * dy + dz * dz) * 1.0001f <= s_max;
+// The band's candidates (32 bytes each, as cs_store_mma writes them) against
+// the warp's pixels, a run of a row at a time: the steps on its left that some
+// windows do not reach, those that all hold, and the rest.  At the end of a run
+// the quad's lanes exchange their values so that lane t has its own pixels,
+// those of tile t.
+__device__ __forceinline__ void cs_scan_mma(const float4* sm, int wu, int xs, int yb, int ca, int cb, int ia, int ib,
+                                            int ya, int yz, const unsigned (&af)[4][4], const int (&first)[8], CsLane& q0,
+                                            CsLane& q1, float eps, const CorrConsts& k) {
+  const unsigned r = (unsigned)k.radius;
+  const int lane = threadIdx.x & 31, t = lane & 3, t2 = 2 * t;
+  for (int yy = ya; yy <= yz; ++yy) {
+    const uint2* row = reinterpret_cast<const uint2*>(sm + (size_t)(yy - yb) * 2 * wu) + lane - 4 * xs;
+    const bool in0 = (unsigned)(yy - q0.pv) + r <= 2 * r, in1 = (unsigned)(yy - q1.pv) + r <= 2 * r;
+    const int base = yy * k.W;
+    for (int g = ca; g <= cb; g += kGroup) {
+      float m[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m[i] = kFarS;
+      const int e = min(cb, g + kGroup - 1);
+      int c = g;
+#pragma unroll 1
+      for (; c <= e && c < ia; c += 8) {
+        if (c + 7 <= ib) cs_step_mma<true, false>(row[4 * c], af, first, c + t2, 0, m);
+        else cs_step_mma<true, true>(row[4 * c], af, first, c + t2, c + t2 - 2 * (int)r, m);
+      }
+      const int n = (min(e, ib) - c + 1) >> 3;  // steps that all windows hold
+      const uint2* at = row + 4 * c;
+#pragma unroll 4
+      for (int j = 0; j < n; ++j, at += 32) cs_step_mma<false, false>(*at, af, first, 0, 0, m);
+      c += 8 * max(n, 0);
+#pragma unroll 1
+      for (; c <= e; c += 8) cs_step_mma<false, true>(row[4 * c], af, first, 0, c + t2 - 2 * (int)r, m);
+      // lane t keeps tile t's two pixels
+      float s[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float send = t & 2 ? m[i] : m[4 + i], keep = t & 2 ? m[4 + i] : m[i];
+        s[i] = fminf(keep, __shfl_xor_sync(0xffffffffu, send, 2));
+      }
+      float v[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float send = t & 1 ? s[i] : s[2 + i], keep = t & 1 ? s[2 + i] : s[i];
+        v[i] = fminf(keep, __shfl_xor_sync(0xffffffffu, send, 1));
+      }
+      // a window that does not reach this row holds nothing of the run
+      cs_track(q0, in0 ? v[0] : kFarS, eps, base + g);
+      cs_track(q1, in1 ? v[1] : kFarS, eps, base + g);
+    }
+  }
 }
 
 // find_correspondences_kernel's loop as it stands (kernels/tsdf_kernels.cu:470-524),
@@ -495,189 +656,483 @@ __device__ __forceinline__ void cs_emit(const CorrConsts& k, const CsPixel& p, b
   }
 }
 
-// One thread per vertically adjacent pixel pair, 32 x 16 pixels per CTA.
-// kDirect: one chunk covers every row, and the kernel resolves each pixel and
-// writes its record itself (no partials, no merge launch).
-template <bool kAngle, bool kDirect>
-__global__ void __launch_bounds__(kCsThreads, kCsCtasPerSm)
-    corr_search_kernel(const CorrConsts k, const float* __restrict__ lv, const float* __restrict__ ln,
-                       const float4* __restrict__ A, const float2* __restrict__ B, const int* __restrict__ flag,
-                       float* __restrict__ part_pd, int* __restrict__ part_idx, const KnnSrc knn,
-                       cf_correspondence* __restrict__ out, int* __restrict__ num_valid, int* __restrict__ stats) {
-  extern __shared__ float4 cs_smem[];
-  __shared__ int s_box[4];  // min pu, max pu, min pv, max pv of the pixels scanned here
-  __shared__ float s_bb[kCsThreads / 32][6];  // per warp: the band's real-point box (min xyz, max xyz)
-  const int tid = threadIdx.y * kCsTx + threadIdx.x;
-  const int x = blockIdx.x * kCsTx + threadIdx.x;
-  const int y0 = blockIdx.y * kCsPy + 2 * threadIdx.y, y1 = y0 + 1;
-  const int chunk = blockIdx.z;
-  const bool img0 = x < k.W && y0 < k.H, img1 = x < k.W && y1 < k.H;
-  const int px0 = img0 ? y0 * k.W + x : 0, px1 = img1 ? y1 * k.W + x : 0;
-  if (tid == 0) {
-    s_box[0] = INT_MAX;
-    s_box[1] = INT_MIN;
-    s_box[2] = INT_MAX;
-    s_box[3] = INT_MIN;
-  }
-  const int frame_flag = *flag;
-  CsScan q0, q1;
-  {
-    CsPixel p;
-    p.search = false;
-    p.special = false;
-    p.pu = p.pv = 0;
-    p.vc = p.nc = make_float3(0.f, 0.f, 0.f);
-    if (img0) p = cs_pixel(k, lv, ln, px0, frame_flag);
-    q0 = cs_scan_state(p, img0 && p.search && !p.special, k.dist_thr);
-    p.search = false;
-    p.special = false;
-    p.pu = p.pv = 0;
-    if (img1) p = cs_pixel(k, lv, ln, px1, frame_flag);
-    q1 = cs_scan_state(p, img1 && p.search && !p.special, k.dist_thr);
-  }
-  __syncthreads();
-  if (q0.on) {
-    atomicMin(&s_box[0], q0.pu);
-    atomicMax(&s_box[1], q0.pu);
-    atomicMin(&s_box[2], q0.pv);
-    atomicMax(&s_box[3], q0.pv);
-  }
-  if (q1.on) {
-    atomicMin(&s_box[0], q1.pu);
-    atomicMax(&s_box[1], q1.pu);
-    atomicMin(&s_box[2], q1.pv);
-    atomicMax(&s_box[3], q1.pv);
-  }
-  __syncthreads();
+// What a chunk of rows leaves of a pixel: its three least values less eps
+// (a: L1, L2, L3, eps) and the runs of the first two.
+struct CsPart {
+  float4* __restrict__ a;
+  int2* __restrict__ g;
+  int2* __restrict__ rows;  // per tile of pixels: its first row, and the rows of a chunk
+};
 
-  if (s_box[0] <= s_box[1]) {  // uniform over the CTA
-    const int r = k.radius;
-    const int xlo = max(0, s_box[0] - r), xhi = min(k.W - 1, s_box[1] + r);
-    const int ylo = max(0, s_box[2] - r), yhi = min(k.H - 1, s_box[3] + r);
-    const int per = (yhi - ylo + k.chunks) / k.chunks;  // ceil(rows / chunks)
-    const int c0 = ylo + chunk * per, c1 = min(yhi, c0 + per - 1);
-    const int wu = xhi - xlo + 1;
-    const int band = kCsSmem / (kCsRecBytes * wu);
-    // rows either pixel's window covers
-    const int plo = min(q0.on ? q0.pv : INT_MAX, q1.on ? q1.pv : INT_MAX) - r;
-    const int phi = max(q0.on ? q0.pv : INT_MIN, q1.on ? q1.pv : INT_MIN) + r;
-    const bool any = q0.on || q1.on;
-    if (c0 <= c1 && band >= 1) {
-      float4* sA = cs_smem;
-      float2* sB = reinterpret_cast<float2*>(cs_smem + (size_t)band * wu);
-      for (int yb = c0; yb <= c1; yb += band) {
-        const int rows = min(band, c1 - yb + 1);
-        // the band's records, and the bounding box of their real points
-        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (int j = tid; j < rows * wu; j += kCsThreads) {
-          const int rr = j / wu;
-          const int g = (yb + rr) * k.W + xlo + (j - rr * wu);
-          const float4 a = A[g];
-          sA[j] = a;
-          sB[j] = B[g];
-          if (a.z > 0.f) {
-            lo[0] = fminf(lo[0], a.x);
-            lo[1] = fminf(lo[1], a.y);
-            lo[2] = fminf(lo[2], a.z);
-            hi[0] = fmaxf(hi[0], a.x);
-            hi[1] = fmaxf(hi[1], a.y);
-            hi[2] = fmaxf(hi[2], a.z);
-          }
+// The band's candidates against the warp's pixels.  Shared memory holds row
+// after row of wu columns from xs (even): for the filter per two columns
+// (nx, nx, ny, ny), (nz, nz, -c, -c), for the exact scan per column (point, nx),
+// (ny, nz, -, -).  [ca, cb]: the warp's columns here, [ia, ib] those that all
+// its pixels' windows hold, [ya, yz] its rows.
+template <bool kAngle, bool kExact>
+__device__ __forceinline__ void cs_scan(const float4* sm, int wu, int xs, int yb, int ca, int cb, int ia, int ib, int ya,
+                                        int yz, CsLane& q0, CsLane& q1, float eps, const CorrConsts& k) {
+  const unsigned r = (unsigned)k.radius;
+  ca &= ~1;  // (xs is even)
+  for (int yy = ya; yy <= yz; ++yy) {
+    const float4* row = sm + (size_t)(yy - yb) * (kExact ? 2 * wu : wu) - (kExact ? 2 * xs : xs);
+    const bool in0 = (unsigned)(yy - q0.pv) + r <= 2 * r, in1 = (unsigned)(yy - q1.pv) + r <= 2 * r;
+    const int base = yy * k.W;
+    for (int g = ca; g <= cb; g += kGroup) {
+      float m0 = kCsNone, m1 = kCsNone;
+      if (kExact) {
+        const int e = min(cb, g + kGroup - 1);
+        const float3 v0 = make_float3(cs_unpack(q0.wx).x, cs_unpack(q0.wy).x, cs_unpack(q0.wz).x);
+        const float3 v1 = make_float3(cs_unpack(q1.wx).x, cs_unpack(q1.wy).x, cs_unpack(q1.wz).x);
+        const float3 n0 = make_float3(cs_unpack(q0.nx).x, cs_unpack(q0.ny).x, cs_unpack(q0.nz).x);
+        const float3 n1 = make_float3(cs_unpack(q1.nx).x, cs_unpack(q1.ny).x, cs_unpack(q1.nz).x);
+#pragma unroll 2
+        for (int c = g; c <= e; ++c) {
+          const float4 a = row[2 * c], bb = row[2 * c + 1];
+          const float2 b = make_float2(bb.x, bb.y);
+          const float f0 = cs_pd<kAngle>(v0, n0, a, b, k), f1 = cs_pd<kAngle>(v1, n1, a, b, k);
+          m0 = fminf(m0, (unsigned)(c - q0.l) <= q0.span ? f0 : kCsNone);
+          m1 = fminf(m1, (unsigned)(c - q1.l) <= q1.span ? f1 : kCsNone);
         }
+      } else {
+        const ulonglong2* pr = reinterpret_cast<const ulonglong2*>(row + g);
+#pragma unroll 1
+        for (int h = 0; h < kGroup / kSub; ++h) {
+          const int c = g + h * kSub;
+          if (c > cb) break;
+          if (c >= ia && c + kSub - 1 <= ib) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          for (int o = 16; o; o >>= 1) {
-            lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-            hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-          }
-        if ((tid & 31) == 0)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            s_bb[tid >> 5][c] = lo[c];
-            s_bb[tid >> 5][3 + c] = hi[c];
-          }
-        __syncthreads();
-        if (any) {
-#pragma unroll
-          for (int w = 0; w < kCsThreads / 32; ++w)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              lo[c] = fminf(lo[c], s_bb[w][c]);
-              hi[c] = fmaxf(hi[c], s_bb[w][3 + c]);
-            }
-          const int ya = max(yb, plo), yz = min(yb + rows - 1, phi);
-          if (cs_within_cap(q0, lo, hi, k.s_max) && cs_within_cap(q1, lo, hi, k.s_max)) {
-            for (int yy = ya; yy <= yz; ++yy) {
-              const int o = (yy - yb) * wu - xlo;
-              cs_pair_row<kAngle, false>(sA + o, sB + o, yy, q0, q1, k);
+            for (int j = 0; j < kSub / 2; ++j) {
+              const ulonglong2 xy = pr[h * kSub + 2 * j], zc = pr[h * kSub + 2 * j + 1];
+              m0 = cs_pair<kAngle, false>(m0, q0, xy, zc, 0, k.angle_thr);
+              m1 = cs_pair<kAngle, false>(m1, q1, xy, zc, 0, k.angle_thr);
             }
           } else {
-            for (int yy = ya; yy <= yz; ++yy) {
-              const int o = (yy - yb) * wu - xlo;
-              cs_pair_row<kAngle, true>(sA + o, sB + o, yy, q0, q1, k);
+#pragma unroll
+            for (int j = 0; j < kSub / 2; ++j) {
+              if (c + 2 * j <= cb) {
+                const ulonglong2 xy = pr[h * kSub + 2 * j], zc = pr[h * kSub + 2 * j + 1];
+                m0 = cs_pair<kAngle, true>(m0, q0, xy, zc, c + 2 * j, k.angle_thr);
+                m1 = cs_pair<kAngle, true>(m1, q1, xy, zc, c + 2 * j, k.angle_thr);
+              }
             }
           }
         }
-        __syncthreads();
       }
-    } else if (c0 <= c1 && any) {  // the union is wider than a band buffer row: read through L1
-      const int ya = max(c0, plo), yz = min(c1, phi);
-      for (int yy = ya; yy <= yz; ++yy)
-        cs_pair_row<kAngle, true>(A + (size_t)yy * k.W, B + (size_t)yy * k.W, yy, q0, q1, k);
-    }
-  }
-  cs_resolve<kAngle>(q0, A, B, k);
-  cs_resolve<kAngle>(q1, A, B, k);
-  if (kDirect) {
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      const bool img = h == 0 ? img0 : img1;
-      const int px = h == 0 ? px0 : px1;
-      const int best_i = h == 0 ? q0.bi : q1.bi;
-      CsPixel p;
-      p.search = false;
-      p.code = -1;
-      if (img) p = cs_pixel(k, lv, ln, px, frame_flag);
-      int code = p.code;
-      int bi = -1;
-      if (p.search) {
-        bool saw_depth = false;
-        if (p.special) {
-          bi = cs_rescan(k, p, A, B, saw_depth);
-        } else {
-          bi = best_i;
-          if (bi < 0 && stats) saw_depth = cs_any_depth(k, p, A);
-        }
-        code = bi >= 0 ? 5 : (saw_depth ? 3 : 2);
-      }
-      // the band buffer is free once every band is scanned: stage the records there
-      cs_emit(k, p, img, px, bi, code, A, B, knn, out, num_valid, stats, threadIdx.x,
-              reinterpret_cast<float*>(cs_smem) + threadIdx.y * (32 * kCsRecWords));
-    }
-  } else {
-    if (img0) {
-      part_pd[(size_t)chunk * k.P + px0] = q0.best;
-      part_idx[(size_t)chunk * k.P + px0] = q0.bi;
-    }
-    if (img1) {
-      part_pd[(size_t)chunk * k.P + px1] = q1.best;
-      part_idx[(size_t)chunk * k.P + px1] = q1.bi;
+      // a window that does not reach this row holds nothing of the run
+      cs_track(q0, in0 ? m0 : kCsNone, eps, base + g);
+      cs_track(q1, in1 ? m1 : kCsNone, eps, base + g);
     }
   }
 }
 
-__global__ void __launch_bounds__(256)
-    corr_merge_kernel(const CorrConsts k, const float* __restrict__ lv, const float* __restrict__ ln,
-                      const float4* __restrict__ A, const float2* __restrict__ B, const int* __restrict__ flag,
-                      const float* __restrict__ part_pd, const int* __restrict__ part_idx, const KnnSrc knn,
-                      cf_correspondence* __restrict__ out, int* __restrict__ num_valid, int* __restrict__ stats) {
-  __shared__ float s_stage[256 / 32][32 * kCsRecWords];
-  const int px = blockIdx.x * blockDim.x + threadIdx.x;
+template <bool kAngle>
+__global__ void __launch_bounds__(kCsThreads, kCsCtasPerSm)
+    corr_search_kernel(const CorrConsts k, const float4* __restrict__ A, const float2* __restrict__ B, const CsPix pix,
+                       const CsBox* __restrict__ box, const int* __restrict__ flag, const CsPart part) {
+  extern __shared__ float4 cs_smem[];
+  __shared__ float s_d[kCsThreads / 32][7];  // per warp: the candidates' part of the boxes
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int x = blockIdx.x * kCsTx + (wid & 3) * 8 + (lane >> 2);
+  const int y0 = blockIdx.y * kCsTy + (wid >> 2) * 8 + 2 * (lane & 3), y1 = y0 + 1;
+  const int chunk = blockIdx.z, r = k.radius;
+  const int px0 = y0 * k.W + x, px1 = px0 + k.W;
+  // the pixels' boxes: the tile is two blocks
+  const int bpr = (k.W + kCsBlock - 1) / kCsBlock;
+  const CsBox* bt = box + (size_t)blockIdx.y * bpr + 2 * blockIdx.x;
+  const bool two = 2 * (int)blockIdx.x + 1 < bpr;
+  int bx[4];
+  float bv[6];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) bx[c] = max(bt[0].p[c], two ? bt[1].p[c] : kCsOff);
+  if (*flag || bx[1] < -bx[0]) return;  // a frame scanned sequentially, or no pixel (uniform over the CTA)
+#pragma unroll
+  for (int c = 0; c < 6; ++c) bv[c] = fmaxf(bt[0].v[c], two ? bt[1].v[c] : -INFINITY);
+  // the CTA's columns, and its rows in this chunk
+  const int xlo = max(0, -bx[0] - r) & ~1, xhi = min(k.W - 1, bx[1] + r);
+  const int ylo = max(0, -bx[2] - r), yhi = min(k.H - 1, bx[3] + r);
+  const int per = (yhi - ylo + k.chunks) / k.chunks;  // ceil(rows / chunks)
+  const int c0 = ylo + chunk * per, c1 = min(yhi, c0 + per - 1);
+  if (chunk == 0 && tid == 0) part.rows[blockIdx.y * gridDim.x + blockIdx.x] = make_int2(ylo, per);
+  {  // their boxes
+    float v[7] = {-INFINITY, -INFINITY, -INFINITY, 0.f, -INFINITY, -INFINITY, -INFINITY};
+    if (c0 <= c1) {
+      const int b0 = xlo / kCsBlock, bw = xhi / kCsBlock - b0 + 1, r0 = c0 / kCsBlock, bh = c1 / kCsBlock - r0 + 1;
+      for (int i = tid; i < bw * bh; i += kCsThreads) {
+        const float4* b = reinterpret_cast<const float4*>(box[(size_t)(r0 + i / bw) * bpr + b0 + i % bw].d);
+        const float4 lo = b[0], hi = b[1];
+        v[0] = fmaxf(v[0], lo.x);
+        v[1] = fmaxf(v[1], lo.y);
+        v[2] = fmaxf(v[2], lo.z);
+        v[3] = fmaxf(v[3], lo.w);
+        v[4] = fmaxf(v[4], hi.x);
+        v[5] = fmaxf(v[5], hi.y);
+        v[6] = fmaxf(v[6], hi.z);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+      v[c] = cs_warp_max(v[c]);
+      if (lane == 0) s_d[wid][c] = v[c];
+    }
+  }
+  CsPixel p0, p1;
+  p0.search = p1.search = p0.special = p1.special = false;
+  p0.pu = p1.pu = p0.pv = p1.pv = 0;
+  p0.vc = p1.vc = p0.nc = p1.nc = make_float3(0.f, 0.f, 0.f);
+  if (x < k.W && y0 < k.H) p0 = cs_load_pixel(pix, px0);
+  if (x < k.W && y1 < k.H) p1 = cs_load_pixel(pix, px1);
+  const bool on0 = p0.search && !p0.special, on1 = p1.search && !p1.special;
+  // the warp's windows: the union of their columns and rows, and the columns common to all
+  constexpr int kFar = 1 << 30;
+  const int wul = __reduce_min_sync(0xffffffffu, min(on0 ? p0.pu : kFar, on1 ? p1.pu : kFar));
+  const int wuh = __reduce_max_sync(0xffffffffu, max(on0 ? p0.pu : -kFar, on1 ? p1.pu : -kFar));
+  const int wvl = __reduce_min_sync(0xffffffffu, min(on0 ? p0.pv : kFar, on1 ? p1.pv : kFar));
+  const int wvh = __reduce_max_sync(0xffffffffu, max(on0 ? p0.pv : -kFar, on1 ? p1.pv : -kFar));
+  __syncthreads();
+  float o[3], eps, sw = 1.f, sn = 1.f;
+  bool filter, any = false;
+  {
+    float v[7];
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+      v[c] = s_d[0][c];
+#pragma unroll
+      for (int w = 1; w < kCsThreads / 32; ++w) v[c] = fmaxf(v[c], s_d[w][c]);
+    }
+    any = v[4] >= -v[0];  // a real candidate
+    float ww = 0.f, aa = 0.f, dd = 0.f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      o[c] = 0.5f * (bv[3 + c] - bv[c]);
+      const float hw = fmaxf(fabsf(bv[3 + c] - o[c]), fabsf(-bv[c] - o[c]));
+      const float ha = fmaxf(fabsf(v[4 + c] - o[c]), fabsf(-v[c] - o[c]));
+      const float d = fmaxf(fabsf(bv[3 + c] + v[c]), fabsf(v[4 + c] + bv[c]));
+      ww += hw * hw;
+      aa += ha * ha;
+      dd += d * d;
+    }
+    const float nn = sqrtf(v[3]), wr = sqrtf(ww), ar = sqrtf(aa);
+    // (a relative margin of 1e-4 over the few-ulp rounding of the squared distances)
+    filter = dd * 1.0001f <= k.s_max && nn >= 1e-6f && nn <= 1e6f && wr + ar >= 1e-6f && wr + ar <= 1e6f;
+    if (kAngle) {
+      eps = 14.f * kU * nn * (wr + ar);
+    } else {
+      // w and n up to 256 each: c then up to 2^16, a quarter of it fits a half
+      const int ew = 7 - ilogbf(wr + ar), en = 7 - ilogbf(nn);
+      sw = filter ? ldexpf(1.f, ew) : 1.f;
+      sn = filter ? ldexpf(1.f, en) : 1.f;
+      eps = kU * nn * (25.f * wr + 20.f * ar) * (sw * sn);
+    }
+    if (!filter) eps = 0.f;
+  }
+  CsLane q0, q1;
+  {
+    const float ox = filter ? o[0] : 0.f, oy = filter ? o[1] : 0.f, oz = filter ? o[2] : 0.f;
+    auto state = [&](const CsPixel& p, bool on) {
+      CsLane q;
+      const float wx = on ? p.vc.x - ox : 0.f, wy = on ? p.vc.y - oy : 0.f, wz = on ? p.vc.z - oz : 0.f;
+      q.wx = cs_pack(wx, wx);
+      q.wy = cs_pack(wy, wy);
+      q.wz = cs_pack(wz, wz);
+      q.nx = q.ny = q.nz = 0ull;
+      if (kAngle && on) {
+        q.nx = cs_pack(p.nc.x, p.nc.x);
+        q.ny = cs_pack(p.nc.y, p.nc.y);
+        q.nz = cs_pack(p.nc.z, p.nc.z);
+      }
+      q.l = on ? max(0, p.pu - r) : kFar;
+      q.span = on ? (unsigned)(min(k.W - 1, p.pu + r) - q.l) : 0u;
+      q.pv = on ? p.pv : -kFar;
+      q.L1 = q.L2 = q.L3 = kCsNone;
+      q.g1 = q.g2 = -1;
+      return q;
+    };
+    q0 = state(p0, on0);
+    q1 = state(p1, on1);
+  }
+  if (any && c0 <= c1) {
+    const bool some = wuh >= wul;
+    const int ua = max(0, wul - r), ub = min(k.W - 1, wuh + r);  // the warp's columns
+    const int ia = max(0, wuh - r), ib = min(k.W - 1, wul + r);  // those of every window
+    const bool mma = !kAngle && filter;
+    unsigned af[4][4];
+    int first[8];
+    if (mma) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int src = (lane & 28) | i;  // the lane that holds this lane's pixels of tile i
+        const float2 a0 = cs_unpack(q0.wx), b0 = cs_unpack(q0.wy), d0 = cs_unpack(q0.wz);
+        const float2 a1 = cs_unpack(q1.wx), b1 = cs_unpack(q1.wy), d1 = cs_unpack(q1.wz);
+        cs_pixel_mma(__shfl_sync(0xffffffffu, a0.x, src) * sw, __shfl_sync(0xffffffffu, b0.x, src) * sw,
+                     __shfl_sync(0xffffffffu, d0.x, src) * sw, lane & 3, af[i][0], af[i][2]);
+        cs_pixel_mma(__shfl_sync(0xffffffffu, a1.x, src) * sw, __shfl_sync(0xffffffffu, b1.x, src) * sw,
+                     __shfl_sync(0xffffffffu, d1.x, src) * sw, lane & 3, af[i][1], af[i][3]);
+        first[2 * i] = __shfl_sync(0xffffffffu, on0 ? p0.pu - r : kFar, src);
+        first[2 * i + 1] = __shfl_sync(0xffffffffu, on1 ? p1.pu - r : kFar, src);
+      }
+    }
+    for (int xs = xlo; xs <= xhi; xs += kSlab) {
+      const int xe = min(xhi, xs + kSlab - 1);
+      const int wu = mma ? xe - xs + 1 + kPad : (xe - xs + 2) & ~1;
+      const int band = kCsSmem / (wu * (filter && kAngle ? 16 : 32));
+      for (int yb = c0; yb <= c1; yb += band) {
+        const int rows = min(band, c1 - yb + 1);
+        __syncthreads();
+        if (mma) {
+          const float sc = -0.25f * sw * sn;
+          for (int j = tid; j < rows * wu; j += kCsThreads) {
+            const int rr = j / wu, c = j - rr * wu;
+            float nx = 0.f, ny = 0.f, nz = 0.f, mc = 0.25f * kFarS * 0.8f;
+            if (xs + c <= xe) {
+              const int g = (yb + rr) * k.W + xs + c;
+              const float4 a = A[g];
+              if (a.z > 0.f) {
+                const float2 b = B[g];
+                nx = a.w * sn;
+                ny = b.x * sn;
+                nz = b.y * sn;
+                mc = sc * cs_dot(a.w, b.x, b.y, a.x - o[0], a.y - o[1], a.z - o[2]);
+              }
+            }
+            cs_store_mma(cs_smem + 2 * j, nx, ny, nz, mc);
+          }
+        } else if (filter) {
+          for (int j = tid; j < rows * (wu >> 1); j += kCsThreads) {
+            const int rr = j / (wu >> 1), c = 2 * (j - rr * (wu >> 1));
+            float nx[2], ny[2], nz[2], mc[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              nx[h] = ny[h] = nz[h] = 0.f;
+              mc[h] = kCsNone;
+              if (xs + c + h <= xe) {
+                const int g = (yb + rr) * k.W + xs + c + h;
+                const float4 a = A[g];
+                if (a.z > 0.f) {
+                  const float2 b = B[g];
+                  nx[h] = a.w;
+                  ny[h] = b.x;
+                  nz[h] = b.y;
+                  mc[h] = -cs_dot(a.w, b.x, b.y, a.x - o[0], a.y - o[1], a.z - o[2]);
+                }
+              }
+            }
+            cs_smem[2 * j] = make_float4(nx[0], nx[1], ny[0], ny[1]);
+            cs_smem[2 * j + 1] = make_float4(nz[0], nz[1], mc[0], mc[1]);
+          }
+        } else {
+          for (int j = tid; j < rows * wu; j += kCsThreads) {
+            const int rr = j / wu, c = j - rr * wu;
+            float4 a = make_float4(kCsFar, kCsFar, 0.f, kCsFar);
+            float2 b = make_float2(0.f, 0.f);
+            if (xs + c <= xe) {
+              const int g = (yb + rr) * k.W + xs + c;
+              a = A[g];
+              b = B[g];
+            }
+            cs_smem[2 * j] = a;
+            cs_smem[2 * j + 1] = make_float4(b.x, b.y, 0.f, 0.f);
+          }
+        }
+        __syncthreads();
+        if (some) {
+          const int ca = max(xs, ua), cb = min(xe, ub), ya = max(yb, wvl - r), yz = min(yb + rows - 1, wvh + r);
+          if (ca <= cb) {
+            if (mma)
+              cs_scan_mma(cs_smem, wu, xs, yb, ca, cb, ia, ib, ya, yz, af, first, q0, q1, eps, k);
+            else if (kAngle && filter)
+              cs_scan<kAngle, false>(cs_smem, wu, xs, yb, ca, cb, ia, min(ib, cb), ya, yz, q0, q1, eps, k);
+            else
+              cs_scan<kAngle, true>(cs_smem, wu, xs, yb, ca, cb, ia, ib, ya, yz, q0, q1, 0.f, k);
+          }
+        }
+      }
+    }
+    if (mma) {  // back to metres (powers of two); what is not there has no value
+      const float un = 1.f / (sw * sn);
+      eps *= un;
+      auto unscale = [&](CsLane& q) {
+        q.g1 = q.L1 < 0.5f * kFarS ? q.g1 : -1;
+        q.g2 = q.L2 < 0.5f * kFarS ? q.g2 : -1;
+        q.L1 = q.L1 < 0.5f * kFarS ? q.L1 * un : kCsNone;
+        q.L2 = q.L2 < 0.5f * kFarS ? q.L2 * un : kCsNone;
+        q.L3 = q.L3 < 0.5f * kFarS ? q.L3 * un : kCsNone;
+      };
+      unscale(q0);
+      unscale(q1);
+    }
+  }
+  if (on0) {
+    part.a[(size_t)chunk * k.P + px0] = make_float4(q0.L1, q0.L2, q0.L3, eps);
+    part.g[(size_t)chunk * k.P + px0] = make_int2(q0.g1, q0.g2);
+  }
+  if (on1) {
+    part.a[(size_t)chunk * k.P + px1] = make_float4(q1.L1, q1.L2, q1.L3, eps);
+    part.g[(size_t)chunk * k.P + px1] = make_int2(q1.g1, q1.g2);
+  }
+}
+
+// A candidate taken so far; of equal distances the first in row-major order.
+struct CsBest {
+  float pd;
+  int i;
+  __device__ __forceinline__ void take(float d, int j) {
+    if (j >= 0 && (d < pd || (d == pd && i >= 0 && j < i))) {
+      pd = d;
+      i = j;
+    }
+  }
+};
+
+// Eight lanes per pixel evaluate its runs (the loads of a run's columns are then
+// in flight together, and four pixels' runs per warp; a warp per run took
+// three times as long).  Pixels whose third value is within the bound are left
+// to the CTA, a row of the window per warp at a time.
+// kDirect: no search went before, each lane scans its pixel's window (rule at
+// kCsDirect).
+constexpr int kMergeThreads = 256;
+template <bool kAngle, bool kDirect>
+__global__ void __launch_bounds__(kMergeThreads)
+    corr_merge_kernel(const CorrConsts k, const float* __restrict__ lv, const float4* __restrict__ A,
+                      const float2* __restrict__ B, const CsPix pix, const int* __restrict__ flag, const CsPart part,
+                      const KnnSrc knn, cf_correspondence* __restrict__ out, int* __restrict__ num_valid,
+                      int* __restrict__ stats) {
+  __shared__ float s_stage[kMergeThreads / 32][32 * kCsRecWords];
+  __shared__ int s_again[kMergeThreads], s_count;
+  __shared__ float s_p[12];
+  __shared__ CsBest s_best[kMergeThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int px = blockIdx.x * kMergeThreads + tid;
   const bool inimg = px < k.P;
   CsPixel p;
   p.search = false;
+  p.special = false;
   p.code = -1;
-  if (inimg) p = cs_pixel(k, lv, ln, px, *flag);
+  p.pu = p.pv = 0;
+  p.vl = p.vc = p.nc = make_float3(0.f, 0.f, 0.f);
+  p.view_cos = 0.f;
+  if (tid == 0) s_count = 0;
+  if (inimg) {
+    p = cs_load_pixel(pix, px);
+    if (p.search) {
+      p.special |= *flag != 0;
+      p.vl = make_float3(lv[3 * px], lv[3 * px + 1], lv[3 * px + 2]);
+    }
+  }
+  const bool on = p.search && !p.special;
+  // an upper bound of the winner's distance, and the runs that can hold it: bit
+  // 2 c + s the chunk's s-th
+  float U = k.dist_thr;
+  unsigned runs = 0, again = 0;  // again: the chunks of which more runs could
+  if (!kDirect && on) {
+    for (int c = 0; c < k.chunks; ++c) {
+      const float4 a = part.a[(size_t)c * k.P + px];
+      U = fminf(U, a.x + 2.25f * a.w);
+    }
+    for (int c = 0; c < k.chunks; ++c) {
+      const float4 a = part.a[(size_t)c * k.P + px];
+      runs |= (a.x <= U ? 1u : 0u) << (2 * c) | (a.y <= U ? 2u : 0u) << (2 * c);
+      again |= (a.z <= U ? 1u : 0u) << c;
+    }
+  }
+  CsBest best = {k.dist_thr, -1};
+  if (kDirect && on) {
+    const int l = max(0, p.pu - k.radius), h = min(k.W - 1, p.pu + k.radius);
+    const int ya = max(0, p.pv - k.radius), yz = min(k.H - 1, p.pv + k.radius);
+    for (int yy = ya; yy <= yz; ++yy)
+#pragma unroll 4
+      for (int c = l; c <= h; ++c) {
+        const float d = cs_pd<kAngle>(p.vc, p.nc, A[yy * k.W + c], B[yy * k.W + c], k);
+        if (d < best.pd) {
+          best.pd = d;
+          best.i = yy * k.W + c;
+        }
+      }
+  }
+  for (unsigned todo; !kDirect && (todo = __ballot_sync(0xffffffffu, runs != 0)) != 0;) {
+    const unsigned mine = (todo >> (lane & 24)) & 0xffu;  // of this lane's eight pixels
+    const int src = (lane & 24) + (mine ? __ffs(mine) - 1 : 0);
+    int gs = -1;
+    if (mine && lane == src) {
+      const int e = __ffs(runs) - 1;
+      runs &= runs - 1;
+      const int2 g = part.g[(size_t)(e >> 1) * k.P + px];
+      gs = e & 1 ? g.y : g.x;
+    }
+    const int gg = __shfl_sync(0xffffffffu, gs, src), pu = __shfl_sync(0xffffffffu, p.pu, src);
+    const float3 v = make_float3(__shfl_sync(0xffffffffu, p.vc.x, src), __shfl_sync(0xffffffffu, p.vc.y, src),
+                                 __shfl_sync(0xffffffffu, p.vc.z, src));
+    float3 nc = v;
+    if (kAngle)
+      nc = make_float3(__shfl_sync(0xffffffffu, p.nc.x, src), __shfl_sync(0xffffffffu, p.nc.y, src),
+                       __shfl_sync(0xffffffffu, p.nc.z, src));
+    CsBest b = {INFINITY, -1};
+    if (mine && gg >= 0) {
+      const int row0 = gg / k.W * k.W, c0 = gg - row0;
+      const int l = max(c0, pu - k.radius), h = min(min(c0 + kGroup - 1, k.W - 1), pu + k.radius);
+#pragma unroll 4
+      for (int col = l + (lane & 7); col <= h; col += 8) {
+        const float d = cs_pd<kAngle>(v, nc, A[row0 + col], B[row0 + col], k);
+        if (d < b.pd) {
+          b.pd = d;
+          b.i = row0 + col;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 4; o; o >>= 1) {
+      const float d = __shfl_xor_sync(0xffffffffu, b.pd, o);
+      const int i = __shfl_xor_sync(0xffffffffu, b.i, o);
+      b.take(d, i);
+    }
+    if (mine && lane == src) best.take(b.pd, b.i);
+  }
+  __syncthreads();
+  if (!kDirect && again) s_again[atomicAdd(&s_count, 1)] = tid;
+  __syncthreads();
+  for (int t = 0; !kDirect && t < s_count; ++t) {
+    const int src = s_again[t];
+    if (tid == src) {
+      s_p[0] = p.vc.x; s_p[1] = p.vc.y; s_p[2] = p.vc.z;
+      s_p[3] = p.nc.x; s_p[4] = p.nc.y; s_p[5] = p.nc.z;
+      s_p[6] = __int_as_float(p.pu); s_p[7] = __int_as_float(p.pv);
+      const int y = px / k.W, x = px - y * k.W;
+      const int2 rw = part.rows[y / kCsTy * ((k.W + kCsTx - 1) / kCsTx) + x / kCsTx];
+      s_p[8] = __uint_as_float(again); s_p[9] = __int_as_float(rw.x); s_p[10] = __int_as_float(rw.y);
+    }
+    __syncthreads();
+    const float3 v = make_float3(s_p[0], s_p[1], s_p[2]), nc = make_float3(s_p[3], s_p[4], s_p[5]);
+    const int pu = __float_as_int(s_p[6]), pv = __float_as_int(s_p[7]);
+    const int l = max(0, pu - k.radius), h = min(k.W - 1, pu + k.radius);
+    const int ch = __float_as_int(s_p[8]), y0 = __float_as_int(s_p[9]), per = __float_as_int(s_p[10]);
+    CsBest b = {k.dist_thr, -1};
+    for (int cc = 0; cc < k.chunks; ++cc) {
+      if (!((ch >> cc) & 1)) continue;
+      const int ya = max(max(0, pv - k.radius), y0 + cc * per), yz = min(min(k.H - 1, pv + k.radius), y0 + cc * per + per - 1);
+      for (int yy = ya + wid; yy <= yz; yy += kMergeThreads / 32) {
+#pragma unroll 4
+        for (int c = l + lane; c <= h; c += 32) {
+          const float d = cs_pd<kAngle>(v, nc, A[yy * k.W + c], B[yy * k.W + c], k);
+          if (d < b.pd) {
+            b.pd = d;
+            b.i = yy * k.W + c;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float d = __shfl_xor_sync(0xffffffffu, b.pd, o);
+      const int i = __shfl_xor_sync(0xffffffffu, b.i, o);
+      b.take(d, i);
+    }
+    if (lane == 0) s_best[wid] = b;
+    __syncthreads();
+    if (tid == src) {
+#pragma unroll
+      for (int w = 0; w < kMergeThreads / 32; ++w) best.take(s_best[w].pd, s_best[w].i);
+    }
+  }
   int code = p.code;
   int bi = -1;
   if (p.search) {
@@ -685,20 +1140,12 @@ __global__ void __launch_bounds__(256)
     if (p.special) {
       bi = cs_rescan(k, p, A, B, saw_depth);
     } else {
-      float best = k.dist_thr;
-      for (int c = 0; c < k.chunks; ++c) {
-        const int i = part_idx[(size_t)c * k.P + px];
-        const float pd = part_pd[(size_t)c * k.P + px];
-        if (i >= 0 && pd < best) {
-          best = pd;
-          bi = i;
-        }
-      }
+      bi = best.i;
       if (bi < 0 && stats) saw_depth = cs_any_depth(k, p, A);
     }
     code = bi >= 0 ? 5 : (saw_depth ? 3 : 2);
   }
-  cs_emit(k, p, inimg, px, bi, code, A, B, knn, out, num_valid, stats, threadIdx.x & 31, s_stage[threadIdx.x >> 5]);
+  cs_emit(k, p, inimg, px, bi, code, A, B, knn, out, num_valid, stats, lane, s_stage[threadIdx.x >> 5]);
 }
 
 __global__ void pixel_knn_kernel(const int* __restrict__ hit, int P, const int* __restrict__ vk,
@@ -734,19 +1181,18 @@ float sqrt_bound(float cap) {
 
 }  // namespace
 
-// Row chunks per tile.  Rough model in SM clocks: a CTA scans 512 pixels x
-// S/C candidates at about 1.9 candidates per clock (7.5 per SM, 4 CTAs) after
-// a fixed ~3000-clock set-up, the CTAs run in ceil(tiles x C / slots) waves,
-// and more than one chunk adds the merge launch (~20000 clocks).  One chunk
-// writes the records from the search kernel itself.
+// Row chunks per tile.  Rough model in SM clocks, from 640 x 480 at radii 8, 20
+// and 50 with 1 to 8 chunks: a CTA's set-up takes 9000, its scan of 512 pixels x
+// S/C candidates goes at 9 per clock (3 CTAs per SM), the CTAs run in
+// ceil(tiles x C / slots) waves, and the merge reads each chunk for 5000.
 int corr_pick_chunks(int tiles, int sms, int radius, int W, int H) {
   const double slots = (double)(sms > 0 ? sms : 1) * kCsCtasPerSm;
-  const double side_x = std::fmin(2.0 * radius + 1.0, (double)W), side_y = std::fmin(2.0 * radius + 1.0, (double)H);
-  const double scan = 512.0 * side_x * side_y / 1.9;
+  const double side_x = std::fmin(2.0 * radius + 8.0, (double)W), side_y = std::fmin(2.0 * radius + 8.0, (double)H);
+  const double scan = 512.0 * side_x * side_y / 9.0;
   int best_c = 1;
   double best = 1e300;
   for (int c = 1; c <= kCorrMaxChunks; ++c) {
-    const double t = std::ceil((double)tiles * c / slots) * (3000.0 + scan / c) + (c > 1 ? 20000.0 : 0.0);
+    const double t = std::ceil((double)tiles * c / slots) * (9000.0 + scan / c) + 5000.0 * c;
     if (t < best * (1.0 - 1e-9)) {
       best = t;
       best_c = c;
@@ -754,6 +1200,15 @@ int corr_pick_chunks(int tiles, int sms, int radius, int W, int H) {
   }
   return best_c;
 }
+
+// Row chunks that the partials of frames of up to P pixels have room for.
+int corr_chunk_cap(size_t P) {
+  return (int)std::fmax(1.0, std::fmin((double)kCorrMaxChunks, std::floor((double)(1u << 27) / (double)P)));
+}
+
+// Blocks of frames of up to P pixels, whatever their sides.
+size_t corr_box_cap(size_t P) { return P / (kCsBlock * kCsBlock) + (P + 1) / kCsBlock + 2; }
+size_t corr_box_bytes() { return sizeof(CsBox); }
 
 cudaError_t launch_corr_search(const cf_corr_frame* f, const cf_camera* cam, const cf_mat4* Tcw, const cf_mat4* Twc,
                                const cf_corr_params* p, const CorrScratch& sc, int chunks, cf_correspondence* out,
@@ -797,41 +1252,39 @@ cudaError_t launch_corr_search(const cf_corr_frame* f, const cf_camera* cam, con
   knn.pixel_knn_out = f->d_pixel_knn ? nullptr : f->d_pixel_knn_out;
   knn.pixel_knn_w_out = f->d_pixel_knn ? nullptr : f->d_pixel_knn_w_out;
 
-  e = cudaMemsetAsync(num_valid, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  if (stats) {
-    e = cudaMemsetAsync(stats, 0, 6 * sizeof(int), s);
-    if (e != cudaSuccess) return e;
+  if (W == 0 || H == 0) {
+    e = cudaMemsetAsync(num_valid, 0, sizeof(int), s);
+    if (e == cudaSuccess && stats) e = cudaMemsetAsync(stats, 0, 6 * sizeof(int), s);
+    return e;
   }
-  if (W == 0 || H == 0) return cudaSuccess;
   // a NaN bound defeats the strict-less rule (the reference then accepts every
   // candidate it reaches) and an infinite one lets a skip record pass the
   // Euclidean test: such calls take the sequential scan throughout
   e = cudaMemsetAsync(sc.flag, std::isfinite(p->dist_threshold) ? 0 : 1, sizeof(int), s);
   if (e != cudaSuccess) return e;
 
-  const dim3 tiles((W + kCsTx - 1) / kCsTx, (H + kCsPy - 1) / kCsPy);
-  // the partials hold kCorrMaxChunks entries per pixel of the largest frame
-  k.chunks = chunks > 0 ? (chunks > kCorrMaxChunks ? kCorrMaxChunks : chunks)
-                        : corr_pick_chunks((int)(tiles.x * tiles.y), sc.sms, k.radius, W, H);
-  const bool angle = p->angle_threshold > 0.f, direct = k.chunks == 1;
-  auto kern = angle ? (direct ? corr_search_kernel<true, true> : corr_search_kernel<true, false>)
-                    : (direct ? corr_search_kernel<false, true> : corr_search_kernel<false, false>);
+  const dim3 tiles((W + kCsTx - 1) / kCsTx, (H + kCsTy - 1) / kCsTy);
+  const int want = chunks > 0 ? chunks : corr_pick_chunks((int)(tiles.x * tiles.y), sc.sms, k.radius, W, H);
+  k.chunks = want < sc.chunk_cap ? want : sc.chunk_cap;
+  const bool angle = p->angle_threshold > 0.f;
+  auto kern = angle ? corr_search_kernel<true> : corr_search_kernel<false>;
+  const bool direct = k.radius <= kCsDirect;
+  auto merge = direct ? (angle ? corr_merge_kernel<true, true> : corr_merge_kernel<false, true>)
+                      : (angle ? corr_merge_kernel<true, false> : corr_merge_kernel<false, false>);
   // per device and cheap: set on every call rather than cached per device
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCsSmem);
   if (e != cudaSuccess) return e;
+  const CsPart part = {sc.part_a, sc.part_g, sc.rows};
 
-  corr_prep_kernel<<<(k.P + 255) / 256, 256, 0, s>>>(f->d_depth, f->d_depth_normals, W, H, k.fx, k.fy, k.cx, k.cy,
-                                                      sc.A, sc.B, sc.flag);
-  const dim3 grid(tiles.x, tiles.y, k.chunks);
-  kern<<<grid, dim3(kCsTx, kCsTy), kCsSmem, s>>>(k, f->d_live_vertices, f->d_live_normals, sc.A, sc.B, sc.flag,
-                                                 sc.part_pd, sc.part_idx, knn, out, num_valid, stats);
-  *launches += 2;
-  if (!direct) {
-    corr_merge_kernel<<<(k.P + 255) / 256, 256, 0, s>>>(k, f->d_live_vertices, f->d_live_normals, sc.A, sc.B,
-                                                        sc.flag, sc.part_pd, sc.part_idx, knn, out, num_valid, stats);
-    *launches += 1;
-  }
+  const CsPix pix = {sc.pix_v, sc.pix_n, sc.pix_row};
+  CsBox* box = static_cast<CsBox*>(sc.box);
+  corr_prep_kernel<<<dim3((W + kCsBlock - 1) / kCsBlock, (H + kCsBlock - 1) / kCsBlock), kCsBlock * kCsBlock, 0, s>>>(
+      k, f->d_depth, f->d_depth_normals, f->d_live_vertices, f->d_live_normals, sc.A, sc.B, pix, box, sc.flag, num_valid,
+      stats);
+  if (!direct) kern<<<dim3(tiles.x, tiles.y, k.chunks), kCsThreads, kCsSmem, s>>>(k, sc.A, sc.B, pix, box, sc.flag, part);
+  merge<<<(k.P + kMergeThreads - 1) / kMergeThreads, kMergeThreads, 0, s>>>(k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag,
+                                                                            part, knn, out, num_valid, stats);
+  *launches += direct ? 2 : 3;
   return cudaGetLastError();
 }
 

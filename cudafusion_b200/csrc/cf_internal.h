@@ -259,12 +259,20 @@ constexpr int kCorrMaxChunks = 8;
 struct CorrScratch {
   float4* A;       // per pixel: unprojected point (x, y, z) and normal x
   float2* B;       // per pixel: normal y, z
-  float* part_pd;  // [kCorrMaxChunks][pixels]: each row chunk's best distance ...
-  int* part_idx;   // ... and candidate
+  float4* part_a;  // [chunk_cap][pixels]: each row chunk's three least values, and their error bound
+  int2* part_g;    // [chunk_cap][pixels]: the runs of the first two
+  int2* rows;      // per tile of pixels: the rows that it scans, by chunk
+  void* box;       // [blocks]: what is known of each block of 16 x 16 pixels
+  float4 *pix_v, *pix_n;  // per pixel: its camera-frame point, normal, projection ...
+  int* pix_row;           // ... and state
+  int chunk_cap;
   int* flag;       // set when a value could make a distance NaN
   int sms;
 };
 int corr_pick_chunks(int tiles, int sms, int radius, int W, int H);
+int corr_chunk_cap(size_t P);
+size_t corr_box_cap(size_t P);
+size_t corr_box_bytes();
 // cf_linesearch.cu: the GN step's acceptance
 cudaError_t launch_update_stats(const float* dx, int N, float update_scale, float max_rot, float max_trans,
                                 double* sums, unsigned* maxima, int* finite, cudaStream_t s);

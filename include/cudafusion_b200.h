@@ -496,7 +496,7 @@ CF_API cf_status cf_compute_pixel_knn(const int* d_hit_voxel_idx, int width, int
 CF_API cf_status cf_corr_search_launch_count(const cf_corr_search* h, long long* launches);
 
 /* Tuning knob (no reference counterpart): the search splits the rows each
- * 32 x 8 tile of pixels scans into `chunks` parts run by separate CTAs
+ * 32 x 16 tile of pixels scans into `chunks` parts run by separate CTAs
  * (1..8; 0, the default, picks the count per frame from the tile count and
  * the SM count).  Results do not depend on it. */
 CF_API cf_status cf_corr_search_set_chunks(cf_corr_search* h, int chunks);
