@@ -93,6 +93,7 @@ static_assert(pair_at(3, 3) + 27 <= kRecFloats, "record layout");
 // through shared memory; 128 threads instead of 256: 17) and by shared memory
 // (33M correspondences: 1.8 ms, 2.3).
 __global__ void __launch_bounds__(kSortThreads) bucket_sort_kernel(Table tb, Work w, int N) {
+  after_previous();
   __shared__ unsigned long long key[kSortMax];
   __shared__ int cidx[kSortMax];
   const int tid = threadIdx.x;
@@ -203,6 +204,7 @@ __global__ void __launch_bounds__(kSortThreads) bucket_sort_kernel(Table tb, Wor
 // (its correspondences are read one by one), else 0 (it has a record).
 constexpr int kPermThreads = 128;
 __global__ void __launch_bounds__(kPermThreads) permute_kernel(Table tb, Work w) {
+  after_previous();
   __shared__ float stage[kPermThreads / 32][32 * 23];
   const int lane = lane_id(), wid = threadIdx.x >> 5;
   const int q0 = (blockIdx.x * (kPermThreads / 32) + wid) * 32;
@@ -328,6 +330,7 @@ __device__ __forceinline__ uint4 list_desc(const Work& w, const Pattern& pt, int
 // 64 tasks, by rank; the CTA together for the others.
 constexpr int kListSmem = 4096;
 __global__ void __launch_bounds__(kThreads) list_sort_kernel(Work w, Pattern pt, int N) {
+  after_previous();
   __shared__ int big[kWarps];
   __shared__ int buf[kListSmem];
   const int lane = lane_id(), wid = threadIdx.x >> 5;
@@ -512,6 +515,7 @@ __device__ __forceinline__ void reduce_energy(const Work& w, const double* part,
   }
 }
 __global__ void energy_reduce_kernel(Table tb, Work w, int slot) {
+  after_previous();
   const ProbDesc d = tb.desc[blockIdx.x];
   reduce_energy(w, w.e_data_part + d.e_cta0, d.e_ctas, blockIdx.x, slot);
 }
@@ -682,6 +686,7 @@ __global__ void __launch_bounds__(kThreads, 2) cells_kernel(Table tb, Work w, Pa
   extern __shared__ __align__(16) unsigned char cells_smem[];
   __shared__ double red[kWarps];
   if (kAcc && (int)blockIdx.x < ea.edge_ctas) {
+    after_previous();
     edge_terms_cta(ea, blockIdx.x);
     return;
   }
@@ -758,6 +763,9 @@ __global__ void __launch_bounds__(kThreads, 2) cells_kernel(Table tb, Work w, Pa
     }
   };
   enter(w0, size);
+  // what the lists' kernels left is read already (at least one kernel lies
+  // between), the transforms and records from here on
+  after_previous();
   for (; w0 < qb || left > 0; w0 += 32) {
     const int q = w0 + lane;
     float3 src = f3(0.f, 0.f, 0.f);
@@ -1032,6 +1040,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) gather_kernel(Work w, Pattern 
     if (tid >= 32 && tid - 32 <= kn) m.edge[tid - 32] = __ldg(pt.arap_blk_ptr + u0 + 1 + k0 + tid - 32);
     for (int i = lane; i < kn * kSums; i += 32) (&m.sum[wid][0][0])[i] = 0.f;
     __syncthreads();
+    if (k0 == 0) after_previous();  // (so far the pattern and the lists)
     float(*sum)[kSums] = m.sum[wid];
     for (int i0 = b0; i0 < b1; i0 += 32) {
       // a lane per task: the run, and the pass's blocks of the nodes after the row's
@@ -1236,14 +1245,14 @@ EdgeArgs edge_args(const Pattern& p, const SolveArgs& a, const cf_dual_quat* T, 
 
 cudaError_t launch_bucket_sort(const Work& w, const Table& tb, cudaStream_t s) {
   if (tb.N <= 0) return cudaSuccess;
-  bucket_sort_kernel<<<tb.N + tb.M / kSortChunk, kSortThreads, 0, s>>>(tb, w, tb.N);
+  launch_next(bucket_sort_kernel, tb.N + tb.M / kSortChunk, kSortThreads, 0, s, tb, w, tb.N);
   return cudaGetLastError();
 }
 
 cudaError_t launch_node_lists(const Work& w, const Table& tb, const Pattern& p, cudaStream_t s) {
   if (tb.N <= 0 || tb.M <= 0) return cudaSuccess;
-  permute_kernel<<<(tb.M + kPermThreads - 1) / kPermThreads, kPermThreads, 0, s>>>(tb, w);
-  list_sort_kernel<<<(tb.N + kWarps - 1) / kWarps, kThreads, 0, s>>>(w, p, tb.N);
+  launch_next(permute_kernel, (tb.M + kPermThreads - 1) / kPermThreads, kPermThreads, 0, s, tb, w);
+  launch_next(list_sort_kernel, (tb.N + kWarps - 1) / kWarps, kThreads, 0, s, w, p, tb.N);
   return cudaGetLastError();
 }
 
@@ -1255,7 +1264,7 @@ cudaError_t launch_residual(const Work& w, const Table& tb, const Pattern& p, co
   auto kern = skin ? cells_kernel<true, true> : cells_kernel<false, true>;
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCellsSmem);
   if (e != cudaSuccess) return e;
-  kern<<<grid, kThreads, kCellsSmem, s>>>(tb, w, p, ea, 0);
+  launch_next(kern, grid, kThreads, kCellsSmem, s, tb, w, p, ea, 0);
   return cudaGetLastError();
 }
 
@@ -1264,8 +1273,9 @@ cudaError_t launch_final_energy(const Work& w, const Pattern& p, const SolveArgs
                                 bool stats) {
   const Table& tb = a.tb;
   if (tb.n_e <= 0) return cudaSuccess;
-  cells_kernel<true, false><<<tb.n_e, kThreads, 0, s>>>(tb, w, p, edge_args(p, a, a.transforms, stats), slot);
-  if (tb.P > 1) energy_reduce_kernel<<<tb.P, 32, 0, s>>>(tb, w, slot);
+  launch_next(cells_kernel<true, false>, tb.n_e, kThreads, 0, s, tb, w, p, edge_args(p, a, a.transforms, stats),
+              slot);
+  if (tb.P > 1) launch_next(energy_reduce_kernel, tb.P, 32, 0, s, tb, w, slot);
   return cudaGetLastError();
 }
 
@@ -1275,9 +1285,9 @@ cudaError_t launch_assemble(const Work& w, const Pattern& p, const SolveArgs& a,
   // row is then four times shorter; 256 rows: 14.8 us against 18.9), two beyond
   // (less work per row; 2048 rows: 23 us against 26, 255k rows: 1.61 against 2.12 ms).
   if (p.N <= 1024)
-    gather_kernel<4><<<p.N, 128, 0, s>>>(w, p, a.lambda_damping);
+    launch_next(gather_kernel<4>, p.N, 128, 0, s, w, p, a.lambda_damping);
   else
-    gather_kernel<2><<<p.N, 64, 0, s>>>(w, p, a.lambda_damping);
+    launch_next(gather_kernel<2>, p.N, 64, 0, s, w, p, a.lambda_damping);
   return cudaGetLastError();
 }
 

@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(kCsBlock* kCsBlock)
                      const float* __restrict__ lv, const float* __restrict__ ln, float4* __restrict__ A,
                      float2* __restrict__ B, const CsPix pix, CsBox* __restrict__ box, int* __restrict__ flag,
                      int* __restrict__ num_valid, int* __restrict__ stats) {
+  after_previous();
   __shared__ float s_f[kCsBlock * kCsBlock / 32][13];
   __shared__ int s_i[kCsBlock * kCsBlock / 32][4];
   const int tid = threadIdx.x;
@@ -997,6 +998,7 @@ __global__ void __launch_bounds__(kMergeThreads)
                       const float2* __restrict__ B, const CsPix pix, const int* __restrict__ flag, const CsPart part,
                       const KnnSrc knn, cf_correspondence* __restrict__ out, int* __restrict__ num_valid,
                       int* __restrict__ stats) {
+  after_previous();
   __shared__ float s_stage[kMergeThreads / 32][32 * kCsRecWords];
   __shared__ int s_again[kMergeThreads], s_count;
   __shared__ float s_p[12];
@@ -1151,6 +1153,7 @@ __global__ void __launch_bounds__(kMergeThreads)
 __global__ void pixel_knn_kernel(const int* __restrict__ hit, int P, const int* __restrict__ vk,
                                  const float* __restrict__ vw, long long num_voxels, int* __restrict__ pk,
                                  float* __restrict__ pw) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P) return;
   const int v = hit[i];
@@ -1278,12 +1281,19 @@ cudaError_t launch_corr_search(const cf_corr_frame* f, const cf_camera* cam, con
 
   const CsPix pix = {sc.pix_v, sc.pix_n, sc.pix_row};
   CsBox* box = static_cast<CsBox*>(sc.box);
-  corr_prep_kernel<<<dim3((W + kCsBlock - 1) / kCsBlock, (H + kCsBlock - 1) / kCsBlock), kCsBlock * kCsBlock, 0, s>>>(
-      k, f->d_depth, f->d_depth_normals, f->d_live_vertices, f->d_live_normals, sc.A, sc.B, pix, box, sc.flag, num_valid,
-      stats);
-  if (!direct) kern<<<dim3(tiles.x, tiles.y, k.chunks), kCsThreads, kCsSmem, s>>>(k, sc.A, sc.B, pix, box, sc.flag, part);
-  merge<<<(k.P + kMergeThreads - 1) / kMergeThreads, kMergeThreads, 0, s>>>(k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag,
-                                                                            part, knn, out, num_valid, stats);
+  launch_next(corr_prep_kernel, dim3((W + kCsBlock - 1) / kCsBlock, (H + kCsBlock - 1) / kCsBlock),
+              kCsBlock * kCsBlock, 0, s, k, f->d_depth, f->d_depth_normals, f->d_live_vertices, f->d_live_normals,
+              sc.A, sc.B, pix, box, sc.flag, num_valid, stats);
+  // (launch_next only for the short calls: CTAs of the merge that wait beside a
+  // running search cost 15 of 573 us at radius 50)
+  const int mg = (k.P + kMergeThreads - 1) / kMergeThreads;
+  if (direct) {
+    launch_next(merge, mg, kMergeThreads, 0, s, k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag, part, knn, out,
+                num_valid, stats);
+  } else {
+    kern<<<dim3(tiles.x, tiles.y, k.chunks), kCsThreads, kCsSmem, s>>>(k, sc.A, sc.B, pix, box, sc.flag, part);
+    merge<<<mg, kMergeThreads, 0, s>>>(k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag, part, knn, out, num_valid, stats);
+  }
   *launches += direct ? 2 : 3;
   return cudaGetLastError();
 }
@@ -1291,7 +1301,7 @@ cudaError_t launch_corr_search(const cf_corr_frame* f, const cf_camera* cam, con
 cudaError_t launch_pixel_knn(const int* hit, int P, const int* vk, const float* vw, long long num_voxels, int* pk,
                              float* pw, cudaStream_t s) {
   if (P <= 0) return cudaSuccess;
-  pixel_knn_kernel<<<(P + 255) / 256, 256, 0, s>>>(hit, P, vk, vw, num_voxels, pk, pw);
+  launch_next(pixel_knn_kernel, (P + 255) / 256, 256, 0, s, hit, P, vk, vw, num_voxels, pk, pw);
   return cudaGetLastError();
 }
 

@@ -43,6 +43,7 @@ __device__ __forceinline__ int key_node(unsigned lo) {
 }
 
 __global__ void __launch_bounds__(kThreads) key_count_kernel(Table tb, Work w) {
+  after_previous();
   extern __shared__ int hist[];
   __shared__ __align__(16) uint32_t stage2[2][kThreads * kWords];  // double-buffered tiles of records
   const int tid = threadIdx.x;
@@ -133,6 +134,7 @@ __device__ __forceinline__ void setup_node(const Table& tb, const Work& w, int n
 //
 // The launch also resets the solve's statistics and sets up its nodes.
 __global__ void __launch_bounds__(kThreads) bin_scan_nodes_kernel(Table tb, Work w, int reset_stats) {
+  after_previous();
   __shared__ int seg[kThreads / 32][32];
   if (blockIdx.x == 0) reset_state(tb, w, reset_stats);
   const int lane = lane_id(), wid = threadIdx.x >> 5;
@@ -179,6 +181,7 @@ __global__ void __launch_bounds__(kThreads) bin_scan_nodes_kernel(Table tb, Work
 
 // the node set-up alone, for a table without correspondences
 __global__ void __launch_bounds__(kThreads) node_setup_kernel(Table tb, Work w, int reset_stats) {
+  after_previous();
   if (blockIdx.x == 0) reset_state(tb, w, reset_stats);
   const int n = blockIdx.x * kThreads + threadIdx.x;
   if (n < tb.N) setup_node(tb, w, n);
@@ -188,6 +191,7 @@ __global__ void __launch_bounds__(kThreads) node_setup_kernel(Table tb, Work w, 
 // round, the next round's totals in flight); cursor, when given, a copy of it.
 __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ total, int* __restrict__ start,
                                                     int* __restrict__ cursor, int N) {
+  after_previous();
   __shared__ int wsum[32];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   auto load = [&](int i0) {
@@ -238,6 +242,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ tota
 // Stable scatter of the correspondences by their key's first node: order
 // within a node = (tile, correspondence).
 __global__ void __launch_bounds__(kThreads) bin_scatter_kernel(Table tb, Work w) {
+  after_previous();
   extern __shared__ int cursor[];
   __shared__ int wkey[kThreads / 32][32];
   __shared__ int wcnt[kThreads / 32][32];
@@ -294,6 +299,7 @@ __global__ void __launch_bounds__(kThreads) bin_scatter_kernel(Table tb, Work w)
 constexpr int kScatterWarps = kThreads / 32;
 constexpr int kWarpScatterSmem = 200 * 1024;
 __global__ void __launch_bounds__(kThreads) bin_scatter_warp_kernel(Table tb, Work w) {
+  after_previous();
   extern __shared__ int sbase[];  // [N] CTA base of each node, then [8][N] 16-bit warp offsets
   const int tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
   const ProbDesc d = tb.desc[tb.bin_prob[blockIdx.x]];
@@ -346,6 +352,7 @@ __global__ void __launch_bounds__(kThreads) bin_scatter_warp_kernel(Table tb, Wo
 // Batched solves: each problem's nodes (neighbour ids made global) and
 // transforms into the concatenated arrays.
 __global__ void batch_gather_kernel(Table tb, Work w) {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= tb.N) return;
   const ProbDesc d = tb.desc[tb.node_prob[n]];
@@ -362,6 +369,7 @@ __global__ void batch_gather_kernel(Table tb, Work w) {
 }
 
 __global__ void batch_scatter_kernel(Table tb, Work w) {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= tb.N) return;
   const ProbDesc d = tb.desc[tb.node_prob[n]];
@@ -371,6 +379,7 @@ __global__ void batch_scatter_kernel(Table tb, Work w) {
 // WarpField::apply_twist_increment (src/warp_field.cu:250-291).
 __global__ void apply_twist_kernel(cf_dual_quat* __restrict__ T, const float* __restrict__ dx, int N, float max_rot,
                                    float max_trans, float scale) {
+  after_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   float d[6];
@@ -383,6 +392,7 @@ __global__ void apply_twist_kernel(cf_dual_quat* __restrict__ T, const float* __
 __global__ void skin_points_kernel(const float* __restrict__ pts, const int* __restrict__ ids,
                                    const float* __restrict__ ws, int M, const cf_deform_node* __restrict__ nodes,
                                    const cf_dual_quat* __restrict__ T, int N, float* out) {
+  after_previous();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= M) return;
   const float3 o = skin_point_centered(f3(pts[3 * c], pts[3 * c + 1], pts[3 * c + 2]), ids + 4 * c, ws + 4 * c,
@@ -404,26 +414,26 @@ cudaError_t launch_key_count(const Work& w, const Table& tb, cudaStream_t s) {
   const int smem = tb.max_N * (int)sizeof(int);
   cudaError_t e = cudaFuncSetAttribute(key_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  key_count_kernel<<<tb.n_bin, kThreads, smem, s>>>(tb, w);
+  launch_next(key_count_kernel, tb.n_bin, kThreads, smem, s, tb, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bin_scan(const Work& w, const Table& tb, bool reset_stats, cudaStream_t s) {
   if (tb.N <= 0) return cudaSuccess;
-  bin_scan_nodes_kernel<<<cdiv(tb.N, 32), kThreads, 0, s>>>(tb, w, reset_stats ? 1 : 0);
-  scan_kernel<<<1, 1024, 0, s>>>(w.node_total, w.inc_start, nullptr, tb.N);
+  launch_next(bin_scan_nodes_kernel, cdiv(tb.N, 32), kThreads, 0, s, tb, w, reset_stats ? 1 : 0);
+  launch_next(scan_kernel, 1, 1024, 0, s, w.node_total, w.inc_start, nullptr, tb.N);
   return cudaGetLastError();
 }
 
 cudaError_t launch_node_setup(const Work& w, const Table& tb, bool reset_stats, cudaStream_t s) {
   if (tb.N <= 0) return cudaSuccess;
-  node_setup_kernel<<<cdiv(tb.N, kThreads), kThreads, 0, s>>>(tb, w, reset_stats ? 1 : 0);
+  launch_next(node_setup_kernel, cdiv(tb.N, kThreads), kThreads, 0, s, tb, w, reset_stats ? 1 : 0);
   return cudaGetLastError();
 }
 
 cudaError_t launch_list_scan(const Work& w, const Table& tb, cudaStream_t s) {
   if (tb.N <= 0) return cudaSuccess;
-  scan_kernel<<<1, 1024, 0, s>>>(w.cl_total, w.cl_start, w.cl_cur, tb.N);
+  launch_next(scan_kernel, 1, 1024, 0, s, w.cl_total, w.cl_start, w.cl_cur, tb.N);
   return cudaGetLastError();
 }
 
@@ -435,32 +445,32 @@ cudaError_t launch_bin_scatter(const Work& w, const Table& tb, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(bin_scatter_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kWarpScatterSmem);
     if (e != cudaSuccess) return e;
-    bin_scatter_warp_kernel<<<tb.n_bin, kThreads, wsmem, s>>>(tb, w);
+    launch_next(bin_scatter_warp_kernel, tb.n_bin, kThreads, wsmem, s, tb, w);
     return cudaGetLastError();
   }
   const int smem = tb.max_N * (int)sizeof(int);
   cudaError_t e = cudaFuncSetAttribute(bin_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  bin_scatter_kernel<<<tb.n_bin, kThreads, smem, s>>>(tb, w);
+  launch_next(bin_scatter_kernel, tb.n_bin, kThreads, smem, s, tb, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_gather(const Work& w, const Table& tb, cudaStream_t s) {
   if (tb.N <= 0) return cudaSuccess;
-  batch_gather_kernel<<<cdiv(tb.N, 128), 128, 0, s>>>(tb, w);
+  launch_next(batch_gather_kernel, cdiv(tb.N, 128), 128, 0, s, tb, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_scatter(const Work& w, const Table& tb, cudaStream_t s) {
   if (tb.N <= 0) return cudaSuccess;
-  batch_scatter_kernel<<<cdiv(tb.N, 128), 128, 0, s>>>(tb, w);
+  launch_next(batch_scatter_kernel, cdiv(tb.N, 128), 128, 0, s, tb, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_apply_twist(cf_dual_quat* T, const float* dx, int N, float max_rot, float max_trans,
                                float scale, cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  apply_twist_kernel<<<cdiv(N, 128), 128, 0, s>>>(T, dx, N, max_rot, max_trans, scale);
+  launch_next(apply_twist_kernel, cdiv(N, 128), 128, 0, s, T, dx, N, max_rot, max_trans, scale);
   return cudaGetLastError();
 }
 
@@ -468,7 +478,7 @@ cudaError_t launch_skin_points(const float* pts, const int* ids, const float* ws
                                const cf_deform_node* nodes, const cf_dual_quat* T, int N, float* out,
                                cudaStream_t s) {
   if (M <= 0) return cudaSuccess;
-  skin_points_kernel<<<cdiv(M, 256), 256, 0, s>>>(pts, ids, ws, M, nodes, T, N, out);
+  launch_next(skin_points_kernel, cdiv(M, 256), 256, 0, s, pts, ids, ws, M, nodes, T, N, out);
   return cudaGetLastError();
 }
 

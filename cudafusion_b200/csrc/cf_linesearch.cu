@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(kLsThreads) update_stats_kernel(const float* _
                                                                    float max_trans, double* __restrict__ sums,
                                                                    unsigned* __restrict__ maxima,
                                                                    int* __restrict__ finite) {
+  after_previous();
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   float m[4] = {0.f, 0.f, 0.f, 0.f};
   bool fin = true;
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(kLsThreads) update_stats_kernel(const float* _
 // dx[k] * (rs * scale) and dx[k] * (ts * scale).
 __global__ void scale_delta_kernel(const float* __restrict__ dx, int N, float max_rot, float max_trans, float scale,
                                    float* __restrict__ out) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const float* d = dx + 6 * (size_t)i;
@@ -105,6 +107,7 @@ __global__ void scale_delta_kernel(const float* __restrict__ dx, int N, float ma
 // order; rmse_final_kernel adds the blocks in block order.  Deterministic.
 __global__ void __launch_bounds__(kLsThreads) rmse_partial_kernel(const cf_correspondence* __restrict__ corrs, int M,
                                                                    double* __restrict__ part) {
+  after_previous();
   const int per = (M + gridDim.x - 1) / gridDim.x;
   const int lo = blockIdx.x * per, hi = min(M, lo + per);
   double s = 0.0, ws = 0.0;
@@ -133,6 +136,7 @@ __global__ void __launch_bounds__(kLsThreads) rmse_partial_kernel(const cf_corre
 // search's valid count (the line search keeps each trial's in its slot).
 __global__ void rmse_final_kernel(const double* __restrict__ part, int blocks, double* __restrict__ out,
                                   const int* __restrict__ valid) {
+  after_previous();
   if (threadIdx.x < 2) {
     double v = 0.0;
     for (int b = 0; b < blocks; ++b) v += part[2 * b + threadIdx.x];
@@ -149,6 +153,7 @@ __global__ void rmse_final_kernel(const double* __restrict__ part, int blocks, d
 // copied aside, so that the accepted trial need not be predicted and searched
 // again.
 __global__ void __launch_bounds__(256) ls_keep_kernel(LsKeepArgs a) {
+  after_previous();
   const double sum = a.slot[0], wsum = a.slot[1];
   const int valid = (int)a.slot[2];
   const double rmse = wsum > 0.0 ? sqrt(sum / wsum) : (double)INFINITY;
@@ -170,7 +175,7 @@ __global__ void __launch_bounds__(256) ls_keep_kernel(LsKeepArgs a) {
 }  // namespace
 
 cudaError_t launch_ls_keep(const LsKeepArgs& a, cudaStream_t s) {
-  ls_keep_kernel<<<296, 256, 0, s>>>(a);
+  launch_next(ls_keep_kernel, 296, 256, 0, s, a);
   return cudaGetLastError();
 }
 
@@ -179,21 +184,22 @@ cudaError_t launch_update_stats(const float* dx, int N, float update_scale, floa
   if (N <= 0) return cudaSuccess;
   int blocks = (N + kLsThreads - 1) / kLsThreads;
   if (blocks > 148) blocks = 148;
-  update_stats_kernel<<<blocks, kLsThreads, 0, s>>>(dx, N, update_scale, max_rot, max_trans, sums, maxima, finite);
+  launch_next(update_stats_kernel, blocks, kLsThreads, 0, s, dx, N, update_scale, max_rot, max_trans, sums, maxima,
+              finite);
   return cudaGetLastError();
 }
 
 cudaError_t launch_scale_delta(const float* dx, int N, float max_rot, float max_trans, float scale, float* out,
                                cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  scale_delta_kernel<<<(N + 255) / 256, 256, 0, s>>>(dx, N, max_rot, max_trans, scale, out);
+  launch_next(scale_delta_kernel, (N + 255) / 256, 256, 0, s, dx, N, max_rot, max_trans, scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_corr_rmse(const cf_correspondence* corrs, int M, double* partials, double* out, const int* valid,
                              cudaStream_t s) {
-  rmse_partial_kernel<<<CF_RMSE_BLOCKS, kLsThreads, 0, s>>>(corrs, M, partials);
-  rmse_final_kernel<<<1, 32, 0, s>>>(partials, CF_RMSE_BLOCKS, out, valid);
+  launch_next(rmse_partial_kernel, CF_RMSE_BLOCKS, kLsThreads, 0, s, corrs, M, partials);
+  launch_next(rmse_final_kernel, 1, 32, 0, s, partials, CF_RMSE_BLOCKS, out, valid);
   return cudaGetLastError();
 }
 

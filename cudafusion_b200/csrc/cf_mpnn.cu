@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
                                                       const __nv_bfloat16* __restrict__ W,
                                                       const __nv_bfloat16* __restrict__ b, void* out_,
                                                       const float* __restrict__ x_skip, int N) {
+  after_previous();
   using S = FwdShape<DIN, DOUT, AGG>;
   constexpr int CAT = S::CAT, CATP = S::CATP, DINP = S::DINP, DOUTP = S::DOUTP, LD = S::LD, LDL = S::LDL;
   static_assert(CAT % 8 == 0, "weight rows in 16-B chunks");
@@ -386,6 +387,7 @@ __global__ void reduce_loss(const double* __restrict__ part, int n, double* __re
 __global__ void adam_step(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
                           const float* __restrict__ g, __nv_bfloat16* __restrict__ wb, int n, float lr, float b1,
                           float b2, float c1, float c2, float eps) {
+  after_previous();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float gg = g[q];
@@ -399,6 +401,7 @@ __global__ void adam_step(float* __restrict__ w, float* __restrict__ m, float* _
 }
 
 __global__ void to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__ wb, int n) {
+  after_previous();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < n) wb[q] = tobf(w[q]);
 }
@@ -406,6 +409,7 @@ __global__ void to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__
 // graph of a problem's nodes: neighbour lists (-1 = none) and 1/degree
 __global__ void graph_from_nodes(const cf_deform_node* __restrict__ nodes, int N, int* __restrict__ nbr,
                                  float* __restrict__ inv_deg) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const int nn = min(max(nodes[i].num_neighbors, 0), CF_K_GRAPH);
@@ -464,6 +468,7 @@ __device__ __forceinline__ DQ dq_apply_increment(DQ T, const float* o) {
 
 __global__ void increments_kernel(const cf_dual_quat* __restrict__ to, const cf_dual_quat* __restrict__ from, int n,
                                   float* __restrict__ out) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float o[6];
@@ -479,6 +484,7 @@ __global__ void increments_kernel(const cf_dual_quat* __restrict__ to, const cf_
 __global__ void features_kernel(const cf_dual_quat* __restrict__ T, const cf_dual_quat* __restrict__ hist, int N,
                                 const int* __restrict__ cl_start, const int* __restrict__ clist,
                                 const float4* __restrict__ cstat, float* __restrict__ feat) {
+  after_previous();
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= N) return;
   float s = 0.f, mx = 0.f;
@@ -516,6 +522,7 @@ __global__ void features_kernel(const cf_dual_quat* __restrict__ T, const cf_dua
 __global__ void apply_prediction(cf_dual_quat* __restrict__ T, cf_dual_quat* __restrict__ T_save,
                                  cf_dual_quat* __restrict__ plain, const cf_deform_node* __restrict__ nodes,
                                  const float* __restrict__ pred, int N) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const DQ t0 = load_dq_cg(T + i);
@@ -538,6 +545,7 @@ __global__ void apply_prediction(cf_dual_quat* __restrict__ T, cf_dual_quat* __r
 __global__ void gate_prediction(cf_dual_quat* __restrict__ T, const cf_dual_quat* __restrict__ T_save,
                                 cf_dual_quat* __restrict__ plain, const cf_deform_node* __restrict__ nodes,
                                 DevStats* __restrict__ st, int N) {
+  after_previous();
   const bool reject = !(st->gate[1] <= st->gate[0]);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) st->init_rejected = reject ? 1 : 0;
@@ -595,14 +603,14 @@ void mpnn_free(Mpnn& m) {
 }
 
 cudaError_t mpnn_refresh_bf16(const Mpnn& m, cudaStream_t s) {
-  to_bf16<<<cdiv(kParams, 256), 256, 0, s>>>(m.w, reinterpret_cast<__nv_bfloat16*>(m.wb), kParams);
+  launch_next(to_bf16, cdiv(kParams, 256), 256, 0, s, m.w, reinterpret_cast<__nv_bfloat16*>(m.wb), kParams);
   return cudaGetLastError();
 }
 
 cudaError_t mpnn_graph_from_nodes(Mpnn& m, const cf_deform_node* nodes, int N, cudaStream_t s) {
   m.N = N;
   if (N <= 0) return cudaSuccess;
-  graph_from_nodes<<<cdiv(N, 128), 128, 0, s>>>(nodes, N, m.nbr, m.inv_deg);
+  launch_next(graph_from_nodes, cdiv(N, 128), 128, 0, s, nodes, N, m.nbr, m.inv_deg);
   return cudaGetLastError();
 }
 
@@ -616,14 +624,14 @@ cudaError_t mpnn_forward(const Mpnn& m, const float* feat, float* out, cudaStrea
   cudaError_t e = cudaFuncSetAttribute(layer_fwd<kHid, kHid, false, true, true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, s1);
   if (e != cudaSuccess) return e;
-  layer_fwd<kIn, kHid, true, true, true><<<g, kThreads, s0, s>>>(feat, m.nbr, m.inv_deg, wb + kW0, wb + kB0, m.h1,
-                                                                  nullptr, N);
-  layer_fwd<kHid, kHid, false, true, true><<<g, kThreads, s1, s>>>(m.h1, m.nbr, m.inv_deg, wb + kW1, wb + kB1, m.h2,
-                                                                    nullptr, N);
-  layer_fwd<kHid, kHid, false, true, true><<<g, kThreads, s1, s>>>(m.h2, m.nbr, m.inv_deg, wb + kW2, wb + kB2, m.h3,
-                                                                    nullptr, N);
-  layer_fwd<kHid, kOut, false, false, false><<<g, kThreads, so, s>>>(m.h3, nullptr, nullptr, wb + kWo, wb + kBo, out,
-                                                                      feat, N);
+  launch_next(layer_fwd<kIn, kHid, true, true, true>, g, kThreads, s0, s, feat, m.nbr, m.inv_deg, wb + kW0, wb + kB0,
+              m.h1, nullptr, N);
+  launch_next(layer_fwd<kHid, kHid, false, true, true>, g, kThreads, s1, s, m.h1, m.nbr, m.inv_deg, wb + kW1,
+              wb + kB1, m.h2, nullptr, N);
+  launch_next(layer_fwd<kHid, kHid, false, true, true>, g, kThreads, s1, s, m.h2, m.nbr, m.inv_deg, wb + kW2,
+              wb + kB2, m.h3, nullptr, N);
+  launch_next(layer_fwd<kHid, kOut, false, false, false>, g, kThreads, so, s, m.h3, nullptr, nullptr, wb + kWo,
+              wb + kBo, out, feat, N);
   return cudaGetLastError();
 }
 
@@ -665,35 +673,35 @@ cudaError_t mpnn_adam(Mpnn& m, float lr, cudaStream_t s) {
   m.step++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)m.step), c2 = 1.f - powf(b2, (float)m.step);
-  adam_step<<<cdiv(kParams, 256), 256, 0, s>>>(m.w, m.m, m.v, m.g, reinterpret_cast<__nv_bfloat16*>(m.wb), kParams,
-                                                lr, b1, b2, c1, c2, 1e-8f);
+  launch_next(adam_step, cdiv(kParams, 256), 256, 0, s, m.w, m.m, m.v, m.g, reinterpret_cast<__nv_bfloat16*>(m.wb),
+              kParams, lr, b1, b2, c1, c2, 1e-8f);
   return cudaGetLastError();
 }
 
 cudaError_t launch_increments(const cf_dual_quat* to, const cf_dual_quat* from, int n, float* out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  increments_kernel<<<cdiv(n, 128), 128, 0, s>>>(to, from, n, out);
+  launch_next(increments_kernel, cdiv(n, 128), 128, 0, s, to, from, n, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_features(const Work& w, const cf_dual_quat* T, const cf_dual_quat* hist, int N, float* feat,
                             cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  features_kernel<<<cdiv(N * 32, 256), 256, 0, s>>>(T, hist, N, w.cl_start, w.clist, w.cstat, feat);
+  launch_next(features_kernel, cdiv(N * 32, 256), 256, 0, s, T, hist, N, w.cl_start, w.clist, w.cstat, feat);
   return cudaGetLastError();
 }
 
 cudaError_t launch_apply_prediction(const Work& w, cf_dual_quat* T, const cf_deform_node* nodes, const float* pred,
                                     int N, cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  apply_prediction<<<cdiv(N, 128), 128, 0, s>>>(T, w.T_save, w.plain, nodes, pred, N);
+  launch_next(apply_prediction, cdiv(N, 128), 128, 0, s, T, w.T_save, w.plain, nodes, pred, N);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gate_prediction(const Work& w, cf_dual_quat* T, const cf_deform_node* nodes, int N,
                                    cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  gate_prediction<<<cdiv(N, 128), 128, 0, s>>>(T, w.T_save, w.plain, nodes, w.stats, N);
+  launch_next(gate_prediction, cdiv(N, 128), 128, 0, s, T, w.T_save, w.plain, nodes, w.stats, N);
   return cudaGetLastError();
 }
 

@@ -166,7 +166,12 @@ __global__ void __launch_bounds__(kSpl == 1 ? 1024 : 768, 1) pcg_cluster_kernel(
   asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
 
   // ---- prologue ----
-  // the diagonal blocks, by cp.async, and everything small
+  // the plan, while the assembly may still run; then the diagonal blocks, by
+  // cp.async, and everything small
+  for (int k = tid; k < nblk; k += nthreads) sVidx[k] = (unsigned short)__ldg(pt.clu_vidx + b0 + k);
+  for (int k = tid; k < nhalo; k += nthreads) sHalo[k] = __ldg(pt.clu_halo + h0 + k);
+  for (int i = tid; i <= nrows; i += nthreads) sRow[i] = __ldg(pt.row_ptr + r0 + i) - b0;
+  after_previous();
   const float* gA = pt.values + (size_t)b0 * 36;
   float* sD = sA;
   unsigned char* scr0 = smem + L.a + al16(nrows * 36 * 4);
@@ -186,9 +191,6 @@ __global__ void __launch_bounds__(kSpl == 1 ? 1024 : 768, 1) pcg_cluster_kernel(
       cp_async4(sp + 2, np + 2);
     }
   cp_async_commit();
-  for (int k = tid; k < nblk; k += nthreads) sVidx[k] = (unsigned short)__ldg(pt.clu_vidx + b0 + k);
-  for (int k = tid; k < nhalo; k += nthreads) sHalo[k] = __ldg(pt.clu_halo + h0 + k);
-  for (int i = tid; i <= nrows; i += nthreads) sRow[i] = __ldg(pt.row_ptr + r0 + i) - b0;
   // this lane's row, its element and its share of the element's blocks
   const int rl = lane / kRowLanes, c = (lane - rl * kRowLanes) / kSpl, ks = lane % kSpl;
   const int row = wid * kRowsPerWarp + rl;
@@ -442,18 +444,21 @@ cudaError_t config_kernel(int C, int rows_max, int smem) {
   return e;
 }
 
+// (attr: two; the second lets it start as launch_next does)
 cudaLaunchConfig_t launch_config(int C, int threads, int smem, cudaLaunchAttribute* attr, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = C;
-  attr->val.clusterDim.y = 1;
-  attr->val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -472,8 +477,8 @@ int pcg_cluster_max_active(int C, int rows_max, int smem) {
     cudaGetLastError();
     return 0;
   }
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = launch_config(C, threads, smem, &attr, nullptr);
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = launch_config(C, threads, smem, attr, nullptr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kernel_of(rows_max), &cfg) != cudaSuccess) {
     cudaGetLastError();
@@ -490,8 +495,8 @@ cudaError_t launch_pcg_cluster(const Work& w, const Pattern& p, const SolveArgs&
   P.a = a;
   P.slot = gn_slot;
   const int threads = pick_threads(p.clu_rows_max);
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = launch_config(p.clu_C, threads, p.clu_smem, &attr, s);
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = launch_config(p.clu_C, threads, p.clu_smem, attr, s);
   return cudaLaunchKernelEx(&cfg, kernel_of(p.clu_rows_max), P);
 }
 

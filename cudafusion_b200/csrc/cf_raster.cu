@@ -128,6 +128,7 @@ __global__ void mesh_skin_kernel(const float* __restrict__ canon, float* __restr
                                  const RasterConsts k, const cf_deform_node* __restrict__ nodes,
                                  const cf_dual_quat* __restrict__ T, int N, const int* __restrict__ vk,
                                  const float* __restrict__ vw) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
   const float3 p = rs_ld3(canon, i);
@@ -148,6 +149,7 @@ __global__ void mesh_skin_kernel(const float* __restrict__ canon, float* __restr
 __global__ void mesh_skin_plain_kernel(const float* __restrict__ canon, float* __restrict__ warped, int V,
                                        const RasterConsts k, const cf_dual_quat* __restrict__ plain, int N,
                                        const int4* __restrict__ vk, const float4* __restrict__ vw) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
   const float3 p = rs_ld3(canon, i);
@@ -367,6 +369,7 @@ __global__ void __launch_bounds__(128, 9) raster_kernel(const float* __restrict_
                                                         unsigned long long* __restrict__ ztri,
                                                         float4* __restrict__ cache, int2* __restrict__ big,
                                                         unsigned long long* __restrict__ big_ctr) {
+  after_previous();
   const int ti = blockIdx.x * blockDim.x + threadIdx.x;
   if (ti >= NT) return;
   RsTri r;
@@ -395,6 +398,7 @@ __global__ void __launch_bounds__(256) raster_big_kernel(const float4* __restric
                                                          int G, unsigned long long* __restrict__ ztri,
                                                          const int2* __restrict__ big,
                                                          const unsigned long long* __restrict__ big_ctr) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
   const unsigned long long ctr = *big_ctr;
@@ -463,6 +467,7 @@ __global__ void __launch_bounds__(256) resolve_kernel(const RasterConsts k, unsi
                                                       const float4* __restrict__ cache, float* __restrict__ lv,
                                                       float* __restrict__ ln, int* __restrict__ hit,
                                                       unsigned long long* __restrict__ big_ctr) {
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t == 0) *big_ctr = 0;  // the big list is consumed: ready for the next frame
   const int P = k.W * k.H, half = (P + 1) >> 1;
@@ -514,7 +519,7 @@ cudaError_t launch_mesh_skin(const float* canon, float* warped, int V, const cf_
                              cudaStream_t s) {
   if (V <= 0) return cudaSuccess;
   const RasterConsts k = raster_consts(nullptr, nullptr, grid);
-  mesh_skin_kernel<<<(V + 255) / 256, 256, 0, s>>>(canon, warped, V, k, nodes, T, N, vk, vw);
+  launch_next(mesh_skin_kernel, (V + 255) / 256, 256, 0, s, canon, warped, V, k, nodes, T, N, vk, vw);
   return cudaGetLastError();
 }
 
@@ -522,9 +527,8 @@ cudaError_t launch_mesh_skin_plain(const float* canon, float* warped, int V, con
                                    const cf_dual_quat* plain, int N, const int* vk, const float* vw, cudaStream_t s) {
   if (V <= 0) return cudaSuccess;
   const RasterConsts k = raster_consts(nullptr, nullptr, grid);
-  mesh_skin_plain_kernel<<<(V + 255) / 256, 256, 0, s>>>(canon, warped, V, k, plain, N,
-                                                         reinterpret_cast<const int4*>(vk),
-                                                         reinterpret_cast<const float4*>(vw));
+  launch_next(mesh_skin_plain_kernel, (V + 255) / 256, 256, 0, s, canon, warped, V, k, plain, N,
+              reinterpret_cast<const int4*>(vk), reinterpret_cast<const float4*>(vw));
   return cudaGetLastError();
 }
 
@@ -550,11 +554,12 @@ cudaError_t launch_raster(const float* canon, const float* warped, const int* tr
       if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       sms_times_2 = 2 * sms;
     }
-    raster_kernel<<<(NT + 127) / 128, 128, 0, s>>>(canon, warped, t3, V, NT, k, G, ztri, cache, big2, big_ctr);
-    raster_big_kernel<<<sms_times_2, 256, 0, s>>>(cache, k, G, ztri, big2, big_ctr);
+    launch_next(raster_kernel, (NT + 127) / 128, 128, 0, s, canon, warped, t3, V, NT, k, G, ztri, cache, big2,
+                big_ctr);
+    launch_next(raster_big_kernel, sms_times_2, 256, 0, s, cache, k, G, ztri, big2, big_ctr);
     *launches += 2;
   }
-  resolve_kernel<<<((P + 1) / 2 + 255) / 256, 256, 0, s>>>(k, ztri, cache, lv, ln, hit, big_ctr);
+  launch_next(resolve_kernel, ((P + 1) / 2 + 255) / 256, 256, 0, s, k, ztri, cache, lv, ln, hit, big_ctr);
   *launches += 1;
   return cudaGetLastError();
 }

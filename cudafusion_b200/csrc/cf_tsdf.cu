@@ -74,6 +74,7 @@ __device__ __forceinline__ float3 ts_centre(const TsdfConsts& k, unsigned i) {
 
 __global__ void tsdf_plain_kernel(const cf_deform_node* __restrict__ nodes, const cf_dual_quat* __restrict__ T,
                                   cf_dual_quat* __restrict__ plain, int N) {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < N) store_dq(plain + i, dq_centered(load_dq_cg(T + i), node_pos(nodes, i)));
 }
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(kTsThreads)
     tsdf_integrate_kernel(const TsdfConsts k, float* __restrict__ vox, unsigned V, const float* __restrict__ depth,
                           const int4* __restrict__ knn, const float4* __restrict__ knn_w,
                           const cf_dual_quat* __restrict__ plain, int N, const int* __restrict__ counts) {
+  after_previous();
   const unsigned i = blockIdx.x * kTsThreads + threadIdx.x;
   if (i >= V) return;
   if (kGate && __ldcs(counts + i) < k.min_opt) return;
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(kTsThreads)
     tsdf_gated_kernel(const TsdfConsts k, float* __restrict__ vox, unsigned V, const float* __restrict__ depth,
                       const int4* __restrict__ knn, const float4* __restrict__ knn_w,
                       const cf_dual_quat* __restrict__ plain, int N, const int* __restrict__ counts) {
+  after_previous();
   __shared__ unsigned s_queue[kTsThreads / 32][kTsQueue];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   unsigned* q = s_queue[wl];
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(kTsThreads)
 __global__ void __launch_bounds__(kTsThreads)
     tsdf_centres_kernel(const TsdfConsts k, float* __restrict__ out, unsigned V, const int4* __restrict__ knn,
                         const float4* __restrict__ knn_w, const cf_dual_quat* __restrict__ plain, int N) {
+  after_previous();
   const unsigned i = blockIdx.x * kTsThreads + threadIdx.x;
   if (i >= V) return;
   float3 p = ts_centre(k, i);
@@ -268,6 +272,7 @@ __global__ void __launch_bounds__(kTsThreads)
 __global__ void mark_opt_kernel(const cf_correspondence* __restrict__ corrs, const int* __restrict__ vidx_map,
                                 int P, int dx, int dy, int dz, int frame, int* __restrict__ counts,
                                 int* __restrict__ frames) {
+  after_previous();
   const int px = blockIdx.x * blockDim.x + threadIdx.x;
   if (px >= P) return;
   const cf_correspondence& c = corrs[px];
@@ -292,6 +297,7 @@ __global__ void mark_opt_kernel(const cf_correspondence* __restrict__ corrs, con
 }
 
 __global__ void tsdf_init_kernel(cf_tsdf_voxel* __restrict__ vox, unsigned V) {
+  after_previous();
   const unsigned i = blockIdx.x * kTsThreads + threadIdx.x;
   if (i >= V) return;
   float* f = reinterpret_cast<float*>(vox + i);
@@ -336,7 +342,7 @@ unsigned blocks_of(unsigned V) { return (V + kTsThreads - 1) / kTsThreads; }
 cudaError_t launch_tsdf_plain(const cf_deform_node* nodes, const cf_dual_quat* T, cf_dual_quat* plain, int N,
                               cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
-  tsdf_plain_kernel<<<(N + 127) / 128, 128, 0, s>>>(nodes, T, plain, N);
+  launch_next(tsdf_plain_kernel, (N + 127) / 128, 128, 0, s, nodes, T, plain, N);
   return cudaGetLastError();
 }
 
@@ -365,14 +371,16 @@ cudaError_t launch_tsdf_integrate(float* vox, const cf_tsdf_params* p, const flo
     }
     const unsigned tiles = (V + kTsTile - 1) / kTsTile;
     const unsigned ctas = std::min<unsigned>(resident, (tiles + kTsThreads / 32 - 1) / (kTsThreads / 32));
-    tsdf_gated_kernel<<<ctas, kTsThreads, 0, s>>>(k, vox, V, depth, kn, kw, plain, N, counts);
+    launch_next(tsdf_gated_kernel, ctas, kTsThreads, 0, s, k, vox, V, depth, kn, kw, plain, N, counts);
   } else if (warp && counts)
-    tsdf_integrate_kernel<true, true><<<blocks_of(V), kTsThreads, 0, s>>>(k, vox, V, depth, kn, kw, plain, N, counts);
+    launch_next(tsdf_integrate_kernel<true, true>, blocks_of(V), kTsThreads, 0, s, k, vox, V, depth, kn, kw, plain, N,
+                counts);
   else if (warp)
-    tsdf_integrate_kernel<true, false><<<blocks_of(V), kTsThreads, 0, s>>>(k, vox, V, depth, kn, kw, plain, N, nullptr);
+    launch_next(tsdf_integrate_kernel<true, false>, blocks_of(V), kTsThreads, 0, s, k, vox, V, depth, kn, kw, plain,
+                N, nullptr);
   else
-    tsdf_integrate_kernel<false, false><<<blocks_of(V), kTsThreads, 0, s>>>(k, vox, V, depth, nullptr, nullptr,
-                                                                             nullptr, 0, nullptr);
+    launch_next(tsdf_integrate_kernel<false, false>, blocks_of(V), kTsThreads, 0, s, k, vox, V, depth, nullptr,
+                nullptr, nullptr, 0, nullptr);
   return cudaGetLastError();
 }
 
@@ -381,21 +389,22 @@ cudaError_t launch_tsdf_centres(float* out, const cf_tsdf_params* p, const int* 
   const unsigned V = (unsigned)p->dims[0] * (unsigned)p->dims[1] * (unsigned)p->dims[2];
   if (V == 0) return cudaSuccess;
   const TsdfConsts k = make_consts(p, nullptr, nullptr, 0);
-  tsdf_centres_kernel<<<blocks_of(V), kTsThreads, 0, s>>>(k, out, V, reinterpret_cast<const int4*>(knn),
-                                                          reinterpret_cast<const float4*>(knn_w), plain, N);
+  launch_next(tsdf_centres_kernel, blocks_of(V), kTsThreads, 0, s, k, out, V, reinterpret_cast<const int4*>(knn),
+              reinterpret_cast<const float4*>(knn_w), plain, N);
   return cudaGetLastError();
 }
 
 cudaError_t launch_mark_optimized(const cf_correspondence* corrs, const int* vidx, int P, const int dims[3],
                                   int frame, int* counts, int* frames, cudaStream_t s) {
   if (P <= 0) return cudaSuccess;
-  mark_opt_kernel<<<(P + 255) / 256, 256, 0, s>>>(corrs, vidx, P, dims[0], dims[1], dims[2], frame, counts, frames);
+  launch_next(mark_opt_kernel, (P + 255) / 256, 256, 0, s, corrs, vidx, P, dims[0], dims[1], dims[2], frame, counts,
+              frames);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tsdf_init(cf_tsdf_voxel* vox, unsigned V, cudaStream_t s) {
   if (V == 0) return cudaSuccess;
-  tsdf_init_kernel<<<blocks_of(V), kTsThreads, 0, s>>>(vox, V);
+  launch_next(tsdf_init_kernel, blocks_of(V), kTsThreads, 0, s, vox, V);
   return cudaGetLastError();
 }
 
