@@ -380,7 +380,7 @@ struct Mpnn {
   int *rev_ptr = nullptr, *rev_idx = nullptr;  // reverse graph (training)
   float *feat = nullptr, *tgt = nullptr, *out = nullptr;
   void *h1 = nullptr, *h2 = nullptr, *h3 = nullptr;  // BF16 activations [N][64]
-  float *dh = nullptr, *dh2 = nullptr, *dcat = nullptr, *part = nullptr;
+  float *dh = nullptr, *dcat2 = nullptr, *dcat = nullptr, *part = nullptr;
   double *loss_part = nullptr, *loss = nullptr;
 };
 int mpnn_param_count();

@@ -17,8 +17,8 @@
 // rounded to BF16 after every step); every sum accumulates in FP32, in a
 // fixed order, so forward and gradients are deterministic.  The layers are
 // tiny (N x 128 x 64): the forward runs on the tensor cores (BF16 mma.sync
-// over shared-memory tiles of 16 nodes), the gradients on CUDA cores over
-// tiles of 32 (per-CTA partial sums reduced in CTA order).
+// over shared-memory tiles of 16 nodes), the gradients on CUDA cores (FP32)
+// over tiles of 32 (per-CTA partial sums reduced in CTA order).
 #include <cuda_bf16.h>
 
 #include "cf_device.cuh"
@@ -80,6 +80,37 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], unsigned a0, unsig
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Features k..k+3 of node i's neighbour mean, summed in list order in FP32.
+__device__ __forceinline__ float4 bf4(uint2 v) {
+  const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(v.x)),
+               b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(v.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <int DIN>
+__device__ __forceinline__ float4 mean_of(const __nv_bfloat16* in, const int* __restrict__ nbr,
+                                          const float* __restrict__ inv_deg, int i, int k) {
+  const int4 n0 = __ldg(reinterpret_cast<const int4*>(nbr + (size_t)i * CF_K_GRAPH)),
+             n1 = __ldg(reinterpret_cast<const int4*>(nbr + (size_t)i * CF_K_GRAPH) + 1);
+  const int jn[CF_K_GRAPH] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
+  uint2 x[CF_K_GRAPH];
+#pragma unroll
+  for (int q = 0; q < CF_K_GRAPH; q++)
+    x[q] = jn[q] >= 0 ? *reinterpret_cast<const uint2*>(in + (size_t)jn[q] * DIN + k) : make_uint2(0u, 0u);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int q = 0; q < CF_K_GRAPH; q++)
+    if (jn[q] >= 0) {
+      const float4 v = bf4(x[q]);
+      a.x += v.x;
+      a.y += v.y;
+      a.z += v.z;
+      a.w += v.w;
+    }
+  const float d = inv_deg[i];
+  return make_float4(a.x * d, a.y * d, a.z * d, a.w * d);
+}
+static_assert(CF_K_GRAPH == 8, "a node's list is two int4");
+
 template <int DIN, int DOUT, bool FIRST, bool AGG, bool RELU>
 __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int* __restrict__ nbr,
                                                       const float* __restrict__ inv_deg,
@@ -96,7 +127,6 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
   __nv_bfloat16* sLo = sX + kFwdTile * LD;                        // [kFwdTile][LDL]: mean (lo)
   float* sB = reinterpret_cast<float*>(sLo + (AGG ? kFwdTile * LDL : 0));  // [DOUTP]
   const int tid = threadIdx.x;
-  const int n0 = blockIdx.x * kFwdTile;
   const __nv_bfloat16 zero = tobf(0.f);
   // column c of a global weight row -> its padded column
   auto wcol = [](int c) { return c < DIN ? c : DINP + (c - DIN); };
@@ -111,7 +141,9 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
 #pragma unroll
     for (int j = 0; j < PER; j++) {
       const int q = tid + j * kThreads;
-      if (q < NCH) {
+      if (q < NCH && CAT == CATP) {  // no padding: rows keep their 16-byte chunks
+        *reinterpret_cast<uint4*>(sW + 8 * q / CAT * LD + 8 * q % CAT) = wv[j];
+      } else if (q < NCH) {
         const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&wv[j]);
 #pragma unroll
         for (int t = 0; t < 8; t++) {
@@ -136,7 +168,33 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
     if (FIRST) return bf(tobf(reinterpret_cast<const float*>(in_)[(size_t)i * DIN + k]));
     return bf(reinterpret_cast<const __nv_bfloat16*>(in_)[(size_t)i * DIN + k]);
   };
-  {
+  for (int n0 = blockIdx.x * kFwdTile; n0 < N; n0 += gridDim.x * kFwdTile) {
+  if (n0 != (int)blockIdx.x * kFwdTile) __syncthreads();
+  if constexpr (!FIRST) {  // four features a thread: 8-byte loads, all in flight
+    constexpr int NCH = kFwdTile * DIN / 4, PER = (NCH + kThreads - 1) / kThreads;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      const int e = tid + j * kThreads, sl = e / (DIN / 4), k = 4 * (e % (DIN / 4)), i = n0 + sl;
+      if (e >= NCH) continue;
+      const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(in_);
+      uint2 own = make_uint2(0u, 0u);
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < N) {
+        own = *reinterpret_cast<const uint2*>(in + (size_t)i * DIN + k);
+        if constexpr (AGG) a = mean_of<DIN>(in, nbr, inv_deg, i, k);
+      }
+      *reinterpret_cast<uint2*>(sX + sl * LD + k) = own;
+      if constexpr (AGG) {
+        const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          const __nv_bfloat16 hi = tobf(v[c]);
+          sX[sl * LD + DINP + k + c] = hi;
+          sLo[sl * LDL + k + c] = tobf(v[c] - bf(hi));
+        }
+      }
+    }
+  } else {
     constexpr int NE = kFwdTile * DIN, EPT = (NE + kThreads - 1) / kThreads;
     int jn[EPT][CF_K_GRAPH];
 #pragma unroll
@@ -224,6 +282,7 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
       }
     }
   }
+  }
 }
 
 // Output layer backward over a tile: loss = mean over N*6 of (out - target)^2;
@@ -232,6 +291,7 @@ __global__ void __launch_bounds__(kThreads) out_bwd(const float* __restrict__ ou
                                                     const __nv_bfloat16* __restrict__ h3,
                                                     const __nv_bfloat16* __restrict__ Wo, float* __restrict__ dh3,
                                                     float* __restrict__ part, double* __restrict__ loss_part, int N) {
+  after_previous();
   __shared__ float sdy[kTileNodes * kOut];
   __shared__ float sh[kTileNodes * kHid];
   __shared__ float sW[kOut * kHid];
@@ -284,103 +344,238 @@ __global__ void __launch_bounds__(kThreads) out_bwd(const float* __restrict__ ou
   }
 }
 
-// Hidden layer backward over a tile: dz = dh * (h > 0); partial gradients of
-// W (DOUT x 2 DIN) and b; dcat = W^T dz (FP32, [N][2 DIN]).
-template <int DIN, bool FIRST>
-__global__ void __launch_bounds__(kThreads) layer_bwd(const void* in_, const int* __restrict__ nbr,
-                                                      const float* __restrict__ inv_deg,
-                                                      const __nv_bfloat16* __restrict__ W,
-                                                      const __nv_bfloat16* __restrict__ h,
-                                                      const float* __restrict__ dh, float* __restrict__ dcat,
-                                                      float* __restrict__ part, int N) {
-  constexpr int CAT = 2 * DIN, DOUT = kHid;
-  extern __shared__ float smem[];
+// Hidden layer backward: dz = dh * (h > 0); partial gradients of W (DOUT x 2 DIN)
+// and b; dcat = W^T dz (FP32, [N][2 DIN]; not for the first layer, whose
+// inputs have no gradient).  TOP: dh is given; else it is gathered from the next
+// layer's dcat: dh_j = dcat_j[0:64] + sum over the nodes i that list j (reverse
+// graph, fixed order) of inv_deg_i * dcat_i[64:128].
+// A CTA takes consecutive tiles of 32 nodes and keeps its part of dW in
+// registers, so a partial is written per CTA (at most kBwdCtas).  Both products
+// are register tiles over shared memory, 32 (dW) and 16 (dcat) FMAs to three and two
+// 16-byte loads: for 16384 nodes a layer takes 25-31 us; with one output per
+// thread (two loads to an FMA) it took 75, and 9 for the gather as a launch of
+// its own.  What bounds it now is the gathers' latency before each tile.
+constexpr int kBwdCtas = 296;
+struct BwdArgs {
+  const void* in;
+  const int* nbr;
+  const float* inv_deg;
+  const __nv_bfloat16* W;
+  const __nv_bfloat16* h;
+  const float* dh;         // TOP: [N][64]
+  const float* dnext;      // else: [N][128], with the reverse graph
+  const int* rev_ptr;
+  const int* rev_idx;
+  float* dcat;
+  float* part;
+  int N;
+};
+template <int DIN>
+struct BwdShape {
+  static constexpr int CAT = 2 * DIN, DOUT = kHid;
+  static constexpr int TU = CAT == 128 ? 4 : 2, TK = CAT == 128 ? 8 : 5;  // a thread's part of dW
+  static constexpr int KG = CAT / TK;                                     // threads across k
+  static constexpr int ZS = DOUT + 4;                                     // row stride of sZ
+  static_assert((DOUT / TU) * KG == kThreads, "one part per thread");
+  static constexpr int SMEM = (DOUT * CAT + kTileNodes * (CAT + ZS + DOUT)) * 4;
+};
+template <int DIN, bool FIRST, bool TOP>
+__global__ void __launch_bounds__(kThreads) layer_bwd(const BwdArgs a) {
+  using S = BwdShape<DIN>;
+  constexpr int CAT = S::CAT, DOUT = S::DOUT, TU = S::TU, TK = S::TK, KG = S::KG, ZS = S::ZS;
+  extern __shared__ __align__(16) float smem[];
   float* sW = smem;                       // [DOUT][CAT]
   float* sX = sW + DOUT * CAT;            // [32][CAT]
-  float* sZ = sX + kTileNodes * CAT;      // [32][DOUT]
-  const int n0 = blockIdx.x * kTileNodes;
-  for (int k = threadIdx.x; k < DOUT * CAT; k += kThreads) sW[k] = bf(W[k]);
-  auto load_in = [&](int i, int k) -> float {
-    if (FIRST) return bf(tobf(reinterpret_cast<const float*>(in_)[(size_t)i * DIN + k]));
-    return bf(reinterpret_cast<const __nv_bfloat16*>(in_)[(size_t)i * DIN + k]);
-  };
-  for (int e = threadIdx.x; e < kTileNodes * DIN; e += kThreads) {
-    const int s = e / DIN, k = e % DIN, i = n0 + s;
-    float v = 0.f, a = 0.f;
-    if (i < N) {
-      v = load_in(i, k);
+  float* sZ = sX + kTileNodes * CAT;      // [32][ZS]
+  float* sT = sZ + kTileNodes * ZS;       // [DOUT][32], its transpose
+  const int tid = threadIdx.x, N = a.N;
+  if (!FIRST)
+    for (int k = tid; k < DOUT * CAT / 4; k += kThreads)
+      reinterpret_cast<float4*>(sW)[k] = bf4(__ldg(reinterpret_cast<const uint2*>(a.W) + k));
+  after_previous();  // (the weights are older)
+  const int tk = tid % KG, u0 = tid / KG * TU;
+  // a thread's columns: two runs of four (CAT 128), or five
+  auto col = [&](int c) { return CAT == 128 ? 4 * tk + (c & 3) + (c >> 2) * 64 : TK * tk + c; };
+  float g[TU][TK], gb[TU];
 #pragma unroll
-      for (int q = 0; q < CF_K_GRAPH; q++) {
-        const int j = nbr[(size_t)i * CF_K_GRAPH + q];
-        if (j >= 0) a += load_in(j, k);
+  for (int u = 0; u < TU; u++) {
+    gb[u] = 0.f;
+#pragma unroll
+    for (int c = 0; c < TK; c++) g[u][c] = 0.f;
+  }
+  const int tiles = (N + kTileNodes - 1) / kTileNodes, per = (tiles + gridDim.x - 1) / gridDim.x;
+  const int t1 = min(tiles, ((int)blockIdx.x + 1) * per);
+  for (int tile = blockIdx.x * per; tile < t1; tile++) {
+    const int n0 = tile * kTileNodes;
+    __syncthreads();
+    // the inputs and their neighbour means
+    if constexpr (FIRST) {
+      const float* in = reinterpret_cast<const float*>(a.in);
+      for (int e = tid; e < kTileNodes * DIN / 4; e += kThreads) {  // (the caller's rows: single loads, all in flight)
+        const int s = e / (DIN / 4), k = 4 * (e % (DIN / 4)), i = n0 + s;
+        float v[4] = {}, m[4] = {};
+        if (i < N) {
+          const int4 l0 = __ldg(reinterpret_cast<const int4*>(a.nbr + (size_t)i * CF_K_GRAPH)),
+                     l1 = __ldg(reinterpret_cast<const int4*>(a.nbr + (size_t)i * CF_K_GRAPH) + 1);
+          const int jn[CF_K_GRAPH] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+          float x[CF_K_GRAPH][4];
+#pragma unroll
+          for (int q = 0; q < CF_K_GRAPH; q++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) x[q][c] = jn[q] >= 0 ? in[(size_t)jn[q] * DIN + k + c] : 0.f;
+          const float d = a.inv_deg[i];
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            v[c] = bf(tobf(in[(size_t)i * DIN + k + c]));
+#pragma unroll
+            for (int q = 0; q < CF_K_GRAPH; q++)
+              if (jn[q] >= 0) m[c] += bf(tobf(x[q][c]));
+            m[c] *= d;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          sX[s * CAT + k + c] = v[c];
+          sX[s * CAT + DIN + k + c] = m[c];
+        }
       }
-      a *= inv_deg[i];
-    }
-    sX[s * CAT + k] = v;
-    sX[s * CAT + DIN + k] = a;
-  }
-  for (int e = threadIdx.x; e < kTileNodes * DOUT; e += kThreads) {
-    const int i = n0 + e / DOUT;
-    float z = 0.f;
-    if (i < N) {
-      const size_t o = (size_t)i * DOUT + e % DOUT;
-      z = bf(h[o]) > 0.f ? dh[o] : 0.f;
-    }
-    sZ[e] = z;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < kTileNodes * CAT; e += kThreads) {
-    const int s = e / CAT, k = e % CAT, i = n0 + s;
-    if (i >= N) continue;
-    float a = 0.f;
-#pragma unroll 8
-    for (int u = 0; u < DOUT; u++) a = fmaf(sW[u * CAT + k], sZ[s * DOUT + u], a);
-    dcat[(size_t)i * CAT + k] = a;
-  }
-  float* p = part + (size_t)blockIdx.x * (DOUT * CAT + DOUT);
-  for (int q = threadIdx.x; q < DOUT * CAT + DOUT; q += kThreads) {
-    float a = 0.f;
-    if (q < DOUT * CAT) {
-      const int u = q / CAT, k = q % CAT;
-      for (int s = 0; s < kTileNodes; s++) a = fmaf(sZ[s * DOUT + u], sX[s * CAT + k], a);
     } else {
-      for (int s = 0; s < kTileNodes; s++) a += sZ[s * DOUT + (q - DOUT * CAT)];
+      const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(a.in);
+#pragma unroll
+      for (int e = tid; e < kTileNodes * DIN / 4; e += kThreads) {
+        const int s = e / (DIN / 4), k = 4 * (e % (DIN / 4)), i = n0 + s;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), m = v;
+        if (i < N) {
+          v = bf4(*reinterpret_cast<const uint2*>(in + (size_t)i * DIN + k));
+          m = mean_of<DIN>(in, a.nbr, a.inv_deg, i, k);
+        }
+        *reinterpret_cast<float4*>(sX + s * CAT + k) = v;
+        *reinterpret_cast<float4*>(sX + s * CAT + DIN + k) = m;
+      }
     }
-    p[q] = a;
+#pragma unroll
+    for (int e = tid; e < kTileNodes * DOUT / 4; e += kThreads) {
+      const int s = e / (DOUT / 4), k = 4 * (e % (DOUT / 4)), i = n0 + s;
+      float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < N) {
+        if (TOP) {
+          z = *reinterpret_cast<const float4*>(a.dh + (size_t)i * DOUT + k);
+        } else {
+          z = __ldg(reinterpret_cast<const float4*>(a.dnext + (size_t)i * 2 * DOUT + k));
+          const int q1 = a.rev_ptr[i + 1];
+#pragma unroll 4
+          for (int q = a.rev_ptr[i]; q < q1; q++) {
+            const int j = __ldg(a.rev_idx + q);
+            const float w = __ldg(a.inv_deg + j);
+            const float4 d = __ldg(reinterpret_cast<const float4*>(a.dnext + (size_t)j * 2 * DOUT + DOUT + k));
+            z.x = fmaf(w, d.x, z.x);
+            z.y = fmaf(w, d.y, z.y);
+            z.z = fmaf(w, d.z, z.z);
+            z.w = fmaf(w, d.w, z.w);
+          }
+        }
+        const float4 h = bf4(*reinterpret_cast<const uint2*>(a.h + (size_t)i * DOUT + k));
+        z.x = h.x > 0.f ? z.x : 0.f;
+        z.y = h.y > 0.f ? z.y : 0.f;
+        z.z = h.z > 0.f ? z.z : 0.f;
+        z.w = h.w > 0.f ? z.w : 0.f;
+      }
+      *reinterpret_cast<float4*>(sZ + s * ZS + k) = z;
+    }
+    __syncthreads();
+    if constexpr (!FIRST) {  // four nodes by four columns per thread
+      for (int e = tid; e < kTileNodes * DOUT; e += kThreads)
+        sT[e] = sZ[e % kTileNodes * ZS + e / kTileNodes];
+      __syncthreads();
+      const int k = 4 * (tid & 31), s0 = 4 * (tid >> 5);
+      float4 o[4];
+#pragma unroll
+      for (int s = 0; s < 4; s++) o[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int u = 0; u < DOUT; u++) {
+        const float4 w = *reinterpret_cast<const float4*>(sW + u * CAT + k);
+        const float4 z = *reinterpret_cast<const float4*>(sT + u * kTileNodes + s0);
+        const float zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          o[s].x = fmaf(w.x, zs[s], o[s].x);
+          o[s].y = fmaf(w.y, zs[s], o[s].y);
+          o[s].z = fmaf(w.z, zs[s], o[s].z);
+          o[s].w = fmaf(w.w, zs[s], o[s].w);
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < 4; s++)
+        if (n0 + s0 + s < N) *reinterpret_cast<float4*>(a.dcat + (size_t)(n0 + s0 + s) * CAT + k) = o[s];
+    }
+#pragma unroll 4
+    for (int s = 0; s < kTileNodes; s++) {
+      float z[TU], x[TK];
+#pragma unroll
+      for (int u = 0; u < TU; u++) z[u] = sZ[s * ZS + u0 + u];
+#pragma unroll
+      for (int c = 0; c < TK; c++) x[c] = sX[s * CAT + col(c)];
+#pragma unroll
+      for (int u = 0; u < TU; u++) {
+        gb[u] += z[u];
+#pragma unroll
+        for (int c = 0; c < TK; c++) g[u][c] = fmaf(z[u], x[c], g[u][c]);
+      }
+    }
+  }
+  float* p = a.part + (size_t)blockIdx.x * (DOUT * CAT + DOUT);
+#pragma unroll
+  for (int u = 0; u < TU; u++) {
+#pragma unroll
+    for (int c = 0; c < TK; c++) p[(u0 + u) * CAT + col(c)] = g[u][c];
+    if (tk == 0) p[DOUT * CAT + u0 + u] = gb[u];
   }
 }
 
-// d in_j = dcat_j[0:DIN] + sum over the nodes i that list j (reverse graph,
-// fixed order) of inv_deg_i * dcat_i[DIN:2 DIN]
-template <int DIN>
-__global__ void grad_gather(const float* __restrict__ dcat, const int* __restrict__ rev_ptr,
-                            const int* __restrict__ rev_idx, const float* __restrict__ inv_deg,
-                            float* __restrict__ din, int N) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= N * DIN) return;
-  const int j = e / DIN, k = e % DIN;
-  float a = dcat[(size_t)j * 2 * DIN + k];
-  for (int q = rev_ptr[j]; q < rev_ptr[j + 1]; q++) {
-    const int i = rev_idx[q];
-    a = fmaf(inv_deg[i], dcat[(size_t)i * 2 * DIN + DIN + k], a);
+// The gradients of all layers: grad[p] = sum over CTAs of part[cta][p], 32 values
+// per CTA and eight threads to a value (each a run of the CTAs, then in order);
+// the last CTA adds the loss.  One launch of short sums for all layers instead
+// of one per layer, whose threads each added all CTAs' values: 8 us against four
+// times 20 at 16384 nodes.
+struct ReduceArgs {
+  const float* part[4];
+  float* grad[4];
+  int ctas[4], np[4], first[5];  // first: the first CTA of each layer's
+  const double* loss_part;
+  double* loss;
+  int loss_n, N;
+};
+__global__ void __launch_bounds__(kThreads) reduce_parts(const ReduceArgs r) {
+  after_previous();
+  __shared__ float s_sum[8][32];
+  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  const int b = blockIdx.x;
+  if (b == r.first[4]) {
+    if (sl) return;
+    double a = 0.0;
+    for (int k = lane; k < r.loss_n; k += 32) a += r.loss_part[k];
+    a = warp_sum_d(a);
+    if (lane == 0) *r.loss = a / (6.0 * r.N);
+    return;
   }
-  din[e] = a;
-}
-
-// grad[p] = sum over CTAs (in order) of part[cta][p]
-__global__ void reduce_parts(const float* __restrict__ part, int ctas, int np, float* __restrict__ grad) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= np) return;
+  int L = 0;
+#pragma unroll
+  for (int l = 1; l < 4; l++) L = b >= r.first[l] ? l : L;
+  const int np = r.np[L], n = r.ctas[L], q = (b - r.first[L]) * 32 + lane;
   float a = 0.f;
-  for (int c = 0; c < ctas; c++) a += part[(size_t)c * np + q];
-  grad[q] = a;
-}
-
-__global__ void reduce_loss(const double* __restrict__ part, int n, double* __restrict__ out, int N) {
-  double a = 0.0;
-  for (int k = threadIdx.x; k < n; k += 32) a += part[k];
-  a = warp_sum_d(a);
-  if (threadIdx.x == 0) *out = a / (6.0 * N);
+  if (q < np) {
+    const float* p = r.part[L] + q;
+    const int c1 = n * (sl + 1) / 8;
+#pragma unroll 8
+    for (int c = n * sl / 8; c < c1; c++) a += p[(size_t)c * np];
+  }
+  s_sum[sl][lane] = a;
+  __syncthreads();
+  if (sl == 0 && q < np) {
+#pragma unroll
+    for (int k = 1; k < 8; k++) a += s_sum[k][lane];
+    r.grad[L][q] = a;
+  }
 }
 
 // Adam (FP32 master weights), then the BF16 copy
@@ -565,8 +760,6 @@ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 int mpnn_param_count() { return kParams; }
 
-static int layer_bwd_smem(int din) { return (kHid * 2 * din + kTileNodes * 2 * din + kTileNodes * kHid) * 4; }
-
 template <typename T>
 static cudaError_t alloc_n(T** p, size_t n) {
   *p = nullptr;
@@ -587,8 +780,8 @@ cudaError_t mpnn_alloc(Mpnn& m, int max_nodes) {
   if ((e = cudaMalloc(&m.h1, sizeof(__nv_bfloat16) * N * kHid)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&m.h2, sizeof(__nv_bfloat16) * N * kHid)) != cudaSuccess) return e;
   if ((e = cudaMalloc(&m.h3, sizeof(__nv_bfloat16) * N * kHid)) != cudaSuccess) return e;
-  A_(m.dh, N * kHid); A_(m.dh2, N * kHid); A_(m.dcat, N * 2 * kHid);
-  A_(m.part, (size_t)ctas * (kHid * 2 * kHid + kHid)); A_(m.loss_part, (size_t)ctas); A_(m.loss, 1);
+  A_(m.dh, N * kHid); A_(m.dcat, N * 2 * kHid); A_(m.dcat2, N * 2 * kHid);
+  A_(m.part, (size_t)ctas * (kOut * kHid + kOut) + (size_t)min(ctas, kBwdCtas) * kWo); A_(m.loss_part, (size_t)ctas); A_(m.loss, 1);
 #undef A_
   if ((e = cudaMemset(m.m, 0, sizeof(float) * kParams)) != cudaSuccess) return e;
   return cudaMemset(m.v, 0, sizeof(float) * kParams);
@@ -596,7 +789,7 @@ cudaError_t mpnn_alloc(Mpnn& m, int max_nodes) {
 
 void mpnn_free(Mpnn& m) {
   void* ps[] = {m.w, m.m, m.v, m.g, m.wb, m.nbr, m.inv_deg, m.rev_ptr, m.rev_idx, m.feat, m.tgt, m.out,
-                m.h1, m.h2, m.h3, m.dh, m.dh2, m.dcat, m.part, m.loss_part, m.loss};
+                m.h1, m.h2, m.h3, m.dh, m.dcat, m.dcat2, m.part, m.loss_part, m.loss};
   for (void* p : ps)
     if (p) cudaFree(p);
   m = Mpnn();
@@ -617,7 +810,8 @@ cudaError_t mpnn_graph_from_nodes(Mpnn& m, const cf_deform_node* nodes, int N, c
 cudaError_t mpnn_forward(const Mpnn& m, const float* feat, float* out, cudaStream_t s) {
   const int N = m.N;
   if (N <= 0) return cudaSuccess;
-  const int g = cdiv(N, kFwdTile);
+  // tiles share the weights past four CTAs per SM
+  const int g = min(cdiv(N, kFwdTile), 4 * 148);
   const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(m.wb);
   const int s0 = FwdShape<kIn, kHid, true>::SMEM, s1 = FwdShape<kHid, kHid, true>::SMEM,
             so = FwdShape<kHid, kOut, false>::SMEM;
@@ -640,32 +834,78 @@ cudaError_t mpnn_forward(const Mpnn& m, const float* feat, float* out, cudaStrea
 cudaError_t mpnn_gradients(Mpnn& m, const float* feat, const float* tgt, cudaStream_t s) {
   const int N = m.N;
   if (N <= 0) return cudaSuccess;
-  const int g = cdiv(N, kTileNodes);
+  const int g = cdiv(N, kTileNodes), gb = min(g, kBwdCtas);
   cudaError_t e = mpnn_forward(m, feat, m.out, s);
   if (e != cudaSuccess) return e;
   const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(m.wb);
-  out_bwd<<<g, kThreads, 0, s>>>(m.out, tgt, reinterpret_cast<const __nv_bfloat16*>(m.h3), wb + kWo, m.dh, m.part,
-                                 m.loss_part, N);
-  reduce_parts<<<cdiv(kOut * kHid + kOut, 128), 128, 0, s>>>(m.part, g, kOut * kHid + kOut, m.g + kWo);
-  reduce_loss<<<1, 32, 0, s>>>(m.loss_part, g, m.loss, N);
-  const int sm64 = layer_bwd_smem(kHid), sm20 = layer_bwd_smem(kIn);
-  if ((e = cudaFuncSetAttribute(layer_bwd<kHid, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64)) !=
-      cudaSuccess)
+  const int smem = BwdShape<kHid>::SMEM;
+  if ((e = cudaFuncSetAttribute(layer_bwd<kHid, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) !=
+          cudaSuccess ||
+      (e = cudaFuncSetAttribute(layer_bwd<kHid, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) !=
+          cudaSuccess)
     return e;
+  constexpr int nh = kHid * 2 * kHid + kHid, n0 = kHid * 2 * kIn + kHid, no = kOut * kHid + kOut;
+  float* part2 = m.part + (size_t)g * no;
+  float* part1 = part2 + (size_t)gb * nh;
+  float* part0 = part1 + (size_t)gb * nh;
+  // With more tiles than SMs the kernels are long enough to hide a launch, and
+  // CTAs let in early settle unevenly (16384 nodes: 202 us, 216 with launch_next
+  // throughout; 2048 nodes: 130 and 119).
+  auto run = [&](auto kernel, int grid, int sm, auto... args) {
+    if (g <= 148)
+      launch_next(kernel, grid, kThreads, sm, s, args...);
+    else
+      kernel<<<grid, kThreads, sm, s>>>(args...);
+  };
+  run(out_bwd, g, 0, m.out, tgt, reinterpret_cast<const __nv_bfloat16*>(m.h3), wb + kWo, m.dh, m.part, m.loss_part, N);
+  BwdArgs a = {};
+  a.nbr = m.nbr;
+  a.inv_deg = m.inv_deg;
+  a.rev_ptr = m.rev_ptr;
+  a.rev_idx = m.rev_idx;
+  a.N = N;
   // layer 3 (h2 -> h3)
-  layer_bwd<kHid, false><<<g, kThreads, sm64, s>>>(m.h2, m.nbr, m.inv_deg, wb + kW2,
-                                                   reinterpret_cast<const __nv_bfloat16*>(m.h3), m.dh, m.dcat, m.part, N);
-  reduce_parts<<<cdiv(kHid * 2 * kHid + kHid, 128), 128, 0, s>>>(m.part, g, kHid * 2 * kHid + kHid, m.g + kW2);
-  grad_gather<kHid><<<cdiv(N * kHid, 256), 256, 0, s>>>(m.dcat, m.rev_ptr, m.rev_idx, m.inv_deg, m.dh2, N);
+  a.in = m.h2;
+  a.W = wb + kW2;
+  a.h = reinterpret_cast<const __nv_bfloat16*>(m.h3);
+  a.dh = m.dh;
+  a.dcat = m.dcat;
+  a.part = part2;
+  run(layer_bwd<kHid, false, true>, gb, smem, a);
   // layer 2 (h1 -> h2)
-  layer_bwd<kHid, false><<<g, kThreads, sm64, s>>>(m.h1, m.nbr, m.inv_deg, wb + kW1,
-                                                   reinterpret_cast<const __nv_bfloat16*>(m.h2), m.dh2, m.dcat, m.part, N);
-  reduce_parts<<<cdiv(kHid * 2 * kHid + kHid, 128), 128, 0, s>>>(m.part, g, kHid * 2 * kHid + kHid, m.g + kW1);
-  grad_gather<kHid><<<cdiv(N * kHid, 256), 256, 0, s>>>(m.dcat, m.rev_ptr, m.rev_idx, m.inv_deg, m.dh, N);
+  a.in = m.h1;
+  a.W = wb + kW1;
+  a.h = reinterpret_cast<const __nv_bfloat16*>(m.h2);
+  a.dnext = m.dcat;
+  a.dcat = m.dcat2;
+  a.part = part1;
+  run(layer_bwd<kHid, false, false>, gb, smem, a);
   // layer 1 (x -> h1)
-  layer_bwd<kIn, true><<<g, kThreads, sm20, s>>>(feat, m.nbr, m.inv_deg, wb + kW0,
-                                                 reinterpret_cast<const __nv_bfloat16*>(m.h1), m.dh, m.dcat, m.part, N);
-  reduce_parts<<<cdiv(kHid * 2 * kIn + kHid, 128), 128, 0, s>>>(m.part, g, kHid * 2 * kIn + kHid, m.g + kW0);
+  a.in = feat;
+  a.W = wb + kW0;
+  a.h = reinterpret_cast<const __nv_bfloat16*>(m.h1);
+  a.dnext = m.dcat2;
+  a.dcat = nullptr;
+  a.part = part0;
+  run(layer_bwd<kIn, true, false>, gb, BwdShape<kIn>::SMEM, a);
+  ReduceArgs r = {};
+  const float* parts[4] = {part0, part1, part2, m.part};
+  const int nps[4] = {n0, nh, nh, no}, at[4] = {kW0, kW1, kW2, kWo};
+  int first = 0;
+  for (int l = 0; l < 4; l++) {
+    r.part[l] = parts[l];
+    r.grad[l] = m.g + at[l];
+    r.ctas[l] = l < 3 ? gb : g;
+    r.np[l] = nps[l];
+    r.first[l] = first;
+    first += cdiv(nps[l], 32);
+  }
+  r.first[4] = first;
+  r.loss_part = m.loss_part;
+  r.loss = m.loss;
+  r.loss_n = g;
+  r.N = N;
+  run(reduce_parts, first + 1, 0, r);
   return cudaGetLastError();
 }
 
