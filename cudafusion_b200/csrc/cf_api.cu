@@ -2105,7 +2105,7 @@ cf_status cf_scale_delta(const float* d_delta_x, int num_nodes, float max_rot, f
 cf_status cf_correspondence_rmse(const cf_correspondence* d_corrs, int num_corrs, double* d_partials, double* d_out,
                                  void* stream) {
   if (num_corrs < 0 || !d_partials || !d_out || (num_corrs > 0 && !d_corrs)) return CF_ERR_INVALID_ARG;
-  CF_TRY(launch_corr_rmse(d_corrs, num_corrs, d_partials, d_out, nullptr, (cudaStream_t)stream));
+  CF_TRY(launch_corr_rmse(d_corrs, num_corrs, d_partials, d_out, (cudaStream_t)stream));
   return CF_OK;
 }
 
@@ -2145,13 +2145,15 @@ cf_status cf_line_search(cf_raster* raster, cf_corr_search* search, const float*
   double* partials = d_scratch_rmse;
   double* slots = d_scratch_rmse + 2 * CF_RMSE_BLOCKS;
   cf_status st = CF_OK;
-  // one trial, or the final application: restore, scale, apply, predict, search
+  // the saved transforms with the increment at a scale
+  auto transforms = [&](float scale) -> cf_status {
+    if (num_nodes > 0 && (reinterpret_cast<uintptr_t>(d_transforms) & 15u)) return CF_ERR_INVALID_ARG;
+    return from_cuda(launch_trial_transforms(d_scratch_transforms, d_delta_x, num_nodes, params->max_update_rot,
+                                             params->max_update_trans, scale, d_scratch_delta, d_transforms, s));
+  };
+  // one trial, or the final application: transforms, predict, search
   auto apply = [&](float scale) -> cf_status {
-    cf_status r = from_cuda(cudaMemcpyAsync(d_transforms, d_scratch_transforms, tbytes, cudaMemcpyDeviceToDevice, s));
-    if (r == CF_OK) r = cf_scale_delta(d_delta_x, num_nodes, params->max_update_rot, params->max_update_trans, scale,
-                                       d_scratch_delta, stream);
-    if (r == CF_OK) r = cf_warp_apply_twist(d_transforms, d_scratch_delta, num_nodes, params->max_update_rot,
-                                            params->max_update_trans, 1.0f, stream);
+    cf_status r = transforms(scale);
     if (r == CF_OK) r = cf_predict_live_surface(raster, d_mesh_canonical, d_mesh_warped, d_mesh_triangles,
                                                 num_vertices, num_triangles, d_nodes, d_transforms, num_nodes,
                                                 d_voxel_knn, d_voxel_knn_w, cam, T_cam_world, grid, lv, ln, hit,
@@ -2214,8 +2216,10 @@ cf_status cf_line_search(cf_raster* raster, cf_corr_search* search, const float*
   CF_TRY(cudaMemcpyAsync(d_scratch_transforms, d_transforms, tbytes, cudaMemcpyDeviceToDevice, s));  // save
   for (int t = 0; t < CF_LINE_SEARCH_TRIALS && st == CF_OK; ++t) {
     st = apply(scales[t]);
-    if (st == CF_OK) st = from_cuda(launch_corr_rmse(d_corrs, P, partials, slots + 3 * t, d_num_valid, s));
+    if (st == CF_OK) st = from_cuda(launch_corr_rmse(d_corrs, P, partials, nullptr, s));
     if (st == CF_OK) {
+      ka.part = partials;
+      ka.valid = d_num_valid;
       ka.slot = slots + 3 * t;
       ka.best_in = t > 0 ? best_chain + t : nullptr;
       ka.best_out = best_chain + t + 1;
@@ -2251,12 +2255,7 @@ cf_status cf_line_search(cf_raster* raster, cf_corr_search* search, const float*
   } else if (h_kept == best_t) {
     // the accepted trial's transforms (as apply computes them), its skinned
     // mesh (the prediction's skinning launches), its records and maps
-    CF_TRY(cudaMemcpyAsync(d_transforms, d_scratch_transforms, tbytes, cudaMemcpyDeviceToDevice, s));
-    st = cf_scale_delta(d_delta_x, num_nodes, params->max_update_rot, params->max_update_trans, *best_scale,
-                        d_scratch_delta, stream);
-    if (st == CF_OK) st = cf_warp_apply_twist(d_transforms, d_scratch_delta, num_nodes, params->max_update_rot,
-                                              params->max_update_trans, 1.0f, stream);
-    if (st != CF_OK) return st;
+    if ((st = transforms(*best_scale)) != CF_OK) return st;
     RasterCall c{};
     c.skin = true;
     c.canon = d_mesh_canonical;

@@ -1185,17 +1185,18 @@ float sqrt_bound(float cap) {
 }  // namespace
 
 // Row chunks per tile.  Rough model in SM clocks, from 640 x 480 at radii 8, 20
-// and 50 with 1 to 8 chunks: a CTA's set-up takes 9000, its scan of 512 pixels x
-// S/C candidates goes at 9 per clock (3 CTAs per SM), the CTAs run in
-// ceil(tiles x C / slots) waves, and the merge reads each chunk for 5000.
+// and 50 and 320 x 240 at 20, each with 1 to 8 chunks: a CTA's set-up takes 9000,
+// its scan of 512 pixels x S/C candidates goes at 9 per clock beside two others,
+// the last CTAs run with fewer beside them, so the waves count as
+// tiles x C / slots + 0.4; the merge reads each chunk for 5000 at 640 x 480.
 int corr_pick_chunks(int tiles, int sms, int radius, int W, int H) {
   const double slots = (double)(sms > 0 ? sms : 1) * kCsCtasPerSm;
   const double side_x = std::fmin(2.0 * radius + 8.0, (double)W), side_y = std::fmin(2.0 * radius + 8.0, (double)H);
-  const double scan = 512.0 * side_x * side_y / 9.0;
+  const double scan = 512.0 * side_x * side_y / 9.0, merge = 5000.0 * ((double)W * H / 307200.0);
   int best_c = 1;
   double best = 1e300;
   for (int c = 1; c <= kCorrMaxChunks; ++c) {
-    const double t = std::ceil((double)tiles * c / slots) * (9000.0 + scan / c) + 5000.0 * c;
+    const double t = ((double)tiles * c / slots + 0.4) * (9000.0 + scan / c) + merge * c;
     if (t < best * (1.0 - 1e-9)) {
       best = t;
       best_c = c;

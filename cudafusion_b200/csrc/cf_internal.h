@@ -313,7 +313,9 @@ cudaError_t launch_scale_delta(const float* dx, int N, float max_rot, float max_
                                cudaStream_t s);
 // The line search's record of its best trial (ls_keep_kernel).
 struct LsKeepArgs {
-  const double* slot;
+  const double* part;  // the trial's block sums
+  const int* valid;    // and valid count
+  double* slot;        // where both go
   const double* best_in;  // nullptr: best0
   double best0;
   double* best_out;
@@ -324,8 +326,10 @@ struct LsKeepArgs {
   size_t words[8];
 };
 cudaError_t launch_ls_keep(const LsKeepArgs& a, cudaStream_t s);
-cudaError_t launch_corr_rmse(const cf_correspondence* corrs, int M, double* partials, double* out, const int* valid,
-                             cudaStream_t s);
+// out: nullptr leaves the block sums alone
+cudaError_t launch_corr_rmse(const cf_correspondence* corrs, int M, double* partials, double* out, cudaStream_t s);
+cudaError_t launch_trial_transforms(const cf_dual_quat* saved, const float* dx, int N, float max_rot, float max_trans,
+                                    float scale, float* delta, cf_dual_quat* T, cudaStream_t s);
 cudaError_t launch_tsdf_plain(const cf_deform_node* nodes, const cf_dual_quat* T, cf_dual_quat* plain, int N,
                               cudaStream_t s);
 cudaError_t launch_tsdf_integrate(float* vox, const cf_tsdf_params* p, const float* depth, const cf_camera* cam,

@@ -10,6 +10,7 @@
 // without a host round trip (cf_line_search in cf_api.cu drives it).
 #include <cmath>
 
+#include "cf_device.cuh"
 #include "cf_internal.h"
 
 namespace cf {
@@ -84,22 +85,62 @@ __global__ void __launch_bounds__(kLsThreads) update_stats_kernel(const float* _
 // upload_scaled_delta_x (fusion_app.h:1352-1375): per node rs = max_rot / rn
 // when rn exceeds a positive max_rot (else 1), ts likewise, then
 // dx[k] * (rs * scale) and dx[k] * (ts * scale).
-__global__ void scale_delta_kernel(const float* __restrict__ dx, int N, float max_rot, float max_trans, float scale,
-                                   float* __restrict__ out) {
-  after_previous();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const float* d = dx + 6 * (size_t)i;
+__device__ __forceinline__ void ls_scale(const float* __restrict__ d, float max_rot, float max_trans, float scale,
+                                         float (&o)[6]) {
   const float rn = ls_norm3(d[0], d[1], d[2]), tn = ls_norm3(d[3], d[4], d[5]);
   float rs = 1.f, ts = 1.f;
   if (max_rot > 0.f && rn > max_rot) rs = __fdiv_rn(max_rot, rn);
   if (max_trans > 0.f && tn > max_trans) ts = __fdiv_rn(max_trans, tn);
   const float fr = __fmul_rn(rs, scale), ft = __fmul_rn(ts, scale);
-  float* o = out + 6 * (size_t)i;
 #pragma unroll
   for (int k = 0; k < 3; ++k) o[k] = __fmul_rn(d[k], fr);
 #pragma unroll
   for (int k = 3; k < 6; ++k) o[k] = __fmul_rn(d[k], ft);
+}
+__global__ void scale_delta_kernel(const float* __restrict__ dx, int N, float max_rot, float max_trans, float scale,
+                                   float* __restrict__ out) {
+  after_previous();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  float o[6];
+  ls_scale(dx + 6 * (size_t)i, max_rot, max_trans, scale, o);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) out[6 * (size_t)i + k] = o[k];
+}
+
+// A trial's transforms: the saved ones with the scaled increment applied (the
+// restore, scale_delta and apply_twist of the host flow, in one launch: the
+// copy and two launches took 8 us a trial, this 3).
+__global__ void trial_transforms_kernel(const cf_dual_quat* __restrict__ saved, const float* __restrict__ dx, int N,
+                                        float max_rot, float max_trans, float scale, float* __restrict__ delta,
+                                        cf_dual_quat* __restrict__ T) {
+  after_previous();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  float o[6];
+  ls_scale(dx + 6 * (size_t)i, max_rot, max_trans, scale, o);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) delta[6 * (size_t)i + k] = o[k];
+  const float* q = reinterpret_cast<const float*>(saved + i);  // (the caller's scratch: whole floats)
+  DQ t;
+  t.r = make_float4(q[0], q[1], q[2], q[3]);
+  t.d = make_float4(q[4], q[5], q[6], q[7]);
+  store_dq(T + i, twist_update(t, o, max_rot, max_trans, 1.f));
+}
+
+// v[0] + v[1] + ... in order, by one thread, the reads ahead of the adds.
+__device__ __forceinline__ double ls_sum(const double* v, int n) {
+  double s = 0.0;
+  int j = 0;
+  for (; j + 16 <= n; j += 16) {
+    double x[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = v[j + k];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s += x[k];
+  }
+  for (; j < n; ++j) s += v[j];
+  return s;
 }
 
 // correspondence_rmse's sums (fusion_app.h:1336-1347): block b sums the
@@ -125,41 +166,46 @@ __global__ void __launch_bounds__(kLsThreads) rmse_partial_kernel(const cf_corre
   sh[0][threadIdx.x] = s;
   sh[1][threadIdx.x] = ws;
   __syncthreads();
-  if (threadIdx.x < 2) {
-    double v = 0.0;
-    for (int j = 0; j < kLsThreads; ++j) v += sh[threadIdx.x][j];
-    part[2 * blockIdx.x + threadIdx.x] = v;
-  }
+  if (threadIdx.x < 2) part[2 * blockIdx.x + threadIdx.x] = ls_sum(sh[threadIdx.x], kLsThreads);
 }
 
-// out[0..1] = the block sums in block order; with `valid` also out[2] = the
-// search's valid count (the line search keeps each trial's in its slot).
-__global__ void rmse_final_kernel(const double* __restrict__ part, int blocks, double* __restrict__ out,
-                                  const int* __restrict__ valid) {
+// The block sums in block order, for the whole CTA (256 threads).
+__device__ __forceinline__ void ls_total(const double* __restrict__ part, double (&out)[2]) {
+  __shared__ double sh[2][CF_RMSE_BLOCKS];
+  __shared__ double tot[2];
+  for (int b = threadIdx.x; b < 2 * CF_RMSE_BLOCKS; b += blockDim.x) sh[b & 1][b >> 1] = part[b];
+  __syncthreads();
+  if (threadIdx.x < 2) tot[threadIdx.x] = ls_sum(sh[threadIdx.x], CF_RMSE_BLOCKS);
+  __syncthreads();
+  out[0] = tot[0];
+  out[1] = tot[1];
+}
+__global__ void __launch_bounds__(256) rmse_final_kernel(const double* __restrict__ part, double* __restrict__ out) {
   after_previous();
-  if (threadIdx.x < 2) {
-    double v = 0.0;
-    for (int b = 0; b < blocks; ++b) v += part[2 * b + threadIdx.x];
-    out[threadIdx.x] = v;
-  }
-  if (threadIdx.x == 2 && valid) out[2] = (double)*valid;
+  double t[2];
+  ls_total(part, t);
+  if (threadIdx.x < 2) out[threadIdx.x] = t[threadIdx.x];
 }
 
-// After a trial's RMSE (slot: its sum, wsum and valid count): whether the
-// trial is the best so far under the line search's acceptance rule
-// (fusion_app.h:575-582, the host's arithmetic: IEEE double quotient and
-// square root), chaining the best RMSE from best_in (or best0) to best_out;
-// a kept trial's index goes to *kept and its outputs (4-byte words) are
-// copied aside, so that the accepted trial need not be predicted and searched
-// again.
+// After a trial's records: its sums (every CTA adds the block sums itself;
+// slot: sum, wsum and valid count) and whether the trial is the best so far
+// under the line search's acceptance rule (fusion_app.h:575-582, the host's
+// arithmetic: IEEE double quotient and square root), chaining the best RMSE from
+// best_in (or best0) to best_out; a kept trial's index goes to *kept and its
+// outputs (4-byte words) are copied aside, so that the accepted trial need not
+// be predicted and searched again.
 __global__ void __launch_bounds__(256) ls_keep_kernel(LsKeepArgs a) {
   after_previous();
-  const double sum = a.slot[0], wsum = a.slot[1];
-  const int valid = (int)a.slot[2];
-  const double rmse = wsum > 0.0 ? sqrt(sum / wsum) : (double)INFINITY;
+  double t[2];
+  ls_total(a.part, t);
+  const int valid = *a.valid;
+  const double rmse = t[1] > 0.0 ? sqrt(t[0] / t[1]) : (double)INFINITY;
   const double best = a.best_in ? *a.best_in : a.best0;
   const bool take = valid >= a.min_valid && valid >= a.need && isfinite(rmse) && rmse < best;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.slot[0] = t[0];
+    a.slot[1] = t[1];
+    a.slot[2] = (double)valid;
     *a.best_out = take ? rmse : best;
     if (take) *a.kept = a.trial;
   }
@@ -196,10 +242,16 @@ cudaError_t launch_scale_delta(const float* dx, int N, float max_rot, float max_
   return cudaGetLastError();
 }
 
-cudaError_t launch_corr_rmse(const cf_correspondence* corrs, int M, double* partials, double* out, const int* valid,
-                             cudaStream_t s) {
+cudaError_t launch_trial_transforms(const cf_dual_quat* saved, const float* dx, int N, float max_rot, float max_trans,
+                                    float scale, float* delta, cf_dual_quat* T, cudaStream_t s) {
+  if (N <= 0) return cudaSuccess;
+  launch_next(trial_transforms_kernel, (N + 63) / 64, 64, 0, s, saved, dx, N, max_rot, max_trans, scale, delta, T);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_corr_rmse(const cf_correspondence* corrs, int M, double* partials, double* out, cudaStream_t s) {
   launch_next(rmse_partial_kernel, CF_RMSE_BLOCKS, kLsThreads, 0, s, corrs, M, partials);
-  launch_next(rmse_final_kernel, 1, 32, 0, s, partials, CF_RMSE_BLOCKS, out, valid);
+  if (out) launch_next(rmse_final_kernel, 1, 256, 0, s, partials, out);
   return cudaGetLastError();
 }
 
