@@ -122,7 +122,7 @@ void free_work(Work& w) {
   dfree(w.key); dfree(w.order); dfree(w.sorted); dfree(w.npos); dfree(w.sp_src); dfree(w.sp_dst); dfree(w.sp_nrm); dfree(w.sp_uw); dfree(w.task);
   dfree(w.cell_ids); dfree(w.rec); dfree(w.raw); dfree(w.cstat); dfree(w.cl_total); dfree(w.cl_start);
   dfree(w.cl_cur); dfree(w.clist); dfree(w.cdesc); dfree(w.cnt); dfree(w.node_total); dfree(w.inc_start); dfree(w.rhs); dfree(w.plain); dfree(w.x); dfree(w.z); dfree(w.p0); dfree(w.p1);
-  dfree(w.partials); dfree(w.barrier); dfree(w.err); dfree(w.done); dfree(w.e_data_part); dfree(w.e_arap_part); dfree(w.stats); dfree(w.timers);
+  dfree(w.partials); dfree(w.barrier); dfree(w.dots); dfree(w.err); dfree(w.done); dfree(w.e_data_part); dfree(w.e_arap_part); dfree(w.stats); dfree(w.timers);
   dfree(w.nodes_cat); dfree(w.T_cat); dfree(w.r); dfree(w.ap); dfree(w.minv32);
   w.cnt_cap = 0;
 }
@@ -144,10 +144,11 @@ cudaError_t alloc_work(Work& w, int max_nodes, int max_corrs, int bin_ctas_max) 
   A_(w.node_total, N); A_(w.inc_start, N + 1);
   A_(w.cl_total, N); A_(w.cl_start, N + 1); A_(w.cl_cur, N); A_(w.clist, 4 * M); A_(w.cdesc, 4 * M);
   A_(w.rhs, 6 * N); A_(w.plain, N); A_(w.x, 6 * N); A_(w.z, 6 * N); A_(w.p0, 6 * N); A_(w.p1, 6 * N);
-  A_(w.partials, (size_t)2 * 3 * kMaxPcgCtas); A_(w.barrier, (size_t)kMaxPcgCtas); A_(w.err, 1);
+  A_(w.partials, (size_t)2 * 3 * kMaxPcgCtas); A_(w.barrier, (size_t)kMaxPcgCtas); A_(w.dots, (size_t)kMaxPcgCtas * 48); A_(w.err, 1);
   A_(w.e_data_part, (size_t)(kMaxEnergyCtas + kMaxProblems)); A_(w.e_arap_part, N); A_(w.stats, (size_t)kMaxProblems);
   A_(w.timers, (size_t)kTimerSlots); A_(w.done, 1);
 #undef A_
+  if ((e = cudaMemset(w.dots, 0, sizeof(unsigned long long) * (size_t)kMaxPcgCtas * 48)) != cudaSuccess) return e;
   return cudaMemset(w.done, 0, sizeof(unsigned));
 }
 

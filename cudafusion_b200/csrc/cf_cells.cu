@@ -1040,7 +1040,11 @@ __global__ void __launch_bounds__(32 * kRowWarps) gather_kernel(Work w, Pattern 
     if (tid >= 32 && tid - 32 <= kn) m.edge[tid - 32] = __ldg(pt.arap_blk_ptr + u0 + 1 + k0 + tid - 32);
     for (int i = lane; i < kn * kSums; i += 32) (&m.sum[wid][0][0])[i] = 0.f;
     __syncthreads();
-    if (k0 == 0) after_previous();  // (so far the pattern and the lists)
+    if (k0 == 0) {
+      after_previous();  // (so far the pattern and the lists)
+      if (r == 0)  // the barriers of the PCG that follows
+        for (int i = tid; i < pt.P; i += kRowThreads) w.barrier[i] = 0u;
+    }
     float(*sum)[kSums] = m.sum[wid];
     for (int i0 = b0; i0 < b1; i0 += 32) {
       // a lane per task: the run, and the pass's blocks of the nodes after the row's

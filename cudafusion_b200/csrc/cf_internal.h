@@ -177,7 +177,8 @@ struct Work {
   float* p0 = nullptr;
   float* p1 = nullptr;
   double* partials = nullptr;  // [2 bufs][3 slots][max pcg ctas]
-  unsigned* barrier = nullptr;  // [max pcg ctas] one arrival counter per PCG CTA group
+  unsigned* barrier = nullptr;  // [max pcg ctas] one arrival counter per PCG CTA group (zeroed by the gather)
+  unsigned long long* dots = nullptr;  // [max pcg ctas][3 lines] per group: exchanged sums (cf_pcg_grid.cu)
   int* err = nullptr;
   unsigned* done = nullptr;       // CTAs of an energy launch that have finished (0 between launches)
   double* e_data_part = nullptr;  // [kMaxEnergyCtas + kMaxProblems] one partial per energy CTA

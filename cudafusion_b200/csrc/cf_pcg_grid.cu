@@ -5,20 +5,22 @@
 // for the whole solve, its block-Jacobi inverses are computed in FP64 in the
 // prologue, and its state vectors never leave shared memory.  Only the
 // exchange vector of the halo (the columns of other CTAs' rows that this
-// CTA's blocks touch, a deduplicated per-CTA list) and the dot-product
-// partials go through global memory, around a fence-free release/acquire
-// grid barrier with a bounded wait.
+// CTA's blocks touch, a deduplicated per-CTA list) and the dot products go
+// through global memory: the sums as integer atomics whose count of arrivals is
+// the barrier (dot_arrive, dot_wait), or as stored partials around a release /
+// acquire counter barrier; every wait is bounded.
 //
 // Two schedules (kernels/solver_kernels.cu:616-687 semantics in both: x0 = 0,
 // |p.Ap| < 1e-12 stops before the update, ||r|| < tol after it):
 //   standard   the reference's PCG; FP32 vectors, FP64 dot products; two
-//              reductions per iteration.  p of the halo is formed locally as
-//              z + beta*p_old from the exchanged z and p_old, so p itself is
-//              never waited for.
+//              reductions per iteration.  p of the halo is kept locally, as
+//              z + beta*p_old from the exchanged z, so p is never exchanged.
 //   pipelined  Ghysels-Vanroose pipelined PCG: the same iterates in exact
 //              arithmetic with ONE reduction (gamma, delta, ||r||^2) per
 //              iteration overlapped with the SpMV operand exchange; its
 //              recurrences run in FP64 (the SpMV stays FP32).
+#include <climits>
+
 #include "cf_device.cuh"
 #include "cf_internal.h"
 
@@ -166,6 +168,97 @@ __device__ __forceinline__ void wsum_parts(const double* parts, int G, int strid
   }
 }
 
+// The exchange of a dot product: the CTAs' FP64 sums added as integers by
+// L2 atomics, so that the sum arrives with the last arrival's count and its bits
+// do not depend on the order.  A line holds two words, each a sum << kDotCount with
+// the number of arrivals below it; a sum v goes in units of 2^(e - 30) (high word)
+// and what is left in units of 2^(e - 62) (low word), e the exponent of a value
+// that every CTA knows to be of v's size.  |v| < 2^(e + 12), so that kMaxPcgCtas of
+// them fit; any other (or no usable e) counts in the low word's top bits and the
+// exchange is repeated with stored partials behind the counter barrier.  The total
+// is within G 2^(e - 62) of the partials' exact sum: what G additions in FP64 lose.
+// The words only grow: a CTA remembers them as it last saw them, and none can
+// run an exchange ahead of another.  (Four lines, each for a quarter of the CTAs,
+// are no faster: 81.6 us per launch at 2048 nodes against 78.7 with one.)
+struct DotLine {
+  unsigned long long hi, lo;
+};
+constexpr int kDotStride = 16;  // words: a line of its own for each exchange
+constexpr int kDotCount = 11;   // bits of the count
+constexpr int kDotOver = 42;    // bit of the low sum from which "does not fit" is counted
+static_assert(kMaxPcgCtas < (1 << kDotCount) && kDotCount + kDotOver + 10 < 64, "the counts fit their bits");
+
+// kAcquire: what was released with the counts is seen after it.
+template <bool kAcquire>
+__device__ __forceinline__ DotLine dot_load(const unsigned long long* p) {
+  DotLine v;
+  if (kAcquire)
+    asm volatile("{\n\t.reg .b128 t;\n\tld.acquire.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(v.hi), "=l"(v.lo)
+                 : "l"(p)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(v.hi), "=l"(v.lo)
+                 : "l"(p)
+                 : "memory");
+  return v;
+}
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+// The exponent for sums of about v's size; kNoExp: none.
+constexpr int kNoExp = INT_MIN;
+__device__ __forceinline__ int dot_exp(double v) {
+  const int e = (int)((__double_as_longlong(v) >> 52) & 0x7ff) - 1023;
+  return e > -900 && e < 900 ? e : kNoExp;  // (0, infinities and NaN are outside)
+}
+// kRelease: what the CTA wrote before (by a barrier of its threads) is seen by those who wait.
+template <bool kRelease>
+__device__ __forceinline__ void dot_arrive(unsigned long long* p, double v, int e) {
+  unsigned long long h = 1, l = 1;
+  if (e != kNoExp && fabs(v) < pow2(e + 12)) {
+    const double x = v * pow2(30 - e), f = floor(x);
+    h += (unsigned long long)(long long)f << kDotCount;
+    l += (unsigned long long)((x - f) * pow2(32)) << kDotCount;
+  } else {
+    l += 1ull << (kDotOver + kDotCount);
+  }
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p + 1), "l"(l) : "memory");
+  if (kRelease)
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(h) : "memory");
+  else
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(h) : "memory");
+}
+// Waits (bounded, as arrive_wait) for G arrivals past `base`; the total into v.
+// False: it does not fit.
+template <bool kAcquire>
+__device__ __forceinline__ bool dot_wait(const unsigned long long* p, DotLine& base, int G, int e, double& v, int* err,
+                                         unsigned spin_limit, unsigned extra) {
+  constexpr unsigned kMask = (1u << kDotCount) - 1u;
+  const unsigned want = ((unsigned)G + extra) & kMask;
+  unsigned polls = 0;
+  DotLine d;
+  for (;;) {
+    const DotLine now = dot_load<kAcquire>(p);
+    d.hi = now.hi - base.hi;
+    d.lo = now.lo - base.lo;
+    if (((unsigned)d.hi & kMask) == want && ((unsigned)d.lo & kMask) == want) {
+      base = now;
+      break;
+    }
+    if ((polls & 31) == 31 && *(volatile int*)err != 0) break;
+    if (++polls > spin_limit) {
+      atomicOr(err, kErrTimeout);
+      break;
+    }
+    if (polls > 256) __nanosleep(polls > 8192 ? 256 : 20);
+  }
+  const long long h = (long long)(d.hi - (unsigned)G) >> kDotCount;
+  const unsigned long long l = (d.lo - (unsigned)G) >> kDotCount;
+  if (e == kNoExp || (l >> kDotOver)) return false;
+  v = (double)h * pow2(e - 30) + (double)l * pow2(e - 62);
+  return true;
+}
+
 template <bool A_SMEM, bool PIPE>
 __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -199,7 +292,6 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
   double* part = w.partials;  // [2 bufs][3 slots][GT], this group's at [gb, gb + G)
   unsigned gen = 0;
   PhaseClock clk((a.timers && cta == 0 && tid == 0) ? a.timers : nullptr);
-  (void)gcta;
 
   // ---- prologue: A rows, indices, halo list, FP64 block inverses ----
   // staged with cp.async: every copy of the CTA in flight at once, one wait
@@ -309,6 +401,12 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
     float* sPn = sAp + vs;
     // lanes per row element of the SpMV: 4, 2 or 1, as many as the CTA's threads allow
     const int spl_log = (n6 * 4 <= kThreads) ? 2 : (n6 * 2 <= kThreads) ? 1 : 0, spl = 1 << spl_log;
+    // this problem's lines: p.Ap, r.z, r.r, and their words before the first arrival
+    unsigned long long* dots = w.dots + (size_t)prob * 3 * kDotStride;
+    DotLine baseA = {0, 0}, baseB = {0, 0};  // thread 0: p.Ap and r.z; thread 1: r.r
+    if (tid == 0) baseA = dot_load<false>(dots);
+    if (tid < 2) baseB = dot_load<false>(dots + (1 + tid) * kDotStride);
+    volatile int* sFit = reinterpret_cast<volatile int*>(sRed + 60);  // whether the exchange's totals fit
     double prz = 0.0, pbb = 0.0;
     for (int t = tid; t < n6; t += kThreads) {
       const float rt = __ldcg(w.rhs + r0 * 6 + t);
@@ -324,9 +422,8 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
       prz += (double)sR[t] * zf;
     }
     {
-      const int buf = gen & 1;
       const double v2[2] = {prz, pbb};
-      double* const d2[2] = {part + (buf * 3 + 0) * GT + cta, part + (buf * 3 + 1) * GT + cta};
+      double* const d2[2] = {part + GT + cta, part + 2 * GT + cta};
       publish_sums<2>(v2, sRed, d2);
     }
     clk.mark(0);  // prologue
@@ -340,20 +437,25 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
     clk.mark(1);  // first barrier
     double rz = 0.0;
     float betaf = 0.f;
+    // the partials of the last exchange behind the counter barrier: the first
+    // one, and those whose totals did not fit
+    auto repeat = [&](int slots, int dst) {
+      gbar(bar, gen++, G, cta, err, a.spin_limit, a.bar_extra);
+      if (tid < 32) {
+        if (slots == 1) wsum_parts<1>(part + gb, G, GT, sRed, dst);
+        else wsum_parts<2>(part + GT + gb, G, GT, sRed, dst);
+      }
+      __syncthreads();
+    };
     for (int it = 0;; it++) {
-      const float* pold = (it & 1) ? w.p0 : w.p1;  // p_{it-1} lives in buffer (it-1)&1
-      float* pnew = (it & 1) ? w.p1 : w.p0;
-      // ---- one round trip: the reduction behind the last barrier and the halo ----
+      // ---- the halo's z, and behind the first barrier its partials ----
       {
-        const int buf = (gen - 1) & 1;
-        if (tid < 32) {
-          wsum_parts<2>(part + (buf * 3 + 0) * GT + gb, G, GT, sRed, 16);
+        const bool parts = it == 0;
+        if (parts && tid < 32) {
+          wsum_parts<2>(part + GT + gb, G, GT, sRed, 16);
         } else {
-          for (int e = tid - 32; e < h6; e += kThreads - 32) {
-            const int col = sHalo[e / 6], c = e % 6;
-            sZ[n6 + e] = __ldcg(w.z + col * 6 + c);
-            if (it > 0) sV[n6 + e] = __ldcg(pold + col * 6 + c);
-          }
+          const int t0 = parts ? tid - 32 : tid, dt = parts ? kThreads - 32 : kThreads;
+          for (int e = t0; e < h6; e += dt) sZ[n6 + e] = __ldcg(w.z + sHalo[e / 6] * 6 + e % 6);
         }
         __syncthreads();
       }
@@ -362,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
         rz = sRed[16];
         rr_last = sRed[17];
       } else {
-        const double rr = sRed[16], rzn = sRed[17];
+        const double rzn = sRed[16], rr = sRed[17];
         used = it;
         rr_last = rr;
         if (sqrt(rr) < (double)a.pcg_tolerance) break;  // solver_kernels.cu:669
@@ -384,14 +486,16 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
         if (t < n6) {
           const int i = t / 6, c = t % 6;
           for (int bl = sRow[i] + k; bl < sRow[i + 1]; bl += spl) {
-            const float* Ab = A_SMEM ? (sA + bl * 36 + c * 6) : (gA + bl * 36 + c * 6);
+            // (8-byte loads: rows of blocks and operands are 24 bytes)
+            const float2* Ab = reinterpret_cast<const float2*>(A_SMEM ? (sA + bl * 36 + c * 6) : (gA + bl * 36 + c * 6));
             const int o = sVidx[bl] * 6;
-            const float* zz = sZ + o;
-            const float* pp = sV + o;
+            const float2* zz = reinterpret_cast<const float2*>(sZ + o);
+            const float2* pp = reinterpret_cast<const float2*>(sV + o);
 #pragma unroll
-            for (int q = 0; q < 6; q++) {
-              const float pv = first ? zz[q] : __fmaf_rn(betaf, pp[q], zz[q]);
-              y = __fmaf_rn(A_SMEM ? Ab[q] : __ldcg(Ab + q), pv, y);
+            for (int q = 0; q < 3; q++) {
+              const float2 av = A_SMEM ? Ab[q] : __ldcg(Ab + q), zv = zz[q], po = pp[q];
+              y = __fmaf_rn(av.x, first ? zv.x : __fmaf_rn(betaf, po.x, zv.x), y);
+              y = __fmaf_rn(av.y, first ? zv.y : __fmaf_rn(betaf, po.y, zv.y), y);
             }
           }
         }
@@ -399,7 +503,6 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
         if (k == 0 && t < n6) {
           const float pt_ = first ? sZ[t] : __fmaf_rn(betaf, sV[t], sZ[t]);
           sPn[t] = pt_;
-          pnew[r0 * 6 + t] = pt_;
           sAp[t] = y;
           ppap += (double)pt_ * y;
         }
@@ -407,19 +510,22 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
       clk.mark(4);  // spmv
       {
         const double v1[1] = {ppap};
-        double* const d1[1] = {part + ((gen & 1) * 3 + 0) * GT + cta};
+        double* const d1[1] = {sRed + 50};
         publish_sums<1>(v1, sRed, d1);
       }
       clk.mark(5);  // block sum
-      if (tid < 32) {  // warp 0 waits and reads the partials; the others wait at the CTA barrier
-        if (tid == 0) arrive_wait(bar, gen, G, err, a.spin_limit, a.bar_extra);
-        clk.mark(6);  // barrier A
-        __syncwarp();
-        wsum_parts<1>(part + ((gen & 1) * 3 + 0) * GT + gb, G, GT, sRed, 18);
+      if (tid == 0) {  // nothing but the sum is exchanged here: no release
+        const int e = dot_exp(rz);
+        double v = 0.0;
+        part[cta] = sRed[50];  // (for a repeat)
+        dot_arrive<false>(dots, sRed[50], e);
+        *sFit = dot_wait<false>(dots, baseA, G, e, v, err, a.spin_limit, a.bar_extra);
+        sRed[18] = v;
       }
-      gen++;
+      clk.mark(6);  // exchange A
       __syncthreads();
-      clk.mark(7);  // pAp partials
+      if (!*sFit) repeat(1, 18);
+      clk.mark(7);
       const double pAp = sRed[18];
       if (fabs(pAp) < 1e-12) break;  // solver_kernels.cu:647-653
       const float af = (float)(rz / pAp);
@@ -428,6 +534,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
         sR[t] = __fmaf_rn(-af, sAp[t], sR[t]);
         sV[t] = sPn[t];  // p_old of the next iteration
       }
+      for (int e = n6 + tid; e < n6 + h6; e += kThreads) sV[e] = first ? sZ[e] : __fmaf_rn(betaf, sV[e], sZ[e]);
       __syncthreads();
       double prr = 0.0, przn = 0.0;
       for (int t = tid; t < n6; t += kThreads) {
@@ -439,16 +546,32 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_grid_kernel(GridArgs P) {
       }
       clk.mark(8);  // x, r, z updates
       {
-        const int buf = gen & 1;
-        const double v2[2] = {prr, przn};
-        double* const d2[2] = {part + (buf * 3 + 0) * GT + cta, part + (buf * 3 + 1) * GT + cta};
+        const double v2[2] = {przn, prr};
+        double* const d2[2] = {sRed + 50, sRed + 51};
         publish_sums<2>(v2, sRed, d2);
       }
       clk.mark(9);  // block sums
-      if (tid == 0) arrive_wait(bar, gen, G, err, a.spin_limit, a.bar_extra);
-      gen++;
+      if (tid < 32) {
+        const int er = dot_exp(rr_last), ez = dot_exp(rz);
+        if (tid == 0) {
+          part[GT + cta] = sRed[50];
+          part[2 * GT + cta] = sRed[51];
+          dot_arrive<false>(dots + 2 * kDotStride, sRed[51], er);
+          dot_arrive<true>(dots + kDotStride, sRed[50], ez);  // with z of the CTA's rows
+        }
+        __syncwarp();
+        double v = 0.0;
+        bool fit = true;
+        if (tid < 2) {
+          fit = dot_wait<true>(dots + (1 + tid) * kDotStride, baseB, G, tid ? er : ez, v, err, a.spin_limit, a.bar_extra);
+          sRed[16 + tid] = v;
+        }
+        fit = __all_sync(0xffffffffu, fit);
+        if (tid == 0) *sFit = fit;
+      }
       __syncthreads();
-      clk.mark(10);  // barrier B
+      clk.mark(10);  // exchange B
+      if (!*sFit) repeat(2, 16);
     }
     // ---- epilogue ----
     bool bad = false;
@@ -658,8 +781,6 @@ int pcg_max_active_ctas(int smem, bool a_in_smem, bool pipelined) {
 
 cudaError_t launch_pcg(const Work& w, const Pattern& p, const SolveArgs& a, int gn_slot, cudaStream_t s) {
   if (a.N <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(w.barrier, 0, sizeof(unsigned) * (size_t)p.P, s);
-  if (e != cudaSuccess) return e;
   GridArgs P;
   P.w = w;
   P.pt = p;

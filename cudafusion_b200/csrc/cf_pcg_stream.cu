@@ -458,8 +458,6 @@ int pcg_stream_max_active_ctas(int tb) {
 
 cudaError_t launch_pcg_stream(const Work& w, const Pattern& p, const SolveArgs& a, int gn_slot, cudaStream_t s) {
   if (a.N <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(w.barrier, 0, sizeof(unsigned) * (size_t)p.P, s);
-  if (e != cudaSuccess) return e;
   StreamArgs P;
   P.w = w;
   P.pt = p;
