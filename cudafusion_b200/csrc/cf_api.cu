@@ -123,7 +123,7 @@ void free_work(Work& w) {
   dfree(w.cell_ids); dfree(w.rec); dfree(w.raw); dfree(w.cstat); dfree(w.cl_total); dfree(w.cl_start);
   dfree(w.cl_cur); dfree(w.clist); dfree(w.cdesc); dfree(w.cnt); dfree(w.node_total); dfree(w.inc_start); dfree(w.rhs); dfree(w.plain); dfree(w.x); dfree(w.z); dfree(w.p0); dfree(w.p1);
   dfree(w.partials); dfree(w.barrier); dfree(w.dots); dfree(w.err); dfree(w.done); dfree(w.e_data_part); dfree(w.e_arap_part); dfree(w.stats); dfree(w.timers);
-  dfree(w.nodes_cat); dfree(w.T_cat); dfree(w.r); dfree(w.ap); dfree(w.minv32);
+  dfree(w.nodes_cat); dfree(w.T_cat); dfree(w.r); dfree(w.ap); dfree(w.zp); dfree(w.minv32);
   w.cnt_cap = 0;
 }
 
@@ -629,6 +629,7 @@ cf_status build_pattern_host(cf_gn* h, const std::vector<cf_deform_node>& nodes,
     if (!w.minv32) {
       CF_TRY(dalloc(&w.r, 6 * (size_t)w.max_nodes));
       CF_TRY(dalloc(&w.ap, 6 * (size_t)w.max_nodes));
+      CF_TRY(dalloc(&w.zp, 24 * (size_t)w.max_nodes));
       CF_TRY(dalloc(&w.minv32, 36 * (size_t)w.max_nodes));
     }
   }

@@ -1001,8 +1001,9 @@ struct RowMem {
   int edge[kRowBlocks + 4];     // the blocks' first ARAP edges
   float raw[kRowWarps][32][12];  // (u, n), g w_a, -g r, g w_b of the three nodes after a; g = fw w_a
 };
+// (18 CTAs of two warps per SM need 56 registers: 255k rows take 1.52 ms, with 64 1.66)
 template <int kRowWarps>
-__global__ void __launch_bounds__(32 * kRowWarps) gather_kernel(Work w, Pattern pt, float lambda_damping) {
+__global__ void __launch_bounds__(32 * kRowWarps, kRowWarps == 2 ? 18 : 8) gather_kernel(Work w, Pattern pt, float lambda_damping) {
   constexpr int kRowThreads = 32 * kRowWarps;
   __shared__ __align__(16) RowMem<kRowWarps> m;
   const int tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;

@@ -13,6 +13,8 @@ namespace cf {
 
 constexpr int kThreads = 256;
 
+constexpr unsigned kEarlyCtas = 32 * 148;
+
 // A kernel that may be set up while the one before it in the stream still runs:
 // its CTAs take what room there is and wait in after_previous() until all of
 // that kernel, and so all before it, is done and visible.  A call is a row of
@@ -31,7 +33,8 @@ inline cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, dim3 block,
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  // (past that many CTAs the launch no longer matters, and a wait per CTA does)
+  cfg.numAttrs = (unsigned long long)grid.x * grid.y * grid.z <= kEarlyCtas ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
@@ -176,6 +179,7 @@ struct Work {
   float* z = nullptr;
   float* p0 = nullptr;
   float* p1 = nullptr;
+  float* zp = nullptr;        // [2][max_nodes][12] z and p of the streaming PCG
   double* partials = nullptr;  // [2 bufs][3 slots][max pcg ctas]
   unsigned* barrier = nullptr;  // [max pcg ctas] one arrival counter per PCG CTA group (zeroed by the gather)
   unsigned long long* dots = nullptr;  // [max pcg ctas][3 lines] per group: exchanged sums (cf_pcg_grid.cu)

@@ -23,7 +23,13 @@
 // copies still in flight when the loop ends are drained before exit.  Each
 // stage also brings the tile's column indices (a padded copy made with the
 // pattern), so the SpMV operand of tile t + 1 is gathered while tile t's rows
-// are summed: one exposed gather per iteration instead of one per tile.
+// are summed: one exposed gather per iteration instead of one per tile; the row
+// sums' own operands are read during the products.
+//
+// What bounds it (B200, 64 problems, 255k rows, 12.2 iterations: 1.86 ms per
+// launch, A alone would be 0.85 at the copy rate): the gathered operands cross
+// L2 like A does, and two CTAs per SM wait for them a tile at a time.  z and p in
+// arrays of their own, and the row sums' operands read after the products: 2.05.
 #include "cf_device.cuh"
 #include "cf_internal.h"
 
@@ -221,6 +227,10 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
   __syncthreads();
   top_up();  // the first tiles stream in during the first reduction
 
+  // z and p of a node side by side, two buffers: an iteration reads z with the
+  // p before it from one (48 bytes per gathered node instead of 24 in each of
+  // two arrays, which straddle sectors) and leaves p and the next z in the other
+  float *zp0 = w.zp, *zp1 = w.zp + (size_t)12 * w.max_nodes;
   // r = b, x = 0, z = M^-1 r; r.z and b.b
   double prz = 0.0, pbb = 0.0;
   for (int i = r0 + tid; i < r1; i += kThreads) {
@@ -239,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
     const float zero[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     st6(w.r + (size_t)i * 6, rr);
     st6(w.x + (size_t)i * 6, zero);
-    st6(w.z + (size_t)i * 6, zz);
+    st6(zp1 + (size_t)i * 12, zz);  // (the first iteration reads the second buffer)
   }
   {
     const double t1 = bsum_s(prz, sRed), t2 = bsum_s(pbb, sRed + 8);
@@ -283,8 +293,8 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
       rz = rzn;
     }
     if (it >= a.pcg_iterations || *(volatile int*)err) break;
-    const float* pold = (it & 1) ? w.p0 : w.p1;
-    float* pnew = (it & 1) ? w.p1 : w.p0;
+    const float* zpo = (it & 1) ? zp0 : zp1;
+    float* zpn = (it & 1) ? zp1 : zp0;
     // ---- Ap = A (z + beta p_old), p = z + beta p_old, p.Ap ----
     double ppap = 0.0;
     // the operand of the tile in stage s (its column indices came with A;
@@ -293,18 +303,51 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
     auto gather = [&](int s) {
       const int j = stageC(s)[tid < TB ? tid : 0];
       if (tid < TB && j >= 0) {
-        ld6(w.z + (size_t)j * 6, gz);
-        if (it > 0) ld6(pold + (size_t)j * 6, gp);
+        const float4* q = reinterpret_cast<const float4*>(zpo + (size_t)j * 12);
+        const float4 f0 = __ldcg(q), f1 = __ldcg(q + 1), f2 = __ldcg(q + 2);  // (p: of no use in the first iteration)
+        gz[0] = f0.x; gz[1] = f0.y; gz[2] = f0.z; gz[3] = f0.w; gz[4] = f1.x; gz[5] = f1.y;
+        gp[0] = f1.z; gp[1] = f1.w; gp[2] = f2.x; gp[3] = f2.y; gp[4] = f2.z; gp[5] = f2.w;
       }
     };
+    // what thread e of a tile's row sums needs besides the products: the row's
+    // blocks, z and p_old
+    struct RowOwn {
+      int q0, q1;
+      float z, p;
+    };
+    auto load_own = [&](int ra, int e, int b0) -> RowOwn {
+      const int i = ra + e / 6, c = e % 6;
+      RowOwn o;
+      o.q0 = pt.row_ptr[i] - b0;
+      o.q1 = pt.row_ptr[i + 1] - b0;
+      o.z = __ldcg(zpo + (size_t)i * 12 + c);
+      o.p = it > 0 ? __ldcg(zpo + (size_t)i * 12 + 6 + c) : 0.f;
+      return o;
+    };
+    // the next tile's rows and blocks, read a tile ahead
+    int ra_n = 0, rb_n = 0, b0_n = 0, b1_n = 0;
+    if (n_tiles > 0) {
+      ra_n = trow[0];
+      rb_n = trow[1];
+      b0_n = pt.row_ptr[ra_n];
+      b1_n = pt.row_ptr[rb_n];
+    }
     for (int t = 0; t < n_tiles; t++) {
       const int s = (int)(consumed % kStages);
       if (!mbar_wait(&mbar[s], (phase_bits >> s) & 1u, err, kCopyWaitLimit)) ok = false;
       if (t == 0) gather(s);  // (later tiles were gathered during the previous one)
       phase_bits ^= 1u << s;
       const float* A = stageA(s);
-      const int ra = trow[t], rb_ = trow[t + 1];
-      const int b0 = pt.row_ptr[ra], nb = pt.row_ptr[rb_] - b0;
+      const int ra = ra_n, b0 = b0_n, ne = (rb_n - ra) * 6, nb = b1_n - b0;
+      // the row sums' operands, in flight during the products
+      RowOwn own = {0, 0, 0.f, 0.f};
+      if (tid < ne) own = load_own(ra, tid, b0);
+      if (t + 1 < n_tiles) {
+        ra_n = rb_n;
+        b0_n = b1_n;
+        rb_n = trow[t + 2];
+        b1_n = pt.row_ptr[rb_n];
+      }
       if (tid < nb) {
         float v[6];
 #pragma unroll
@@ -332,14 +375,13 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
       __syncthreads();
       consumed++;
       top_up();  // stage s is free: refill it (tiles wrap into the next iteration)
-      for (int e = tid; e < (rb_ - ra) * 6; e += kThreads) {
+      for (int e = tid; e < ne; e += kThreads) {
+        if (e >= kThreads) own = load_own(ra, e, b0);  // (more than a value per thread: short rows)
         const int i = ra + e / 6, c = e % 6;
-        const int q0 = pt.row_ptr[i] - b0, q1 = pt.row_ptr[i + 1] - b0;
         float y = 0.f;
-        for (int q = q0; q < q1; q++) y += sPart[q * kPartStride + c];
-        const float zi = __ldcg(w.z + (size_t)i * 6 + c);
-        const float pi = (it > 0) ? __fmaf_rn(betaf, __ldcg(pold + (size_t)i * 6 + c), zi) : zi;
-        pnew[(size_t)i * 6 + c] = pi;
+        for (int q = own.q0; q < own.q1; q++) y += sPart[q * kPartStride + c];
+        const float pi = (it > 0) ? __fmaf_rn(betaf, own.p, own.z) : own.z;
+        zpn[(size_t)i * 12 + 6 + c] = pi;
         w.ap[(size_t)i * 6 + c] = y;
         ppap += (double)pi * y;
       }
@@ -366,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
       float xx[6], rr[6], pp[6], ap[6], zz[6], M[36];
       ld6(w.x + (size_t)i * 6, xx);
       ld6(w.r + (size_t)i * 6, rr);
-      ld6(pnew + (size_t)i * 6, pp);
+      ld6(zpn + (size_t)i * 12 + 6, pp);
       ld6(w.ap + (size_t)i * 6, ap);
       const float4* m4 = reinterpret_cast<const float4*>(w.minv32 + (size_t)i * 36);
 #pragma unroll
@@ -390,7 +432,7 @@ __global__ void __launch_bounds__(kThreads, 2) pcg_stream_kernel(StreamArgs P) {
       }
       st6(w.x + (size_t)i * 6, xx);
       st6(w.r + (size_t)i * 6, rr);
-      st6(w.z + (size_t)i * 6, zz);
+      st6(zpn + (size_t)i * 12, zz);
     }
     {
       const double t1 = bsum_s(prr, sRed), t2 = bsum_s(przn, sRed + 8);
