@@ -27,8 +27,9 @@
 // entry, of which a correspondence has ten, and the gather reads a record per
 // task instead of every correspondence of a row.  Per GN iteration on B200 (data
 // term + assembly, event times; before: one record per correspondence, gathered
-// entry by entry): 2048 nodes, 306k correspondences 38 + 23 us (before 20 + 56),
-// 8192 nodes, 1.2M 107 + 62 (46 + 192), 64 problems, 33M 3.2 + 1.5 ms (1.7 + 7.1);
+// entry by entry): 2048 nodes, 306k correspondences 37 + 23 us (before 20 + 56),
+// 8192 nodes, 1.2M 103 + 62 (46 + 192), 64 problems, 33M 3.1 + 1.57 ms (1.7 + 7.1);
+// three CTAs per SM at 80 registers spill (4.0 ms);
 // the sort costs 98 us against 80 at 306k and 7 ms against 10 at 33M.
 // Restates kernels/solver_kernels.cu:52-352 (data term, ARAP, damping).
 #include "cf_device.cuh"
@@ -682,7 +683,7 @@ __device__ __forceinline__ void close_task(const unsigned long long (&acc)[10], 
 // (and the raw records of small tasks); otherwise the energy alone, with the
 // problem's ARAP edges.
 template <bool kSkin, bool kAcc>
-__global__ void __launch_bounds__(kThreads, 2) cells_kernel(Table tb, Work w, Pattern pt, EdgeArgs ea, int slot) {
+__global__ void __launch_bounds__(kThreads, kAcc ? 2 : 3) cells_kernel(Table tb, Work w, Pattern pt, EdgeArgs ea, int slot) {
   extern __shared__ __align__(16) unsigned char cells_smem[];
   __shared__ double red[kWarps];
   if (kAcc && (int)blockIdx.x < ea.edge_ctas) {
@@ -693,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, 2) cells_kernel(Table tb, Work w, Pa
   const int lane = lane_id(), wid = threadIdx.x >> 5;
   const int cta = kAcc ? blockIdx.x - ea.edge_ctas : blockIdx.x;
   // (a single problem's share needs no table: one load instead of three in a row)
-  int prob = 0, lc = cta, e_ctas = tb.n_e, n0 = 0, n1 = tb.N;
+  int prob = 0, lc = cta, e_ctas = kAcc ? tb.n_e : (int)gridDim.x, n0 = 0, n1 = tb.N;
   if (tb.P > 1) {
     prob = tb.e_prob[cta];
     const ProbDesc& d = tb.desc[prob];
@@ -884,7 +885,7 @@ __global__ void __launch_bounds__(kThreads, 2) cells_kernel(Table tb, Work w, Pa
         const float *cp = colp + first * kStageWords, *wp = wgtp + first * kStageWords;
         const float* wq = m.stage + (first + half) * kStageWords;
         int j = half;
-#pragma unroll 2
+#pragma unroll 4  // (2: 3.21 ms against 3.10 at 33M correspondences; 8: the same as 4)
         for (; j < (n & ~1); j += 2, cp += 2 * kStageWords, wp += 2 * kStageWords, wq += 2 * kStageWords) {
           const float2 L = *reinterpret_cast<const float2*>(cp);
           const ulonglong2 g01 = *reinterpret_cast<const ulonglong2*>(wp);
@@ -963,12 +964,12 @@ __global__ void __launch_bounds__(kThreads, 2) cells_kernel(Table tb, Work w, Pa
     __shared__ bool final_cta;
     if (threadIdx.x == 0) {
       __threadfence();
-      final_cta = atomicAdd(w.done, 1u) == (unsigned)tb.n_e - 1u;
+      final_cta = atomicAdd(w.done, 1u) == gridDim.x - 1u;
     }
     __syncthreads();
     if (final_cta && wid == 0) {
       __threadfence();
-      reduce_energy(w, w.e_data_part, tb.n_e, 0, slot);
+      reduce_energy(w, w.e_data_part, (int)gridDim.x, 0, slot);
       if (lane == 0) *w.done = 0u;
     }
   }
@@ -1278,8 +1279,10 @@ cudaError_t launch_final_energy(const Work& w, const Pattern& p, const SolveArgs
                                 bool stats) {
   const Table& tb = a.tb;
   if (tb.n_e <= 0) return cudaSuccess;
-  launch_next(cells_kernel<true, false>, tb.n_e, kThreads, 0, s, tb, w, p, edge_args(p, a, a.transforms, stats),
-              slot);
+  // the energy alone needs no records and fits three CTAs per SM (1.2M
+  // correspondences: 39 us, 47 with the two of the data term)
+  launch_next(cells_kernel<true, false>, tb.P > 1 ? tb.n_e : 3 * 148, kThreads, 0, s, tb, w, p,
+              edge_args(p, a, a.transforms, stats), slot);
   if (tb.P > 1) launch_next(energy_reduce_kernel, tb.P, 32, 0, s, tb, w, slot);
   return cudaGetLastError();
 }
