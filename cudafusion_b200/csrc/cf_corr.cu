@@ -60,9 +60,10 @@
 // candidates of a row a lane takes the least |n . w - c| and keeps of these the
 // least L1, the second L2 (with their runs) and the third L3, each less eps.  The
 // winner's distance is at most U = min(L1 + 2 eps), so it is in a run of L <= U:
-// usually one, and if a chunk's L3 <= U its rows are scanned again.  A surface
-// with many equal distances (a plane seen head on) takes that path, at about
-// the cost of one exact scan.
+// usually one, and if a chunk's L3 <= U the merge scans the chunk's rows for that
+// pixel, the CTA's warps taking such pixels from a list.  Surfaces whose distances
+// are equal along lines (a cylinder without noise) do that for half their pixels
+// (radius 50: 982 us per call), a plane for all of them.
 // With an angle threshold the values come from packed FP32 FMAs on the lane's own
 // two pixels (one shared-memory broadcast per candidate; eps = 14 u N (max |w| +
 // max |p - o|)), since that test needs each candidate's normal.  Where the boxes
@@ -74,7 +75,8 @@
 // and instruction issue (two lane-minima per step and 16 pixels, the masks of
 // the windows' edges).  Measured on B200, 640 x 480: radius 50 585 us per call
 // (1825 with a thread per two pixels scanning its own windows in the reference's
-// arithmetic: its shared-memory reads and 11 instructions per candidate), with an
+// arithmetic: its shared-memory reads and 11 instructions per candidate; 1142 on the
+// cylinders), with an
 // angle threshold 1411 (2656), past the cap 2122 (2868), radius 20 272 (463).
 #include <cfloat>
 #include <climits>
@@ -327,12 +329,13 @@ __global__ void __launch_bounds__(kCsBlock* kCsBlock)
 // A candidate's point-to-plane distance, +inf where the reference would skip
 // it (finite values only).  A skip record's far-away point and huge normal
 // make its distance +inf by themselves.  kAngle: apply the angle threshold.
-template <bool kAngle>
+// kCap: apply the Euclidean cap (left out where every candidate is within it).
+template <bool kAngle, bool kCap = true>
 __device__ __forceinline__ float cs_pd(const float3& v, const float3& n, const float4& a, const float2& b,
                                        const CorrConsts& k) {
   const float ex = __fsub_rn(v.x, a.x), ey = __fsub_rn(v.y, a.y), ez = __fsub_rn(v.z, a.z);
   float pd = fabsf(cs_dot(a.w, b.x, b.y, ex, ey, ez));
-  pd = cs_dot(ex, ey, ez, ex, ey, ez) <= k.s_max ? pd : INFINITY;
+  if (kCap) pd = cs_dot(ex, ey, ez, ex, ey, ez) <= k.s_max ? pd : INFINITY;
   if (kAngle) pd = fabsf(cs_dot(n.x, n.y, n.z, a.w, b.x, b.y)) < k.angle_thr ? INFINITY : pd;
   return pd;
 }
@@ -985,13 +988,39 @@ struct CsBest {
   }
 };
 
+// A pixel's n rows of w candidates from row0 (columns from l), the warp's lanes
+// on consecutive ones of them: the lane's first least in row-major order.
+template <bool kAngle, bool kCap>
+__device__ __forceinline__ void cs_rows(const CorrConsts& k, const float3& v, const float3& nc, int row0, int n, int l,
+                                        int w, int lane, const float4* __restrict__ A, const float2* __restrict__ B,
+                                        CsBest& b) {
+  const int total = n * w, dy = 32 / w, dx = 32 - dy * w;
+  int y = lane / w, x = lane - y * w;
+#pragma unroll 8
+  for (int t = lane; t < total; t += 32) {
+    const int i = (row0 + y) * k.W + l + x;
+    const float d = cs_pd<kAngle, kCap>(v, nc, A[i], B[i], k);
+    if (d < b.pd) {
+      b.pd = d;
+      b.i = i;
+    }
+    x += dx;
+    y += dy;
+    if (x >= w) {
+      x -= w;
+      ++y;
+    }
+  }
+}
+
 // Eight lanes per pixel evaluate its runs (the loads of a run's columns are then
 // in flight together, and four pixels' runs per warp; a warp per run took
-// three times as long).  Pixels whose third value is within the bound are left
-// to the CTA, a row of the window per warp at a time.
+// three times as long).  Pixels whose third value is within the bound have those
+// chunks' rows evaluated by the CTA's warps.
 // kDirect: no search went before, each lane scans its pixel's window (rule at
 // kCsDirect).
 constexpr int kMergeThreads = 256;
+static_assert(kMergeThreads <= 256 && kCorrMaxChunks <= 8, "an item: pixel, chunk");
 template <bool kAngle, bool kDirect>
 __global__ void __launch_bounds__(kMergeThreads)
     corr_merge_kernel(const CorrConsts k, const float* __restrict__ lv, const float4* __restrict__ A,
@@ -1000,9 +1029,9 @@ __global__ void __launch_bounds__(kMergeThreads)
                       int* __restrict__ stats) {
   after_previous();
   __shared__ float s_stage[kMergeThreads / 32][32 * kCsRecWords];
-  __shared__ int s_again[kMergeThreads], s_count;
-  __shared__ float s_p[12];
-  __shared__ CsBest s_best[kMergeThreads / 32];
+  __shared__ unsigned long long s_key[kMergeThreads];  // distance bits, candidate: the least first
+  __shared__ unsigned short s_items[kMergeThreads * kCorrMaxChunks];
+  __shared__ int s_count, s_next;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int px = blockIdx.x * kMergeThreads + tid;
   const bool inimg = px < k.P;
@@ -1013,7 +1042,8 @@ __global__ void __launch_bounds__(kMergeThreads)
   p.pu = p.pv = 0;
   p.vl = p.vc = p.nc = make_float3(0.f, 0.f, 0.f);
   p.view_cos = 0.f;
-  if (tid == 0) s_count = 0;
+  if (tid == 0) s_count = s_next = 0;
+  if (!kDirect) __syncthreads();
   if (inimg) {
     p = cs_load_pixel(pix, px);
     if (p.search) {
@@ -1089,51 +1119,53 @@ __global__ void __launch_bounds__(kMergeThreads)
     }
     if (mine && lane == src) best.take(b.pd, b.i);
   }
-  __syncthreads();
-  if (!kDirect && again) s_again[atomicAdd(&s_count, 1)] = tid;
-  __syncthreads();
-  for (int t = 0; !kDirect && t < s_count; ++t) {
-    const int src = s_again[t];
-    if (tid == src) {
-      s_p[0] = p.vc.x; s_p[1] = p.vc.y; s_p[2] = p.vc.z;
-      s_p[3] = p.nc.x; s_p[4] = p.nc.y; s_p[5] = p.nc.z;
-      s_p[6] = __int_as_float(p.pu); s_p[7] = __int_as_float(p.pv);
-      const int y = px / k.W, x = px - y * k.W;
+  // The pixels left: the rows of their chunks, a chunk at a time to the CTA's
+  // next free warp (a surface of equal distances leaves whole CTAs of them).
+  if (!kDirect) {
+    float* q = s_stage[0] + 8 * tid;  // (the records' staging is not in use yet)
+    if (again) {
+      q[0] = p.vc.x; q[1] = p.vc.y; q[2] = p.vc.z;
+      q[3] = p.nc.x; q[4] = p.nc.y; q[5] = p.nc.z;
+      q[6] = __int_as_float(p.pu); q[7] = __int_as_float(p.pv);
+      s_key[tid] = best.i < 0 ? ~0ull : (unsigned long long)__float_as_uint(best.pd) << 32 | (unsigned)best.i;
+      for (unsigned m = again; m; m &= m - 1)
+        s_items[atomicAdd(&s_count, 1)] = (unsigned short)(tid | (__ffs(m) - 1) << 8);
+    }
+    __syncthreads();
+    const int items = s_count;
+    for (;;) {
+      int t = 0;
+      if (lane == 0) t = atomicAdd(&s_next, 1);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      if (t >= items) break;
+      const int src = s_items[t] & 255, cc = s_items[t] >> 8;
+      const float* r = s_stage[0] + 8 * src;
+      const float3 v = make_float3(r[0], r[1], r[2]), nc = make_float3(r[3], r[4], r[5]);
+      const int pu = __float_as_int(r[6]), pv = __float_as_int(r[7]);
+      const int spx = blockIdx.x * kMergeThreads + src, y = spx / k.W, x = spx - y * k.W;
       const int2 rw = part.rows[y / kCsTy * ((k.W + kCsTx - 1) / kCsTx) + x / kCsTx];
-      s_p[8] = __uint_as_float(again); s_p[9] = __int_as_float(rw.x); s_p[10] = __int_as_float(rw.y);
-    }
-    __syncthreads();
-    const float3 v = make_float3(s_p[0], s_p[1], s_p[2]), nc = make_float3(s_p[3], s_p[4], s_p[5]);
-    const int pu = __float_as_int(s_p[6]), pv = __float_as_int(s_p[7]);
-    const int l = max(0, pu - k.radius), h = min(k.W - 1, pu + k.radius);
-    const int ch = __float_as_int(s_p[8]), y0 = __float_as_int(s_p[9]), per = __float_as_int(s_p[10]);
-    CsBest b = {k.dist_thr, -1};
-    for (int cc = 0; cc < k.chunks; ++cc) {
-      if (!((ch >> cc) & 1)) continue;
-      const int ya = max(max(0, pv - k.radius), y0 + cc * per), yz = min(min(k.H - 1, pv + k.radius), y0 + cc * per + per - 1);
-      for (int yy = ya + wid; yy <= yz; yy += kMergeThreads / 32) {
-#pragma unroll 4
-        for (int c = l + lane; c <= h; c += 32) {
-          const float d = cs_pd<kAngle>(v, nc, A[yy * k.W + c], B[yy * k.W + c], k);
-          if (d < b.pd) {
-            b.pd = d;
-            b.i = yy * k.W + c;
-          }
-        }
+      const bool within = part.a[(size_t)cc * k.P + spx].w > 0.f;  // the chunk's candidates are within the cap
+      const int l = max(0, pu - k.radius), w = min(k.W - 1, pu + k.radius) - l + 1;
+      const int ya = max(max(0, pv - k.radius), rw.x + cc * rw.y),
+                n = min(min(k.H - 1, pv + k.radius), rw.x + cc * rw.y + rw.y - 1) - ya + 1;
+      CsBest b = {k.dist_thr, -1};
+      if (within) cs_rows<kAngle, false>(k, v, nc, ya, n, l, w, lane, A, B, b);
+      else cs_rows<kAngle, true>(k, v, nc, ya, n, l, w, lane, A, B, b);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        const float d = __shfl_xor_sync(0xffffffffu, b.pd, o);
+        const int i = __shfl_xor_sync(0xffffffffu, b.i, o);
+        b.take(d, i);
       }
+      if (lane == 0 && b.i >= 0)
+        atomicMin(&s_key[src], (unsigned long long)__float_as_uint(b.pd) << 32 | (unsigned)b.i);
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const float d = __shfl_xor_sync(0xffffffffu, b.pd, o);
-      const int i = __shfl_xor_sync(0xffffffffu, b.i, o);
-      b.take(d, i);
-    }
-    if (lane == 0) s_best[wid] = b;
     __syncthreads();
-    if (tid == src) {
-#pragma unroll
-      for (int w = 0; w < kMergeThreads / 32; ++w) best.take(s_best[w].pd, s_best[w].i);
+    if (again && s_key[tid] != ~0ull) {
+      best.pd = __uint_as_float((unsigned)(s_key[tid] >> 32));
+      best.i = (int)(unsigned)s_key[tid];
     }
+    __syncthreads();  // (the staging is the records' again)
   }
   int code = p.code;
   int bi = -1;
