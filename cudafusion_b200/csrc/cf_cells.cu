@@ -265,11 +265,13 @@ __global__ void __launch_bounds__(kPermThreads) permute_kernel(Table tb, Work w)
   __syncwarp();
   if (lane >= m) return;
   const float* r = st + lane * 23;
-  // per slot, which of the key's nodes it names (3 bits; 7: none); a node
-  // named twice blends once, with both weights
-  const unsigned u0 = kk.x & 0xffffu, u1 = kk.x >> 16, u2 = kk.y & 0xffffu;
+  // Per slot, which of the key's nodes it names (3 bits; 7: none), and the sum
+  // of each node's weights.  A node that a later slot names again (codes 4..6,
+  // which node in bits 12 + 2 s, bit 20: there are such) is blended again there,
+  // with that slot's weight, which goes to one of the entries past the last node.
+  const unsigned u0 = kk.x & 0xffffu, u1 = kk.x >> 16, u2 = kk.y & 0xffffu, u3 = kk.y >> 16;
   float uw[4] = {0.f, 0.f, 0.f, 0.f};
-  unsigned perm = 0, seen = 0;
+  unsigned perm = 0, seen = 0, spare = 1u + (u1 != kNone) + (u2 != kNone) + (u3 != kNone);
 #pragma unroll
   for (int s = 0; s < kK; s++) {
     const int id = __float_as_int(r[9 + s]);
@@ -277,10 +279,19 @@ __global__ void __launch_bounds__(kPermThreads) permute_kernel(Table tb, Work w)
     unsigned p = 7u;
     if (id >= 0 && id < d.N && !(ws < 1e-8f)) {
       const unsigned at = (unsigned)id == u0 ? 0u : (unsigned)id == u1 ? 1u : (unsigned)id == u2 ? 2u : 3u;
-      if (!((seen >> at) & 1u)) p = at;
+      p = at;
+      const bool again = (seen >> at) & 1u;
+      if (again) {
+        perm |= 1u << 20 | at << (12 + 2 * s);
+        p = 3u + spare;
+      }
       seen |= 1u << at;
 #pragma unroll
-      for (unsigned a = 0; a < 4; a++) uw[a] += a == at ? ws : 0.f;
+      for (unsigned a = 0; a < 4; a++) {
+        uw[a] += a == at ? ws : 0.f;
+        if (again && a == spare) uw[a] = ws;
+      }
+      spare += again ? 1u : 0u;
     }
     perm |= p << (3 * s);
   }
@@ -556,29 +567,48 @@ static_assert(sizeof(WarpMem) % 16 == 0, "16-byte rows");
 constexpr int kCellsSmem = kWarps * (int)sizeof(WarpMem);
 
 // blend_warp (cf_device.cuh) over the nodes of the task, in the order of the
-// correspondence's slots; the four nodes' loads are issued together.
+// correspondence's slots; the four nodes' loads are issued together.  A node
+// that two slots name enters at both places: the sign that it gets at the second
+// depends on what was blended in between.
 __device__ __forceinline__ float3 blend_cell(float3 p, unsigned perm, const float4& uw, const int4& ids,
                                              const cf_dual_quat* plain) {
-  DQ q[kK];
-  float wt[kK];
-#pragma unroll
-  for (int k = 0; k < kK; k++) {
-    const int a = (perm >> (3 * k)) & 7;
-    q[k].r = q[k].d = make_float4(0.f, 0.f, 0.f, 0.f);
-    wt[k] = 0.f;
-    if (a < 4) {
-      q[k] = load_dq_ldg(plain + sel4i(ids, a));  // (the plain DQs come from an earlier launch)
-      wt[k] = sel4(uw, a);
-    }
-  }
   float4 br = make_float4(0.f, 0.f, 0.f, 0.f), bd = br;
   float wsum = 0.f;
+  auto add = [&](const DQ& q, float w) {
+    wsum += w;
+    const float s = qdot(q.r, br) < 0.f ? -w : w;
+    br.x += s * q.r.x; br.y += s * q.r.y; br.z += s * q.r.z; br.w += s * q.r.w;
+    bd.x += s * q.d.x; bd.y += s * q.d.y; bd.z += s * q.d.z; bd.w += s * q.d.w;
+  };
+  if (perm >> 20) {  // slot by slot; uw has the sum of a node's weights, so the first slot's is what the others leave
+#pragma unroll 1
+    for (int k = 0; k < kK; k++) {
+      const int c = (perm >> (3 * k)) & 7, a = c < 4 ? c : (perm >> (12 + 2 * k)) & 3;
+      if (c == 7) continue;
+      float w = sel4(uw, c < 4 ? c : c - 3);
+      if (c < 4)
+#pragma unroll 1
+        for (int j = k + 1; j < kK; j++) {
+          const int cj = (perm >> (3 * j)) & 7;
+          if (cj >= 4 && cj < 7 && (int)((perm >> (12 + 2 * j)) & 3) == a) w -= sel4(uw, cj - 3);
+        }
+      add(load_dq_ldg(plain + sel4i(ids, a)), w);
+    }
+  } else {
+    DQ q[kK];
+    float wt[kK];
 #pragma unroll
-  for (int k = 0; k < kK; k++) {
-    wsum += wt[k];
-    const float s = qdot(q[k].r, br) < 0.f ? -wt[k] : wt[k];
-    br.x += s * q[k].r.x; br.y += s * q[k].r.y; br.z += s * q[k].r.z; br.w += s * q[k].r.w;
-    bd.x += s * q[k].d.x; bd.y += s * q[k].d.y; bd.z += s * q[k].d.z; bd.w += s * q[k].d.w;
+    for (int k = 0; k < kK; k++) {
+      const int a = (perm >> (3 * k)) & 7;
+      q[k].r = q[k].d = make_float4(0.f, 0.f, 0.f, 0.f);
+      wt[k] = 0.f;
+      if (a < 4) {
+        q[k] = load_dq_ldg(plain + sel4i(ids, a));  // (the plain DQs come from an earlier launch)
+        wt[k] = sel4(uw, a);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kK; k++) add(q[k], wt[k]);
   }
   if (wsum < 1e-8f) return p;
   DQ b;
