@@ -1644,6 +1644,7 @@ void corr_free(cf_corr_search* h) {
   cudaFree(h->sc.part_a);
   cudaFree(h->sc.part_g);
   cudaFree(h->sc.rows);
+  cudaFree(h->sc.todo);
   cudaFree(h->sc.box);
   cudaFree(h->sc.pix_v);
   cudaFree(h->sc.pix_n);
@@ -1671,6 +1672,7 @@ cf_status cf_corr_search_create(int max_width, int max_height, cf_corr_search** 
   if (e == cudaSuccess) e = dalloc(&h->sc.part_a, P * h->sc.chunk_cap);
   if (e == cudaSuccess) e = dalloc(&h->sc.part_g, P * h->sc.chunk_cap);
   if (e == cudaSuccess) e = dalloc(&h->sc.rows, corr_box_cap(P));
+  if (e == cudaSuccess) e = dalloc(&h->sc.todo, 1 + corr_box_cap(P) * kCorrMaxChunks);
   if (e == cudaSuccess) e = cudaMalloc(&h->sc.box, corr_box_cap(P) * corr_box_bytes());
   if (e == cudaSuccess) e = dalloc(&h->sc.pix_v, P);
   if (e == cudaSuccess) e = dalloc(&h->sc.pix_n, P);

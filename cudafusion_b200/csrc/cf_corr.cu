@@ -32,9 +32,13 @@
 //                      divisions, for every (pixel, candidate) pair.
 //                      The live pixels' camera-frame points, projections and
 //                      rejections are made here as well.
-//  corr_search_kernel  finds, for each pixel and chunk of image rows, the runs
-//                      of kGroup candidates that can hold the winner (below).
-//  corr_merge_kernel   evaluates those runs with the reference's arithmetic,
+//  corr_search_kernel  (wide windows) finds, for each pixel and chunk of image
+//                      rows, the runs of kGroup candidates that can hold the
+//                      winner (below).
+//  corr_exact_kernel   all candidates in the reference's arithmetic: every chunk
+//                      where windows are narrower or an angle threshold is
+//                      given, else those that the search leaves to it.
+//  corr_merge_kernel   evaluates the runs with the reference's arithmetic,
 //                      takes the least distance (of equal ones the first
 //                      candidate in row-major order: the strict-less rule of
 //                      one sequential scan, as no distance can be NaN: every
@@ -43,7 +47,7 @@
 //                      record.  A pixel or frame holding any other value is
 //                      rescanned sequentially with the reference's rule as it
 //                      stands (a NaN distance is accepted).  Small windows it
-//                      scans itself, without a search before.
+//                      scans itself, without a scan before.
 //
 // The search.  A CTA takes 32 x 16 pixels, a warp 8 x 8 of them, a lane two.
 // The warp scans the union of its pixels' windows.  With o the centre of the
@@ -61,23 +65,28 @@
 // least L1, the second L2 (with their runs) and the third L3, each less eps.  The
 // winner's distance is at most U = min(L1 + 2 eps), so it is in a run of L <= U:
 // usually one, and if a chunk's L3 <= U the merge scans the chunk's rows for that
-// pixel, the CTA's warps taking such pixels from a list.  Surfaces whose distances
-// are equal along lines (a cylinder without noise) do that for half their pixels
-// (radius 50: 982 us per call), a plane for all of them.
-// With an angle threshold the values come from packed FP32 FMAs on the lane's own
-// two pixels (one shared-memory broadcast per candidate; eps = 14 u N (max |w| +
-// max |p - o|)), since that test needs each candidate's normal.  Where the boxes
-// do not prove every candidate within the Euclidean cap, or the values' ranges
-// leave no room in halfs, the CTA scans with the reference's arithmetic and cap
-// test instead (eps = 0).
+// pixel, the CTA's warps taking such pixels from a list.
 //
-// What bounds it: the legacy tensor path (8.2 clocks per step and SM quarter)
-// and instruction issue (two lane-minima per step and 16 pixels, the masks of
-// the windows' edges).  Measured on B200, 640 x 480: radius 50 585 us per call
-// (1825 with a thread per two pixels scanning its own windows in the reference's
-// arithmetic: its shared-memory reads and 11 instructions per candidate; 1142 on the
-// cylinders), with an
-// angle threshold 1411 (2656), past the cap 2122 (2868), radius 20 272 (463).
+// Surfaces of equal distances (a plane, a cylinder along its axis) put the third
+// run of most pixels in reach, and such a scan per pixel costs twelve times the
+// search.  So a CTA counts these pixels, first after a few rows of its middle, and
+// past kCsTies threads with them leaves the chunk to the exact scan.  It also does
+// where the boxes do not prove every candidate within the Euclidean cap, or the
+// values' ranges leave no room in halfs.
+//
+// What bounds the search: the legacy tensor path (8.2 clocks per step and SM
+// quarter) and instruction issue (two lane-minima per step and 16 pixels, the
+// masks of the windows' edges); the exact scan: instruction issue (6.5 per pixel
+// and candidate) and shared memory's data path.  Measured on B200, us per call, in
+// brackets a thread per two pixels with the reference's arithmetic throughout:
+//                        noisy       plane       plane, third runs scanned per pixel
+//   640 x 480 r 50       565 (1771)  1132 (1104)   4272
+//             r 36       380 (1027)   700  (645)   2498
+//             r 28       425  (692)   395  (441)   1688
+//             r 20       280  (430)   264  (286)   1123
+//             r 50 angle 1500 (2594) 1467 (1645)   5453
+//   320 x 240 r 20       103  (152)    98  (103)    508
+//   160 x 120 r 20        69   (72)    65   (57)    512
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -95,16 +104,30 @@ constexpr int kCsTy = 16;
 constexpr int kCsThreads = 256;
 constexpr int kCsSmem = 72 * 1024;  // one band of records; 3 CTAs per SM with the 1 KB reserve each
 constexpr int kCsCtasPerSm = 3;
+constexpr int kExSmem = 104 * 1024;  // the exact scan's; 2 CTAs per SM, whose 128 registers a lane's four pixels need
+constexpr int kExCtasPerSm = 2;
+constexpr int kCsTieRows = 4;  // rows after which ties are looked for first
+// Threads of a CTA (two pixels each; of those that have any, as many in
+// proportion) with ties beyond which its chunk is scanned exactly.  640 x 480,
+// radius 50: a noise-free wavy surface 700 us with 64, 633 with 112 (one chunk alone
+// takes the exact scan 77); a tilted plane in FP32 depth 1202 and 1263, radius 36 a
+// plane 699 and 739.
+constexpr int kCsTies = 64;
 constexpr int kCsBlock = 16;  // side of the blocks whose boxes are known
 constexpr int kGroup = 128;   // candidates of a run at most
-constexpr int kSub = 8;       // columns scanned with or without window masks together
 constexpr int kSlab = 768;    // columns staged at a time at most
 constexpr int kPad = 8;       // and the columns past them that a step may read
 constexpr float kFarS = 3e5f;  // (scaled) distance of what is not there, above every real one
 // Largest radius whose windows the merge scans itself, a lane per pixel: 640 x
-// 480 takes 84 us at radius 3 and 118 at 6 that way, 137 and 150 with the
-// search's fixed costs; at 8 152 (from the candidates' share) and 165.
-constexpr int kCsDirect = 8;
+// 480 takes 80 us at radius 5 that way and 127 at 8; with the exact scan before
+// it 103 and 125.
+constexpr int kCsDirect = 7;
+// Pixels times candidates past which the search goes before the exact scan: its
+// fixed costs, and those of a surface that it leaves to the exact scan, weigh on
+// narrower windows.  640 x 480 at radius 20 (5.2e8): 250 us with the search, 280
+// without, on a plane 314 and 264; at 28 (1e9) 310 and 425, 519 and 395; at 36
+// (1.6e9) 380 and 590, 700 and 560.
+constexpr double kCsFilter = 1.2e9;
 constexpr float kCsNone = 1e30f;  // distance of what is not there
 constexpr float kU = 5.9604645e-8f;  // 2^-24
 constexpr float kCsBig = 1e18f;  // squares and three-term sums of such values stay finite in FP32
@@ -253,14 +276,14 @@ __global__ void __launch_bounds__(kCsBlock* kCsBlock)
     corr_prep_kernel(const CorrConsts k, const float* __restrict__ depth, const float* __restrict__ dn,
                      const float* __restrict__ lv, const float* __restrict__ ln, float4* __restrict__ A,
                      float2* __restrict__ B, const CsPix pix, CsBox* __restrict__ box, int* __restrict__ flag,
-                     int* __restrict__ num_valid, int* __restrict__ stats) {
+                     int* __restrict__ todo, int* __restrict__ num_valid, int* __restrict__ stats) {
   after_previous();
   __shared__ float s_f[kCsBlock * kCsBlock / 32][13];
   __shared__ int s_i[kCsBlock * kCsBlock / 32][4];
   const int tid = threadIdx.x;
   const int x = blockIdx.x * kCsBlock + (tid & (kCsBlock - 1)), y = blockIdx.y * kCsBlock + tid / kCsBlock;
-  if (blockIdx.x == 0 && blockIdx.y == 0) {  // (counted by the merge)
-    if (tid == 0) *num_valid = 0;
+  if (blockIdx.x == 0 && blockIdx.y == 0) {  // (counted by the merge, and by the search)
+    if (tid == 0) *num_valid = *todo = 0;
     if (stats && tid < 6) stats[tid] = 0;
   }
   const float none = -INFINITY;
@@ -340,60 +363,17 @@ __device__ __forceinline__ float cs_pd(const float3& v, const float3& n, const f
   return pd;
 }
 
-__device__ __forceinline__ unsigned long long cs_pack(float x, float y) {
-  unsigned long long d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-  return d;
-}
-__device__ __forceinline__ float2 cs_unpack(unsigned long long v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ unsigned long long cs_fma2(unsigned long long a, unsigned long long b,
-                                                      unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ unsigned long long cs_mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 // One of a lane's two pixels.
 struct CsLane {
-  unsigned long long wx, wy, wz;  // its point less the origin, twice (filter), or its point (exact)
-  unsigned long long nx, ny, nz;  // its normal, twice (angle test)
-  int l;                          // its window's first column and the columns after it
-  unsigned span;
-  int pv;                         // its projection's row; off the image when it is not scanned
+  int pv;  // its projection's row; off the image when it is not scanned
   float L1, L2, L3;
-  int g1, g2;                     // the runs of L1 and L2: their first pixel
+  int g1, g2;  // the runs of L1 and L2: their first pixel
 };
 
 __device__ __forceinline__ float cs_min_abs(float a, float b, float c) {
   float d;
   asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
-}
-// Two candidates' distances from a pixel into m.  (col: the first one's
-// column, for the window mask.)
-template <bool kAngle, bool kMask>
-__device__ __forceinline__ float cs_pair(float m, const CsLane& q, const ulonglong2& xy, const ulonglong2& zc, int col,
-                                         float angle_thr) {
-  float2 f = cs_unpack(cs_fma2(xy.x, q.wx, cs_fma2(xy.y, q.wy, cs_fma2(zc.x, q.wz, zc.y))));
-  if (kAngle) {
-    const float2 t = cs_unpack(cs_fma2(q.nz, zc.x, cs_fma2(q.ny, xy.y, cs_mul2(q.nx, xy.x))));
-    f.x = fabsf(t.x) < angle_thr ? kCsNone : f.x;
-    f.y = fabsf(t.y) < angle_thr ? kCsNone : f.y;
-  }
-  if (kMask) {
-    f.x = (unsigned)(col - q.l) <= q.span ? f.x : kCsNone;
-    f.y = (unsigned)(col + 1 - q.l) <= q.span ? f.y : kCsNone;
-  }
-  return cs_min_abs(m, f.x, f.y);
 }
 
 // A run's least value into the pixel's three least.
@@ -661,129 +641,131 @@ __device__ __forceinline__ void cs_emit(const CorrConsts& k, const CsPixel& p, b
 }
 
 // What a chunk of rows leaves of a pixel: its three least values less eps
-// (a: L1, L2, L3, eps) and the runs of the first two.
+// (a: L1, L2, L3, eps) and the runs of the first two; from the exact scan the
+// least distance and the first run that has it, with eps 0.
 struct CsPart {
   float4* __restrict__ a;
   int2* __restrict__ g;
   int2* __restrict__ rows;  // per tile of pixels: its first row, and the rows of a chunk
+  int* __restrict__ todo;   // the exact scan's share: how many, then each (chunk * tiles + tile) * 2 + near
 };
 
-// The band's candidates against the warp's pixels.  Shared memory holds row
-// after row of wu columns from xs (even): for the filter per two columns
-// (nx, nx, ny, ny), (nz, nz, -c, -c), for the exact scan per column (point, nx),
-// (ny, nz, -, -).  [ca, cb]: the warp's columns here, [ia, ib] those that all
-// its pixels' windows hold, [ya, yz] its rows.
-template <bool kAngle, bool kExact>
-__device__ __forceinline__ void cs_scan(const float4* sm, int wu, int xs, int yb, int ca, int cb, int ia, int ib, int ya,
-                                        int yz, CsLane& q0, CsLane& q1, float eps, const CorrConsts& k) {
-  const unsigned r = (unsigned)k.radius;
-  ca &= ~1;  // (xs is even)
-  for (int yy = ya; yy <= yz; ++yy) {
-    const float4* row = sm + (size_t)(yy - yb) * (kExact ? 2 * wu : wu) - (kExact ? 2 * xs : xs);
-    const bool in0 = (unsigned)(yy - q0.pv) + r <= 2 * r, in1 = (unsigned)(yy - q1.pv) + r <= 2 * r;
-    const int base = yy * k.W;
-    for (int g = ca; g <= cb; g += kGroup) {
-      float m0 = kCsNone, m1 = kCsNone;
-      if (kExact) {
-        const int e = min(cb, g + kGroup - 1);
-        const float3 v0 = make_float3(cs_unpack(q0.wx).x, cs_unpack(q0.wy).x, cs_unpack(q0.wz).x);
-        const float3 v1 = make_float3(cs_unpack(q1.wx).x, cs_unpack(q1.wy).x, cs_unpack(q1.wz).x);
-        const float3 n0 = make_float3(cs_unpack(q0.nx).x, cs_unpack(q0.ny).x, cs_unpack(q0.nz).x);
-        const float3 n1 = make_float3(cs_unpack(q1.nx).x, cs_unpack(q1.ny).x, cs_unpack(q1.nz).x);
-#pragma unroll 2
-        for (int c = g; c <= e; ++c) {
-          const float4 a = row[2 * c], bb = row[2 * c + 1];
-          const float2 b = make_float2(bb.x, bb.y);
-          const float f0 = cs_pd<kAngle>(v0, n0, a, b, k), f1 = cs_pd<kAngle>(v1, n1, a, b, k);
-          m0 = fminf(m0, (unsigned)(c - q0.l) <= q0.span ? f0 : kCsNone);
-          m1 = fminf(m1, (unsigned)(c - q1.l) <= q1.span ? f1 : kCsNone);
-        }
-      } else {
-        const ulonglong2* pr = reinterpret_cast<const ulonglong2*>(row + g);
-#pragma unroll 1
-        for (int h = 0; h < kGroup / kSub; ++h) {
-          const int c = g + h * kSub;
-          if (c > cb) break;
-          if (c >= ia && c + kSub - 1 <= ib) {
+// The exact scan and the merge start as the kernel before them ends (their
+// CTAs beside a running search cost more than the launch).
+__device__ __forceinline__ void cs_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A CTA's tile of pixels and chunk of rows: the columns and rows that its windows cover.
+struct CsTile {
+  int xlo, xhi, ylo, yhi, per, c0, c1;
+  float v[6];  // the live pixels' box: maxima of -x, -y, -z, x, y, z
+};
+// False (over the CTA): nothing is scanned here.
+__device__ __forceinline__ bool cs_tile(const CorrConsts& k, const CsBox* __restrict__ box, const int* __restrict__ flag,
+                                        int tx, int ty, int chunk, CsTile& t) {
+  // the pixels' boxes: the tile is two blocks
+  const int r = k.radius, bpr = (k.W + kCsBlock - 1) / kCsBlock;
+  const CsBox* bt = box + (size_t)ty * bpr + 2 * tx;
+  const bool two = 2 * tx + 1 < bpr;
+  int bx[4];
 #pragma unroll
-            for (int j = 0; j < kSub / 2; ++j) {
-              const ulonglong2 xy = pr[h * kSub + 2 * j], zc = pr[h * kSub + 2 * j + 1];
-              m0 = cs_pair<kAngle, false>(m0, q0, xy, zc, 0, k.angle_thr);
-              m1 = cs_pair<kAngle, false>(m1, q1, xy, zc, 0, k.angle_thr);
-            }
-          } else {
+  for (int c = 0; c < 4; ++c) bx[c] = max(bt[0].p[c], two ? bt[1].p[c] : kCsOff);
+  if (*flag || bx[1] < -bx[0]) return false;  // a frame scanned sequentially, or no pixel
 #pragma unroll
-            for (int j = 0; j < kSub / 2; ++j) {
-              if (c + 2 * j <= cb) {
-                const ulonglong2 xy = pr[h * kSub + 2 * j], zc = pr[h * kSub + 2 * j + 1];
-                m0 = cs_pair<kAngle, true>(m0, q0, xy, zc, c + 2 * j, k.angle_thr);
-                m1 = cs_pair<kAngle, true>(m1, q1, xy, zc, c + 2 * j, k.angle_thr);
-              }
-            }
-          }
-        }
-      }
-      // a window that does not reach this row holds nothing of the run
-      cs_track(q0, in0 ? m0 : kCsNone, eps, base + g);
-      cs_track(q1, in1 ? m1 : kCsNone, eps, base + g);
+  for (int c = 0; c < 6; ++c) t.v[c] = fmaxf(bt[0].v[c], two ? bt[1].v[c] : -INFINITY);
+  t.xlo = max(0, -bx[0] - r) & ~1;
+  t.xhi = min(k.W - 1, bx[1] + r);
+  t.ylo = max(0, -bx[2] - r);
+  t.yhi = min(k.H - 1, bx[3] + r);
+  t.per = (t.yhi - t.ylo + k.chunks) / k.chunks;  // ceil(rows / chunks)
+  t.c0 = t.ylo + chunk * t.per;
+  t.c1 = min(t.yhi, t.c0 + t.per - 1);
+  return true;
+}
+// The box of the chunk's real candidates (CsBox::d) and what follows from it.
+struct CsReach {
+  float o[3];     // the centre of the live pixels' points
+  float wr, ar;   // the largest |v - o| and |p - o|
+  float nn;       // the longest normal
+  bool any, cap;  // a real candidate; all of them within the Euclidean cap of all pixels
+};
+__device__ __forceinline__ CsReach cs_reach(const CorrConsts& k, const CsBox* __restrict__ box, const CsTile& t) {
+  __shared__ float s_d[kCsThreads / 32][7];
+  const int tid = threadIdx.x, bpr = (k.W + kCsBlock - 1) / kCsBlock;
+  float v[7] = {-INFINITY, -INFINITY, -INFINITY, 0.f, -INFINITY, -INFINITY, -INFINITY};
+  if (t.c0 <= t.c1) {
+    const int b0 = t.xlo / kCsBlock, bw = t.xhi / kCsBlock - b0 + 1, r0 = t.c0 / kCsBlock,
+              bh = t.c1 / kCsBlock - r0 + 1;
+    for (int i = tid; i < bw * bh; i += kCsThreads) {
+      const float4* b = reinterpret_cast<const float4*>(box[(size_t)(r0 + i / bw) * bpr + b0 + i % bw].d);
+      const float4 lo = b[0], hi = b[1];
+      v[0] = fmaxf(v[0], lo.x);
+      v[1] = fmaxf(v[1], lo.y);
+      v[2] = fmaxf(v[2], lo.z);
+      v[3] = fmaxf(v[3], lo.w);
+      v[4] = fmaxf(v[4], hi.x);
+      v[5] = fmaxf(v[5], hi.y);
+      v[6] = fmaxf(v[6], hi.z);
     }
   }
+#pragma unroll
+  for (int c = 0; c < 7; ++c) {
+    v[c] = cs_warp_max(v[c]);
+    if ((tid & 31) == 0) s_d[tid >> 5][c] = v[c];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 7; ++c) {
+    v[c] = s_d[0][c];
+#pragma unroll
+    for (int w = 1; w < kCsThreads / 32; ++w) v[c] = fmaxf(v[c], s_d[w][c]);
+  }
+  CsReach q;
+  q.any = v[4] >= -v[0];
+  float ww = 0.f, aa = 0.f, dd = 0.f;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    q.o[c] = 0.5f * (t.v[3 + c] - t.v[c]);
+    const float hw = fmaxf(fabsf(t.v[3 + c] - q.o[c]), fabsf(-t.v[c] - q.o[c]));
+    const float ha = fmaxf(fabsf(v[4 + c] - q.o[c]), fabsf(-v[c] - q.o[c]));
+    const float d = fmaxf(fabsf(t.v[3 + c] + v[c]), fabsf(v[4 + c] + t.v[c]));
+    ww += hw * hw;
+    aa += ha * ha;
+    dd += d * d;
+  }
+  q.nn = sqrtf(v[3]);
+  q.wr = sqrtf(ww);
+  q.ar = sqrtf(aa);
+  // (a relative margin of 1e-4 over the few-ulp rounding of the squared distances)
+  q.cap = dd * 1.0001f <= k.s_max;
+  return q;
 }
 
-template <bool kAngle>
 __global__ void __launch_bounds__(kCsThreads, kCsCtasPerSm)
     corr_search_kernel(const CorrConsts k, const float4* __restrict__ A, const float2* __restrict__ B, const CsPix pix,
                        const CsBox* __restrict__ box, const int* __restrict__ flag, const CsPart part) {
   extern __shared__ float4 cs_smem[];
-  __shared__ float s_d[kCsThreads / 32][7];  // per warp: the candidates' part of the boxes
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int x = blockIdx.x * kCsTx + (wid & 3) * 8 + (lane >> 2);
   const int y0 = blockIdx.y * kCsTy + (wid >> 2) * 8 + 2 * (lane & 3), y1 = y0 + 1;
   const int chunk = blockIdx.z, r = k.radius;
   const int px0 = y0 * k.W + x, px1 = px0 + k.W;
-  // the pixels' boxes: the tile is two blocks
-  const int bpr = (k.W + kCsBlock - 1) / kCsBlock;
-  const CsBox* bt = box + (size_t)blockIdx.y * bpr + 2 * blockIdx.x;
-  const bool two = 2 * (int)blockIdx.x + 1 < bpr;
-  int bx[4];
-  float bv[6];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) bx[c] = max(bt[0].p[c], two ? bt[1].p[c] : kCsOff);
-  if (*flag || bx[1] < -bx[0]) return;  // a frame scanned sequentially, or no pixel (uniform over the CTA)
-#pragma unroll
-  for (int c = 0; c < 6; ++c) bv[c] = fmaxf(bt[0].v[c], two ? bt[1].v[c] : -INFINITY);
-  // the CTA's columns, and its rows in this chunk
-  const int xlo = max(0, -bx[0] - r) & ~1, xhi = min(k.W - 1, bx[1] + r);
-  const int ylo = max(0, -bx[2] - r), yhi = min(k.H - 1, bx[3] + r);
-  const int per = (yhi - ylo + k.chunks) / k.chunks;  // ceil(rows / chunks)
-  const int c0 = ylo + chunk * per, c1 = min(yhi, c0 + per - 1);
-  if (chunk == 0 && tid == 0) part.rows[blockIdx.y * gridDim.x + blockIdx.x] = make_int2(ylo, per);
-  {  // their boxes
-    float v[7] = {-INFINITY, -INFINITY, -INFINITY, 0.f, -INFINITY, -INFINITY, -INFINITY};
-    if (c0 <= c1) {
-      const int b0 = xlo / kCsBlock, bw = xhi / kCsBlock - b0 + 1, r0 = c0 / kCsBlock, bh = c1 / kCsBlock - r0 + 1;
-      for (int i = tid; i < bw * bh; i += kCsThreads) {
-        const float4* b = reinterpret_cast<const float4*>(box[(size_t)(r0 + i / bw) * bpr + b0 + i % bw].d);
-        const float4 lo = b[0], hi = b[1];
-        v[0] = fmaxf(v[0], lo.x);
-        v[1] = fmaxf(v[1], lo.y);
-        v[2] = fmaxf(v[2], lo.z);
-        v[3] = fmaxf(v[3], lo.w);
-        v[4] = fmaxf(v[4], hi.x);
-        v[5] = fmaxf(v[5], hi.y);
-        v[6] = fmaxf(v[6], hi.z);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 7; ++c) {
-      v[c] = cs_warp_max(v[c]);
-      if (lane == 0) s_d[wid][c] = v[c];
-    }
+  const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+  CsTile t;
+  if (!cs_tile(k, box, flag, blockIdx.x, blockIdx.y, chunk, t)) return;
+  if (chunk == 0 && tid == 0) part.rows[tile] = make_int2(t.ylo, t.per);
+  const CsReach q = cs_reach(k, box, t);
+  auto leave_to_exact = [&]() {
+    if (tid == 0)
+      part.todo[1 + atomicAdd(part.todo, 1)] = 2 * (chunk * (int)(gridDim.x * gridDim.y) + tile) + (q.cap ? 1 : 0);
+  };
+  if (q.any && !(q.cap && q.nn >= 1e-6f && q.nn <= 1e6f && q.wr + q.ar >= 1e-6f && q.wr + q.ar <= 1e6f)) {
+    leave_to_exact();
+    return;
   }
   CsPixel p0, p1;
   p0.search = p1.search = p0.special = p1.special = false;
   p0.pu = p1.pu = p0.pv = p1.pv = 0;
-  p0.vc = p1.vc = p0.nc = p1.nc = make_float3(0.f, 0.f, 0.f);
+  p0.vc = p1.vc = make_float3(0.f, 0.f, 0.f);
   if (x < k.W && y0 < k.H) p0 = cs_load_pixel(pix, px0);
   if (x < k.W && y1 < k.H) p1 = cs_load_pixel(pix, px1);
   const bool on0 = p0.search && !p0.special, on1 = p1.search && !p1.special;
@@ -793,186 +775,269 @@ __global__ void __launch_bounds__(kCsThreads, kCsCtasPerSm)
   const int wuh = __reduce_max_sync(0xffffffffu, max(on0 ? p0.pu : -kFar, on1 ? p1.pu : -kFar));
   const int wvl = __reduce_min_sync(0xffffffffu, min(on0 ? p0.pv : kFar, on1 ? p1.pv : kFar));
   const int wvh = __reduce_max_sync(0xffffffffu, max(on0 ? p0.pv : -kFar, on1 ? p1.pv : -kFar));
-  __syncthreads();
-  float o[3], eps, sw = 1.f, sn = 1.f;
-  bool filter, any = false;
-  {
-    float v[7];
-#pragma unroll
-    for (int c = 0; c < 7; ++c) {
-      v[c] = s_d[0][c];
-#pragma unroll
-      for (int w = 1; w < kCsThreads / 32; ++w) v[c] = fmaxf(v[c], s_d[w][c]);
-    }
-    any = v[4] >= -v[0];  // a real candidate
-    float ww = 0.f, aa = 0.f, dd = 0.f;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      o[c] = 0.5f * (bv[3 + c] - bv[c]);
-      const float hw = fmaxf(fabsf(bv[3 + c] - o[c]), fabsf(-bv[c] - o[c]));
-      const float ha = fmaxf(fabsf(v[4 + c] - o[c]), fabsf(-v[c] - o[c]));
-      const float d = fmaxf(fabsf(bv[3 + c] + v[c]), fabsf(v[4 + c] + bv[c]));
-      ww += hw * hw;
-      aa += ha * ha;
-      dd += d * d;
-    }
-    const float nn = sqrtf(v[3]), wr = sqrtf(ww), ar = sqrtf(aa);
-    // (a relative margin of 1e-4 over the few-ulp rounding of the squared distances)
-    filter = dd * 1.0001f <= k.s_max && nn >= 1e-6f && nn <= 1e6f && wr + ar >= 1e-6f && wr + ar <= 1e6f;
-    if (kAngle) {
-      eps = 14.f * kU * nn * (wr + ar);
-    } else {
-      // w and n up to 256 each: c then up to 2^16, a quarter of it fits a half
-      const int ew = 7 - ilogbf(wr + ar), en = 7 - ilogbf(nn);
-      sw = filter ? ldexpf(1.f, ew) : 1.f;
-      sn = filter ? ldexpf(1.f, en) : 1.f;
-      eps = kU * nn * (25.f * wr + 20.f * ar) * (sw * sn);
-    }
-    if (!filter) eps = 0.f;
-  }
+  // w and n up to 256 each: c then up to 2^16, a quarter of it fits a half
+  const float sw = q.any ? ldexpf(1.f, 7 - ilogbf(q.wr + q.ar)) : 1.f, sn = q.any ? ldexpf(1.f, 7 - ilogbf(q.nn)) : 1.f;
+  const float eps = q.any ? kU * q.nn * (25.f * q.wr + 20.f * q.ar) * (sw * sn) : 0.f;
   CsLane q0, q1;
-  {
-    const float ox = filter ? o[0] : 0.f, oy = filter ? o[1] : 0.f, oz = filter ? o[2] : 0.f;
-    auto state = [&](const CsPixel& p, bool on) {
-      CsLane q;
-      const float wx = on ? p.vc.x - ox : 0.f, wy = on ? p.vc.y - oy : 0.f, wz = on ? p.vc.z - oz : 0.f;
-      q.wx = cs_pack(wx, wx);
-      q.wy = cs_pack(wy, wy);
-      q.wz = cs_pack(wz, wz);
-      q.nx = q.ny = q.nz = 0ull;
-      if (kAngle && on) {
-        q.nx = cs_pack(p.nc.x, p.nc.x);
-        q.ny = cs_pack(p.nc.y, p.nc.y);
-        q.nz = cs_pack(p.nc.z, p.nc.z);
-      }
-      q.l = on ? max(0, p.pu - r) : kFar;
-      q.span = on ? (unsigned)(min(k.W - 1, p.pu + r) - q.l) : 0u;
-      q.pv = on ? p.pv : -kFar;
-      q.L1 = q.L2 = q.L3 = kCsNone;
-      q.g1 = q.g2 = -1;
-      return q;
-    };
-    q0 = state(p0, on0);
-    q1 = state(p1, on1);
-  }
-  if (any && c0 <= c1) {
+  q0.pv = on0 ? p0.pv : -kFar;
+  q1.pv = on1 ? p1.pv : -kFar;
+  q0.L1 = q0.L2 = q0.L3 = q1.L1 = q1.L2 = q1.L3 = kCsNone;
+  q0.g1 = q0.g2 = q1.g1 = q1.g2 = -1;
+  if (q.any && t.c0 <= t.c1) {
     const bool some = wuh >= wul;
+    const int most = __syncthreads_count(on0 || on1) * kCsTies / kCsThreads;
     const int ua = max(0, wul - r), ub = min(k.W - 1, wuh + r);  // the warp's columns
     const int ia = max(0, wuh - r), ib = min(k.W - 1, wul + r);  // those of every window
-    const bool mma = !kAngle && filter;
     unsigned af[4][4];
     int first[8];
-    if (mma) {
+    {
+      const float3 a0 = on0 ? make_float3((p0.vc.x - q.o[0]) * sw, (p0.vc.y - q.o[1]) * sw, (p0.vc.z - q.o[2]) * sw)
+                            : make_float3(0.f, 0.f, 0.f);
+      const float3 a1 = on1 ? make_float3((p1.vc.x - q.o[0]) * sw, (p1.vc.y - q.o[1]) * sw, (p1.vc.z - q.o[2]) * sw)
+                            : make_float3(0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int src = (lane & 28) | i;  // the lane that holds this lane's pixels of tile i
-        const float2 a0 = cs_unpack(q0.wx), b0 = cs_unpack(q0.wy), d0 = cs_unpack(q0.wz);
-        const float2 a1 = cs_unpack(q1.wx), b1 = cs_unpack(q1.wy), d1 = cs_unpack(q1.wz);
-        cs_pixel_mma(__shfl_sync(0xffffffffu, a0.x, src) * sw, __shfl_sync(0xffffffffu, b0.x, src) * sw,
-                     __shfl_sync(0xffffffffu, d0.x, src) * sw, lane & 3, af[i][0], af[i][2]);
-        cs_pixel_mma(__shfl_sync(0xffffffffu, a1.x, src) * sw, __shfl_sync(0xffffffffu, b1.x, src) * sw,
-                     __shfl_sync(0xffffffffu, d1.x, src) * sw, lane & 3, af[i][1], af[i][3]);
+        cs_pixel_mma(__shfl_sync(0xffffffffu, a0.x, src), __shfl_sync(0xffffffffu, a0.y, src),
+                     __shfl_sync(0xffffffffu, a0.z, src), lane & 3, af[i][0], af[i][2]);
+        cs_pixel_mma(__shfl_sync(0xffffffffu, a1.x, src), __shfl_sync(0xffffffffu, a1.y, src),
+                     __shfl_sync(0xffffffffu, a1.z, src), lane & 3, af[i][1], af[i][3]);
         first[2 * i] = __shfl_sync(0xffffffffu, on0 ? p0.pu - r : kFar, src);
         first[2 * i + 1] = __shfl_sync(0xffffffffu, on1 ? p1.pu - r : kFar, src);
       }
     }
-    for (int xs = xlo; xs <= xhi; xs += kSlab) {
-      const int xe = min(xhi, xs + kSlab - 1);
-      const int wu = mma ? xe - xs + 1 + kPad : (xe - xs + 2) & ~1;
-      const int band = kCsSmem / (wu * (filter && kAngle ? 16 : 32));
-      for (int yb = c0; yb <= c1; yb += band) {
-        const int rows = min(band, c1 - yb + 1);
-        __syncthreads();
-        if (mma) {
-          const float sc = -0.25f * sw * sn;
-          for (int j = tid; j < rows * wu; j += kCsThreads) {
-            const int rr = j / wu, c = j - rr * wu;
-            float nx = 0.f, ny = 0.f, nz = 0.f, mc = 0.25f * kFarS * 0.8f;
-            if (xs + c <= xe) {
-              const int g = (yb + rr) * k.W + xs + c;
-              const float4 a = A[g];
-              if (a.z > 0.f) {
-                const float2 b = B[g];
-                nx = a.w * sn;
-                ny = b.x * sn;
-                nz = b.y * sn;
-                mc = sc * cs_dot(a.w, b.x, b.y, a.x - o[0], a.y - o[1], a.z - o[2]);
-              }
+    // (in shared memory: registers are what the scan is short of)
+    __shared__ float s_k[6];
+    if (tid == 0) {
+      s_k[0] = q.o[0];
+      s_k[1] = q.o[1];
+      s_k[2] = q.o[2];
+      s_k[3] = sn;
+      s_k[4] = -0.25f * sw * sn;
+      s_k[5] = k.dist_thr * (sw * sn);
+    }
+    __syncthreads();
+    // a third run in reach: the merge would scan the chunk's rows for the pixel
+    auto tied = [&]() {
+      const float reach = 2.25f * eps, thr = s_k[5];
+      const bool tie = q0.L3 <= fminf(q0.L1 + reach, thr) || q1.L3 <= fminf(q1.L1 + reach, thr);
+      return __syncthreads_count(tie) > most;
+    };
+    for (int xs = t.xlo; xs <= t.xhi; xs += kSlab) {
+      const int xe = min(t.xhi, xs + kSlab - 1);
+      const int wu = xe - xs + 1 + kPad;
+      const int band = kCsSmem / (wu * 32);
+      // The bands from the middle one on, whose rows most windows hold, and its
+      // first rows alone: ties show there.
+      const int n = (t.c1 - t.c0 + band) / band;
+      int at = n / 2, yb = t.c0 + at * band, step = min(band, kCsTieRows);
+      for (int left = n; left > 0;) {
+        const int end = min(t.c1, t.c0 + at * band + band - 1);
+        const int rows = min(step, end - yb + 1);
+        if (tied()) {
+          leave_to_exact();
+          return;
+        }
+        for (int j = tid; j < rows * wu; j += kCsThreads) {
+          const int rr = j / wu, c = j - rr * wu;
+          float nx = 0.f, ny = 0.f, nz = 0.f, mc = 0.25f * kFarS * 0.8f;
+          if (xs + c <= xe) {
+            const int g = (yb + rr) * k.W + xs + c;
+            const float4 a = A[g];
+            if (a.z > 0.f) {
+              const float2 b = B[g];
+              nx = a.w * s_k[3];
+              ny = b.x * s_k[3];
+              nz = b.y * s_k[3];
+              mc = s_k[4] * cs_dot(a.w, b.x, b.y, a.x - s_k[0], a.y - s_k[1], a.z - s_k[2]);
             }
-            cs_store_mma(cs_smem + 2 * j, nx, ny, nz, mc);
           }
-        } else if (filter) {
-          for (int j = tid; j < rows * (wu >> 1); j += kCsThreads) {
-            const int rr = j / (wu >> 1), c = 2 * (j - rr * (wu >> 1));
-            float nx[2], ny[2], nz[2], mc[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              nx[h] = ny[h] = nz[h] = 0.f;
-              mc[h] = kCsNone;
-              if (xs + c + h <= xe) {
-                const int g = (yb + rr) * k.W + xs + c + h;
-                const float4 a = A[g];
-                if (a.z > 0.f) {
-                  const float2 b = B[g];
-                  nx[h] = a.w;
-                  ny[h] = b.x;
-                  nz[h] = b.y;
-                  mc[h] = -cs_dot(a.w, b.x, b.y, a.x - o[0], a.y - o[1], a.z - o[2]);
-                }
-              }
-            }
-            cs_smem[2 * j] = make_float4(nx[0], nx[1], ny[0], ny[1]);
-            cs_smem[2 * j + 1] = make_float4(nz[0], nz[1], mc[0], mc[1]);
-          }
-        } else {
-          for (int j = tid; j < rows * wu; j += kCsThreads) {
-            const int rr = j / wu, c = j - rr * wu;
-            float4 a = make_float4(kCsFar, kCsFar, 0.f, kCsFar);
-            float2 b = make_float2(0.f, 0.f);
-            if (xs + c <= xe) {
-              const int g = (yb + rr) * k.W + xs + c;
-              a = A[g];
-              b = B[g];
-            }
-            cs_smem[2 * j] = a;
-            cs_smem[2 * j + 1] = make_float4(b.x, b.y, 0.f, 0.f);
-          }
+          cs_store_mma(cs_smem + 2 * j, nx, ny, nz, mc);
         }
         __syncthreads();
         if (some) {
           const int ca = max(xs, ua), cb = min(xe, ub), ya = max(yb, wvl - r), yz = min(yb + rows - 1, wvh + r);
-          if (ca <= cb) {
-            if (mma)
-              cs_scan_mma(cs_smem, wu, xs, yb, ca, cb, ia, ib, ya, yz, af, first, q0, q1, eps, k);
-            else if (kAngle && filter)
-              cs_scan<kAngle, false>(cs_smem, wu, xs, yb, ca, cb, ia, min(ib, cb), ya, yz, q0, q1, eps, k);
-            else
-              cs_scan<kAngle, true>(cs_smem, wu, xs, yb, ca, cb, ia, ib, ya, yz, q0, q1, 0.f, k);
-          }
+          if (ca <= cb) cs_scan_mma(cs_smem, wu, xs, yb, ca, cb, ia, ib, ya, yz, af, first, q0, q1, eps, k);
+        }
+        yb += step;
+        step = band;
+        if (yb > end) {
+          --left;
+          if (++at == n) at = 0;
+          yb = t.c0 + at * band;
         }
       }
     }
-    if (mma) {  // back to metres (powers of two); what is not there has no value
-      const float un = 1.f / (sw * sn);
-      eps *= un;
-      auto unscale = [&](CsLane& q) {
-        q.g1 = q.L1 < 0.5f * kFarS ? q.g1 : -1;
-        q.g2 = q.L2 < 0.5f * kFarS ? q.g2 : -1;
-        q.L1 = q.L1 < 0.5f * kFarS ? q.L1 * un : kCsNone;
-        q.L2 = q.L2 < 0.5f * kFarS ? q.L2 * un : kCsNone;
-        q.L3 = q.L3 < 0.5f * kFarS ? q.L3 * un : kCsNone;
-      };
-      unscale(q0);
-      unscale(q1);
+    if (tied()) {
+      leave_to_exact();
+      return;
     }
   }
-  if (on0) {
-    part.a[(size_t)chunk * k.P + px0] = make_float4(q0.L1, q0.L2, q0.L3, eps);
-    part.g[(size_t)chunk * k.P + px0] = make_int2(q0.g1, q0.g2);
+  // back to metres (powers of two); what is not there has no value
+  const float un = 1.f / (sw * sn);
+  auto leave = [&](CsLane& l, int px) {
+    const size_t at = (size_t)chunk * k.P + px;
+    part.a[at] = make_float4(l.L1 < 0.5f * kFarS ? l.L1 * un : kCsNone, l.L2 < 0.5f * kFarS ? l.L2 * un : kCsNone,
+                             l.L3 < 0.5f * kFarS ? l.L3 * un : kCsNone, eps * un);
+    part.g[at] = make_int2(l.L1 < 0.5f * kFarS ? l.g1 : -1, l.L2 < 0.5f * kFarS ? l.g2 : -1);
+  };
+  if (on0) leave(q0, px0);
+  if (on1) leave(q1, px1);
+}
+
+// ----------------------------------------------------------------------------
+// exact scan
+// ----------------------------------------------------------------------------
+constexpr int kExPx = 4;  // a lane's pixels, one below the other
+
+// The rows [yb, yb + rows) of the columns [xs, xe], of which the lane takes every
+// second row, against the lane's pixels.
+template <bool kAngle, bool kCap>
+__device__ __forceinline__ void cs_scan_exact(const float4* sA, const float2* sB, int wu, int xs, int xe, int yb, int rows,
+                                              int half, int lo, int hi, int il, int ih, int pl, int ph,
+                                              const float3 (&v)[kExPx], const float3 (&n)[kExPx],
+                                              const int (&pu)[kExPx], const int (&pv)[kExPx], float (&L)[kExPx],
+                                              int (&G)[kExPx], const CorrConsts& k) {
+  const int r = k.radius, ca = max(lo, xs), cb = min(hi, xe), yz = min(yb + rows - 1, ph);
+  int yy = max(yb, pl);
+  yy += (yy ^ half) & 1;
+  for (; yy <= yz; yy += 2) {
+    const float4* ra = sA + (yy - yb) * wu - xs;
+    const float2* rb = sB + (yy - yb) * wu - xs;
+    for (int g = ca; g <= cb; g += kGroup) {
+      const int e = min(cb, g + kGroup - 1);
+      float m[kExPx];
+#pragma unroll
+      for (int i = 0; i < kExPx; ++i) m[i] = INFINITY;
+      auto edge = [&](int c) {  // a column that some of the windows hold
+        const float4 a = ra[c];
+        const float2 b = rb[c];
+#pragma unroll
+        for (int i = 0; i < kExPx; ++i) {
+          const float d = cs_pd<kAngle, kCap>(v[i], n[i], a, b, k);
+          m[i] = (unsigned)(c - pu[i] + r) <= 2u * r ? fminf(m[i], d) : m[i];
+        }
+      };
+      int c = g;
+      for (; c < il && c <= e; ++c) edge(c);
+      const int z = min(e, ih);
+#pragma unroll 2
+      for (; c < z; c += 2) {
+        const float4 a0 = ra[c], a1 = ra[c + 1];
+        const float2 b0 = rb[c], b1 = rb[c + 1];
+#pragma unroll
+        for (int i = 0; i < kExPx; ++i)
+          m[i] = cs_min_abs(m[i], cs_pd<kAngle, kCap>(v[i], n[i], a0, b0, k), cs_pd<kAngle, kCap>(v[i], n[i], a1, b1, k));
+      }
+      for (; c <= e; ++c) edge(c);
+      const int at = yy * k.W + g;
+#pragma unroll
+      for (int i = 0; i < kExPx; ++i)
+        if ((unsigned)(yy - pv[i] + r) <= 2u * r && (m[i] < L[i] || (m[i] == L[i] && at < G[i]))) {
+          L[i] = m[i];
+          G[i] = at;
+        }
+    }
   }
-  if (on1) {
-    part.a[(size_t)chunk * k.P + px1] = make_float4(q1.L1, q1.L2, q1.L3, eps);
-    part.g[(size_t)chunk * k.P + px1] = make_int2(q1.g1, q1.g2);
+}
+
+// The reference's arithmetic on every candidate.  A lane's four pixels share each
+// candidate's load; shared memory's data path (six cycles per 32 records) is
+// what bounds it with two.  The CTA's halves take every second row each.  Leaves of each
+// pixel the least distance and the first run in row-major order that has it.
+// all: the whole frame; otherwise the chunks that the search has left.
+template <bool kAngle>
+__global__ void __launch_bounds__(kCsThreads, kExCtasPerSm)
+    corr_exact_kernel(const CorrConsts k, const float4* __restrict__ A, const float2* __restrict__ B, const CsPix pix,
+                      const CsBox* __restrict__ box, const int* __restrict__ flag, const CsPart part, int tiles_x,
+                      int tiles, bool all) {
+  cs_after_previous();
+  extern __shared__ float4 cs_smem[];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, half = wid >> 2, r = k.radius;
+  const int items = all ? tiles * k.chunks : *part.todo;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int what = all ? 2 * item : part.todo[1 + item];
+    const int chunk = (what >> 1) / tiles, tile = (what >> 1) - chunk * tiles, ty = tile / tiles_x,
+              tx = tile - ty * tiles_x;
+    CsTile t;
+    if (!cs_tile(k, box, flag, tx, ty, chunk, t)) continue;
+    bool any = true, cap = what & 1;
+    if (all) {
+      const CsReach q = cs_reach(k, box, t);
+      any = q.any;
+      cap = q.cap;
+    }
+    const int x = tx * kCsTx + lane, y0 = ty * kCsTy + kExPx * (wid & 3), px = y0 * k.W + x;
+    float3 v[kExPx], n[kExPx];
+    int pu[kExPx], pv[kExPx], G[kExPx];
+    float L[kExPx];
+    unsigned on = 0;
+    // the windows' union, the columns common to them, their rows
+    int lo = k.W, hi = -1, il = 0, ih = k.W, pl = k.H, ph = -1;
+#pragma unroll
+    for (int i = 0; i < kExPx; ++i) {
+      CsPixel p;
+      p.search = p.special = false;
+      if (x < k.W && y0 + i < k.H) p = cs_load_pixel(pix, px + i * k.W);
+      v[i] = n[i] = make_float3(0.f, 0.f, 0.f);
+      pu[i] = 0;
+      pv[i] = -(1 << 30);
+      if (p.search && !p.special) {
+        on |= 1u << i;
+        v[i] = p.vc;
+        if (kAngle) n[i] = p.nc;
+        pu[i] = p.pu;
+        pv[i] = p.pv;
+        lo = min(lo, max(0, p.pu - r));
+        hi = max(hi, min(k.W - 1, p.pu + r));
+        il = max(il, p.pu - r);
+        ih = min(ih, p.pu + r);
+        pl = min(pl, p.pv - r);
+        ph = max(ph, p.pv + r);
+      }
+      L[i] = INFINITY;
+      G[i] = -1;
+    }
+    for (int xs = t.xlo; xs <= t.xhi && any; xs += kSlab) {
+      const int xe = min(t.xhi, xs + kSlab - 1), wu = xe - xs + 1, band = kExSmem / (wu * 24);
+      float2* sB = reinterpret_cast<float2*>(cs_smem + (size_t)band * wu);
+      for (int yb = t.c0; yb <= t.c1; yb += band) {
+        const int rows = min(band, t.c1 - yb + 1);
+        __syncthreads();
+        for (int j = tid; j < rows * wu; j += kCsThreads) {
+          const int rr = j / wu, g = (yb + rr) * k.W + xs + j - rr * wu;
+          cs_smem[j] = A[g];
+          sB[j] = B[g];
+        }
+        __syncthreads();
+        if (cap) cs_scan_exact<kAngle, false>(cs_smem, sB, wu, xs, xe, yb, rows, half, lo, hi, il, ih, pl, ph, v, n, pu, pv, L, G, k);
+        else cs_scan_exact<kAngle, true>(cs_smem, sB, wu, xs, xe, yb, rows, half, lo, hi, il, ih, pl, ph, v, n, pu, pv, L, G, k);
+      }
+    }
+    // the halves together
+    __syncthreads();
+    float2* both = reinterpret_cast<float2*>(cs_smem) + (tid & 127);
+    if (half) {
+#pragma unroll
+      for (int i = 0; i < kExPx; ++i) both[128 * i] = make_float2(L[i], __int_as_float(G[i]));
+    }
+    __syncthreads();
+    if (!half) {
+#pragma unroll
+      for (int i = 0; i < kExPx; ++i) {
+        if (!((on >> i) & 1u)) continue;
+        const float2 h = both[128 * i];
+        const int g = __float_as_int(h.y);
+        if (h.x < L[i] || (h.x == L[i] && g < G[i])) {
+          L[i] = h.x;
+          G[i] = g;
+        }
+        const size_t at = (size_t)chunk * k.P + px + i * k.W;
+        part.a[at] = make_float4(L[i], INFINITY, INFINITY, 0.f);
+        part.g[at] = make_int2(G[i], -1);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -988,27 +1053,37 @@ struct CsBest {
   }
 };
 
-// A pixel's n rows of w candidates from row0 (columns from l), the warp's lanes
-// on consecutive ones of them: the lane's first least in row-major order.
-template <bool kAngle, bool kCap>
-__device__ __forceinline__ void cs_rows(const CorrConsts& k, const float3& v, const float3& nc, int row0, int n, int l,
-                                        int w, int lane, const float4* __restrict__ A, const float2* __restrict__ B,
-                                        CsBest& b) {
+constexpr int kFly = 6;  // loads in flight
+// A pixel's n rows of w candidates from row0 (columns from l), all within the
+// cap, the warp's lanes on consecutive ones of them: the lane's first least in
+// row-major order.
+__device__ __forceinline__ void cs_rows(const CorrConsts& k, const float3& v, int row0, int n, int l, int w, int lane,
+                                        const float4* __restrict__ A, const float2* __restrict__ B, CsBest& b) {
   const int total = n * w, dy = 32 / w, dx = 32 - dy * w;
   int y = lane / w, x = lane - y * w;
-#pragma unroll 8
-  for (int t = lane; t < total; t += 32) {
-    const int i = (row0 + y) * k.W + l + x;
-    const float d = cs_pd<kAngle, kCap>(v, nc, A[i], B[i], k);
-    if (d < b.pd) {
-      b.pd = d;
-      b.i = i;
+  for (int t = lane; t < total; t += 32 * kFly) {
+    int at[kFly];
+    float4 a[kFly];
+    float2 c[kFly];
+#pragma unroll
+    for (int h = 0; h < kFly; ++h) {  // the loads together (one by one they take three times as long)
+      at[h] = t + 32 * h < total ? (row0 + y) * k.W + l + x : -1;
+      a[h] = at[h] >= 0 ? A[at[h]] : make_float4(kCsFar, kCsFar, 0.f, kCsFar);
+      c[h] = at[h] >= 0 ? B[at[h]] : make_float2(0.f, 0.f);
+      x += dx;
+      y += dy;
+      if (x >= w) {
+        x -= w;
+        ++y;
+      }
     }
-    x += dx;
-    y += dy;
-    if (x >= w) {
-      x -= w;
-      ++y;
+#pragma unroll
+    for (int h = 0; h < kFly; ++h) {
+      const float d = cs_pd<false, false>(v, v, a[h], c[h], k);
+      if (d < b.pd) {
+        b.pd = d;
+        b.i = at[h];
+      }
     }
   }
 }
@@ -1017,7 +1092,11 @@ __device__ __forceinline__ void cs_rows(const CorrConsts& k, const float3& v, co
 // in flight together, and four pixels' runs per warp; a warp per run took
 // three times as long).  Pixels whose third value is within the bound have those
 // chunks' rows evaluated by the CTA's warps.
-// kDirect: no search went before, each lane scans its pixel's window (rule at
+// own: the exact scan saw every chunk, and a lane evaluates its own pixel's one
+// run.  Shorter while the merge is at most two CTAs per SM and its chain of loads
+// is what it takes (160 x 120 at radius 20: 70 us a call with eight lanes, 63), longer
+// beyond (640 x 480: 282 and 290).
+// kDirect: no scan went before, each lane scans its pixel's window (rule at
 // kCsDirect).
 constexpr int kMergeThreads = 256;
 static_assert(kMergeThreads <= 256 && kCorrMaxChunks <= 8, "an item: pixel, chunk");
@@ -1025,14 +1104,14 @@ template <bool kAngle, bool kDirect>
 __global__ void __launch_bounds__(kMergeThreads)
     corr_merge_kernel(const CorrConsts k, const float* __restrict__ lv, const float4* __restrict__ A,
                       const float2* __restrict__ B, const CsPix pix, const int* __restrict__ flag, const CsPart part,
-                      const KnnSrc knn, cf_correspondence* __restrict__ out, int* __restrict__ num_valid,
+                      const KnnSrc knn, bool own, cf_correspondence* __restrict__ out, int* __restrict__ num_valid,
                       int* __restrict__ stats) {
   after_previous();
   __shared__ float s_stage[kMergeThreads / 32][32 * kCsRecWords];
   __shared__ unsigned long long s_key[kMergeThreads];  // distance bits, candidate: the least first
   __shared__ unsigned short s_items[kMergeThreads * kCorrMaxChunks];
   __shared__ int s_count, s_next;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int px = blockIdx.x * kMergeThreads + tid;
   const bool inimg = px < k.P;
   CsPixel p;
@@ -1054,6 +1133,7 @@ __global__ void __launch_bounds__(kMergeThreads)
   const bool on = p.search && !p.special;
   // an upper bound of the winner's distance, and the runs that can hold it: bit
   // 2 c + s the chunk's s-th
+  CsBest best = {k.dist_thr, -1};
   float U = k.dist_thr;
   unsigned runs = 0, again = 0;  // again: the chunks of which more runs could
   if (!kDirect && on) {
@@ -1061,13 +1141,23 @@ __global__ void __launch_bounds__(kMergeThreads)
       const float4 a = part.a[(size_t)c * k.P + px];
       U = fminf(U, a.x + 2.25f * a.w);
     }
+    unsigned only = 0;
+    float found = INFINITY;  // the least of the exact scan: one run, the first that has it
     for (int c = 0; c < k.chunks; ++c) {
       const float4 a = part.a[(size_t)c * k.P + px];
+      if (a.w == 0.f) {
+        if (a.x <= U && a.x < found) {
+          found = a.x;
+          runs &= ~only;
+          only = 1u << (2 * c);
+          runs |= only;
+        }
+        continue;
+      }
       runs |= (a.x <= U ? 1u : 0u) << (2 * c) | (a.y <= U ? 2u : 0u) << (2 * c);
       again |= (a.z <= U ? 1u : 0u) << c;
     }
   }
-  CsBest best = {k.dist_thr, -1};
   if (kDirect && on) {
     const int l = max(0, p.pu - k.radius), h = min(k.W - 1, p.pu + k.radius);
     const int ya = max(0, p.pv - k.radius), yz = min(k.H - 1, p.pv + k.radius);
@@ -1081,7 +1171,29 @@ __global__ void __launch_bounds__(kMergeThreads)
         }
       }
   }
-  for (unsigned todo; !kDirect && (todo = __ballot_sync(0xffffffffu, runs != 0)) != 0;) {
+  if (!kDirect && own && runs) {  // the one run that the exact scan has found
+    const int g = part.g[(size_t)((__ffs(runs) - 1) >> 1) * k.P + px].x, row0 = g / k.W * k.W, c0 = g - row0;
+    const int l = max(c0, p.pu - k.radius), h = min(min(c0 + kGroup - 1, k.W - 1), p.pu + k.radius);
+    for (int col = l; col <= h; col += kFly) {
+      float4 a[kFly];
+      float2 b[kFly];
+#pragma unroll
+      for (int j = 0; j < kFly; ++j) {
+        const int i = row0 + min(col + j, h);
+        a[j] = A[i];
+        b[j] = B[i];
+      }
+#pragma unroll
+      for (int j = 0; j < kFly; ++j) {
+        const float d = cs_pd<kAngle>(p.vc, p.nc, a[j], b[j], k);
+        if (d < best.pd) {
+          best.pd = d;
+          best.i = row0 + min(col + j, h);
+        }
+      }
+    }
+  }
+  for (unsigned todo; !kDirect && !own && (todo = __ballot_sync(0xffffffffu, runs != 0)) != 0;) {
     const unsigned mine = (todo >> (lane & 24)) & 0xffu;  // of this lane's eight pixels
     const int src = (lane & 24) + (mine ? __ffs(mine) - 1 : 0);
     int gs = -1;
@@ -1121,12 +1233,11 @@ __global__ void __launch_bounds__(kMergeThreads)
   }
   // The pixels left: the rows of their chunks, a chunk at a time to the CTA's
   // next free warp (a surface of equal distances leaves whole CTAs of them).
-  if (!kDirect) {
-    float* q = s_stage[0] + 8 * tid;  // (the records' staging is not in use yet)
+  if (!kDirect && !kAngle && !own) {  // (only the search leaves such, and it knows no angle)
+    float* q = s_stage[0] + 5 * tid;  // (the records' staging is not in use yet)
     if (again) {
       q[0] = p.vc.x; q[1] = p.vc.y; q[2] = p.vc.z;
-      q[3] = p.nc.x; q[4] = p.nc.y; q[5] = p.nc.z;
-      q[6] = __int_as_float(p.pu); q[7] = __int_as_float(p.pv);
+      q[3] = __int_as_float(p.pu); q[4] = __int_as_float(p.pv);
       s_key[tid] = best.i < 0 ? ~0ull : (unsigned long long)__float_as_uint(best.pd) << 32 | (unsigned)best.i;
       for (unsigned m = again; m; m &= m - 1)
         s_items[atomicAdd(&s_count, 1)] = (unsigned short)(tid | (__ffs(m) - 1) << 8);
@@ -1139,18 +1250,16 @@ __global__ void __launch_bounds__(kMergeThreads)
       t = __shfl_sync(0xffffffffu, t, 0);
       if (t >= items) break;
       const int src = s_items[t] & 255, cc = s_items[t] >> 8;
-      const float* r = s_stage[0] + 8 * src;
-      const float3 v = make_float3(r[0], r[1], r[2]), nc = make_float3(r[3], r[4], r[5]);
-      const int pu = __float_as_int(r[6]), pv = __float_as_int(r[7]);
+      const float* r = s_stage[0] + 5 * src;
+      const float3 v = make_float3(r[0], r[1], r[2]);
+      const int pu = __float_as_int(r[3]), pv = __float_as_int(r[4]);
       const int spx = blockIdx.x * kMergeThreads + src, y = spx / k.W, x = spx - y * k.W;
       const int2 rw = part.rows[y / kCsTy * ((k.W + kCsTx - 1) / kCsTx) + x / kCsTx];
-      const bool within = part.a[(size_t)cc * k.P + spx].w > 0.f;  // the chunk's candidates are within the cap
       const int l = max(0, pu - k.radius), w = min(k.W - 1, pu + k.radius) - l + 1;
       const int ya = max(max(0, pv - k.radius), rw.x + cc * rw.y),
                 n = min(min(k.H - 1, pv + k.radius), rw.x + cc * rw.y + rw.y - 1) - ya + 1;
       CsBest b = {k.dist_thr, -1};
-      if (within) cs_rows<kAngle, false>(k, v, nc, ya, n, l, w, lane, A, B, b);
-      else cs_rows<kAngle, true>(k, v, nc, ya, n, l, w, lane, A, B, b);
+      cs_rows(k, v, ya, n, l, w, lane, A, B, b);
 #pragma unroll
       for (int o = 16; o; o >>= 1) {
         const float d = __shfl_xor_sync(0xffffffffu, b.pd, o);
@@ -1221,14 +1330,17 @@ float sqrt_bound(float cap) {
 // its scan of 512 pixels x S/C candidates goes at 9 per clock beside two others,
 // the last CTAs run with fewer beside them, so the waves count as
 // tiles x C / slots + 0.4; the merge reads each chunk for 5000 at 640 x 480.
-int corr_pick_chunks(int tiles, int sms, int radius, int W, int H) {
-  const double slots = (double)(sms > 0 ? sms : 1) * kCsCtasPerSm;
+// The exact scan: 6000, 6.4 beside one other, 0.3 (80 x 60 to 1280 x 960 at radii
+// 4 to 50: within 2 % of the best number of chunks, 7 % at most).
+int corr_pick_chunks(int tiles, int sms, int radius, int W, int H, bool filter) {
+  const double slots = (double)(sms > 0 ? sms : 1) * (filter ? kCsCtasPerSm : kExCtasPerSm);
   const double side_x = std::fmin(2.0 * radius + 8.0, (double)W), side_y = std::fmin(2.0 * radius + 8.0, (double)H);
-  const double scan = 512.0 * side_x * side_y / 9.0, merge = 5000.0 * ((double)W * H / 307200.0);
+  const double setup = filter ? 9000.0 : 6000.0, tail = filter ? 0.4 : 0.3;
+  const double scan = 512.0 * side_x * side_y / (filter ? 9.0 : 6.4), merge = 5000.0 * ((double)W * H / 307200.0);
   int best_c = 1;
   double best = 1e300;
   for (int c = 1; c <= kCorrMaxChunks; ++c) {
-    const double t = ((double)tiles * c / slots + 0.4) * (9000.0 + scan / c) + merge * c;
+    const double t = ((double)tiles * c / slots + tail) * (setup + scan / c) + merge * c;
     if (t < best * (1.0 - 1e-9)) {
       best = t;
       best_c = c;
@@ -1300,34 +1412,42 @@ cudaError_t launch_corr_search(const cf_corr_frame* f, const cf_camera* cam, con
   if (e != cudaSuccess) return e;
 
   const dim3 tiles((W + kCsTx - 1) / kCsTx, (H + kCsTy - 1) / kCsTy);
-  const int want = chunks > 0 ? chunks : corr_pick_chunks((int)(tiles.x * tiles.y), sc.sms, k.radius, W, H);
-  k.chunks = want < sc.chunk_cap ? want : sc.chunk_cap;
   const bool angle = p->angle_threshold > 0.f;
-  auto kern = angle ? corr_search_kernel<true> : corr_search_kernel<false>;
+  const double side = 2.0 * k.radius + 1.0;
+  const bool filter = !angle && (double)k.P * std::fmin(side, W) * std::fmin(side, H) > kCsFilter;
+  const int want = chunks > 0 ? chunks : corr_pick_chunks((int)(tiles.x * tiles.y), sc.sms, k.radius, W, H, filter);
+  k.chunks = want < sc.chunk_cap ? want : sc.chunk_cap;
+  auto exact = angle ? corr_exact_kernel<true> : corr_exact_kernel<false>;
   const bool direct = k.radius <= kCsDirect;
   auto merge = direct ? (angle ? corr_merge_kernel<true, true> : corr_merge_kernel<false, true>)
                       : (angle ? corr_merge_kernel<true, false> : corr_merge_kernel<false, false>);
   // per device and cheap: set on every call rather than cached per device
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCsSmem);
+  e = cudaFuncSetAttribute(corr_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCsSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(exact, cudaFuncAttributeMaxDynamicSharedMemorySize, kExSmem);
   if (e != cudaSuccess) return e;
-  const CsPart part = {sc.part_a, sc.part_g, sc.rows};
+  const CsPart part = {sc.part_a, sc.part_g, sc.rows, sc.todo};
 
   const CsPix pix = {sc.pix_v, sc.pix_n, sc.pix_row};
   CsBox* box = static_cast<CsBox*>(sc.box);
   launch_next(corr_prep_kernel, dim3((W + kCsBlock - 1) / kCsBlock, (H + kCsBlock - 1) / kCsBlock),
               kCsBlock * kCsBlock, 0, s, k, f->d_depth, f->d_depth_normals, f->d_live_vertices, f->d_live_normals,
-              sc.A, sc.B, pix, box, sc.flag, num_valid, stats);
+              sc.A, sc.B, pix, box, sc.flag, sc.todo, num_valid, stats);
   // (launch_next only for the short calls: CTAs of the merge that wait beside a
   // running search cost 15 of 573 us at radius 50)
   const int mg = (k.P + kMergeThreads - 1) / kMergeThreads;
   if (direct) {
-    launch_next(merge, mg, kMergeThreads, 0, s, k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag, part, knn, out,
+    launch_next(merge, mg, kMergeThreads, 0, s, k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag, part, knn, true, out,
                 num_valid, stats);
   } else {
-    kern<<<dim3(tiles.x, tiles.y, k.chunks), kCsThreads, kCsSmem, s>>>(k, sc.A, sc.B, pix, box, sc.flag, part);
-    merge<<<mg, kMergeThreads, 0, s>>>(k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag, part, knn, out, num_valid, stats);
+    const dim3 grid(tiles.x, tiles.y, k.chunks);
+    if (filter) corr_search_kernel<<<grid, kCsThreads, kCsSmem, s>>>(k, sc.A, sc.B, pix, box, sc.flag, part);
+    const int n = (int)(tiles.x * tiles.y), items = n * k.chunks, slots = kExCtasPerSm * (sc.sms > 0 ? sc.sms : 1);
+    launch_next(exact, filter && items > slots ? slots : items, kCsThreads, kExSmem, s, k, sc.A, sc.B, pix, box, sc.flag,
+                part, (int)tiles.x, n, !filter);
+    launch_next(merge, mg, kMergeThreads, 0, s, k, f->d_live_vertices, sc.A, sc.B, pix, sc.flag, part, knn,
+                !filter && mg <= 2 * sc.sms, out, num_valid, stats);
   }
-  *launches += direct ? 2 : 3;
+  *launches += direct ? 2 : filter ? 4 : 3;
   return cudaGetLastError();
 }
 

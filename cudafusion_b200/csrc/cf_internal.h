@@ -300,6 +300,7 @@ struct CorrScratch {
   float4* part_a;  // [chunk_cap][pixels]: each row chunk's three least values, and their error bound
   int2* part_g;    // [chunk_cap][pixels]: the runs of the first two
   int2* rows;      // per tile of pixels: the rows that it scans, by chunk
+  int* todo;       // [1 + kCorrMaxChunks * tiles]: what is left to the exact scan
   void* box;       // [blocks]: what is known of each block of 16 x 16 pixels
   float4 *pix_v, *pix_n;  // per pixel: its camera-frame point, normal, projection ...
   int* pix_row;           // ... and state
@@ -307,7 +308,7 @@ struct CorrScratch {
   int* flag;       // set when a value could make a distance NaN
   int sms;
 };
-int corr_pick_chunks(int tiles, int sms, int radius, int W, int H);
+int corr_pick_chunks(int tiles, int sms, int radius, int W, int H, bool filter);
 int corr_chunk_cap(size_t P);
 size_t corr_box_cap(size_t P);
 size_t corr_box_bytes();
