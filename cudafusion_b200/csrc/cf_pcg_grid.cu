@@ -173,10 +173,13 @@ __device__ __forceinline__ void wsum_parts(const double* parts, int G, int strid
 // do not depend on the order.  A line holds two words, each a sum << kDotCount with
 // the number of arrivals below it; a sum v goes in units of 2^(e - 30) (high word)
 // and what is left in units of 2^(e - 62) (low word), e the exponent of a value
-// that every CTA knows to be of v's size.  |v| < 2^(e + 12), so that kMaxPcgCtas of
-// them fit; any other (or no usable e) counts in the low word's top bits and the
-// exchange is repeated with stored partials behind the counter barrier.  The total
-// is within G 2^(e - 62) of the partials' exact sum: what G additions in FP64 lose.
+// that every CTA knows and that is usually of v's size (the sum before it).  |v| <
+// 2^(e + 12), so that kMaxPcgCtas of them fit; any other (or no usable e) counts in
+// the low word's top bits.  Each CTA's low word is rounded down, so the total is up
+// to G 2^(e - 62) below the partials' exact sum: no more than G additions in FP64
+// may lose while the total is at least 2^(e - 9).  A smaller total, or one that does not
+// fit, is taken again from stored partials behind the counter barrier; all CTAs
+// decide so, from the same words.
 // The words only grow: a CTA remembers them as it last saw them, and none can
 // run an exchange ahead of another.  (Four lines, each for a quarter of the CTAs,
 // are no faster: 81.6 us per launch at 2048 nodes against 78.7 with one.)
@@ -186,6 +189,7 @@ struct DotLine {
 constexpr int kDotStride = 16;  // words: a line of its own for each exchange
 constexpr int kDotCount = 11;   // bits of the count
 constexpr int kDotOver = 42;    // bit of the low sum from which "does not fit" is counted
+constexpr int kDotFall = 9;     // binary orders that a total may be below the one before it
 static_assert(kMaxPcgCtas < (1 << kDotCount) && kDotCount + kDotOver + 10 < 64, "the counts fit their bits");
 
 // kAcquire: what was released with the counts is seen after it.
@@ -229,7 +233,7 @@ __device__ __forceinline__ void dot_arrive(unsigned long long* p, double v, int 
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(h) : "memory");
 }
 // Waits (bounded, as arrive_wait) for G arrivals past `base`; the total into v.
-// False: it does not fit.
+// False: it does not fit, or is so small that the units show.
 template <bool kAcquire>
 __device__ __forceinline__ bool dot_wait(const unsigned long long* p, DotLine& base, int G, int e, double& v, int* err,
                                          unsigned spin_limit, unsigned extra) {
@@ -256,7 +260,7 @@ __device__ __forceinline__ bool dot_wait(const unsigned long long* p, DotLine& b
   const unsigned long long l = (d.lo - (unsigned)G) >> kDotCount;
   if (e == kNoExp || (l >> kDotOver)) return false;
   v = (double)h * pow2(e - 30) + (double)l * pow2(e - 62);
-  return true;
+  return fabs(v) >= pow2(e - kDotFall);
 }
 
 template <bool A_SMEM, bool PIPE>
