@@ -23,7 +23,9 @@
 // Schedule and guards follow kernels/solver_kernels.cu:616-687 (PCG from
 // x = 0, |p.Ap| < 1e-12 stops before the update, ||r|| < tol after it); FP64
 // block inverses and dot products, FP32 matrix and vectors.  The waits are
-// bounded: past the limit the kernel records kErrTimeout and runs out.
+// bounded (polls, and time): past the limit a CTA records kErrTimeout and leaves the
+// iterations, the others follow when they see that, and none exits while a message
+// may still be under way to it.
 //
 // Measured (B200, event time of a launch less its fixed 10-20 us): 2.8 us per
 // iteration at 256 nodes, 3.1 at 512, 4.6 at 1024, 6.4 at 2048; with upper blocks
@@ -116,7 +118,8 @@ __device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
   return ok != 0;
 }
 
-constexpr long long kClWaitCycles = 1ll << 32;  // a wait gives up after about two seconds
+constexpr long long kClWaitCycles = 1ll << 32;  // a wait gives up after about two seconds, or spin_limit polls
+constexpr long long kClDrainCycles = 1ll << 17;  // far longer than a message takes
 
 // A row's residual, x, z and its row of the inverse live with the first of its
 // kSpl lanes per element.
@@ -155,8 +158,8 @@ __global__ void __launch_bounds__(kSpl == 1 ? 1024 : 768, 1) pcg_cluster_kernel(
   const int n6 = nrows * 6, h6 = nhalo * 6;
   int* err = w.err;
   if (tid == 0) {
-    bar_init(barA, 1);
-    bar_init(barB, 1);
+    bar_init(barA, 1 + min(a.bar_extra, 1024u));
+    bar_init(barB, 1 + min(a.bar_extra, 1024u));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -238,7 +241,7 @@ __global__ void __launch_bounds__(kSpl == 1 ? 1024 : 768, 1) pcg_cluster_kernel(
     const long long t0 = clock64();
     for (unsigned tries = 1; !bar_try(bar, parity); tries++) {
       if (tries & 63) continue;
-      if (clock64() - t0 > kClWaitCycles) atomicOr(err, kErrTimeout);
+      if (tries > a.spin_limit || clock64() - t0 > kClWaitCycles) atomicOr(err, kErrTimeout);
       if (*(volatile int*)err & kErrTimeout) {
         dead = true;
         return;
@@ -321,7 +324,7 @@ __global__ void __launch_bounds__(kSpl == 1 ? 1024 : 768, 1) pcg_cluster_kernel(
       used = it;
       float beta = 0.f;
       // (the root only where it can be below the tolerance) solver_kernels.cu:669
-      bool stop = it >= a.pcg_iterations;
+      bool stop = it >= a.pcg_iterations || dead;  // (lane 0's; after the other exchange this one ends the loop)
       if (it > 0) {
         stop |= !(srr >= tol2) && sqrt(srr) < tol;
         beta = (float)(srz / rz);
@@ -414,6 +417,9 @@ __global__ void __launch_bounds__(kSpl == 1 ? 1024 : 768, 1) pcg_cluster_kernel(
     st->pcg_iters[P.slot] = used;
     st->pcg_res[P.slot] = sqrt(rr_last);
   }
+  if (dead)  // messages that were not waited for (who never gave up has received all of its own)
+    for (const long long t0 = clock64(); clock64() - t0 < kClDrainCycles;) {
+    }
 }
 
 // Lanes per row element: four while that takes at most 24 warps per CTA, else
