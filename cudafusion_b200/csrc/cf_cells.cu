@@ -592,7 +592,7 @@ __device__ __forceinline__ float3 blend_cell(float3 p, unsigned perm, const floa
           const int cj = (perm >> (3 * j)) & 7;
           if (cj >= 4 && cj < 7 && (int)((perm >> (12 + 2 * j)) & 3) == a) w -= sel4(uw, cj - 3);
         }
-      add(load_dq_ldg(plain + sel4i(ids, a)), w);
+      add(load_dq(plain + sel4i(ids, a)), w);
     }
   } else {
     DQ q[kK];
@@ -603,7 +603,7 @@ __device__ __forceinline__ float3 blend_cell(float3 p, unsigned perm, const floa
       q[k].r = q[k].d = make_float4(0.f, 0.f, 0.f, 0.f);
       wt[k] = 0.f;
       if (a < 4) {
-        q[k] = load_dq_ldg(plain + sel4i(ids, a));  // (the plain DQs come from an earlier launch)
+        q[k] = load_dq(plain + sel4i(ids, a));
         wt[k] = sel4(uw, a);
       }
     }
@@ -794,8 +794,8 @@ __global__ void __launch_bounds__(kThreads, kAcc ? 2 : 3) cells_kernel(Table tb,
     }
   };
   enter(w0, size);
-  // what the lists' kernels left is read already (at least one kernel lies
-  // between), the transforms and records from here on
+  // read already: the sorted streams, task sizes and nodes (bucket_sort and permute;
+  // list_sort lies between); from here on the transforms, positions and records
   after_previous();
   for (; w0 < qb || left > 0; w0 += 32) {
     const int q = w0 + lane;
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowWarps == 2 ? 18 : 8) gathe
     for (int i = lane; i < kn * kSums; i += 32) (&m.sum[wid][0][0])[i] = 0.f;
     __syncthreads();
     if (k0 == 0) {
-      after_previous();  // (so far the pattern and the lists)
+      after_previous();  // (so far the pattern and the lists of list_sort; the data term lies between)
       if (r == 0)  // the barriers of the PCG that follows
         for (int i = tid; i < pt.P; i += kRowThreads) w.barrier[i] = 0u;
     }

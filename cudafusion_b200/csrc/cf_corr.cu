@@ -186,8 +186,8 @@ struct CsPixel {
   float view_cos;
 };
 
-__device__ __forceinline__ CsPixel cs_pixel(const CorrConsts& k, const float* __restrict__ lv,
-                                            const float* __restrict__ ln, int px) {
+__device__ __forceinline__ CsPixel cs_pixel(const CorrConsts& k, const float* lv,
+                                            const float* ln, int px) {
   CsPixel p;
   p.code = -1;
   p.search = false;
@@ -273,8 +273,8 @@ constexpr int kCsOff = -(1 << 30);
 // One thread per pixel: the depth's candidate record, the live pixel's record,
 // and the block's box.
 __global__ void __launch_bounds__(kCsBlock* kCsBlock)
-    corr_prep_kernel(const CorrConsts k, const float* __restrict__ depth, const float* __restrict__ dn,
-                     const float* __restrict__ lv, const float* __restrict__ ln, float4* __restrict__ A,
+    corr_prep_kernel(const CorrConsts k, const float* depth, const float* dn,
+                     const float* lv, const float* ln, float4* __restrict__ A,
                      float2* __restrict__ B, const CsPix pix, CsBox* __restrict__ box, int* __restrict__ flag,
                      int* __restrict__ todo, int* __restrict__ num_valid, int* __restrict__ stats) {
   after_previous();
@@ -497,8 +497,8 @@ __device__ __forceinline__ void cs_scan_mma(const float4* sm, int wu, int xs, in
 
 // find_correspondences_kernel's loop as it stands (kernels/tsdf_kernels.cu:470-524),
 // for pixels or frames whose values could make a distance NaN.
-__device__ __forceinline__ int cs_rescan(const CorrConsts& k, const CsPixel& p, const float4* __restrict__ A,
-                                         const float2* __restrict__ B, bool& saw_depth) {
+__device__ __forceinline__ int cs_rescan(const CorrConsts& k, const CsPixel& p, const float4* A,
+                                         const float2* B, bool& saw_depth) {
   const int r = k.radius;
   const int x0 = max(0, p.pu - r), x1 = min(k.W - 1, p.pu + r);
   const int y0 = max(0, p.pv - r), y1 = min(k.H - 1, p.pv + r);
@@ -524,7 +524,7 @@ __device__ __forceinline__ int cs_rescan(const CorrConsts& k, const CsPixel& p, 
 
 // Whether the pixel's window holds any depth (no_depth vs far, for the
 // debug counters of a pixel without a pair).
-__device__ __forceinline__ bool cs_any_depth(const CorrConsts& k, const CsPixel& p, const float4* __restrict__ A) {
+__device__ __forceinline__ bool cs_any_depth(const CorrConsts& k, const CsPixel& p, const float4* A) {
   const int r = k.radius;
   const int x0 = max(0, p.pu - r), x1 = min(k.W - 1, p.pu + r);
   const int y0 = max(0, p.pv - r), y1 = min(k.H - 1, p.pv + r);
@@ -544,7 +544,7 @@ __device__ __forceinline__ bool cs_any_depth(const CorrConsts& k, const CsPixel&
 constexpr int kCsRecWords = (int)(sizeof(cf_correspondence) / 4);
 static_assert(sizeof(cf_correspondence) == 4 * kCsRecWords, "a record is whole words");
 __device__ __forceinline__ void cs_emit(const CorrConsts& k, const CsPixel& p, bool inimg, int px, int bi, int code,
-                                        const float4* __restrict__ A, const float2* __restrict__ B,
+                                        const float4* A, const float2* B,
                                         const KnnSrc& knn, cf_correspondence* __restrict__ out,
                                         int* __restrict__ num_valid, int* __restrict__ stats, int lane,
                                         float* __restrict__ stage) {
@@ -660,7 +660,7 @@ struct CsTile {
   float v[6];  // the live pixels' box: maxima of -x, -y, -z, x, y, z
 };
 // False (over the CTA): nothing is scanned here.
-__device__ __forceinline__ bool cs_tile(const CorrConsts& k, const CsBox* __restrict__ box, const int* __restrict__ flag,
+__device__ __forceinline__ bool cs_tile(const CorrConsts& k, const CsBox* box, const int* flag,
                                         int tx, int ty, int chunk, CsTile& t) {
   // the pixels' boxes: the tile is two blocks
   const int r = k.radius, bpr = (k.W + kCsBlock - 1) / kCsBlock;
@@ -688,7 +688,7 @@ struct CsReach {
   float nn;       // the longest normal
   bool any, cap;  // a real candidate; all of them within the Euclidean cap of all pixels
 };
-__device__ __forceinline__ CsReach cs_reach(const CorrConsts& k, const CsBox* __restrict__ box, const CsTile& t) {
+__device__ __forceinline__ CsReach cs_reach(const CorrConsts& k, const CsBox* box, const CsTile& t) {
   __shared__ float s_d[kCsThreads / 32][7];
   const int tid = threadIdx.x, bpr = (k.W + kCsBlock - 1) / kCsBlock;
   float v[7] = {-INFINITY, -INFINITY, -INFINITY, 0.f, -INFINITY, -INFINITY, -INFINITY};
@@ -741,8 +741,8 @@ __device__ __forceinline__ CsReach cs_reach(const CorrConsts& k, const CsBox* __
 }
 
 __global__ void __launch_bounds__(kCsThreads, kCsCtasPerSm)
-    corr_search_kernel(const CorrConsts k, const float4* __restrict__ A, const float2* __restrict__ B, const CsPix pix,
-                       const CsBox* __restrict__ box, const int* __restrict__ flag, const CsPart part) {
+    corr_search_kernel(const CorrConsts k, const float4* A, const float2* B, const CsPix pix,
+                       const CsBox* box, const int* flag, const CsPart part) {
   extern __shared__ float4 cs_smem[];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int x = blockIdx.x * kCsTx + (wid & 3) * 8 + (lane >> 2);
@@ -948,8 +948,8 @@ __device__ __forceinline__ void cs_scan_exact(const float4* sA, const float2* sB
 // all: the whole frame; otherwise the chunks that the search has left.
 template <bool kAngle>
 __global__ void __launch_bounds__(kCsThreads, kExCtasPerSm)
-    corr_exact_kernel(const CorrConsts k, const float4* __restrict__ A, const float2* __restrict__ B, const CsPix pix,
-                      const CsBox* __restrict__ box, const int* __restrict__ flag, const CsPart part, int tiles_x,
+    corr_exact_kernel(const CorrConsts k, const float4* A, const float2* B, const CsPix pix,
+                      const CsBox* box, const int* flag, const CsPart part, int tiles_x,
                       int tiles, bool all) {
   cs_after_previous();
   extern __shared__ float4 cs_smem[];
@@ -1058,7 +1058,7 @@ constexpr int kFly = 6;  // loads in flight
 // cap, the warp's lanes on consecutive ones of them: the lane's first least in
 // row-major order.
 __device__ __forceinline__ void cs_rows(const CorrConsts& k, const float3& v, int row0, int n, int l, int w, int lane,
-                                        const float4* __restrict__ A, const float2* __restrict__ B, CsBest& b) {
+                                        const float4* A, const float2* B, CsBest& b) {
   const int total = n * w, dy = 32 / w, dx = 32 - dy * w;
   int y = lane / w, x = lane - y * w;
   for (int t = lane; t < total; t += 32 * kFly) {
@@ -1102,8 +1102,8 @@ constexpr int kMergeThreads = 256;
 static_assert(kMergeThreads <= 256 && kCorrMaxChunks <= 8, "an item: pixel, chunk");
 template <bool kAngle, bool kDirect>
 __global__ void __launch_bounds__(kMergeThreads)
-    corr_merge_kernel(const CorrConsts k, const float* __restrict__ lv, const float4* __restrict__ A,
-                      const float2* __restrict__ B, const CsPix pix, const int* __restrict__ flag, const CsPart part,
+    corr_merge_kernel(const CorrConsts k, const float* lv, const float4* A,
+                      const float2* B, const CsPix pix, const int* flag, const CsPart part,
                       const KnnSrc knn, bool own, cf_correspondence* __restrict__ out, int* __restrict__ num_valid,
                       int* __restrict__ stats) {
   after_previous();
@@ -1291,8 +1291,8 @@ __global__ void __launch_bounds__(kMergeThreads)
   cs_emit(k, p, inimg, px, bi, code, A, B, knn, out, num_valid, stats, lane, s_stage[threadIdx.x >> 5]);
 }
 
-__global__ void pixel_knn_kernel(const int* __restrict__ hit, int P, const int* __restrict__ vk,
-                                 const float* __restrict__ vw, long long num_voxels, int* __restrict__ pk,
+__global__ void pixel_knn_kernel(const int* hit, int P, const int* vk,
+                                 const float* vw, long long num_voxels, int* __restrict__ pk,
                                  float* __restrict__ pw) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

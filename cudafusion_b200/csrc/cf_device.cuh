@@ -30,19 +30,13 @@ __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
   return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
 
+// through L1, but not as read-only data (__ldg): the launch before may still write
+// them while this one's CTAs start (after_previous)
 __device__ __forceinline__ DQ load_dq(const cf_dual_quat* p) {
   const float4* q = reinterpret_cast<const float4*>(p);
   DQ d;
-  d.r = __ldg(q);
-  d.d = __ldg(q + 1);
-  return d;
-}
-// through L1: for DQs written by an earlier launch and not during this one
-__device__ __forceinline__ DQ load_dq_ldg(const cf_dual_quat* p) {
-  const float4* q = reinterpret_cast<const float4*>(p);
-  DQ d;
-  d.r = __ldg(q);
-  d.d = __ldg(q + 1);
+  d.r = __ldca(q);
+  d.d = __ldca(q + 1);
   return d;
 }
 __device__ __forceinline__ DQ load_dq_cg(const cf_dual_quat* p) {
@@ -197,8 +191,8 @@ __device__ __forceinline__ DQ twist_update(DQ T, const float* dx, float max_rot,
 // ids outside 0..N-1 and weights below 1e-8 are skipped; no weight left
 // copies the point.
 __device__ __forceinline__ float3 skin_point_centered(float3 p, const int* ids, const float* ws,
-                                                      const cf_deform_node* __restrict__ nodes,
-                                                      const cf_dual_quat* __restrict__ T, int N) {
+                                                      const cf_deform_node* nodes,
+                                                      const cf_dual_quat* T, int N) {
   float4 br = make_float4(0.f, 0.f, 0.f, 0.f), bd = make_float4(0.f, 0.f, 0.f, 0.f);
   float wsum = 0.f;
   for (int k = 0; k < kK; k++) {
@@ -233,7 +227,7 @@ __device__ __forceinline__ float3 blend_warp(float3 p, int4 ids, float4 ws, cons
     int nid = idv[k];
     float w = wv[k];
     if (nid < 0 || nid >= N || w < 1e-8f) continue;
-    DQ d = load_dq_ldg(plain + nid);  // (the plain DQs come from an earlier launch)
+    DQ d = load_dq(plain + nid);
     if (qdot(d.r, br) < 0.f) {
       d.r.x = -d.r.x; d.r.y = -d.r.y; d.r.z = -d.r.z; d.r.w = -d.r.w;
       d.d.x = -d.d.x; d.d.y = -d.d.y; d.d.z = -d.d.z; d.d.w = -d.d.w;
@@ -403,7 +397,7 @@ __device__ __forceinline__ Edge eval_edge(const cf_deform_node* nodes, const cf_
   const float* nwp = reinterpret_cast<const float*>(nodes + i) + 15 + k;  // neighbor_w[k]
   float nw = fmaxf(__ldg(nwp), 0.05f);
   float3 xi = node_pos(nodes, i), xj = node_pos(nodes, j);
-  DQ Ti = load_dq_ldg(T + i), Tj = load_dq_ldg(T + j);  // (T comes from an earlier launch)
+  DQ Ti = load_dq(T + i), Tj = load_dq(T + j);
   float3 ti_xj = dq_transform_point_centered(Ti, xj, xi);
   float3 ti_xi = dq_transform_point_centered(Ti, xi, xi);
   float3 tj_xj = dq_transform_point_centered(Tj, xj, xj);

@@ -39,8 +39,12 @@ inline cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, dim3 block,
 }
 
 #ifdef __CUDACC__
-// First statement of every kernel that launch_next launches.  Only then is the
-// next kernel let in, so that what came before this one is done when it starts.
+// Every kernel that launch_next launches calls it, in all its CTAs and before an
+// early return, before its first write and before it reads what the launch before
+// it writes.  Only then is the next kernel let in, so what lies two or more launches
+// back is done when a kernel starts, and that alone may be read ahead of the call.
+// What the launch before writes is not constant for the kernel's life, even though it
+// is read after the call: no __ldg and no const __restrict__ for it.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

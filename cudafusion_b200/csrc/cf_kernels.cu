@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kThreads) node_setup_kernel(Table tb, Work w, 
 
 // start = exclusive scan of total (one CTA of 1024 threads, 4096 nodes per
 // round, the next round's totals in flight); cursor, when given, a copy of it.
-__global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ total, int* __restrict__ start,
+__global__ void __launch_bounds__(1024) scan_kernel(const int* total, int* __restrict__ start,
                                                     int* __restrict__ cursor, int N) {
   after_previous();
   __shared__ int wsum[32];
@@ -377,7 +377,7 @@ __global__ void batch_scatter_kernel(Table tb, Work w) {
 }
 
 // WarpField::apply_twist_increment (src/warp_field.cu:250-291).
-__global__ void apply_twist_kernel(cf_dual_quat* __restrict__ T, const float* __restrict__ dx, int N, float max_rot,
+__global__ void apply_twist_kernel(cf_dual_quat* __restrict__ T, const float* dx, int N, float max_rot,
                                    float max_trans, float scale) {
   after_previous();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -389,9 +389,9 @@ __global__ void apply_twist_kernel(cf_dual_quat* __restrict__ T, const float* __
 }
 
 // warp_point per point (se3_math.cuh:450-510), centring each node DQ on the fly.
-__global__ void skin_points_kernel(const float* __restrict__ pts, const int* __restrict__ ids,
-                                   const float* __restrict__ ws, int M, const cf_deform_node* __restrict__ nodes,
-                                   const cf_dual_quat* __restrict__ T, int N, float* out) {
+__global__ void skin_points_kernel(const float* pts, const int* ids,
+                                   const float* ws, int M, const cf_deform_node* nodes,
+                                   const cf_dual_quat* T, int N, float* out) {
   after_previous();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= M) return;

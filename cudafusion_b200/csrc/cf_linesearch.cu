@@ -27,7 +27,7 @@ __device__ __forceinline__ float ls_norm3(float a, float b, float c) {
 // and of the scaled-and-clamped values (fusion_app.h:434-458); a non-finite
 // rn or tn clears out->finite.  Block partials then atomics: maxima of
 // non-negative floats compare as their bit patterns.
-__global__ void __launch_bounds__(kLsThreads) update_stats_kernel(const float* __restrict__ dx, int N,
+__global__ void __launch_bounds__(kLsThreads) update_stats_kernel(const float* dx, int N,
                                                                    float update_scale, float max_rot,
                                                                    float max_trans, double* __restrict__ sums,
                                                                    unsigned* __restrict__ maxima,
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kLsThreads) update_stats_kernel(const float* _
 // upload_scaled_delta_x (fusion_app.h:1352-1375): per node rs = max_rot / rn
 // when rn exceeds a positive max_rot (else 1), ts likewise, then
 // dx[k] * (rs * scale) and dx[k] * (ts * scale).
-__device__ __forceinline__ void ls_scale(const float* __restrict__ d, float max_rot, float max_trans, float scale,
+__device__ __forceinline__ void ls_scale(const float* d, float max_rot, float max_trans, float scale,
                                          float (&o)[6]) {
   const float rn = ls_norm3(d[0], d[1], d[2]), tn = ls_norm3(d[3], d[4], d[5]);
   float rs = 1.f, ts = 1.f;
@@ -97,7 +97,7 @@ __device__ __forceinline__ void ls_scale(const float* __restrict__ d, float max_
 #pragma unroll
   for (int k = 3; k < 6; ++k) o[k] = __fmul_rn(d[k], ft);
 }
-__global__ void scale_delta_kernel(const float* __restrict__ dx, int N, float max_rot, float max_trans, float scale,
+__global__ void scale_delta_kernel(const float* dx, int N, float max_rot, float max_trans, float scale,
                                    float* __restrict__ out) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -111,7 +111,7 @@ __global__ void scale_delta_kernel(const float* __restrict__ dx, int N, float ma
 // A trial's transforms: the saved ones with the scaled increment applied (the
 // restore, scale_delta and apply_twist of the host flow, in one launch: the
 // copy and two launches took 8 us a trial, this 3).
-__global__ void trial_transforms_kernel(const cf_dual_quat* __restrict__ saved, const float* __restrict__ dx, int N,
+__global__ void trial_transforms_kernel(const cf_dual_quat* saved, const float* dx, int N,
                                         float max_rot, float max_trans, float scale, float* __restrict__ delta,
                                         cf_dual_quat* __restrict__ T) {
   after_previous();
@@ -146,7 +146,7 @@ __device__ __forceinline__ double ls_sum(const double* v, int n) {
 // correspondence_rmse's sums (fusion_app.h:1336-1347): block b sums the
 // records of its fixed slice in index order per thread and then in thread
 // order; rmse_final_kernel adds the blocks in block order.  Deterministic.
-__global__ void __launch_bounds__(kLsThreads) rmse_partial_kernel(const cf_correspondence* __restrict__ corrs, int M,
+__global__ void __launch_bounds__(kLsThreads) rmse_partial_kernel(const cf_correspondence* corrs, int M,
                                                                    double* __restrict__ part) {
   after_previous();
   const int per = (M + gridDim.x - 1) / gridDim.x;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kLsThreads) rmse_partial_kernel(const cf_corre
 }
 
 // The block sums in block order, for the whole CTA (256 threads).
-__device__ __forceinline__ void ls_total(const double* __restrict__ part, double (&out)[2]) {
+__device__ __forceinline__ void ls_total(const double* part, double (&out)[2]) {
   __shared__ double sh[2][CF_RMSE_BLOCKS];
   __shared__ double tot[2];
   for (int b = threadIdx.x; b < 2 * CF_RMSE_BLOCKS; b += blockDim.x) sh[b & 1][b >> 1] = part[b];
@@ -180,7 +180,7 @@ __device__ __forceinline__ void ls_total(const double* __restrict__ part, double
   out[0] = tot[0];
   out[1] = tot[1];
 }
-__global__ void __launch_bounds__(256) rmse_final_kernel(const double* __restrict__ part, double* __restrict__ out) {
+__global__ void __launch_bounds__(256) rmse_final_kernel(const double* part, double* __restrict__ out) {
   after_previous();
   double t[2];
   ls_total(part, t);

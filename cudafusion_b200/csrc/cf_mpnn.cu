@@ -87,10 +87,9 @@ __device__ __forceinline__ float4 bf4(uint2 v) {
   return make_float4(a.x, a.y, b.x, b.y);
 }
 template <int DIN>
-__device__ __forceinline__ float4 mean_of(const __nv_bfloat16* in, const int* __restrict__ nbr,
-                                          const float* __restrict__ inv_deg, int i, int k) {
-  const int4 n0 = __ldg(reinterpret_cast<const int4*>(nbr + (size_t)i * CF_K_GRAPH)),
-             n1 = __ldg(reinterpret_cast<const int4*>(nbr + (size_t)i * CF_K_GRAPH) + 1);
+__device__ __forceinline__ float4 mean_of(const __nv_bfloat16* in, const int* nbr,
+                                          const float* inv_deg, int i, int k) {
+  const int4 *nb = reinterpret_cast<const int4*>(nbr + (size_t)i * CF_K_GRAPH), n0 = nb[0], n1 = nb[1];
   const int jn[CF_K_GRAPH] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
   uint2 x[CF_K_GRAPH];
 #pragma unroll
@@ -112,11 +111,11 @@ __device__ __forceinline__ float4 mean_of(const __nv_bfloat16* in, const int* __
 static_assert(CF_K_GRAPH == 8, "a node's list is two int4");
 
 template <int DIN, int DOUT, bool FIRST, bool AGG, bool RELU>
-__global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int* __restrict__ nbr,
-                                                      const float* __restrict__ inv_deg,
-                                                      const __nv_bfloat16* __restrict__ W,
-                                                      const __nv_bfloat16* __restrict__ b, void* out_,
-                                                      const float* __restrict__ x_skip, int N) {
+__global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int* nbr,
+                                                      const float* inv_deg,
+                                                      const __nv_bfloat16* W,
+                                                      const __nv_bfloat16* b, void* out_,
+                                                      const float* x_skip, int N) {
   after_previous();
   using S = FwdShape<DIN, DOUT, AGG>;
   constexpr int CAT = S::CAT, CATP = S::CATP, DINP = S::DINP, DOUTP = S::DOUTP, LD = S::LD, LDL = S::LDL;
@@ -136,7 +135,7 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
 #pragma unroll
     for (int j = 0; j < PER; j++) {
       const int q = tid + j * kThreads;
-      if (q < NCH) wv[j] = __ldg(reinterpret_cast<const uint4*>(W) + q);
+      if (q < NCH) wv[j] = reinterpret_cast<const uint4*>(W)[q];
     }
 #pragma unroll
     for (int j = 0; j < PER; j++) {
@@ -287,9 +286,9 @@ __global__ void __launch_bounds__(kThreads) layer_fwd(const void* in_, const int
 
 // Output layer backward over a tile: loss = mean over N*6 of (out - target)^2;
 // dh3 = Wo^T dy; per-CTA partial gradients of Wo, bo and the loss.
-__global__ void __launch_bounds__(kThreads) out_bwd(const float* __restrict__ out, const float* __restrict__ tgt,
-                                                    const __nv_bfloat16* __restrict__ h3,
-                                                    const __nv_bfloat16* __restrict__ Wo, float* __restrict__ dh3,
+__global__ void __launch_bounds__(kThreads) out_bwd(const float* out, const float* tgt,
+                                                    const __nv_bfloat16* h3,
+                                                    const __nv_bfloat16* Wo, float* __restrict__ dh3,
                                                     float* __restrict__ part, double* __restrict__ loss_part, int N) {
   after_previous();
   __shared__ float sdy[kTileNodes * kOut];
@@ -392,7 +391,7 @@ __global__ void __launch_bounds__(kThreads) layer_bwd(const BwdArgs a) {
   if (!FIRST)
     for (int k = tid; k < DOUT * CAT / 4; k += kThreads)
       reinterpret_cast<float4*>(sW)[k] = bf4(__ldg(reinterpret_cast<const uint2*>(a.W) + k));
-  after_previous();  // (the weights are older)
+  after_previous();  // (so far the weights, of an optimizer step before the forward pass)
   const int tk = tid % KG, u0 = tid / KG * TU;
   // a thread's columns: two runs of four (CAT 128), or five
   auto col = [&](int c) { return CAT == 128 ? 4 * tk + (c & 3) + (c >> 2) * 64 : TK * tk + c; };
@@ -415,8 +414,7 @@ __global__ void __launch_bounds__(kThreads) layer_bwd(const BwdArgs a) {
         const int s = e / (DIN / 4), k = 4 * (e % (DIN / 4)), i = n0 + s;
         float v[4] = {}, m[4] = {};
         if (i < N) {
-          const int4 l0 = __ldg(reinterpret_cast<const int4*>(a.nbr + (size_t)i * CF_K_GRAPH)),
-                     l1 = __ldg(reinterpret_cast<const int4*>(a.nbr + (size_t)i * CF_K_GRAPH) + 1);
+          const int4 *nb = reinterpret_cast<const int4*>(a.nbr + (size_t)i * CF_K_GRAPH), l0 = nb[0], l1 = nb[1];
           const int jn[CF_K_GRAPH] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
           float x[CF_K_GRAPH][4];
 #pragma unroll
@@ -461,13 +459,13 @@ __global__ void __launch_bounds__(kThreads) layer_bwd(const BwdArgs a) {
         if (TOP) {
           z = *reinterpret_cast<const float4*>(a.dh + (size_t)i * DOUT + k);
         } else {
-          z = __ldg(reinterpret_cast<const float4*>(a.dnext + (size_t)i * 2 * DOUT + k));
+          z = *reinterpret_cast<const float4*>(a.dnext + (size_t)i * 2 * DOUT + k);
           const int q1 = a.rev_ptr[i + 1];
 #pragma unroll 4
           for (int q = a.rev_ptr[i]; q < q1; q++) {
             const int j = __ldg(a.rev_idx + q);
             const float w = __ldg(a.inv_deg + j);
-            const float4 d = __ldg(reinterpret_cast<const float4*>(a.dnext + (size_t)j * 2 * DOUT + DOUT + k));
+            const float4 d = *reinterpret_cast<const float4*>(a.dnext + (size_t)j * 2 * DOUT + DOUT + k);
             z.x = fmaf(w, d.x, z.x);
             z.y = fmaf(w, d.y, z.y);
             z.z = fmaf(w, d.z, z.z);
@@ -580,7 +578,7 @@ __global__ void __launch_bounds__(kThreads) reduce_parts(const ReduceArgs r) {
 
 // Adam (FP32 master weights), then the BF16 copy
 __global__ void adam_step(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                          const float* __restrict__ g, __nv_bfloat16* __restrict__ wb, int n, float lr, float b1,
+                          const float* g, __nv_bfloat16* __restrict__ wb, int n, float lr, float b1,
                           float b2, float c1, float c2, float eps) {
   after_previous();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -595,14 +593,14 @@ __global__ void adam_step(float* __restrict__ w, float* __restrict__ m, float* _
   wb[q] = tobf(ww);
 }
 
-__global__ void to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__ wb, int n) {
+__global__ void to_bf16(const float* w, __nv_bfloat16* __restrict__ wb, int n) {
   after_previous();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < n) wb[q] = tobf(w[q]);
 }
 
 // graph of a problem's nodes: neighbour lists (-1 = none) and 1/degree
-__global__ void graph_from_nodes(const cf_deform_node* __restrict__ nodes, int N, int* __restrict__ nbr,
+__global__ void graph_from_nodes(const cf_deform_node* nodes, int N, int* __restrict__ nbr,
                                  float* __restrict__ inv_deg) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -661,7 +659,7 @@ __device__ __forceinline__ DQ dq_apply_increment(DQ T, const float* o) {
   return out;
 }
 
-__global__ void increments_kernel(const cf_dual_quat* __restrict__ to, const cf_dual_quat* __restrict__ from, int n,
+__global__ void increments_kernel(const cf_dual_quat* to, const cf_dual_quat* from, int n,
                                   float* __restrict__ out) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -676,9 +674,9 @@ __global__ void increments_kernel(const cf_dual_quat* __restrict__ to, const cf_
 // hist = [T_{t-2}, T_{t-3}, T_{t-4}]: the three increments (scaled) and the
 // mean / max |residual| (mm) of the node's valid correspondences (the
 // residual launch at T must have run; warp per node over its tasks).
-__global__ void features_kernel(const cf_dual_quat* __restrict__ T, const cf_dual_quat* __restrict__ hist, int N,
-                                const int* __restrict__ cl_start, const int* __restrict__ clist,
-                                const float4* __restrict__ cstat, float* __restrict__ feat) {
+__global__ void features_kernel(const cf_dual_quat* T, const cf_dual_quat* hist, int N,
+                                const int* cl_start, const int* clist,
+                                const float4* cstat, float* __restrict__ feat) {
   after_previous();
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= N) return;
@@ -686,7 +684,7 @@ __global__ void features_kernel(const cf_dual_quat* __restrict__ T, const cf_dua
   int cnt = 0;
   // the node's tasks (about 28), each with the sum, maximum and count of its |residuals|
   for (int q = cl_start[i] + lane; q < cl_start[i + 1]; q += 32) {
-    const float4 v = __ldg(cstat + (clist[q] >> 2));
+    const float4 v = cstat[clist[q] >> 2];
     s += v.x;
     mx = fmaxf(mx, v.y);
     cnt += (int)v.z;
@@ -715,8 +713,8 @@ __global__ void features_kernel(const cf_dual_quat* __restrict__ T, const cf_dua
 // T <- D(prediction) (x) T for every node (the warm start kept in T_save),
 // and the node-centred plain DQs for the skinning
 __global__ void apply_prediction(cf_dual_quat* __restrict__ T, cf_dual_quat* __restrict__ T_save,
-                                 cf_dual_quat* __restrict__ plain, const cf_deform_node* __restrict__ nodes,
-                                 const float* __restrict__ pred, int N) {
+                                 cf_dual_quat* __restrict__ plain, const cf_deform_node* nodes,
+                                 const float* pred, int N) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -737,8 +735,8 @@ __global__ void apply_prediction(cf_dual_quat* __restrict__ T, cf_dual_quat* __r
 
 // Keeps the predicted start only if its energy is below the warm start's
 // (gate[0] warm start, gate[1] prediction); otherwise restores the warm start.
-__global__ void gate_prediction(cf_dual_quat* __restrict__ T, const cf_dual_quat* __restrict__ T_save,
-                                cf_dual_quat* __restrict__ plain, const cf_deform_node* __restrict__ nodes,
+__global__ void gate_prediction(cf_dual_quat* __restrict__ T, const cf_dual_quat* T_save,
+                                cf_dual_quat* __restrict__ plain, const cf_deform_node* nodes,
                                 DevStats* __restrict__ st, int N) {
   after_previous();
   const bool reject = !(st->gate[1] <= st->gate[0]);

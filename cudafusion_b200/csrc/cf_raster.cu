@@ -91,7 +91,7 @@ __device__ __forceinline__ int rs_voxel(const RasterConsts& k, float3 p) {
 
 // project_triangle (src/mesh_raster_kernels.cu:47-72): the warped corners,
 // their camera-frame points, their projections and the signed area.
-__device__ __forceinline__ bool rs_project(const RasterConsts& k, const float* __restrict__ warped, int3 t,
+__device__ __forceinline__ bool rs_project(const RasterConsts& k, const float* warped, int3 t,
                                            float3 wc[3], float3 cc[3], float2 p[3], float& area) {
   const int ids[3] = {t.x, t.y, t.z};
 #pragma unroll
@@ -125,9 +125,8 @@ __device__ __forceinline__ bool rs_bary(const float2 p[3], float area, float2 q,
 }
 
 __global__ void mesh_skin_kernel(const float* __restrict__ canon, float* __restrict__ warped, int V,
-                                 const RasterConsts k, const cf_deform_node* __restrict__ nodes,
-                                 const cf_dual_quat* __restrict__ T, int N, const int* __restrict__ vk,
-                                 const float* __restrict__ vw) {
+                                 const RasterConsts k, const cf_deform_node* nodes, const cf_dual_quat* T, int N,
+                                 const int* __restrict__ vk, const float* __restrict__ vw) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
@@ -147,7 +146,7 @@ __global__ void mesh_skin_kernel(const float* __restrict__ canon, float* __restr
 // solve's skinning does: no per-vertex centring.  The lists are read as one
 // 16-byte load each.
 __global__ void mesh_skin_plain_kernel(const float* __restrict__ canon, float* __restrict__ warped, int V,
-                                       const RasterConsts k, const cf_dual_quat* __restrict__ plain, int N,
+                                       const RasterConsts k, const cf_dual_quat* plain, int N,
                                        const int4* __restrict__ vk, const float4* __restrict__ vw) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -217,7 +216,7 @@ __device__ __forceinline__ void rs_fragment(const RsTri& r, int ti, int x, int y
 // Set-up of triangle ti (rasterize_triangles_z_kernel up to the pixel loop,
 // src/mesh_raster_kernels.cu:86-110); false when it draws nothing.  A drawn
 // triangle's record goes to the cache (when given).
-__device__ __forceinline__ bool rs_setup(int ti, const float* __restrict__ canon, const float* __restrict__ warped,
+__device__ __forceinline__ bool rs_setup(int ti, const float* __restrict__ canon, const float* warped,
                                          const int3* __restrict__ tris, int V, const RasterConsts& k,
                                          float4* __restrict__ cache, RsTri& r) {
   const int3 t = tris[ti];
@@ -262,7 +261,7 @@ __device__ __forceinline__ bool rs_setup(int ti, const float* __restrict__ canon
 // fields rs_setup computed (the corners and area as stored, the band from the
 // area, each corner's camera depth from its warped corner, the box from the
 // corners), by the same operations.
-__device__ __forceinline__ void rs_from_record(const float4* __restrict__ rec, const RasterConsts& k, RsTri& r) {
+__device__ __forceinline__ void rs_from_record(const float4* rec, const RasterConsts& k, RsTri& r) {
   const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3], r4 = rec[4];
   const float2 p[3] = {make_float2(r0.x, r0.y), make_float2(r0.z, r0.w), make_float2(r1.x, r1.y)};
   const float3 wc[3] = {make_float3(r2.z, r2.w, r3.x), make_float3(r3.y, r3.z, r3.w), make_float3(r4.x, r4.y, r4.z)};
@@ -363,7 +362,7 @@ __device__ __forceinline__ void rs_span_row(const RsTri& r, const RsSpan& sp, in
 // the entry its index and its first item, so the entries' first items
 // increase with their index.  128-thread CTAs at 9 per SM: 5120 warps of a
 // 164k-triangle mesh fit in one wave.
-__global__ void __launch_bounds__(128, 9) raster_kernel(const float* __restrict__ canon, const float* __restrict__ warped,
+__global__ void __launch_bounds__(128, 9) raster_kernel(const float* __restrict__ canon, const float* warped,
                                                         const int3* __restrict__ tris, int V, int NT,
                                                         const RasterConsts k, int G,
                                                         unsigned long long* __restrict__ ztri,
@@ -394,10 +393,10 @@ __global__ void __launch_bounds__(128, 9) raster_kernel(const float* __restrict_
 // entry's set-up from its record (the same values) and shares each row's span
 // out over its lanes.  The 64-bit min is order-free: the keys
 // equal a sequential pass's.
-__global__ void __launch_bounds__(256) raster_big_kernel(const float4* __restrict__ cache, const RasterConsts k,
+__global__ void __launch_bounds__(256) raster_big_kernel(const float4* cache, const RasterConsts k,
                                                          int G, unsigned long long* __restrict__ ztri,
-                                                         const int2* __restrict__ big,
-                                                         const unsigned long long* __restrict__ big_ctr) {
+                                                         const int2* big,
+                                                         const unsigned long long* big_ctr) {
   after_previous();
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);

@@ -72,7 +72,7 @@ __device__ __forceinline__ float3 ts_centre(const TsdfConsts& k, unsigned i) {
                      fmaf(__fadd_rn((float)z, 0.5f), k.vs, k.oz));
 }
 
-__global__ void tsdf_plain_kernel(const cf_deform_node* __restrict__ nodes, const cf_dual_quat* __restrict__ T,
+__global__ void tsdf_plain_kernel(const cf_deform_node* nodes, const cf_dual_quat* T,
                                   cf_dual_quat* __restrict__ plain, int N) {
   after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,7 +93,7 @@ __device__ __forceinline__ float4 ts_qmul(float4 a, float4 b) {
                      fmaf(a.z, b.w, fmaf(-a.y, b.x, fmaf(a.x, b.y, __fmul_rn(a.w, b.z)))),
                      fmaf(-a.z, b.z, fmaf(-a.y, b.y, fmaf(-a.x, b.x, __fmul_rn(a.w, b.w)))));
 }
-__device__ __forceinline__ float3 ts_warp(float3 p, int4 ids, float4 ws, const cf_dual_quat* __restrict__ plain,
+__device__ __forceinline__ float3 ts_warp(float3 p, int4 ids, float4 ws, const cf_dual_quat* plain,
                                           int N) {
   float4 br = make_float4(0.f, 0.f, 0.f, 0.f), bd = br;
   float wsum = 0.f;
@@ -104,7 +104,7 @@ __device__ __forceinline__ float3 ts_warp(float3 p, int4 ids, float4 ws, const c
     const int nid = idv[k];
     const float w = wv[k];
     if (nid < 0 || nid >= N || w < 1e-8f) continue;
-    DQ d = load_dq_ldg(plain + nid);  // (the plain DQs come from an earlier launch)
+    DQ d = load_dq(plain + nid);
     if (ts_qdot(d.r, br) < 0.f) {
       d.r = make_float4(-d.r.x, -d.r.y, -d.r.z, -d.r.w);
       d.d = make_float4(-d.d.x, -d.d.y, -d.d.z, -d.d.w);
@@ -130,8 +130,8 @@ __device__ __forceinline__ float3 ts_warp(float3 p, int4 ids, float4 ws, const c
 // gate: centre, warp, camera, pixel, sdf, weighted average.
 template <bool kWarp>
 __device__ __forceinline__ void ts_update(const TsdfConsts& k, float* __restrict__ vox, unsigned i,
-                                          const float* __restrict__ depth, const int4* __restrict__ knn,
-                                          const float4* __restrict__ knn_w, const cf_dual_quat* __restrict__ plain,
+                                          const float* depth, const int4* knn,
+                                          const float4* knn_w, const cf_dual_quat* plain,
                                           int N) {
   float3 p = ts_centre(k, i);
   if (kWarp) p = ts_warp(p, __ldcs(knn + i), __ldcs(knn_w + i), plain, N);
@@ -161,9 +161,9 @@ __device__ __forceinline__ void ts_update(const TsdfConsts& k, float* __restrict
 // 16-byte aligned).
 template <bool kWarp, bool kGate>
 __global__ void __launch_bounds__(kTsThreads)
-    tsdf_integrate_kernel(const TsdfConsts k, float* __restrict__ vox, unsigned V, const float* __restrict__ depth,
-                          const int4* __restrict__ knn, const float4* __restrict__ knn_w,
-                          const cf_dual_quat* __restrict__ plain, int N, const int* __restrict__ counts) {
+    tsdf_integrate_kernel(const TsdfConsts k, float* __restrict__ vox, unsigned V, const float* depth,
+                          const int4* knn, const float4* knn_w,
+                          const cf_dual_quat* plain, int N, const int* counts) {
   after_previous();
   const unsigned i = blockIdx.x * kTsThreads + threadIdx.x;
   if (i >= V) return;
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kTsThreads)
 // bytes in flight and no lane idles on a gated voxel.  Each voxel's update is
 // ts_update's, so the values equal the one-thread-per-voxel kernel's.
 constexpr int kTsTile = 256, kTsQueue = 32 + kTsTile;
-__device__ __forceinline__ void ts_load_counts(const int* __restrict__ counts, unsigned V, unsigned tile, int lane,
+__device__ __forceinline__ void ts_load_counts(const int* counts, unsigned V, unsigned tile, int lane,
                                                int4 (&c)[2]) {
 #pragma unroll
   for (int h = 0; h < 2; h++) {
@@ -197,9 +197,9 @@ __device__ __forceinline__ void ts_load_counts(const int* __restrict__ counts, u
 }
 
 __global__ void __launch_bounds__(kTsThreads)
-    tsdf_gated_kernel(const TsdfConsts k, float* __restrict__ vox, unsigned V, const float* __restrict__ depth,
-                      const int4* __restrict__ knn, const float4* __restrict__ knn_w,
-                      const cf_dual_quat* __restrict__ plain, int N, const int* __restrict__ counts) {
+    tsdf_gated_kernel(const TsdfConsts k, float* __restrict__ vox, unsigned V, const float* depth,
+                      const int4* knn, const float4* knn_w,
+                      const cf_dual_quat* plain, int N, const int* counts) {
   after_previous();
   __shared__ unsigned s_queue[kTsThreads / 32][kTsQueue];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -253,8 +253,8 @@ __global__ void __launch_bounds__(kTsThreads)
 }
 
 __global__ void __launch_bounds__(kTsThreads)
-    tsdf_centres_kernel(const TsdfConsts k, float* __restrict__ out, unsigned V, const int4* __restrict__ knn,
-                        const float4* __restrict__ knn_w, const cf_dual_quat* __restrict__ plain, int N) {
+    tsdf_centres_kernel(const TsdfConsts k, float* __restrict__ out, unsigned V, const int4* knn,
+                        const float4* knn_w, const cf_dual_quat* plain, int N) {
   after_previous();
   const unsigned i = blockIdx.x * kTsThreads + threadIdx.x;
   if (i >= V) return;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kTsThreads)
 // correspondence and a canonical voxel marks the 3x3x3 voxels around it
 // (those inside the grid) as optimised in this frame; a voxel's count rises
 // once per frame however many pixels mark it.
-__global__ void mark_opt_kernel(const cf_correspondence* __restrict__ corrs, const int* __restrict__ vidx_map,
+__global__ void mark_opt_kernel(const cf_correspondence* corrs, const int* vidx_map,
                                 int P, int dx, int dy, int dz, int frame, int* __restrict__ counts,
                                 int* __restrict__ frames) {
   after_previous();
