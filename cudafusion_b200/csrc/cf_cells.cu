@@ -30,8 +30,13 @@
 // entry by entry): 2048 nodes, 306k correspondences 37 + 23 us (before 20 + 56),
 // 8192 nodes, 1.2M 103 + 62 (46 + 192), 64 problems, 33M 3.1 + 1.57 ms (1.7 + 7.1);
 // three CTAs per SM at 80 registers spill (4.0 ms);
-// the sort costs 98 us against 80 at 306k and 7 ms against 10 at 33M.
+// the sort costs 98 us against 80 at 306k and 7 ms against 10 at 33M.  Sets that occur
+// once each (no surface has them) leave nothing to sum per set: random ones take
+// 530 us a solve at 64 nodes and 20k correspondences (before: 307), 1010 at 2048
+// and 300k (687).
 // Restates kernels/solver_kernels.cu:52-352 (data term, ARAP, damping).
+#include <algorithm>
+
 #include "cf_device.cuh"
 #include "cf_internal.h"
 
@@ -339,16 +344,18 @@ __device__ __forceinline__ uint4 list_desc(const Work& w, const Pattern& pt, int
 
 // Puts each node's list in position order (its entries came in any order; the
 // gather's sums follow it) and describes its entries.  A warp per node up to
-// 64 tasks, by rank; the CTA together for the others.
+// 64 tasks, by rank; the CTA together for the others, one after another, so a CTA
+// has no more nodes (`per`, at most one per warp) than about 1024 CTAs need: 64 nodes
+// with 1250 tasks each take 29 us, 205 with eight to a CTA.
 constexpr int kListSmem = 4096;
-__global__ void __launch_bounds__(kThreads) list_sort_kernel(Work w, Pattern pt, int N) {
+__global__ void __launch_bounds__(kThreads) list_sort_kernel(Work w, Pattern pt, int N, int per) {
   after_previous();
   __shared__ int big[kWarps];
   __shared__ int buf[kListSmem];
   const int lane = lane_id(), wid = threadIdx.x >> 5;
-  const int node = blockIdx.x * kWarps + wid;
+  const int node = blockIdx.x * per + wid;
   int n = 0, b0 = 0;
-  if (node < N) {
+  if (wid < per && node < N) {
     b0 = w.cl_start[node];
     n = w.cl_start[node + 1] - b0;
   }
@@ -378,7 +385,7 @@ __global__ void __launch_bounds__(kThreads) list_sort_kernel(Work w, Pattern pt,
   }
   if (lane == 0) big[wid] = n > 64 ? node : -1;
   __syncthreads();
-  for (int v = 0; v < kWarps; v++) {
+  for (int v = 0; v < per; v++) {
     const int nd = big[v];
     if (nd < 0) continue;
     const int b = w.cl_start[nd], m = w.cl_start[nd + 1] - b;
@@ -1030,7 +1037,8 @@ struct RowMem {
   float4 d[kRowBlocks];         // x_c - x_r
   int4 task[kRowWarps][32];     // run start, its floats, the blocks of its pairs, the row's node of the task
   int edge[kRowBlocks + 4];     // the blocks' first ARAP edges
-  float raw[kRowWarps][32][12];  // (u, n), g w_a, -g r, g w_b of the three nodes after a; g = fw w_a
+  // (u, n), g w_a, -g r, g w_b of the three nodes after a (g = fw w_a), the blocks of its pairs
+  float raw[kRowWarps][32][12];
 };
 // (18 CTAs of two warps per SM need 56 registers: 255k rows take 1.52 ms, with 64 1.66)
 template <int kRowWarps>
@@ -1093,7 +1101,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowWarps == 2 ? 18 : 8) gathe
       m.task[wid][lane] = make_int4((int)ds.x, lane < cnt && !nraw ? 90 - 21 * a : 0, (int)kb, a);
       __syncwarp();
       constexpr int kFly = 4;
-      for (int t = 0; t < cnt; t += kFly) {
+      const int runs = __any_sync(0xffffffffu, lane < cnt && !nraw) ? cnt : 0;
+      for (int t = 0; t < runs; t += kFly) {
         float x[kFly][3];
         unsigned k3[kFly];
 #pragma unroll
@@ -1120,10 +1129,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowWarps == 2 ? 18 : 8) gathe
         }
       }
       // tasks without a record: their correspondences, a lane each, into
-      // shared memory, then added one by one
+      // shared memory side by side, then added one by one, two's operands read together
+      constexpr int kRawFly = 2;
       for (int j = 0; j < kRecMin - 1; j++) {
         const unsigned on = __ballot_sync(0xffffffffu, j < nraw);
         if (!on) break;
+        const int n = __popc(on);
         if ((on >> lane) & 1u) {
           const int q = (int)ds.x + j;
           const float4 sf = __ldcg(w.raw + q), nr = __ldcg(w.sp_nrm + q), uw = __ldg(w.sp_uw + q);
@@ -1140,23 +1151,41 @@ __global__ void __launch_bounds__(32 * kRowWarps, kRowWarps == 2 ? 18 : 8) gathe
             const float wb = sel4(uw, min(a + 1 + b, 3));
             gb[b] = a + 1 + b < 4 && wb > 1e-8f ? g * wb : 0.f;
           }
-          float4* o = reinterpret_cast<float4*>(m.raw[wid][lane]);
+          float4* o = reinterpret_cast<float4*>(m.raw[wid][__popc(on & lanemask_lt())]);
           o[0] = make_float4(u.x, u.y, u.z, nn.x);
           o[1] = make_float4(nn.y, nn.z, g * wa, g != 0.f ? -g * nr.w : 0.f);
-          o[2] = make_float4(gb[0], gb[1], gb[2], 0.f);
+          o[2] = make_float4(gb[0], gb[1], gb[2], __int_as_float((int)kb));
+        }
+        if (lane >= n && lane < ((n + kRawFly - 1) & ~(kRawFly - 1))) {  // whole rounds: zeros, of no block
+          float4* o = reinterpret_cast<float4*>(m.raw[wid][lane]);
+          o[0] = o[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+          o[2] = make_float4(0.f, 0.f, 0.f, __int_as_float(0xffffff));
         }
         __syncwarp();
-        for (unsigned left = on; left; left &= left - 1) {
-          const int t = __ffs(left) - 1;
-          const float* o = m.raw[wid][t];
-          const unsigned k3 = (unsigned)m.task[wid][t].z;
-          const float y = o[li], L = y * o[lj];
-          if (k0 == 0 && lane < 27) kahan_add(tot, comp, lane < kSums ? o[6] * L : o[7] * y);
-          if (lane < kSums) {
+        for (int t = 0; t < n; t += kRawFly) {
+          float y[kRawFly], L[kRawFly];
+          float2 f[kRawFly];
+          float4 e[kRawFly];
 #pragma unroll
-            for (int b = 0; b < 3; b++) {
-              const unsigned kk = (k3 >> (8 * b)) & 0xffu;
-              if (kk != 0xffu) sum[kk][lane] += o[8 + b] * L;
+          for (int h = 0; h < kRawFly; h++) {
+            const float* o = m.raw[wid][t + h];
+            y[h] = o[li];
+            L[h] = o[lj];
+            f[h] = *reinterpret_cast<const float2*>(o + 6);
+            e[h] = *reinterpret_cast<const float4*>(o + 8);
+          }
+#pragma unroll
+          for (int h = 0; h < kRawFly; h++) {
+            L[h] *= y[h];
+            if (k0 == 0 && lane < 27) kahan_add(tot, comp, lane < kSums ? f[h].x * L[h] : f[h].y * y[h]);
+            const unsigned k3 = (unsigned)__float_as_int(e[h].w);
+            if (lane < kSums && k3 != 0xffffffu) {
+              const float gb[3] = {e[h].x, e[h].y, e[h].z};
+#pragma unroll
+              for (int b = 0; b < 3; b++) {
+                const unsigned kk = (k3 >> (8 * b)) & 0xffu;
+                if (kk != 0xffu) sum[kk][lane] += gb[b] * L[h];
+              }
             }
           }
         }
@@ -1288,7 +1317,8 @@ cudaError_t launch_bucket_sort(const Work& w, const Table& tb, cudaStream_t s) {
 cudaError_t launch_node_lists(const Work& w, const Table& tb, const Pattern& p, cudaStream_t s) {
   if (tb.N <= 0 || tb.M <= 0) return cudaSuccess;
   launch_next(permute_kernel, (tb.M + kPermThreads - 1) / kPermThreads, kPermThreads, 0, s, tb, w);
-  launch_next(list_sort_kernel, (tb.N + kWarps - 1) / kWarps, kThreads, 0, s, w, p, tb.N);
+  const int per = std::min(kWarps, std::max(1, (tb.N + 512) / 1024));
+  launch_next(list_sort_kernel, (tb.N + per - 1) / per, kThreads, 0, s, w, p, tb.N, per);
   return cudaGetLastError();
 }
 
