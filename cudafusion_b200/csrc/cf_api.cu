@@ -18,7 +18,8 @@
 
 using namespace cf;
 
-// Phase slots of the profiler (cf_gn_profile_*).
+// Phase slots of the profiler (cf_gn_profile_*).  The nodes are set up by the
+// scan's launch; node_plain is that alone, where there are no correspondences.
 enum ProfSlot {
   kProfPack = 0, kProfBinScan, kProfScatter, kProfSort, kProfNodePlain, kProfResidual, kProfAssemble,
   kProfPcg, kProfEnergy, kProfTwist, kProfLists, kProfOther
@@ -713,7 +714,7 @@ cf_status bin_correspondences(cf_gn* h, bool reset_stats, cudaStream_t s) {
   } else {
     CF_TRY(cudaMemsetAsync(w.inc_start, 0, sizeof(int) * (size_t)(t.N + 1), s));
     CF_TRY(cudaMemsetAsync(w.cl_start, 0, sizeof(int) * (size_t)(t.N + 1), s));
-    { Timed tm(h, s, kProfBinScan, 1); CF_TRY(launch_node_setup(w, t, reset_stats, s)); }
+    { Timed tm(h, s, kProfNodePlain, 1); CF_TRY(launch_node_setup(w, t, reset_stats, s)); }
   }
   return CF_OK;
 }
