@@ -85,18 +85,19 @@
 // brackets a thread per two pixels with the reference's arithmetic throughout:
 //                        noisy       plane       plane, third runs scanned per pixel
 //   640 x 480 r 50       565 (1771)  1132 (1104)   4272
-//             r 36       380 (1027)   700  (645)   2498
-//             r 28       425  (692)   395  (441)   1688
-//             r 20       280  (430)   264  (286)   1123
-//             r 50 angle 1500 (2594) 1467 (1645)   5453
+//             r 36       385 (1027)   700  (645)   2498
+//             r 28       414  (692)   395  (441)   1688
+//             r 20       278  (430)   260  (286)   1123
+//             r 50 angle 1450 (2594) 1402 (1645)   5453
 //   320 x 240 r 20       103  (152)    98  (103)    508
-//   160 x 120 r 20        69   (72)    65   (57)    512
+//   160 x 120 r 20        62   (72)    60   (57)    512
 #include <cfloat>
 #include <climits>
 #include <cmath>
 
 #include <cuda_fp16.h>
 
+#include "cf_device.cuh"
 #include "cf_internal.h"
 
 namespace cf {
@@ -965,6 +966,19 @@ __global__ void __launch_bounds__(kCsThreads, kExCtasPerSm)
               tx = tile - ty * tiles_x;
     CsTile t;
     if (!cs_tile(k, box, flag, tx, ty, chunk, t)) continue;
+    // columns [xs, xe] of the rows from yb on, asynchronously; the first of them come
+    // while the boxes and pixels are read
+    auto stage = [&](int xs, int yb) {
+      const int wu = min(t.xhi, xs + kSlab - 1) - xs + 1, band = kExSmem / (wu * 24), rows = min(band, t.c1 - yb + 1);
+      float2* sB = reinterpret_cast<float2*>(cs_smem + (size_t)band * wu);
+      for (int j = tid; j < rows * wu; j += kCsThreads) {
+        const int rr = j / wu, g = (yb + rr) * k.W + xs + j - rr * wu;
+        cp_async16(cs_smem + j, A + g);
+        cp_async8(sB + j, B + g);
+      }
+      cp_async_commit();
+    };
+    stage(t.xlo, t.c0);
     bool any = true, cap = what & 1;
     if (all) {
       const CsReach q = cs_reach(k, box, t);
@@ -1004,21 +1018,21 @@ __global__ void __launch_bounds__(kCsThreads, kExCtasPerSm)
     }
     for (int xs = t.xlo; xs <= t.xhi && any; xs += kSlab) {
       const int xe = min(t.xhi, xs + kSlab - 1), wu = xe - xs + 1, band = kExSmem / (wu * 24);
-      float2* sB = reinterpret_cast<float2*>(cs_smem + (size_t)band * wu);
+      const float2* sB = reinterpret_cast<const float2*>(cs_smem + (size_t)band * wu);
       for (int yb = t.c0; yb <= t.c1; yb += band) {
         const int rows = min(band, t.c1 - yb + 1);
-        __syncthreads();
-        for (int j = tid; j < rows * wu; j += kCsThreads) {
-          const int rr = j / wu, g = (yb + rr) * k.W + xs + j - rr * wu;
-          cs_smem[j] = A[g];
-          sB[j] = B[g];
+        if (xs > t.xlo || yb > t.c0) {
+          __syncthreads();
+          stage(xs, yb);
         }
+        cp_async_wait<0>();
         __syncthreads();
         if (cap) cs_scan_exact<kAngle, false>(cs_smem, sB, wu, xs, xe, yb, rows, half, lo, hi, il, ih, pl, ph, v, n, pu, pv, L, G, k);
         else cs_scan_exact<kAngle, true>(cs_smem, sB, wu, xs, xe, yb, rows, half, lo, hi, il, ih, pl, ph, v, n, pu, pv, L, G, k);
       }
     }
     // the halves together
+    cp_async_wait<0>();
     __syncthreads();
     float2* both = reinterpret_cast<float2*>(cs_smem) + (tid & 127);
     if (half) {
