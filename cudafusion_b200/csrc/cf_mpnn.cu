@@ -672,8 +672,8 @@ __global__ void increments_kernel(const cf_dual_quat* to, const cf_dual_quat* fr
 
 // Features of every node at the warm start T (= T_{t-1}) with the history
 // hist = [T_{t-2}, T_{t-3}, T_{t-4}]: the three increments (scaled) and the
-// mean / max |residual| (mm) of the node's valid correspondences (the
-// residual launch at T must have run; warp per node over its tasks).
+// mean / max |residual| (mm) of the node's valid correspondences (from the
+// statistics that the energy launch at T leaves per task; a warp per node).
 __global__ void features_kernel(const cf_dual_quat* T, const cf_dual_quat* hist, int N,
                                 const int* cl_start, const int* clist,
                                 const float4* cstat, float* __restrict__ feat) {

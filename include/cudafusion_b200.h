@@ -130,7 +130,9 @@ typedef struct cf_gn cf_gn;
 
 /* GaussNewtonSolver::GaussNewtonSolver(const Params&, int max_nodes),
  * include/solver.h:24.  `max_corrs` bounds num_corrs of later calls (the
- * reference sizes nothing by it because it accumulates with atomics). */
+ * reference sizes nothing by it because it accumulates with atomics).  Device
+ * memory: 445 B per correspondence and about 200 B per node, and with the first
+ * solve the pattern (some 170 B per block, 390 B per graph edge). */
 CF_API cf_status cf_gn_create(const cf_gn_params* params, int max_nodes, int max_corrs,
                        cf_gn** out);
 CF_API cf_status cf_gn_destroy(cf_gn* h);
@@ -460,7 +462,7 @@ typedef struct cf_corr_frame {
 } cf_corr_frame;
 
 /* Opaque search handle: owns the per-pixel candidate records and the row
- * chunks' partial results (88 B per pixel of the largest frame). */
+ * chunks' partial results (253 B per pixel of the largest frame). */
 typedef struct cf_corr_search cf_corr_search;
 CF_API cf_status cf_corr_search_create(int max_width, int max_height, cf_corr_search** out);
 CF_API cf_status cf_corr_search_destroy(cf_corr_search* h);
