@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(kCsThreads, kCsCtasPerSm)
       s_k[2] = q.o[2];
       s_k[3] = sn;
       s_k[4] = -0.25f * sw * sn;
-      s_k[5] = k.dist_thr * (sw * sn);
+      s_k[5] = fminf(k.dist_thr * (sw * sn), 0.5f * kFarS);  // (past that nothing is there)
     }
     __syncthreads();
     // a third run in reach: the merge would scan the chunk's rows for the pixel
