@@ -1232,12 +1232,32 @@ __global__ void __launch_bounds__(kMergeThreads)
     if (mine && gg >= 0) {
       const int row0 = gg / k.W * k.W, c0 = gg - row0;
       const int l = max(c0, pu - k.radius), h = min(min(c0 + kGroup - 1, k.W - 1), pu + k.radius);
+      const int first = l + (lane & 7);
+      if (h - l < 8 * kFly) {  // all loads together (640 x 480 at radius 20: 280 us a call in fours, 271)
+        float4 a[kFly];
+        float2 c[kFly];
+#pragma unroll
+        for (int j = 0; j < kFly; ++j) {
+          const int i = row0 + min(first + 8 * j, h);
+          a[j] = A[i];
+          c[j] = B[i];
+        }
+#pragma unroll
+        for (int j = 0; j < kFly; ++j) {
+          const float d = cs_pd<kAngle>(v, nc, a[j], c[j], k);
+          if (d < b.pd) {
+            b.pd = d;
+            b.i = row0 + min(first + 8 * j, h);
+          }
+        }
+      } else {
 #pragma unroll 4
-      for (int col = l + (lane & 7); col <= h; col += 8) {
-        const float d = cs_pd<kAngle>(v, nc, A[row0 + col], B[row0 + col], k);
-        if (d < b.pd) {
-          b.pd = d;
-          b.i = row0 + col;
+        for (int col = first; col <= h; col += 8) {
+          const float d = cs_pd<kAngle>(v, nc, A[row0 + col], B[row0 + col], k);
+          if (d < b.pd) {
+            b.pd = d;
+            b.i = row0 + col;
+          }
         }
       }
     }
