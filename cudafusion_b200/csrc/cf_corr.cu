@@ -1368,17 +1368,17 @@ float sqrt_bound(float cap) {
 // its scan of 512 pixels x S/C candidates goes at 9 per clock beside two others,
 // the last CTAs run with fewer beside them, so the waves count as
 // tiles x C / slots + 0.4; the merge reads each chunk for 5000 at 640 x 480.
-// The exact scan: 6000, 6.4 beside one other, 0.3 (80 x 60 to 1280 x 960 at radii
-// 4 to 50: within 2 % of the best number of chunks, 7 % at most).
+// The exact scan: 6000, 8 beside one other (80 x 60 to 1280 x 960 at radii 9 to 50:
+// 1.5 % above the best number of chunks on average, 10 % at most).
 int corr_pick_chunks(int tiles, int sms, int radius, int W, int H, bool filter) {
   const double slots = (double)(sms > 0 ? sms : 1) * (filter ? kCsCtasPerSm : kExCtasPerSm);
   const double side_x = std::fmin(2.0 * radius + 8.0, (double)W), side_y = std::fmin(2.0 * radius + 8.0, (double)H);
-  const double setup = filter ? 9000.0 : 6000.0, tail = filter ? 0.4 : 0.3;
-  const double scan = 512.0 * side_x * side_y / (filter ? 9.0 : 6.4), merge = 5000.0 * ((double)W * H / 307200.0);
+  const double setup = filter ? 9000.0 : 6000.0;
+  const double scan = 512.0 * side_x * side_y / (filter ? 9.0 : 8.0), merge = 5000.0 * ((double)W * H / 307200.0);
   int best_c = 1;
   double best = 1e300;
   for (int c = 1; c <= kCorrMaxChunks; ++c) {
-    const double t = ((double)tiles * c / slots + tail) * (setup + scan / c) + merge * c;
+    const double t = ((double)tiles * c / slots + 0.4) * (setup + scan / c) + merge * c;
     if (t < best * (1.0 - 1e-9)) {
       best = t;
       best_c = c;
