@@ -124,9 +124,10 @@ constexpr int kSlab = 768;    // columns staged at a time at most
 constexpr int kPad = 8;       // and the columns past them that a step may read
 constexpr float kFarS = 3e5f;  // (scaled) distance of what is not there, above every real one
 // Largest radius whose windows the merge scans itself, a lane per pixel: 640 x
-// 480 takes 80 us at radius 5 that way and 127 at 8; with the exact scan before
-// it 103 and 125.
-constexpr int kCsDirect = 7;
+// 480 takes 79 us at radius 5 that way and 127 at 8, 103 and 125 with the exact scan
+// before it.  With an angle threshold the exact scan has more to do per candidate,
+// the merge waits for its loads as before: at 8 136 and 147, past the cap 136 and 170.
+constexpr int kCsDirect = 7, kCsDirectAngle = 8;
 // Pixels times candidates past which the search goes before the exact scan: its
 // fixed costs, and those of a surface that it leaves to the exact scan, weigh on
 // narrower windows.  640 x 480 at radius 20 (5.2e8): 250 us with the search, 280
@@ -1456,7 +1457,7 @@ cudaError_t launch_corr_search(const cf_corr_frame* f, const cf_camera* cam, con
   const int want = chunks > 0 ? chunks : corr_pick_chunks((int)(tiles.x * tiles.y), sc.sms, k.radius, W, H, filter);
   k.chunks = want < sc.chunk_cap ? want : sc.chunk_cap;
   auto exact = angle ? corr_exact_kernel<true> : corr_exact_kernel<false>;
-  const bool direct = k.radius <= kCsDirect;
+  const bool direct = k.radius <= (angle ? kCsDirectAngle : kCsDirect);
   auto merge = direct ? (angle ? corr_merge_kernel<true, true> : corr_merge_kernel<false, true>)
                       : (angle ? corr_merge_kernel<true, false> : corr_merge_kernel<false, false>);
   // per device and cheap: set on every call rather than cached per device
