@@ -82,6 +82,14 @@ CASES = [
     (1201, 49, "noisy", 1.0, CorrParams(0.2, 0.0, 0.0, 400), 0),
     (1201, 49, "plane", 1.0, CorrParams(0.2, 0.0, 0.0, 390), 2),
     (1201, 49, "noisy", 1.0, CorrParams(0.2, 0.3, 0.0, 400), 3),
+    # the last radius that the merge scans itself and the next, without and with an angle threshold
+    (97, 71, "noisy", 1.0, CorrParams(0.2, 0.0, 0.0, 7), 0),
+    (97, 71, "plane", 1.0, CorrParams(0.2, 0.0, 0.0, 8), 0),
+    (97, 71, "plane", 1.0, CorrParams(0.2, 0.3, 0.0, 8), 0),
+    (97, 71, "noisy", 1.0, CorrParams(0.2, 0.3, 0.0, 9), 0),
+    # frames whose merge has at most two CTAs per SM and one that has more
+    (320, 236, "noisy", 1.0, CorrParams(0.2, 0.0, 0.0, 20), 0),
+    (320, 240, "tilted", 1.0, CorrParams(0.2, 0.0, 0.0, 20), 0),
 ]
 
 
@@ -93,7 +101,7 @@ def test_bit_exact(oracle, frames, w, h, kind, scale, prm, chunks):
     s.find_correspondences(DeviceCorrFrame(f), prm)
     recs = s.records(w * h)
     side = min(2 * prm.search_radius_px + 1, w) * min(2 * prm.search_radius_px + 1, h)
-    pix = np.sort(np.random.default_rng(w + prm.search_radius_px).choice(w * h, 2 * 10**7 // side, replace=False))
+    pix = np.sort(np.random.default_rng(w + prm.search_radius_px).choice(w * h, min(w * h, 2 * 10**7 // side), replace=False))
     ref, _, _ = oracle.find_correspondences(f, prm.dist_threshold, prm.angle_threshold, prm.view_threshold,
                                             prm.search_radius_px, pixels=pix.astype(np.int32))
     assert ref["valid"].any()
