@@ -84,12 +84,12 @@
 // and candidate) and shared memory's data path.  Measured on B200, us per call, in
 // brackets a thread per two pixels with the reference's arithmetic throughout:
 //                        noisy       plane       plane, third runs scanned per pixel
-//   640 x 480 r 50       565 (1771)  1132 (1104)   4272
-//             r 36       385 (1027)   700  (645)   2498
-//             r 28       414  (692)   395  (441)   1688
-//             r 20       278  (430)   260  (286)   1123
-//             r 50 angle 1450 (2594) 1402 (1645)   5453
-//   320 x 240 r 20       103  (152)    98  (103)    508
+//   640 x 480 r 50       566 (1771)  1126 (1104)   4272
+//             r 36       384 (1027)   694  (645)   2498
+//             r 28       423  (692)   403  (441)   1688
+//             r 20       269  (430)   258  (286)   1123
+//             r 50 angle 1434 (2594) 1404 (1645)   5453
+//   320 x 240 r 20       100  (152)    97  (103)    508
 //   160 x 120 r 20        62   (72)    60   (57)    512
 #include <cfloat>
 #include <climits>
@@ -130,9 +130,9 @@ constexpr float kFarS = 3e5f;  // (scaled) distance of what is not there, above 
 constexpr int kCsDirect = 7, kCsDirectAngle = 8;
 // Pixels times candidates past which the search goes before the exact scan: its
 // fixed costs, and those of a surface that it leaves to the exact scan, weigh on
-// narrower windows.  640 x 480 at radius 20 (5.2e8): 250 us with the search, 280
-// without, on a plane 314 and 264; at 28 (1e9) 310 and 425, 519 and 395; at 36
-// (1.6e9) 380 and 590, 700 and 560.
+// narrower windows.  640 x 480 at radius 20 (5.2e8): 227 us with the search, 269
+// without, on a plane 357 and 258; at 28 (1e9) 312 and 423, 522 and 402; at 36
+// (1.6e9) 384 and 590, 694 and 571.
 constexpr double kCsFilter = 1.2e9;
 constexpr float kCsNone = 1e30f;  // distance of what is not there
 constexpr float kU = 5.9604645e-8f;  // 2^-24
